@@ -135,6 +135,15 @@ int32_t b200_graph_extend_rows(b200_graph* g, const int32_t* ids, int32_t n, con
 int32_t b200_graph_extend_residual(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** residual);
 /* One token for each of n distinct slots in one pass; logits [n][vocab] (DecodeRows :1527, llm/batch.go:45-63). */
 int32_t b200_graph_decode_rows(b200_graph* g, const int32_t* slots, const int32_t* ids, int32_t n, const float** logits);
+/* Where the next of the calls above (or b200_draft_rows) leaves its logits and, for the calls that return every row's
+ * residual, those rows: host memory of the caller's, pinned for the copy to run at the bus's rate. The pointers that
+ * call returns are then these, and the caller keeps the results without a copy of its own. NULL: the graph's own
+ * buffer. Holds for one call, whether it succeeds or not; a call that needs more room is refused (B200_ECAPACITY). */
+int32_t b200_graph_set_outputs(b200_graph* g, float* logits, int64_t logit_floats, float* residual, int64_t residual_floats);
+/* Pinned host blocks for that, from a bounded process-wide cache (any thread). NULL when the bound is reached: use the
+ * graph's buffers then. A block may be released after its graph is gone. */
+void* b200_host_acquire(b200_graph* g, int64_t bytes);
+void b200_host_release(void* p);
 /* Sequence checkpoints (Checkpoint/Restore :1004,:1037): DeltaNet state + conv rings of the
  * current slot; KV cells below the mark stay in place. */
 int32_t b200_graph_checkpoint(b200_graph* g, int32_t* handle_out);

@@ -1,5 +1,7 @@
 // extern "C" surface of libb200llm.so (include/b200_llm.h).
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -22,6 +24,61 @@ struct Scratch {   // device temporaries of one call
     *out = (T*)p;
     return OK;
   }
+};
+
+// Pinned host blocks for results (b200_host_acquire). One cache per process, because what is expensive is pinning the
+// pages (about a millisecond per four megabytes), not handing a block out: blocks go back to it and serve whichever
+// graph asks next. Bounded: at most POOL_MAX bytes exist at a time, in use or not, and at most POOL_IDLE of them idle.
+struct HostPool {
+  static constexpr size_t POOL_MAX = (size_t)1 << 30, POOL_IDLE = (size_t)256 << 20;
+  std::mutex mu;
+  std::multimap<size_t, void*> idle;
+  std::map<void*, size_t> size_of;
+  size_t total = 0, idle_bytes = 0;
+
+  void drop_largest() {   // mu held
+    auto it = std::prev(idle.end());
+    cudaFreeHost(it->second);
+    total -= it->first; idle_bytes -= it->first;
+    size_of.erase(it->second);
+    idle.erase(it);
+  }
+  void* acquire(size_t bytes) {
+    const size_t unit = bytes > ((size_t)1 << 20) ? (size_t)1 << 20 : (size_t)64 << 10, want = (bytes + unit - 1) / unit * unit;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = idle.lower_bound(want);
+    if (it != idle.end() && it->first <= 2 * want) {
+      void* p = it->second;
+      idle_bytes -= it->first;
+      idle.erase(it);
+      return p;
+    }
+    while (!idle.empty() && total + want > POOL_MAX) drop_largest();
+    void* p = nullptr;
+    if (total + want > POOL_MAX || cudaHostAlloc(&p, want, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    total += want;
+    size_of[p] = want;
+    return p;
+  }
+  void release(void* p) {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = size_of.find(p);
+    if (it == size_of.end()) return;
+    idle.emplace(it->second, p);
+    idle_bytes += it->second;
+    while (idle_bytes > POOL_IDLE) drop_largest();
+  }
+};
+HostPool& host_pool() {
+  static HostPool* pool = new HostPool;   // never destroyed: arrays may be given back while the process ends
+  return *pool;
+}
+
+// The output buffers a caller has set hold for one call, however it ends.
+struct OutputsForOneCall {
+  Graph& g;
+  explicit OutputsForOneCall(Graph& graph) : g(graph) {}
+  ~OutputsForOneCall() { g.out_logits = g.out_resid = nullptr; g.out_logits_cap = g.out_resid_cap = 0; }
 };
 }  // namespace
 
@@ -105,35 +162,52 @@ int32_t b200_graph_set_past(b200_graph* g, int32_t past) {
 }
 int32_t b200_graph_past(const b200_graph* g) { return g ? g->g.past[g->g.cur] : 0; }
 
+void* b200_host_acquire(b200_graph* g, int64_t bytes) {
+  if (!g || bytes <= 0 || cudaSetDevice(g->g.m->device) != cudaSuccess) return nullptr;
+  return host_pool().acquire((size_t)bytes);
+}
+void b200_host_release(void* p) { if (p) host_pool().release(p); }
+int32_t b200_graph_set_outputs(b200_graph* g, float* logits, int64_t logit_floats, float* residual, int64_t residual_floats) {
+  if (!g) { set_error("set_outputs: null argument"); return EINVAL_; }
+  g->g.out_logits = logits; g->g.out_logits_cap = logits ? logit_floats : 0;
+  g->g.out_resid = residual; g->g.out_resid_cap = residual ? residual_floats : 0;
+  return OK;
+}
 int32_t b200_graph_forward(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {
   if (!g || !ids) { set_error("forward: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   B200_TRY(g->g.reset_slot(g->g.cur));
   PassFlags f;
   return g->g.extend(ids, n, f, logits, hidden);
 }
 int32_t b200_graph_extend(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {
   if (!g || !ids) { set_error("extend: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   PassFlags f;
   return g->g.extend(ids, n, f, logits, hidden);
 }
 int32_t b200_graph_extend_input(b200_graph* g, const b200_input* in, const float** logits, const float** hidden) {
   if (!g || !in || !in->ids) { set_error("extend_input: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   if (in->n_images != 0) { set_error("extend_input: this library has no vision tower; inputs with images are refused"); return EINVAL_; }
   PassFlags f;
   return g->g.extend(in->ids, in->n, f, logits, hidden);
 }
 int32_t b200_graph_extend_rows(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** residual) {
   if (!g || !ids) { set_error("extend_rows: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   PassFlags f; f.want_all_logits = true; f.want_residual = true; f.spec = g->g.speculating;
   return g->g.extend(ids, n, f, logits, residual);
 }
 int32_t b200_graph_extend_residual(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** residual) {
   if (!g || !ids) { set_error("extend_residual: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   PassFlags f; f.want_residual = true;
   return g->g.extend(ids, n, f, logits, residual);
 }
 int32_t b200_graph_decode_rows(b200_graph* g, const int32_t* slots, const int32_t* ids, int32_t n, const float** logits) {
   if (!g || !slots || !ids) { set_error("decode_rows: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   return g->g.decode_rows(slots, ids, n, logits);
 }
 int32_t b200_graph_checkpoint(b200_graph* g, int32_t* handle) { if (!g || !handle) return EINVAL_; return g->g.checkpoint(handle); }
@@ -226,6 +300,7 @@ int64_t b200_graph_trace(b200_graph* g, int32_t what, void* dst, int64_t nbytes)
 
 int32_t b200_draft_rows(b200_graph* g, const float* hs, const int32_t* ids, int32_t n, int32_t vocab_k, const float** residual, const float** logits) {
   if (!g || !hs || !ids) { set_error("draft_rows: null argument"); return EINVAL_; }
+  OutputsForOneCall once(g->g);
   return g->g.draft_rows(hs, ids, n, vocab_k, residual, logits);
 }
 int32_t b200_draft_past(const b200_graph* g) { return g ? g->g.draft_past[g->g.dcur] : 0; }

@@ -98,8 +98,8 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
     B200_TRY(make_x_tensor_map(y16, MR, vw, tn, tm_y16[i]));
     B200_TRY(make_x_tensor_map(ctx16, MR, qw, tn, tm_ctx[i]));
   }
-  B200_TRY(dalloc(&ids_dev, (size_t)MR)); B200_TRY(dalloc(&next_ids, (size_t)MR)); B200_TRY(dalloc(&row_slot, (size_t)MR));
-  B200_TRY(dalloc(&row_pos, (size_t)MR)); B200_TRY(dalloc(&logit_rows, (size_t)MR)); B200_TRY(dalloc(&seqs, (size_t)MR));
+  const size_t stage_bytes = ((size_t)MR + 31) / 32 * 32 * (4 * sizeof(int32_t) + sizeof(SeqDesc));
+  B200_TRY(dalloc(&stage_dev, stage_bytes)); B200_TRY(dalloc(&next_ids, (size_t)MR));
   B200_TRY(dalloc(&hist_len, 1));
   B200_TRY(dalloc(&distinct_dev, 1));
   if (c.has_draft) { B200_TRY(dalloc(&e_buf, (size_t)MR * H)); B200_TRY(dalloc(&hs_buf, (size_t)MR * H)); B200_TRY(dalloc(&xcat16, (size_t)MR * 2 * H)); }
@@ -137,10 +137,9 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   }
   past.assign(o.slots, 0); draft_past.assign(o.slots, 0);
   // host staging
-  stage_bytes = (size_t)MR * (4 * sizeof(int32_t) + sizeof(SeqDesc));
   B200_CUDA(cudaMallocHost((void**)&stage, stage_bytes));
-  B200_CUDA(cudaMallocHost((void**)&logits_host, (size_t)LR * c.vocab * sizeof(float)));
-  B200_CUDA(cudaMallocHost((void**)&resid_host, (size_t)MR * H * sizeof(float)));
+  resid_host_cap = (int64_t)std::min(MR, 16) * H;
+  B200_CUDA(cudaMallocHost((void**)&resid_host, (size_t)resid_host_cap * sizeof(float)));
   B200_CUDA(cudaMallocHost((void**)&hidden_host, (size_t)H * sizeof(float)));
   B200_CUDA(cudaMallocHost((void**)&err_host, sizeof(int)));
   *err_host = 0;
@@ -543,22 +542,46 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   return OK;
 }
 
-static void fill_stage(uint8_t* stage, int MR, const int32_t* ids, const int* slots, const int* pos, int M, const std::vector<SeqDesc>& sq, const std::vector<int>& lrows) {
-  int32_t* s_ids = (int32_t*)stage; int* s_slot = (int*)stage + MR; int* s_pos = (int*)stage + 2 * MR; int* s_lr = (int*)stage + 3 * MR;
-  SeqDesc* s_sq = (SeqDesc*)((int*)stage + 4 * MR);
+// The pass's small inputs sit next to each other, at a pitch that depends on the row count alone, so that they cross
+// the bus as one copy (five copies of a few bytes each cost about a microsecond apiece in front of the first kernel)
+// and a captured pass of M rows always finds them at the same addresses.
+void Graph::place_stage(int M) {
+  const int P = (M + 31) / 32 * 32;
+  ids_dev = (int32_t*)stage_dev; row_slot = ids_dev + P; row_pos = ids_dev + 2 * P; logit_rows = ids_dev + 3 * P; seqs = (SeqDesc*)(ids_dev + 4 * P);
+}
+
+static void fill_stage(uint8_t* stage, const int32_t* ids, const int* slots, const int* pos, int M, const std::vector<SeqDesc>& sq, const std::vector<int>& lrows) {
+  const int P = (M + 31) / 32 * 32;
+  int32_t* s_ids = (int32_t*)stage; int* s_slot = s_ids + P; int* s_pos = s_ids + 2 * P; int* s_lr = s_ids + 3 * P;
+  SeqDesc* s_sq = (SeqDesc*)(s_ids + 4 * P);
   for (int i = 0; i < M; i++) { s_ids[i] = ids[i]; s_slot[i] = slots[i]; s_pos[i] = pos[i]; }
   for (size_t i = 0; i < lrows.size(); i++) s_lr[i] = lrows[i];
   for (size_t i = 0; i < sq.size(); i++) s_sq[i] = sq[i];
 }
 
-static int upload_stage(Graph* g, int M, int n_seq, int n_lr) {
-  const int MR = g->MR;
-  uint8_t* s = g->stage;
-  B200_CUDA(cudaMemcpyAsync(g->ids_dev, s, M * sizeof(int32_t), cudaMemcpyHostToDevice, g->st));
-  B200_CUDA(cudaMemcpyAsync(g->row_slot, (int*)s + MR, M * sizeof(int), cudaMemcpyHostToDevice, g->st));
-  B200_CUDA(cudaMemcpyAsync(g->row_pos, (int*)s + 2 * MR, M * sizeof(int), cudaMemcpyHostToDevice, g->st));
-  if (n_lr > 0) B200_CUDA(cudaMemcpyAsync(g->logit_rows, (int*)s + 3 * MR, n_lr * sizeof(int), cudaMemcpyHostToDevice, g->st));
-  B200_CUDA(cudaMemcpyAsync(g->seqs, (int*)s + 4 * MR, n_seq * sizeof(SeqDesc), cudaMemcpyHostToDevice, g->st));
+int Graph::upload_stage(int M) {
+  place_stage(M);
+  const size_t P = (size_t)(M + 31) / 32 * 32;
+  B200_CUDA(cudaMemcpyAsync(stage_dev, stage, P * (4 * sizeof(int32_t) + sizeof(SeqDesc)), cudaMemcpyHostToDevice, st));
+  return OK;
+}
+
+// Where this call's logits and residual rows go: the caller's buffers when it has set them, else the graph's own.
+int Graph::result_buffers(int64_t logit_floats, int64_t resid_floats, float** lg, float** rs) {
+  const b200_config& c = m->c;
+  if ((out_logits != nullptr && logit_floats > out_logits_cap) || (out_resid != nullptr && resid_floats > out_resid_cap)) { set_error("the output buffers that were set are too small for this call"); return ECAPACITY; }
+  auto grow = [](float** p, int64_t* cap, int64_t need) {
+    if (need <= *cap) return OK;
+    if (*p != nullptr) cudaFreeHost(*p);
+    *p = nullptr; *cap = 0;
+    B200_CUDA(cudaMallocHost((void**)p, (size_t)need * sizeof(float)));
+    *cap = need;
+    return OK;
+  };
+  if (out_logits == nullptr) B200_TRY(grow(&logits_host, &logits_host_cap, logit_floats));
+  if (out_resid == nullptr) B200_TRY(grow(&resid_host, &resid_host_cap, resid_floats));
+  *lg = out_logits != nullptr ? out_logits : logits_host;
+  *rs = out_resid != nullptr ? out_resid : resid_host;
   return OK;
 }
 
@@ -569,11 +592,13 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   }
   B200_CUDA(cudaSetDevice(m->device));
   const auto host_t0 = std::chrono::steady_clock::now();
-  fill_stage(stage, MR, ids, slots, pos, M, sq, lrows);
+  fill_stage(stage, ids, slots, pos, M, sq, lrows);
   pass_max_n = 1;
   for (const SeqDesc& s : sq) pass_max_n = std::max(pass_max_n, s.n);
   const int n_lr = (int)lrows.size(), n_seq = (int)sq.size();
   const int NV = f.draft && draft_vocab > 0 ? draft_vocab : c.vocab;
+  float *lg_dst = nullptr, *rs_dst = nullptr;
+  B200_TRY(result_buffers((int64_t)n_lr * NV, f.want_residual ? (int64_t)(resid_off + M) * c.n_embd : 0, &lg_dst, &rs_dst));
   bool single = !f.spec && !f.draft && !o.trace && o.use_cuda_graph && n_seq == M && n_lr == M && !f.want_residual;
   B200_CUDA(cudaEventRecord(ev0, st));
   if (single) {
@@ -584,9 +609,8 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
       // (the reference's pre-recorded command buffer: llm/graph.go:238-258)
       cudaGraph_t graph = nullptr;
       B200_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      int s = upload_stage(this, M, n_seq, n_lr);
+      int s = upload_stage(M);
       if (s == OK) s = enqueue_pass(M, n_seq, n_lr, f);
-      if (s == OK && cudaMemcpyAsync(logits_host, logits, (size_t)n_lr * NV * sizeof(float), cudaMemcpyDeviceToHost, st) != cudaSuccess) s = ECUDA;
       cudaError_t e = cudaStreamEndCapture(st, &graph);
       if (s != OK || e != cudaSuccess) { if (graph) cudaGraphDestroy(graph); if (s == OK) { set_error(std::string("graph capture: ") + cudaGetErrorString(e)); s = ECUDA; } return s; }
       cudaGraphExec_t exec = nullptr;
@@ -599,12 +623,12 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
     B200_CUDA(cudaGraphLaunch(it->second, st));
     h = decode_h[gkey];
   } else {
-    B200_TRY(upload_stage(this, M, n_seq, n_lr));
+    B200_TRY(upload_stage(M));
     B200_TRY(enqueue_pass(M, n_seq, n_lr, f));
-    if (n_lr > 0) B200_CUDA(cudaMemcpyAsync(logits_host, logits, (size_t)n_lr * NV * sizeof(float), cudaMemcpyDeviceToHost, st));
   }
-  if (f.want_residual) B200_CUDA(cudaMemcpyAsync(resid_host + (size_t)resid_off * c.n_embd, h, (size_t)M * c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
-  B200_CUDA(cudaMemcpyAsync(hidden_host, h + (size_t)(M - 1) * c.n_embd, (size_t)c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
+  if (n_lr > 0) B200_CUDA(cudaMemcpyAsync(lg_dst, logits, (size_t)n_lr * NV * sizeof(float), cudaMemcpyDeviceToHost, st));
+  if (f.want_residual) B200_CUDA(cudaMemcpyAsync(rs_dst + (size_t)resid_off * c.n_embd, h, (size_t)M * c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
+  else if (f.want_hidden) B200_CUDA(cudaMemcpyAsync(hidden_host, h + (size_t)(M - 1) * c.n_embd, (size_t)c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
   B200_CUDA(cudaEventRecord(ev1, st));
   B200_TRY(finish_pass());
   last_rows = M;
@@ -657,8 +681,8 @@ int Graph::extend(const int32_t* ids, int n, const PassFlags& f, const float** l
     else { past[cur] += M; spec_n = 0; }
     resid_off += M;
   }
-  if (logits_out) *logits_out = logits_host;
-  if (hidden_out) *hidden_out = f.want_residual ? resid_host : hidden_host;
+  if (logits_out) *logits_out = out_logits != nullptr ? out_logits : logits_host;
+  if (hidden_out) *hidden_out = !f.want_residual ? hidden_host : out_resid != nullptr ? out_resid : resid_host;
   return OK;
 }
 
@@ -676,11 +700,11 @@ int Graph::decode_rows(const int32_t* slots_in, const int32_t* ids, int n, const
     seen[s] = 1; slots[i] = s; pos[i] = past[s]; lrows[i] = i; sq[i] = SeqDesc{s, i, 1, past[s]};
   }
   if (ep_on && (int64_t)n * ep.world > MR) { set_error("decode_rows: with expert parallelism the rows of all ranks (" + std::to_string(n) + " x " + std::to_string(ep.world) + ") must fit max_tokens"); return ECAPACITY; }
-  PassFlags f; f.want_all_logits = true;
+  PassFlags f; f.want_all_logits = true; f.want_hidden = false;
   B200_TRY(run_rows(ids, slots.data(), pos.data(), n, sq, lrows, f));
   for (int i = 0; i < n; i++) past[slots[i]] += 1;
   spec_n = 0;
-  if (logits_out) *logits_out = logits_host;
+  if (logits_out) *logits_out = out_logits != nullptr ? out_logits : logits_host;
   return OK;
 }
 
@@ -700,8 +724,8 @@ int Graph::generate_greedy(const int32_t* slots_in, const int32_t* first, int n,
   }
   if (ep_on && (int64_t)n * ep.world > MR) { set_error("generate_greedy: with expert parallelism the rows of all ranks must fit max_tokens"); return ECAPACITY; }
   B200_CUDA(cudaSetDevice(m->device));
-  fill_stage(stage, MR, first, slots.data(), pos.data(), n, sq, lrows);
-  B200_TRY(upload_stage(this, n, n, n));
+  fill_stage(stage, first, slots.data(), pos.data(), n, sq, lrows);
+  B200_TRY(upload_stage(n));
   B200_CUDA(cudaMemsetAsync(hist_len, 0, sizeof(int), st));
   PassFlags f; f.want_all_logits = true; f.greedy = true;
   cudaGraphExec_t exec = nullptr;
@@ -757,8 +781,8 @@ int Graph::draft_rows(const float* hs, const int32_t* ids, int n, int vocab_k, c
   resid_off = 0;
   B200_TRY(run_rows(ids, slots.data(), pos.data(), n, sq, lrows, f));
   draft_past[dcur] += n;
-  if (resid) *resid = resid_host;
-  if (logits_out) *logits_out = logits_host;
+  if (resid) *resid = out_resid != nullptr ? out_resid : resid_host;
+  if (logits_out) *logits_out = out_logits != nullptr ? out_logits : logits_host;
   return OK;
 }
 

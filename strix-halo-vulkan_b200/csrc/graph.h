@@ -17,6 +17,7 @@ struct PassFlags {
   bool spec = false;              // speculative: write per-row state planes, leave the state untouched
   bool greedy = false;            // argmax + advance on the device (no host traffic)
   bool draft = false;             // the pass runs the draft layer only
+  bool want_hidden = true;        // copy the last row's residual to the host (when not every row's)
 };
 
 struct Graph {
@@ -64,9 +65,14 @@ struct Graph {
   int dcur = 0;        // slot whose draft cache the draft calls read and write (MTPHead.UseSlot)
   // running totals over the passes this graph ran (the reference's GraphStats: llm/graph.go:527-589)
   b200_graph_stats stats{};
-  // host staging (pinned)
-  uint8_t* stage = nullptr; size_t stage_bytes = 0;
+  // host staging (pinned) and its image on the device: ids | slots | positions | logit rows | sequences, one copy per pass
+  uint8_t *stage = nullptr, *stage_dev = nullptr;
+  // results land in the graph's own pinned buffers (grown to what calls ask for: a pass may return hundreds of
+  // megabytes of logits) or, for one call, where b200_graph_set_outputs points
   float *logits_host = nullptr, *resid_host = nullptr, *hidden_host = nullptr;
+  int64_t logits_host_cap = 0, resid_host_cap = 0;
+  float *out_logits = nullptr, *out_resid = nullptr;
+  int64_t out_logits_cap = 0, out_resid_cap = 0;
   int32_t* ids_host = nullptr;
   // trace
   float *tr_mid = nullptr, *tr_out = nullptr, *tr_w = nullptr, *tr_margin = nullptr;
@@ -112,6 +118,9 @@ struct Graph {
   int pass_experts(int* out);
   int inject_wait_timeout();
   int finish_pass();
+  void place_stage(int M);
+  int upload_stage(int M);
+  int result_buffers(int64_t logit_floats, int64_t resid_floats, float** lg, float** rs);
   int ep_prepare(int rank, int world);
   int ep_export(int rank, int world, void* handle64);
   int ep_attach(const void* handles64);

@@ -77,6 +77,9 @@ SYMBOLS = {
     "b200_graph_extend_rows": (I32, [P, P, I32, PP, PP]),
     "b200_graph_extend_residual": (I32, [P, P, I32, PP, PP]),
     "b200_graph_decode_rows": (I32, [P, P, P, I32, PP]),
+    "b200_graph_set_outputs": (I32, [P, P, I64, P, I64]),
+    "b200_host_acquire": (P, [P, I64]),
+    "b200_host_release": (None, [P]),
     "b200_graph_checkpoint": (I32, [P, C.POINTER(I32)]),
     "b200_graph_restore": (I32, [P, I32]),
     "b200_graph_checkpoint_free": (I32, [P, I32]),
