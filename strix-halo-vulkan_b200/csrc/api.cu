@@ -383,6 +383,20 @@ int32_t b200_qgemv(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
   if (!host_w || !host_x || !host_y || rows <= 0 || mrows <= 0) { set_error("qgemv: bad argument"); return EINVAL_; }
   Scratch sc; DTensor t; __half* x16 = nullptr; float* y = nullptr; int* err = nullptr;
   B200_TRY(stage_projection(sc, type, host_w, rows, k, host_x, mrows, &t, &x16, &y, &err));
+  if (mrows > QG_MAXCOLS && tgemm_type(type)) {   // as the passes of more than eight rows do
+    __half* sx = nullptr;
+    B200_TRY(sc.get(&sx, (size_t)mrows * (k / 256) * TG_SX * sizeof(__half)));
+    TGemmMaps maps{};
+    B200_TRY(make_w_tensor_map(type, t.data, rows, t.stride, 128, &maps.w));
+    B200_TRY(make_rows_map(x16, mrows, (int)k, tgemm_cols(mrows), &maps.x));
+    B200_TRY(make_rows_map(sx, mrows, (int)(k / 256 * TG_SX), tgemm_cols(mrows), &maps.sx));
+    maps.w2 = maps.w;
+    B200_TRY(launch_row_sums(x16, mrows, (int)k, sx, false, 0));
+    TGemmParams g{};
+    g.K = (int)k; g.N = (int)rows; g.M = mrows; g.seg_end = (int)rows; g.ksplit = 1; g.y = y; g.ldy = rows; g.err = err;
+    B200_TRY(launch_tgemm(type, tgemm_cols(mrows), g, maps, false, 0));
+    return finish_projection("qgemv", y, err, (int64_t)mrows * rows, host_y);
+  }
   QGemvParams p{};
   p.w[0] = t.data; p.seg_end[0] = (int)rows; p.nseg = 1; p.stride = t.stride; p.K = (int)k; p.N = (int)rows; p.M = mrows; p.xcols = mrows < QG_MAXCOLS ? mrows : QG_MAXCOLS;
   p.x = x16; p.ldx = k; p.y = y; p.ldy = rows; p.x_div = 1; p.err = err;

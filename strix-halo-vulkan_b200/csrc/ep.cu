@@ -128,6 +128,7 @@ int Graph::ep_prepare(int rank, int world) {
   B200_CUDA(cudaMemset(p, 0, ep_arena_bytes));
   allocs.push_back(p);
   ep_arena = (uint8_t*)p;
+  B200_TRY(dalloc(&sx_ep, (size_t)MR * (c.n_embd / 256) * TG_SX));   // sub-block sums of the gathered rows
   B200_TRY(dalloc(&ep_epoch, 4));   // epoch, ticket, pair count
   ep.rank = rank; ep.world = world; ep.epoch = ep_epoch; ep.done = ep_epoch + 1; ep.err = err_flag;
   ep.H = c.n_embd; ep.used = c.n_expert_used; ep.limit_ns = 2000000000ll;

@@ -76,7 +76,7 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
     if (m->layers[l].is_attn) attn_index[l] = n_attn++;
     else dn_index[l] = n_dn++;
   }
-  max_entries = std::max(max_entries_for(MR), max_entries_for(std::min(MR, 128)));
+  max_entries = std::max(max_entries_for(MR, false), max_entries_for(std::min(MR, 128), false));
   B200_TRY(dalloc(&hbuf[0], (size_t)MR * H)); B200_TRY(dalloc(&hbuf[1], (size_t)MR * H)); h = hbuf[0]; B200_TRY(dalloc(&proj, (size_t)MR * proj_ld));
   B200_TRY(dalloc(&xn16, (size_t)MR * H)); B200_TRY(dalloc(&q16, (size_t)MR * qw)); B200_TRY(dalloc(&ctx16, (size_t)MR * qw));
   B200_TRY(dalloc(&attn_partial, (size_t)attn_rows * c.n_head * nsplit * (hd + 2)));
@@ -102,6 +102,20 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   B200_TRY(dalloc(&stage_dev, stage_bytes)); B200_TRY(dalloc(&next_ids, (size_t)MR));
   B200_TRY(dalloc(&hist_len, 1));
   B200_TRY(dalloc(&distinct_dev, 1));
+  auto with_sums = [&](const __half* x, int64_t rows, int K, TMap* xm, __half** sx, TMap* sm) {
+    if (K % 256) return (int)OK;
+    B200_TRY(dalloc(sx, (size_t)rows * (K / 256) * TG_SX));
+    for (int i = 0; i < 3 && xm != nullptr; i++) {
+      B200_TRY(make_rows_map(x, rows, K, 16 << i, &xm[i]));
+      B200_TRY(make_rows_map(*sx, rows, K / 256 * TG_SX, 16 << i, &sm[i]));
+    }
+    return (int)OK;
+  };
+  B200_TRY(with_sums(xn16, MR, H, tx_xn, &sx_xn, ts_xn));
+  B200_TRY(with_sums(act16, (int64_t)MR * slots1, c.ffn_expert, nullptr, &sx_act, nullptr));
+  B200_TRY(with_sums(y16, MR, vw, tx_y16, &sx_y, ts_y16));
+  B200_TRY(with_sums(ctx16, MR, qw, tx_ctx, &sx_ctx, ts_ctx));
+  B200_TRY(make_weight_maps());
   if (c.has_draft) { B200_TRY(dalloc(&e_buf, (size_t)MR * H)); B200_TRY(dalloc(&hs_buf, (size_t)MR * H)); B200_TRY(dalloc(&xcat16, (size_t)MR * 2 * H)); }
   // rotary table, angle walked in f64 like the reference (llm/attn.go:554-584, llm/gpu_attn.go:1440-1477)
   {
@@ -154,12 +168,30 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   return OK;
 }
 
-// Columns per work-list entry. A pass of some tens of rows leaves one or two rows per touched expert: entries of
-// four columns halve the activation staging of the expert kernels, which then fit three to an SM.
-int Graph::entry_cols(int M) { return M >= 16 && M <= 128 ? 4 : 8; }
+// Columns per work-list entry. Column-tiled kernel: a pass of some tens of rows leaves one or two rows per touched expert;
+// entries of four columns halve the activation staging of the expert kernels, which then fit three to an SM. Streaming kernel
+// (qlist): an expert's weights cost the same for one column as for eight, a second group of eight about a quarter more, so
+// entries are eight columns while hardly any expert has more (measured over 350 experts of two rows: 180 us against 217).
+int Graph::entry_cols(int M, bool stream) const {
+  if (!stream) return M >= 16 && M <= 128 ? 4 : 8;
+  return M * m->c.n_expert_used <= 4 * m->c.n_expert ? 8 : 16;
+}
+int Graph::make_weight_maps() {
+  wmaps.resize(m->layers.size());
+  auto map = [](const DTensor& w, int box, TMap* out) { return w.ok() && tgemm_type(w.type) ? make_w_tensor_map(w.type, w.data, w.rows, w.stride, box, out) : (int)OK; };
+  for (size_t l = 0; l < m->layers.size(); l++) {
+    const LayerW& L = m->layers[l];
+    LayerMaps& W = wmaps[l];
+    B200_TRY(map(L.gate_exps, 16, &W.gate)); B200_TRY(map(L.up_exps, 16, &W.up)); B200_TRY(map(L.down_exps, 16, &W.down));
+    B200_TRY(map(L.gate_sh, 16, &W.gate_sh)); B200_TRY(map(L.up_sh, 16, &W.up_sh)); B200_TRY(map(L.down_sh, 16, &W.down_sh));
+    B200_TRY(map(L.qkv, 128, &W.qkv)); B200_TRY(map(L.z, 128, &W.z)); B200_TRY(map(L.ssm_out, 128, &W.out));
+    B200_TRY(map(L.q, 128, &W.q)); B200_TRY(map(L.k, 128, &W.k)); B200_TRY(map(L.o, 128, &W.o));
+  }
+  return OK;
+}
 
-int Graph::max_entries_for(int M) const {
-  const int used = m->c.n_expert_used, ec = entry_cols(M);
+int Graph::max_entries_for(int M, bool stream) const {
+  const int used = m->c.n_expert_used, ec = entry_cols(M, stream);
   return std::min(M * used, m->c.n_expert + (M * used + ec - 1) / ec) + (M + ec - 1) / ec;
 }
 
@@ -179,6 +211,17 @@ constexpr int ROUTER_MMA_FROM = 16;
 // rows every CTA of the next projection forms them while it stages (each staged row costs every CTA a trip to L2)
 constexpr int COMBINE_ROWS_FROM = 4;
 static bool pass_uses_gemm(int M, int H) { return !(M <= QG_FUSED_ROWS && H <= QG_COMBINE_MAX_K) && M >= 16; }
+// Dense projections of passes above the fused ones that keep their weights exact - all of them below 16 rows, above that
+// those whose tiles would not fill the device as a GEMM - run on the tensor cores all the same where the type has the kernel
+bool Graph::dense_tg(uint32_t type, int M, int N) const {
+  return !(M <= QG_FUSED_ROWS && m->c.n_embd <= QG_COMBINE_MAX_K) && tgemm_type(type) && !(M >= 16 && gemm_tile_rows(M, N) != 0);
+}
+// The experts of passes above the fused ones: warps that stream the weights (qlist.cu), where its types and shapes allow
+bool Graph::experts_stream(const LayerW& L, int M) const {
+  const b200_config& c = m->c;
+  return !(M <= QG_FUSED_ROWS && c.n_embd <= QG_COMBINE_MAX_K) && qlist_type(L.gate_exps.type) && qlist_type(L.down_exps.type) && L.down_exps.type == L.down_sh.type &&
+         c.ffn_expert % 256 == 0 && qlist_fits(c.n_embd, c.ffn_expert, max_entries) && qlist_fits(c.ffn_expert, c.n_embd, max_entries);
+}
 static bool pass_moe_gemm(const b200_config& c, const LayerW& L, int M, int H) {
   return pass_uses_gemm(M, H) && (int64_t)M * c.n_expert_used >= 32 * (int64_t)c.n_expert && L.gate_exps.type == L.gate_sh.type && L.down_exps.type == L.down_sh.type;
 }
@@ -262,8 +305,24 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   auto row_tail = [&](int mode, const DTensor& gamma) {
     TailParams t{};
     t.mode = mode; t.h = hc; t.gamma = (const float*)gamma.data; t.xn = xn16; t.down = down; t.topk_w = fused ? comb_w : topk_w;
-    t.used = fused ? comb_used : used; t.H = H; t.M = M; t.eps = c.eps;
+    t.used = fused ? comb_used : used; t.H = H; t.M = M; t.eps = c.eps; t.sx = fused ? nullptr : sx_xn;
     return t;
+  };
+  // exact tensor-core projection of the pass's rows: up to two matrices of one type side by side, outputs at pitch ldy; cut > 1
+  // leaves the sum in that many planes
+  auto tdense = [&](uint32_t type, const TMap& w, int N0, const TMap* w2, int N1, int K, const TMap* x, const TMap* sx, float* y, int64_t ldy, int cut) {
+    const int cols_ = tgemm_cols(M), box = cols_ == 16 ? 0 : cols_ == 32 ? 1 : 2;
+    TGemmMaps maps{};
+    maps.w = w; maps.w2 = w2 != nullptr ? *w2 : w; maps.x = x[box]; maps.sx = sx[box];
+    TGemmParams p{};
+    p.K = K; p.N = N0 + N1; p.M = M; p.seg_end = N0; p.ksplit = cut; p.y = y; p.ldy = ldy; p.plane = (int64_t)M * ldy; p.err = err_flag;
+    return launch_tgemm(type, cols_, p, maps, pdl(), st);
+  };
+  int resid_parts = 0;   // planes of the output projection that the row kernel after it still has to add (in `down`)
+  auto tresid = [&](const DTensor& w, const TMap& wm, int K, const __half* x, const TMap* xm, __half* sx, const TMap* sxm) {
+    B200_TRY(launch_row_sums(x, M, K, sx, pdl(), st));
+    resid_parts = std::min(tgemm_ksplit(K, H, M, tgemm_cols(M)), slots1);
+    return tdense(w.type, wm, H, nullptr, 0, K, xm, sxm, down, H, resid_parts);
   };
   // passes of 16 rows and more run their dense projections on the tensor cores
   const bool use_gemm = pass_uses_gemm(M, H);
@@ -285,7 +344,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   if (f.draft) {
     // nextn seed, embedding first: h = eh_proj . concat(rms(embd, enorm), rms(h_prev, hnorm))  (llm/mtp.go:352-384)
     const LayerW& L = m->layers[c.n_layer];
-    EmbedParams ep{m->token_embd, ids_dev, e_buf, M, H, nullptr, nullptr, c.eps, nullptr};
+    EmbedParams ep{m->token_embd, ids_dev, e_buf, M, H, nullptr, nullptr, c.eps, nullptr, nullptr};
     B200_TRY(launch_embed(ep, st)); pdl();
     B200_TRY(launch_concat_norm(e_buf, hs_buf, (const float*)L.enorm.data, (const float*)L.hnorm.data, c.eps, H, M, xcat16, pdl(), st));
     QGemvParams p = base(L.eh_proj, 2 * H, H, xcat16, 2 * H);
@@ -295,7 +354,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.attn_norm), pdl(), st));
   } else {
     const LayerW& L0 = m->layers[0];
-    EmbedParams ep{m->token_embd, ids_dev, hc, M, H, fused ? nullptr : (const float*)L0.attn_norm.data, xn16, c.eps, fused ? ss_part : nullptr};
+    EmbedParams ep{m->token_embd, ids_dev, hc, M, H, fused ? nullptr : (const float*)L0.attn_norm.data, xn16, c.eps, fused ? ss_part : nullptr, fused ? nullptr : sx_xn};
     B200_TRY(launch_embed(ep, st)); pdl();
     ss_n = 1;
   }
@@ -306,9 +365,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       QGemvParams p = base(L.qkv, H, cw + vw, xn16, H);
       p.w[1] = L.z.data; p.seg_end[0] = cw; p.seg_end[1] = cw + vw; p.nseg = 2;
       p.y = proj; p.ldy = proj_ld;
-      if (use_gemm) {
+      if (dense_tg(L.qkv.type, M, cw) && dense_tg(L.z.type, M, vw) && cw % 128 == 0) {
+        B200_TRY(tdense(L.qkv.type, wmaps[l].qkv, cw, &wmaps[l].z, vw, H, tx_xn, ts_xn, proj, proj_ld, 1));
+      } else if (use_gemm) {
         B200_TRY(gemm(L.qkv, H, cw, xn16, tm_xn, proj, proj_ld, GEMM_STORE));
-        B200_TRY(gemm(L.z, H, vw, xn16, tm_xn, proj + cw, proj_ld, GEMM_STORE));
+        if (dense_tg(L.z.type, M, vw)) B200_TRY(tdense(L.z.type, wmaps[l].z, vw, nullptr, 0, H, tx_xn, ts_xn, proj + cw, proj_ld, 1));
+        else B200_TRY(gemm(L.z, H, vw, xn16, tm_xn, proj + cw, proj_ld, GEMM_STORE));
       } else {
         const int pro = normed(p, L.attn_norm, xn16);  // the DeltaNet step reads the fp16 rows for alpha / beta
         B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
@@ -330,7 +392,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       QGemvParams q = base(L.ssm_out, vw, H, y16, vw);
       q.y = hc; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(vw, H); }
-      if (use_gemm) B200_TRY(gemm(L.ssm_out, vw, H, y16, tm_y16, hc, H, GEMM_RESID));
+      if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16, sx_y, ts_y16));
+      else if (use_gemm) B200_TRY(gemm(L.ssm_out, vw, H, y16, tm_y16, hc, H, GEMM_RESID));
       else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
     } else {
       const int ai = attn_index[l];
@@ -339,8 +402,17 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       const int rows[3] = {2 * qw, kvw, kvw};
       int off = 0;
       bool xn_ready = false;
-      for (int s = 0; s < 3 && use_gemm; s++) { B200_TRY(gemm(*seg[s], H, rows[s], xn16, tm_xn, proj + off, proj_ld, GEMM_STORE)); off += rows[s]; }
-      for (int s = 0; s < 3 && !use_gemm;) {
+      int s0 = 0;
+      if (dense_tg(L.q.type, M, 2 * qw) && dense_tg(L.k.type, M, kvw) && L.k.type == L.q.type && 2 * qw % 128 == 0) {
+        B200_TRY(tdense(L.q.type, wmaps[l].q, 2 * qw, &wmaps[l].k, kvw, H, tx_xn, ts_xn, proj, proj_ld, 1));
+        off = 2 * qw + kvw; s0 = 2;
+      }
+      for (int s = s0; s < 3 && use_gemm; s++) {
+        if (s == 1 && dense_tg(L.k.type, M, kvw)) B200_TRY(tdense(L.k.type, wmaps[l].k, kvw, nullptr, 0, H, tx_xn, ts_xn, proj + off, proj_ld, 1));
+        else B200_TRY(gemm(*seg[s], H, rows[s], xn16, tm_xn, proj + off, proj_ld, GEMM_STORE));
+        off += rows[s];
+      }
+      for (int s = s0; s < 3 && !use_gemm;) {
         int e = s + 1;
         while (e < 3 && seg[e]->type == seg[s]->type) e++;
         int n = 0;
@@ -379,10 +451,16 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       QGemvParams q = base(L.o, qw, H, ctx16, qw);
       q.y = hc; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(qw, H); }
-      if (use_gemm) B200_TRY(gemm(L.o, qw, H, ctx16, tm_ctx, hc, H, GEMM_RESID));
+      if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o, qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
+      else if (use_gemm) B200_TRY(gemm(L.o, qw, H, ctx16, tm_ctx, hc, H, GEMM_RESID));
       else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
     }
-    if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.ffn_norm), pdl(), st));
+    if (!fused) {
+      TailParams t = row_tail(1, L.ffn_norm);
+      t.parts = down; t.n_parts = resid_parts; t.part_plane = (int64_t)M * H;
+      resid_parts = 0;
+      B200_TRY(launch_row_tail(t, pdl(), st));
+    }
     if (o.trace) { B200_CUDA(cudaMemcpyAsync(tr_mid + (size_t)l * MR * H, hc, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st)); first = true; }
     // MoE block
     xn_valid = false;  // the router leaves its own normalised rows in xn16
@@ -394,11 +472,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     // passes of at most 8 rows: the router stops after its logits and every row is routed, computed and combined on
     // the single-row schedule, so each row's result is the single-row pass's, bit for bit (the reference's batched
     // decode and verify passes equal their rows stepped alone: llm/graph_batch_test.go:36, llm/spec_slots_test.go:199)
-    r.defer = fused && !epx; r.ecols = entry_cols(M); r.distinct = r.defer ? nullptr : distinct_dev;
+    const bool moe_gemm = pass_moe_gemm(c, L, M, H) && !epx;
+    const bool moe_stream = !moe_gemm && experts_stream(L, M);
+    r.defer = fused && !epx; r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
     if (epx) { r.entries = nullptr; r.gprob = nullptr; }   // routing only: the work list comes from the gathered routing
     // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted
     // rows (below that the column-tiled kernel, which streams each expert's weights in whole tiles, is faster)
-    const bool moe_gemm = pass_moe_gemm(c, L, M, H) && !epx;
     r.gprob = moe_gemm ? gprob : nullptr;
     if (use_gemm && M >= ROUTER_MMA_FROM && L.router.type == T_Q8_0) {
       // many rows: the router logits are one more tensor-core GEMM (the reference's prefill router is an fp16
@@ -413,7 +492,17 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     } else {
       B200_TRY(launch_router(r, pdl(), st));
     }
-    const int ne = max_entries_for(Mg);
+    const int ne = max_entries_for(Mg, moe_stream);
+    // the two expert launches of a work list: activation rows x (ids / x_div), outputs by pair id
+    auto stream_experts = [&](const __half* x, const __half* sx, int cols_) {
+      const LayerMaps& W = wmaps[l];
+      QListParams g{};
+      g.entries = entries; g.n_entries = n_entries; g.cols = cols; g.x_div = slots1; g.K = H; g.N = c.ffn_expert; g.x = x; g.sx = sx; g.y16 = act16; g.ldy = c.ffn_expert; g.sx_out = sx_act; g.err = err_flag;
+      B200_TRY(launch_qlist(L.gate_exps.type, QL_SWIGLU, cols_, g, QListMaps{W.gate, W.up, W.gate_sh, W.up_sh}, pdl(), st));
+      QListParams d{};
+      d.entries = entries; d.n_entries = n_entries; d.cols = cols; d.x_div = 1; d.K = c.ffn_expert; d.N = H; d.x = act16; d.sx = sx_act; d.y = down; d.ldy = H; d.err = err_flag;
+      return launch_qlist(L.down_exps.type, QL_STORE, cols_, d, QListMaps{W.down, W.down, W.down_sh, W.down_sh}, pdl(), st);
+    };
     comb_used = used; comb_w = topk_w;
     float* down_rows = down;   // where the pairs of this rank's rows land
     if (epx) {
@@ -422,11 +511,15 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       e.rows = M; e.xn = xn16; e.topk = topk;
       B200_TRY(launch_ep_dispatch(e, pdl(), st));
       RouterParams w = r;
-      w.M = Mg; w.topk = reinterpret_cast<int32_t*>(ep_arena + ep.off_topk); w.entries = entries; w.ecols = entry_cols(Mg);
+      w.M = Mg; w.topk = reinterpret_cast<int32_t*>(ep_arena + ep.off_topk); w.entries = entries; w.ecols = entry_cols(Mg, moe_stream);
       w.e_lo = ep.rank * (c.n_expert / ep.world); w.e_hi = w.e_lo + c.n_expert / ep.world; w.sh_lo = ep.rank * M; w.sh_hi = w.sh_lo + M;
       w.n_pairs = ep_epoch + 2;
       B200_TRY(launch_ep_worklist(w, pdl(), st));
-      const int ecx = std::min(std::min(Mg, QG_MAXCOLS), entry_cols(Mg));
+      if (moe_stream) {
+        B200_TRY(launch_row_sums(reinterpret_cast<const __half*>(ep_arena + ep.off_xg), Mg, H, sx_ep, pdl(), st));
+        B200_TRY(stream_experts(reinterpret_cast<const __half*>(ep_arena + ep.off_xg), sx_ep, entry_cols(Mg, true)));
+      } else {
+      const int ecx = std::min(std::min(Mg, QG_MAXCOLS), entry_cols(Mg, false));
       QGemvParams p = base(L.gate_exps, H, c.ffn_expert, reinterpret_cast<const __half*>(ep_arena + ep.off_xg), H);
       p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
       p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = ecx; p.M = Mg;
@@ -437,6 +530,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = ecx; q.M = Mg;
       q.y = down; q.ldy = H;     // local: rows by pair id; the combine kernel carries them to the rows' owners
       B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, ne, pdl(), st));
+      }
       e.y_local = down; e.cols = cols; e.n_pairs = ep_epoch + 2; e.pairs_per_rank = M * slots1;
       B200_TRY(launch_ep_combine(e, M * slots1 + (Mg - M) * used, pdl(), st));
       down_rows = reinterpret_cast<float*>(ep_arena + ep.off_down);
@@ -461,16 +555,18 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       ds.one = GemmProblem{0, M * used, M, M * used}; ds.max_problems = 1; ds.max_count = M; ds.w = L.down_sh.data; ds.stride = L.down_sh.stride;
       ds.K = c.ffn_expert; ds.N = H; ds.y = down; ds.ldy = H; ds.y_rows = cols; ds.err = err_flag;
       B200_TRY(launch_qgemm(L.down_sh.type, GEMM_STORE, 64, ds, tm_act[0], pdl(), st));
+    } else if (moe_stream) {
+      B200_TRY(stream_experts(xn16, sx_xn, entry_cols(M, true)));
     } else {
     QGemvParams p = base(L.gate_exps, H, c.ffn_expert, xn16, H);
     p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
-    p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = r.defer ? 1 : std::min(xcols, entry_cols(M));
+    p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = r.defer ? 1 : std::min(xcols, entry_cols(M, false));
     p.y16 = act16; p.ldy = c.ffn_expert;
     p.route_here = r.defer; p.route = r;
     B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, r.defer ? M * slots1 : ne, pdl(), st));
     QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
     q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
-    q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M));
+    q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M, false));
     q.y = down; q.ldy = H;
     if (r.defer && L.down_exps.type == L.down_sh.type && slots1 <= 16) {
       // per row: the routing weights are applied inside the down projection, which leaves a few partial rows

@@ -41,6 +41,11 @@ struct Graph {
   int pass_max_n = 1;                            // longest sequence of the pass being enqueued
   float* ones = nullptr;       // [8] weights 1.0 (the combine of pre-weighted partial rows)
   __half* xperm16 = nullptr;   // [rows * used][H]: activation rows in expert-sorted order
+  // exact tensor-core projections (tgemm.cuh): maps of every weight matrix and of the activation rows, sub-block sums
+  struct LayerMaps { TMap gate, up, down, gate_sh, up_sh, down_sh, qkv, z, out, q, k, o; };
+  std::vector<LayerMaps> wmaps;
+  TMap tx_xn[3], ts_xn[3], tx_y16[3], ts_y16[3], tx_ctx[3], ts_ctx[3];   // activation rows and their sums, boxes of 16 / 32 / 64 rows
+  __half *sx_xn = nullptr, *sx_act = nullptr, *sx_y = nullptr, *sx_ctx = nullptr, *sx_ep = nullptr;
   int4* gprob = nullptr;       // [n_expert] GEMM problem per expert
   int* n_expert_dev = nullptr;
   float* ss_part = nullptr;   // [rows][SS_LD] partial sums of squares of the residual rows
@@ -101,8 +106,11 @@ struct Graph {
   ~Graph();
   int init(Model* model, const b200_graph_opts& opts);
   int enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f);
-  static int entry_cols(int M);
-  int max_entries_for(int M) const;
+  int entry_cols(int M, bool stream) const;
+  int max_entries_for(int M, bool stream) const;
+  bool dense_tg(uint32_t type, int M, int N) const;
+  bool experts_stream(const LayerW& L, int M) const;
+  int make_weight_maps();
   uint32_t fp16_weight_mask(int M, int n_logit_rows) const;
   int run_rows(const int32_t* ids, const int* slots, const int* pos, int M, const std::vector<SeqDesc>& sq, const std::vector<int>& lrows, const PassFlags& f);
   int extend(const int32_t* ids, int n, const PassFlags& f, const float** logits_out, const float** hidden_out);

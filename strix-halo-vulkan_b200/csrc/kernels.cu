@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(QG_THREADS) embed_norm_kernel(EmbedParams p) {
   }
   if (p.gamma != nullptr) {
     __syncthreads();
-    row_rmsnorm_f16(h, p.gamma, p.eps, p.H, p.xn + (size_t)n * p.H, scratch);
+    row_rmsnorm_f16(h, p.gamma, p.eps, p.H, p.xn + (size_t)n * p.H, scratch, p.sx != nullptr ? p.sx + (size_t)n * (p.H / 256 * TG_SX) : nullptr);
   }
 }
 int launch_embed(const EmbedParams& p, cudaStream_t st) {
@@ -603,7 +603,18 @@ __global__ void __launch_bounds__(QG_THREADS) row_tail_kernel(TailParams tp) {
     row_moe_combine(hrow, tp.down + (size_t)n * slots1 * tp.H, tp.topk_w + (size_t)n * slots1, tp.used, tp.H);
     __syncthreads();
   }
-  row_rmsnorm_f16(hrow, tp.gamma, tp.eps, tp.H, tp.xn + (size_t)n * tp.H, scratch);
+  if (tp.n_parts > 0) {   // (a thread normalises the elements it adds here)
+    for (int k = threadIdx.x * 4; k < tp.H; k += QG_THREADS * 4) {
+      float4 v = *reinterpret_cast<float4*>(hrow + k), a = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < tp.n_parts; i++) {
+        const float4 d = __ldcg(reinterpret_cast<const float4*>(tp.parts + i * tp.part_plane + (size_t)n * tp.H + k));
+        a.x += d.x; a.y += d.y; a.z += d.z; a.w += d.w;
+      }
+      v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
+      *reinterpret_cast<float4*>(hrow + k) = v;
+    }
+  }
+  row_rmsnorm_f16(hrow, tp.gamma, tp.eps, tp.H, tp.xn + (size_t)n * tp.H, scratch, tp.sx != nullptr ? tp.sx + (size_t)n * (tp.H / 256 * TG_SX) : nullptr);
 }
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st) {
   return launch_k(row_tail_kernel, dim3(tp.M), dim3(QG_THREADS), 0, pdl, st, tp);

@@ -3,6 +3,8 @@
 #include "common.cuh"
 #include "qgemv.cuh"
 #include "qgemm.cuh"
+#include "tgemm.cuh"
+#include "qlist.cuh"
 
 namespace b200 {
 
@@ -30,6 +32,7 @@ struct EmbedParams {
   __half* xn;          // [M][H] fp16 normalised rows (when gamma is given)
   float eps;
   float* ss_out;       // optional: sum of squares of each row, [M][SS_LD] part 0
+  __half* sx;          // optional, with xn: sub-block sums of the rows (tgemm.cuh)
 };
 int launch_embed(const EmbedParams& p, cudaStream_t st);
 

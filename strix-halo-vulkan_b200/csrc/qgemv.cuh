@@ -21,6 +21,7 @@
 #pragma once
 #include "common.cuh"
 #include "router.cuh"
+#include "tgemm.cuh"
 #ifdef __CUDACC__
 #include <cooperative_groups.h>
 #endif
@@ -373,7 +374,8 @@ __device__ __forceinline__ void block_accumulate(float (&acc)[4], const typename
 // more than QG_FUSED_ROWS rows, the embedding gather and the draft head's input use them.
 
 // xn[k] = fp16(h[k] * gamma[k] / sqrt(mean(h^2) + eps))   (reference: llm/hc.go:176-190)
-__device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gamma, float eps, int H, __half* xn, float* scratch) {
+// and, when asked, the sums of the rounded values over every 32 of them (the eight threads of a sub-block are neighbours)
+__device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gamma, float eps, int H, __half* xn, float* scratch, __half* sx = nullptr) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float s = 0.f;
   for (int k = tid * 4; k < H; k += QG_THREADS * 4) {
@@ -393,6 +395,13 @@ __device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gam
     float4 g = *reinterpret_cast<const float4*>(gamma + k);
     __half2 a = __floats2half2_rn(v.x * scale * g.x, v.y * scale * g.y), b = __floats2half2_rn(v.z * scale * g.z, v.w * scale * g.w);
     *reinterpret_cast<uint2*>(xn + k) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+    if (sx != nullptr) {   // H is a multiple of 256: whole warps take part
+      const float2 fa = __half22float2(a), fb = __half22float2(b);
+      float sum = (fa.x + fa.y) + (fb.x + fb.y);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((lane & 7) == 0) store_sub_sum(sx, k >> 5, sum);
+    }
   }
 }
 
@@ -423,6 +432,11 @@ struct TailParams {
   const float* gamma;
   __half* xn;
   float eps;
+  // mode 1: first h += parts[0] + parts[1] + ... (the planes of a projection whose contraction was cut), in plane order
+  const float* parts;
+  int n_parts;
+  int64_t part_plane;
+  __half* sx;           // optional: sub-block sums of the normalised rows, [M][H / 256][TG_SX]
 };
 
 // ---- activation staging ------------------------------------------------------------------
