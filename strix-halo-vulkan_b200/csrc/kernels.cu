@@ -985,14 +985,15 @@ __device__ __forceinline__ float* dn_pre_v(const DnStepParams& p, int h, int64_t
 __device__ __forceinline__ float* dn_pre_gb(const DnStepParams& p, int h, int64_t row) {
   return p.pre + (size_t)p.pre_rows * ((size_t)p.Hk * 256 + (size_t)p.Hv * 128) + ((size_t)h * p.pre_rows + row) * 2;
 }
-constexpr int DN_PRE_TOKENS = 16;
+constexpr int DN_PRE_TOKENS = 64;
 constexpr int DN_CHUNK_FROM = 64;   // sequences of this many tokens and more run the chunked recurrence, shorter ones the token-by-token scan
 
 // alpha / beta projections of all rows of a pass (llm/deltanet.go:305-318): out[row][o], o = head for alpha, Hv + head
-// for beta. A CTA keeps 16 rows of the normalised input in shared memory and walks the 2*Hv weight rows once for all
-// of them (a warp per weight row, lanes along K), so the weights are read once per 16 tokens instead of once per
-// token and row block. grid ceil(M / 16), block 256, dynamic shared memory 16 * H halves.
-constexpr int DN_AB_ROWS = 16;
+// beta. A CTA keeps 16 rows of the normalised input in shared memory and walks a quarter of the 2*Hv weight rows once for
+// all of them (a warp per pair of weight rows, lanes along K): the weights are read once per 16 tokens, and four CTAs per 16
+// rows fill the device where one each left a 200-row pass with 13 busy SMs (126 us, now 9).
+// grid (ceil(M / 16), 4), block 256, dynamic shared memory 16 * H halves.
+constexpr int DN_AB_ROWS = 16, DN_AB_CUT = 4;
 __global__ void __launch_bounds__(256) dn_ab_kernel(DnStepParams p, int M) {
   extern __shared__ __align__(16) uint8_t dn_ab_smem[];
   __half* xs = reinterpret_cast<__half*>(dn_ab_smem);
@@ -1005,89 +1006,82 @@ __global__ void __launch_bounds__(256) dn_ab_kernel(DnStepParams p, int M) {
     reinterpret_cast<uint4*>(xs)[i] = r < nr ? __ldcg(reinterpret_cast<const uint4*>(p.xn + (size_t)(r0 + r) * H) + c) : make_uint4(0, 0, 0, 0);
   }
   __syncthreads();
-  for (int o = warp; o < 2 * p.Hv; o += 8) {
-    const float* w = o < p.Hv ? p.alpha_w + (size_t)o * H : p.beta_w + (size_t)(o - p.Hv) * H;
-    float acc[DN_AB_ROWS];
+  auto row = [&](int o) { return o < p.Hv ? p.alpha_w + (size_t)o * H : p.beta_w + (size_t)(o - p.Hv) * H; };
+  const int n_out = 2 * p.Hv, per = (n_out + DN_AB_CUT - 1) / DN_AB_CUT, o_end = min(n_out, (int)(blockIdx.y + 1) * per);
+  for (int o = blockIdx.y * per + 2 * warp; o < o_end; o += 16) {
+    const bool two = o + 1 < o_end;
+    const float *wa = row(o), *wb = row(two ? o + 1 : o);
+    float acc[2][DN_AB_ROWS];
 #pragma unroll
-    for (int r = 0; r < DN_AB_ROWS; r++) acc[r] = 0.f;
+    for (int r = 0; r < DN_AB_ROWS; r++) { acc[0][r] = 0.f; acc[1][r] = 0.f; }
     for (int k = lane * 4; k < H; k += 128) {
-      const float4 wv = *reinterpret_cast<const float4*>(w + k);
+      const float4 va = *reinterpret_cast<const float4*>(wa + k), vb = *reinterpret_cast<const float4*>(wb + k);
 #pragma unroll
       for (int r = 0; r < DN_AB_ROWS; r++) {
         const uint2 xv = *reinterpret_cast<const uint2*>(xs + (size_t)r * H + k);
         const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&xv.x)), f23 = __half22float2(*reinterpret_cast<const __half2*>(&xv.y));
-        acc[r] = fmaf(wv.w, f23.y, fmaf(wv.z, f23.x, fmaf(wv.y, f01.y, fmaf(wv.x, f01.x, acc[r]))));
+        acc[0][r] = fmaf(va.w, f23.y, fmaf(va.z, f23.x, fmaf(va.y, f01.y, fmaf(va.x, f01.x, acc[0][r]))));
+        acc[1][r] = fmaf(vb.w, f23.y, fmaf(vb.z, f23.x, fmaf(vb.y, f01.y, fmaf(vb.x, f01.x, acc[1][r]))));
       }
     }
 #pragma unroll
-    for (int r = 0; r < DN_AB_ROWS; r++) {
-      const float v = warp_sum(acc[r]);
-      if (lane == 0 && r < nr) p.ab[(size_t)(r0 + r) * 2 * p.Hv + o] = v;
-    }
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int r = 0; r < DN_AB_ROWS; r++) {
+        const float v = warp_sum(acc[h][r]);
+        if (lane == 0 && r < nr && (h == 0 || two)) p.ab[(size_t)(r0 + r) * n_out + o + h] = v;
+      }
   }
 }
 
-// grid (Hk + Hv, n_seq, 16-token groups), block 128. CTAs [0, Hk): q and k of one key head (conv + SiLU + L2 norm);
-// CTAs [Hk, Hk + Hv): v of one value head (conv + SiLU) and the head's decay and beta from the projected alpha / beta.
-// Conv inputs of the positions before this pass come from the rings the decode kernels keep per (head, row block).
-__global__ void __launch_bounds__(128) dn_pre_kernel(DnStepParams p) {
-  const int D = 128, RB = 4;
-  const bool is_qk = (int)blockIdx.x < p.Hk;
-  const int hd = is_qk ? blockIdx.x : blockIdx.x - p.Hk;     // key head or value head
+// conv + SiLU of q, k and v, L2 norm of q and k, decay and beta: a warp takes one 128-channel head of q, k or v over eight
+// tokens, four channels per lane, so the norm is a warp sum and nothing waits at a barrier (one CTA per head and 16 tokens
+// with two barriers per token measured 148 us at 4096 rows; the bytes take 41). Conv inputs of the positions before this
+// pass come from the rings the decode kernels keep per (head, row block). grid (2 Hk + Hv, n_seq, 64-token groups), block 256.
+__global__ void __launch_bounds__(256) dn_pre_kernel(DnStepParams p) {
+  constexpr int D = 128, RB = 4;
+  const int kind = (int)blockIdx.x < p.Hk ? 0 : (int)blockIdx.x < 2 * p.Hk ? 1 : 2;      // q, k, v
+  const int hd = blockIdx.x - (kind == 0 ? 0 : kind == 1 ? p.Hk : 2 * p.Hk);             // key head or value head
   const SeqDesc sq = p.seqs[blockIdx.y];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int qk = p.Hk * D;
-  __shared__ float red[8];
-  const int i0 = blockIdx.z * DN_PRE_TOKENS, i1 = min(sq.n, i0 + DN_PRE_TOKENS);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = 4 * lane;
+  const int i0 = blockIdx.z * DN_PRE_TOKENS + warp * 8, i1 = min(sq.n, i0 + 8);
   if (i0 >= sq.n) return;
-  // channels of the projection row: two (q, k) for a key head, one (v) for a value head
-  const int ch_a = is_qk ? hd * D + tid : 2 * qk + hd * D + tid, ch_b = qk + hd * D + tid;
-  const float4 cwa = *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch_a * 4);
-  const float4 cwb = is_qk ? *reinterpret_cast<const float4*>(p.conv_w + (size_t)ch_b * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float a_h = is_qk ? 0.f : p.ssm_a[hd], dtb = is_qk ? 0.f : p.dt_bias[hd];
+  const int ch = kind * p.Hk * D + hd * D + c;                                           // channel of the projection row
+  float4 w[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) w[k] = *reinterpret_cast<const float4*>(p.conv_w + (size_t)(ch + k) * 4);
   // ring of the decode kernels' CTA (head, row block): q at 0..127 and k at 128..255 of any CTA of a head whose key head
   // this is (head hd, block 0 is one), v at 256..287 of the block that owns the channel
-  const float* ring_a = p.ring + (size_t)sq.slot * p.ring_slot_stride + (size_t)(is_qk ? hd * RB : hd * RB + (tid >> 5)) * (DN_RING * DN_RING_W) + (is_qk ? tid : 256 + (tid & 31));
-  const float* ring_b = p.ring + (size_t)sq.slot * p.ring_slot_stride + (size_t)(hd * RB) * (DN_RING * DN_RING_W) + 128 + tid;
+  const float* ring = p.ring + (size_t)sq.slot * p.ring_slot_stride + (size_t)(kind < 2 ? hd * RB : hd * RB + (c >> 5)) * (DN_RING * DN_RING_W) + (kind < 2 ? 128 * kind + c : 256 + (c & 31));
+  const float a_h = kind == 2 ? p.ssm_a[hd] : 0.f, dtb = kind == 2 ? p.dt_bias[hd] : 0.f;
   pdl_wait();
   pdl_launch();
-  // conv input of token index ii (may be negative: before this pass): the projection row, else the ring
-  auto input = [&](int ii, int ch, const float* ring) {
-    if (ii >= 0) return p.proj[(size_t)(sq.row0 + ii) * p.ldp + ch];
+  auto input = [&](int ii) {   // conv inputs of token index ii (negative: before this pass)
+    if (ii >= 0) return __ldcg(reinterpret_cast<const float4*>(p.proj + (size_t)(sq.row0 + ii) * p.ldp + ch));
     const int pos = sq.pos0 + ii;
-    return pos >= 0 ? ring[(size_t)(pos & (DN_RING - 1)) * DN_RING_W] : 0.f;
+    return pos >= 0 ? *reinterpret_cast<const float4*>(ring + (size_t)(pos & (DN_RING - 1)) * DN_RING_W) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
-  float ha[3], hb[3] = {0.f, 0.f, 0.f};
+  float4 x[11];
 #pragma unroll
-  for (int j = 0; j < 3; j++) {
-    ha[j] = input(i0 - 3 + j, ch_a, ring_a);
-    if (is_qk) hb[j] = input(i0 - 3 + j, ch_b, ring_b);
-  }
-  for (int i = i0; i < i1; i++) {
-    const int row = sq.row0 + i;
-    const float* pr = p.proj + (size_t)row * p.ldp;
-    const float ca = pr[ch_a];
-    const float va = silu_acc(ha[0] * cwa.x + ha[1] * cwa.y + ha[2] * cwa.z + ca * cwa.w);
-    ha[0] = ha[1]; ha[1] = ha[2]; ha[2] = ca;
-    if (is_qk) {
-      const float cb = pr[ch_b];
-      const float vb = silu_acc(hb[0] * cwb.x + hb[1] * cwb.y + hb[2] * cwb.z + cb * cwb.w);
-      hb[0] = hb[1]; hb[1] = hb[2]; hb[2] = cb;
-      const float sq2 = warp_sum(va * va), sk2 = warp_sum(vb * vb);
-      __syncthreads();
-      if (lane == 0) { red[warp] = sq2; red[4 + warp] = sk2; }
-      __syncthreads();
-      const float qn = 1.0f / sqrtf(red[0] + red[1] + red[2] + red[3] + p.eps);
-      const float kn = 1.0f / sqrtf(red[4] + red[5] + red[6] + red[7] + p.eps);
-      float* out = dn_pre_qk(p, hd, row);
-      out[tid] = va * qn;
-      out[128 + tid] = vb * kn;
+  for (int u = 0; u < 11; u++) x[u] = i0 - 3 + u < i1 ? input(i0 - 3 + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int u = 0; u < 8; u++) {
+    if (i0 + u >= i1) break;
+    const int row = sq.row0 + i0 + u;
+    float4 v;
+    v.x = silu_acc(x[u].x * w[0].x + x[u + 1].x * w[0].y + x[u + 2].x * w[0].z + x[u + 3].x * w[0].w);
+    v.y = silu_acc(x[u].y * w[1].x + x[u + 1].y * w[1].y + x[u + 2].y * w[1].z + x[u + 3].y * w[1].w);
+    v.z = silu_acc(x[u].z * w[2].x + x[u + 1].z * w[2].y + x[u + 2].z * w[2].z + x[u + 3].z * w[2].w);
+    v.w = silu_acc(x[u].w * w[3].x + x[u + 1].w * w[3].y + x[u + 2].w * w[3].z + x[u + 3].w * w[3].w);
+    if (kind < 2) {
+      const float n = 1.0f / sqrtf(warp_sum((v.x * v.x + v.y * v.y) + (v.z * v.z + v.w * v.w)) + p.eps);
+      v.x *= n; v.y *= n; v.z *= n; v.w *= n;
+      *reinterpret_cast<float4*>(dn_pre_qk(p, hd, row) + 128 * kind + c) = v;
     } else {
-      dn_pre_v(p, hd, row)[tid] = va;
-      if (tid == 0) {
+      *reinterpret_cast<float4*>(dn_pre_v(p, hd, row) + c) = v;
+      if (lane == 0) {
         const float alpha = __ldcg(p.ab + (size_t)row * 2 * p.Hv + hd), betar = __ldcg(p.ab + (size_t)row * 2 * p.Hv + p.Hv + hd);
-        float* gb = dn_pre_gb(p, hd, row);
-        gb[0] = expf(softplus_ref(alpha + dtb) * a_h); gb[1] = sigmoid_acc(betar);
+        *reinterpret_cast<float2*>(dn_pre_gb(p, hd, row)) = make_float2(expf(softplus_ref(alpha + dtb) * a_h), sigmoid_acc(betar));
       }
     }
   }
@@ -1177,264 +1171,395 @@ __global__ void __launch_bounds__(128) dn_scan_kernel(DnStepParams p) {
 }
 
 // -----------------------------------------------------------------------------------------
-// The recurrence in chunks of 64 tokens (the chunked form of the gated delta rule). Within a chunk the per-token
-// updates  s_j <- g_t s_j + beta_t (v_t[j] - g_t s_j . k_t) k_t  are solved for all tokens at once: with
-// L_t = sum_{r<=t} log g_r and ratio(t, r) = exp(L_t - L_r),
-//   A[t][r] = beta_t ratio(t, r) (k_t . k_r)  (r < t),      W[t][r] = ratio(t, r) (q_t . k_r)  (r <= t),
-//   R[t][j] = beta_t (v_t[j] - exp(L_t) (S0 k_t)[j]),       D[t][j] = R[t][j] - sum_{r<t} A[t][r] D[r][j],
-//   o_t[j]  = (exp(L_t) (S0 q_t)[j] + sum_{r<=t} W[t][r] D[r][j]) / sqrt(128),
-//   S_C     = exp(L_C) S0 + sum_r ratio(C, r) D[r] k_r^T,
-// which is the token-by-token recurrence re-associated (llm/deltanet.go:365-418 is the sequential form; the
-// reference has no chunked one, llm/gpu_deltanet.go:48-52). Everything stays f32 (the state and the recurrence
-// are f32 throughout in the reference's device path), so the matrix products run on the FMA pipe, register-tiled,
-// from shared memory; only the forward substitution for D is sequential (32 columns wide, solved in four blocks of
-// 16 tokens). A CTA owns 32 state rows of one head, as dn_scan_kernel does, and reads the same inputs.
-// grid (Hv * 4, n_seq), block 512, dynamic shared memory DN_CHUNK_SMEM.
+// The recurrence in chunks of 64 tokens (the WY form of the gated delta rule). Within a chunk the per-token updates
+// s_j <- g_t s_j + beta_t (v_t[j] - g_t s_j . k_t) k_t  are solved for all tokens at once: with L_t = sum_{r<=t} log g_r,
+// Gamma_t = exp(L_t) and ratio(t, r) = exp(L_t - L_r),
+//   A[t][r] = beta_t ratio(t, r) (k_t . k_r)  (r < t),   T = (I + A)^-1,   W[t][r] = ratio(t, r) (q_t . k_r)  (r <= t),
+//   U = T (beta V),   Y = T (beta Gamma K),   D = U - Y S0^T,
+//   o_t = (Gamma_t S0 q_t + sum_r W[t][r] D[r]) / sqrt(128),   S_C = Gamma_C S0 + sum_r ratio(C, r) D[r] k_r^T,
+// the token-by-token recurrence re-associated (llm/deltanet.go:365-418 is the sequential form; the reference has no chunked
+// one, llm/gpu_deltanet.go:48-52). Everything up to Y needs no state: dn_wy_kernel forms it for every chunk in parallel and
+// leaves dn_chunk_kernel, which walks the chunks, three products against the 32 state rows a CTA owns.
+//
+// The state and the recurrence are f32 throughout in the reference's device path, so the products run as split TF32: every
+// operand is hi + lo with hi rounded to TF32 and lo the exact rest, and hi hi + (hi lo + lo hi) is accumulated in f32, an
+// error of 2^-22 relative per product, that of an f32 dot product of this length. mma.sync TF32 runs at 500 multiply-adds per
+// cycle and SM, three to one here: 1.3 times the FMA pipe, at a tenth of its shared-memory reads, which is what bounded the
+// register-tiled form. 4096 tokens, 32 heads: 1706 us as one kernel on the FMA pipe.
 // -----------------------------------------------------------------------------------------
-constexpr int DN_C = 64;                       // tokens per chunk
-constexpr int DN_KP = 132;                     // pitch of the K and Q rows (floats): 16-byte reads of rows tx, tx+16, .. fall on distinct banks
-constexpr int DN_AP = 68;                      // pitch of A and W rows
-constexpr int DN_DP = 68;                      // pitch of the solved deltas, kept transposed: DT[j][r]
-constexpr size_t DN_CHUNK_SMEM = sizeof(float) * (2 * DN_C * DN_KP + 32 * DN_KP + DN_C * 32 + 32 * DN_DP + 2 * DN_C * DN_AP + 4 * DN_C);
+constexpr int DN_C = 64;                            // tokens per chunk
+// pitches (floats) of shared-memory rows: 16-byte reads of rows g at 16 kk + 4 t want 16 mod 32, 4-byte reads of rows t at
+// column g want 8, of rows g at column t want 4
+constexpr int DN_P16 = 144, DN_P8 = 136, DN_P4 = 68, DN_PD = 40, DN_PU = 36;
 
-__global__ void __launch_bounds__(512, 1) dn_chunk_kernel(DnStepParams p) {
-  const int D = 128, RB = 4;
-  const int h = blockIdx.x / RB, rb = blockIdx.x % RB;
-  const SeqDesc sq = p.seqs[blockIdx.y];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // Two halves of eight warps work side by side: the first on what the forward substitution needs (A, then K S0^T
-  // and the right-hand sides) and later on the state, the second on what only the outputs need (Q S0^T, W, then the
-  // outputs). w8 / t2 are a thread's warp and thread index inside its half.
-  const bool second = warp >= 8;
-  const int w8 = warp & 7, t2 = tid & 255;
-  // products of token rows with the state block or the deltas: a lane takes four of the 32 columns j (j8 + 8m) and a
-  // quarter of the contraction range (cq), eight tokens (w8 + 8u) - 128 multiply-adds per twelve 16-byte reads -
-  // and the four lanes of a column add their quarters with two shuffles
-  const int j8 = lane & 7, cq = lane >> 3;
-  extern __shared__ __align__(16) float dc_smem[];
-  float* Ks = dc_smem;                          // [64][DN_KP]
-  float* Qs = Ks + DN_C * DN_KP;                // [64][DN_KP]
-  float* ST = Qs + DN_C * DN_KP;                // [32 j][DN_KP]: the CTA's 32 state rows
-  float* Vs = ST + 32 * DN_KP;                  // [64][32] values, then R
-  float* DT = Vs + DN_C * 32;                   // [32 j][DN_DP] the solved deltas, transposed
-  float* Am = DT + 32 * DN_DP;                  // [64][DN_AP]
-  float* Wm = Am + DN_C * DN_AP;                // [64][DN_AP]
-  float* Lg = Wm + DN_C * DN_AP;                // [64] cumulative log decay
-  float* Bt = Lg + DN_C;                        // [64] beta
-  float* Gm = Bt + DN_C;                        // [64] exp(L_t)
-  float* Cr = Gm + DN_C;                        // [64] exp(L_C - L_r)
-  float* Sg = p.state + (size_t)sq.slot * p.state_slot_stride + (size_t)h * D * D + (size_t)(rb * 32) * D;
-  // the state block does not depend on the producer kernel
-  for (int idx = tid; idx < 32 * D; idx += 512) { const int j = idx >> 7, i = idx & 127; ST[j * DN_KP + i] = Sg[idx]; }
-  const float oscale = 1.0f / sqrtf((float)D);
-  pdl_wait();
-  pdl_launch();
-  const float* pqk = dn_pre_qk(p, h % p.Hk, sq.row0);
-  const float* pv = dn_pre_v(p, h, sq.row0) + rb * 32;
-  const float* pgb = dn_pre_gb(p, h, sq.row0);
-  const int ty = t2 >> 4, tx = t2 & 15;
-  for (int c0 = 0; c0 < sq.n; c0 += DN_C) {
-    const int n = min(DN_C, sq.n - c0);
-    __syncthreads();                            // the previous chunk's readers are done with every buffer
-    // ---- inputs: q, k rows (zero past the end), values, decay and beta ----
-    for (int idx = tid; idx < DN_C * 64; idx += 512) {
-      const int t = idx >> 6, c = idx & 63;     // 64 float4 per token: 32 of q, 32 of k
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (t < n) v = __ldcg(reinterpret_cast<const float4*>(pqk + (size_t)(c0 + t) * 256 + 4 * c));
-      float* dst = (c < 32 ? Qs : Ks) + t * DN_KP + 4 * (c & 31);
-      *reinterpret_cast<float4*>(dst) = v;
-    }
-    for (int idx = tid; idx < DN_C * 32; idx += 512) {
-      const int t = idx >> 5, j = idx & 31;
-      Vs[idx] = t < n ? __ldcg(pv + (size_t)(c0 + t) * 128 + j) : 0.f;
-    }
-    if (warp == 0) {                            // cumulative log decay of the chunk: two tokens per lane
-      const int t0 = 2 * lane, t1 = t0 + 1;
-      const float g0 = t0 < n ? __ldcg(pgb + (size_t)(c0 + t0) * 2) : 1.f, g1 = t1 < n ? __ldcg(pgb + (size_t)(c0 + t1) * 2) : 1.f;
-      Bt[t0] = t0 < n ? __ldcg(pgb + (size_t)(c0 + t0) * 2 + 1) : 0.f;
-      Bt[t1] = t1 < n ? __ldcg(pgb + (size_t)(c0 + t1) * 2 + 1) : 0.f;
-      const float l0 = fmaxf(logf(g0), -87.f), l1 = fmaxf(logf(g1), -87.f);
-      float run = l0 + l1;                      // inclusive scan over the lanes' pair sums
+__device__ __forceinline__ void tf_split(float x, uint32_t& hi, uint32_t& lo) {
+  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  lo = __float_as_uint(x - __uint_as_float(hi));
+}
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+struct TfA { uint32_t hi[4], lo[4]; };
+struct TfB { uint32_t hi[2], lo[2]; };
+__device__ __forceinline__ TfA tf_a(float a0, float a1, float a2, float a3) {
+  TfA r;
+  tf_split(a0, r.hi[0], r.lo[0]); tf_split(a1, r.hi[1], r.lo[1]); tf_split(a2, r.hi[2], r.lo[2]); tf_split(a3, r.hi[3], r.lo[3]);
+  return r;
+}
+__device__ __forceinline__ TfB tf_b(float b0, float b1) {
+  TfB r;
+  tf_split(b0, r.hi[0], r.lo[0]); tf_split(b1, r.hi[1], r.lo[1]);
+  return r;
+}
+// main += hi hi, cross += hi lo + lo hi (two chains, so neither waits for the other)
+__device__ __forceinline__ void mma_split(float (&main)[4], float (&cross)[4], const TfA& a, const TfB& b) {
+  mma_tf32(main, a.hi, b.hi[0], b.hi[1]);
+  mma_tf32(cross, a.hi, b.lo[0], b.lo[1]);
+  mma_tf32(cross, a.lo, b.hi[0], b.hi[1]);
+}
+// One 16 x 8*NT tile over 128 (float4 steps of 16): X rows m0 + g, + 8 and Y rows n0 + 8 nt + g, both at pitch DN_P16. A lane
+// takes four consecutive elements of each row; the mma's k slots are whatever those are, in X and Y alike.
+template <int NT>
+__device__ __forceinline__ void rows_by_rows(const float* X, const float* Y, int g, int t, float (&main)[NT][4], float (&cross)[NT][4], int live = NT) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += up; }
-      Lg[t0] = run - l1; Lg[t1] = run;
-      const float total = __shfl_sync(0xffffffffu, run, 31);
-      Gm[t0] = expf(run - l1); Gm[t1] = expf(run);
-      Cr[t0] = expf(total - (run - l1)); Cr[t1] = expf(total - run);
-    }
-    __syncthreads();
-    // ---- a 64 x 64 product of token rows against the key rows, 4 x 4 per thread: the first half forms
-    //      A = beta ratio (K K^T) below the diagonal, the second W = ratio (Q K^T) on and below it ----
-    auto gram = [&](const float* Xs, float* Out, bool is_a) {
-      float aa[4][4];
+  for (int n = 0; n < NT; n++)
 #pragma unroll
-      for (int a = 0; a < 4; a++)
+    for (int i = 0; i < 4; i++) { main[n][i] = 0.f; cross[n][i] = 0.f; }
+#pragma unroll 2
+  for (int kk = 0; kk < 8; kk++) {
+    const float4 xa = *reinterpret_cast<const float4*>(X + g * DN_P16 + 16 * kk + 4 * t), xb = *reinterpret_cast<const float4*>(X + (g + 8) * DN_P16 + 16 * kk + 4 * t);
+    const TfA a0 = tf_a(xa.x, xb.x, xa.y, xb.y), a1 = tf_a(xa.z, xb.z, xa.w, xb.w);
 #pragma unroll
-        for (int b = 0; b < 4; b++) aa[a][b] = 0.f;
-      for (int i = 0; i < D; i += 4) {
-        float4 xt[4], kr[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-          xt[a] = *reinterpret_cast<const float4*>(Xs + (ty + 16 * a) * DN_KP + i);
-          kr[a] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * a) * DN_KP + i);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++) aa[a][b] += xt[a].x * kr[b].x + xt[a].y * kr[b].y + xt[a].z * kr[b].z + xt[a].w * kr[b].w;
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const int t = ty + 16 * a, r = tx + 16 * b;
-          const float ratio = r <= t ? expf(Lg[t] - Lg[r]) : 0.f;
-          Out[t * DN_AP + r] = is_a ? (r < t ? Bt[t] * ratio * aa[a][b] : 0.f) : ratio * aa[a][b];
-        }
-    };
-    // ---- out[m][u] = sum_c X[w8 + 8u][c] * Y[j8 + 8m][c] over `len` values of c: X rows of pitch xp (token rows
-    //      or W rows), Y rows of pitch yp (the state block or the transposed deltas) ----
-    auto rows_times = [&](const float* X, int xp, const float* Y, int yp, int len, float (&out)[4][8]) {
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) out[m][u] = 0.f;
-      const int cbeg = cq * (len / 4);
-      for (int c = cbeg; c < cbeg + len / 4; c += 4) {
-        float4 yv[4];
-#pragma unroll
-        for (int m = 0; m < 4; m++) yv[m] = *reinterpret_cast<const float4*>(Y + (j8 + 8 * m) * yp + c);
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          const float4 xx = *reinterpret_cast<const float4*>(X + (w8 + 8 * u) * xp + c);
-#pragma unroll
-          for (int m = 0; m < 4; m++) out[m][u] += xx.x * yv[m].x + xx.y * yv[m].y + xx.z * yv[m].z + xx.w * yv[m].w;
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-          out[m][u] += __shfl_xor_sync(0xffffffffu, out[m][u], 8);
-          out[m][u] += __shfl_xor_sync(0xffffffffu, out[m][u], 16);
-        }
-    };
-    float qs[4][8];
-    if (!second) {
-      gram(Ks, Am, true);
-      float ks[4][8];
-      rows_times(Ks, DN_KP, ST, DN_KP, D, ks);
-      // right-hand sides R; of a column's four lanes, lane cq writes the tokens u = cq and cq + 4
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-          if ((u & 3) == cq) {
-            const int t = w8 + 8 * u, j = j8 + 8 * m;
-            Vs[t * 32 + j] = Bt[t] * (Vs[t * 32 + j] - Gm[t] * ks[m][u]);
-          }
-      asm volatile("bar.sync 1, 256;" ::: "memory");   // A and R are complete (the first half wrote them)
-      // ---- forward substitution D[t] = R[t] - sum_{r<t} A[t][r] D[r] in four blocks of 16 tokens: the part of the sum
-      //      that comes from the blocks already solved is taken off the block's right-hand sides by the whole half
-      //      (thread -> token t, columns j0 and j0 + 16), then one warp solves the 16 x 16 triangle with the block's
-      //      deltas in registers (lane = column j; every index is a compile-time constant, so the loads run ahead of
-      //      the chain of dependent multiply-adds) ----
-      for (int b = 0; b < DN_C / 16; b++) {
-        if (b > 0) {
-          const int t = 16 * b + (t2 >> 4), j0 = t2 & 15;
-          float s0 = 0.f, s1 = 0.f;
-          for (int r = 0; r < 16 * b; r += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(Am + t * DN_AP + r);
-            const float4 d0 = *reinterpret_cast<const float4*>(DT + j0 * DN_DP + r), d1 = *reinterpret_cast<const float4*>(DT + (j0 + 16) * DN_DP + r);
-            s0 += a.x * d0.x + a.y * d0.y + a.z * d0.z + a.w * d0.w;
-            s1 += a.x * d1.x + a.y * d1.y + a.z * d1.z + a.w * d1.w;
-          }
-          Vs[t * 32 + j0] -= s0; Vs[t * 32 + j0 + 16] -= s1;
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-        }
-        if (warp == 0) {
-          float d[16];
-#pragma unroll
-          for (int tl = 0; tl < 16; tl++) {
-            const int t = 16 * b + tl;
-            float acc = Vs[t * 32 + lane];
-            float av[16];
-#pragma unroll
-            for (int q4 = 0; q4 < 4; q4++)
-              if (4 * q4 < tl) {
-                const float4 a = *reinterpret_cast<const float4*>(Am + t * DN_AP + 16 * b + 4 * q4);
-                av[4 * q4] = a.x; av[4 * q4 + 1] = a.y; av[4 * q4 + 2] = a.z; av[4 * q4 + 3] = a.w;
-              }
-#pragma unroll
-            for (int r = 0; r < 16; r++)
-              if (r < tl) acc -= av[r] * d[r];
-            d[tl] = acc;
-          }
-          float* dl = DT + lane * DN_DP + 16 * b;
-#pragma unroll
-          for (int q4 = 0; q4 < 4; q4++) *reinterpret_cast<float4*>(dl + 4 * q4) = make_float4(d[4 * q4], d[4 * q4 + 1], d[4 * q4 + 2], d[4 * q4 + 3]);
-        }
-        if (b + 1 < DN_C / 16) asm volatile("bar.sync 1, 256;" ::: "memory");   // the block's deltas are there for the next update
-      }
-    } else {
-      rows_times(Qs, DN_KP, ST, DN_KP, D, qs);
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int u = 0; u < 8; u++) qs[m][u] *= Gm[w8 + 8 * u];
-      gram(Qs, Wm, false);
-    }
-    __syncthreads();
-    if (second) {
-      // ---- outputs: o_t[j] = (Gamma_t QS + W D) / sqrt(D) ----
-      float wd[4][8];
-      rows_times(Wm, DN_AP, DT, DN_DP, DN_C, wd);
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int u = 0; u < 8; u++)
-          if ((u & 3) == cq) {
-            const int t = w8 + 8 * u;
-            if (t < n) p.o_raw[(size_t)(sq.row0 + c0 + t) * (p.Hv * D) + h * D + rb * 32 + j8 + 8 * m] = (qs[m][u] + wd[m][u]) * oscale;
-          }
-    } else {
-      // ---- state: S[j][i] = Gamma_C S[j][i] + sum_r Cr[r] D[r][j] K[r][i]: a thread owns columns j = jp, jp + 16 and
-      //      the i in [i0, i0 + 4) and [i0 + 64, i0 + 68), and nobody else reads or writes them now (the products with the
-      //      old state are done) ----
-      const int jp = t2 >> 4, i0 = 4 * (t2 & 15);
-      float acc[2][8];
-      const float gc = Gm[DN_C - 1];
-#pragma unroll
-      for (int jj = 0; jj < 2; jj++) {
-        const float4 s0 = *reinterpret_cast<const float4*>(ST + (jp + 16 * jj) * DN_KP + i0), s1 = *reinterpret_cast<const float4*>(ST + (jp + 16 * jj) * DN_KP + i0 + 64);
-        acc[jj][0] = gc * s0.x; acc[jj][1] = gc * s0.y; acc[jj][2] = gc * s0.z; acc[jj][3] = gc * s0.w;
-        acc[jj][4] = gc * s1.x; acc[jj][5] = gc * s1.y; acc[jj][6] = gc * s1.z; acc[jj][7] = gc * s1.w;
-      }
-      for (int r = 0; r < DN_C; r += 4) {
-        const float4 cr = *reinterpret_cast<const float4*>(Cr + r);
-        const float4 d0 = *reinterpret_cast<const float4*>(DT + jp * DN_DP + r), d1 = *reinterpret_cast<const float4*>(DT + (jp + 16) * DN_DP + r);
-        const float c0v[4] = {cr.x * d0.x, cr.y * d0.y, cr.z * d0.z, cr.w * d0.w}, c1v[4] = {cr.x * d1.x, cr.y * d1.y, cr.z * d1.z, cr.w * d1.w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float4 k0 = *reinterpret_cast<const float4*>(Ks + (r + e) * DN_KP + i0), k1 = *reinterpret_cast<const float4*>(Ks + (r + e) * DN_KP + i0 + 64);
-          acc[0][0] += k0.x * c0v[e]; acc[0][1] += k0.y * c0v[e]; acc[0][2] += k0.z * c0v[e]; acc[0][3] += k0.w * c0v[e];
-          acc[0][4] += k1.x * c0v[e]; acc[0][5] += k1.y * c0v[e]; acc[0][6] += k1.z * c0v[e]; acc[0][7] += k1.w * c0v[e];
-          acc[1][0] += k0.x * c1v[e]; acc[1][1] += k0.y * c1v[e]; acc[1][2] += k0.z * c1v[e]; acc[1][3] += k0.w * c1v[e];
-          acc[1][4] += k1.x * c1v[e]; acc[1][5] += k1.y * c1v[e]; acc[1][6] += k1.z * c1v[e]; acc[1][7] += k1.w * c1v[e];
-        }
-      }
-#pragma unroll
-      for (int jj = 0; jj < 2; jj++) {
-        *reinterpret_cast<float4*>(ST + (jp + 16 * jj) * DN_KP + i0) = make_float4(acc[jj][0], acc[jj][1], acc[jj][2], acc[jj][3]);
-        *reinterpret_cast<float4*>(ST + (jp + 16 * jj) * DN_KP + i0 + 64) = make_float4(acc[jj][4], acc[jj][5], acc[jj][6], acc[jj][7]);
+    for (int n = 0; n < NT; n++) {
+      if (n < live) {
+        const float4 y = *reinterpret_cast<const float4*>(Y + (8 * n + g) * DN_P16 + 16 * kk + 4 * t);
+        mma_split(main[n], cross[n], a0, tf_b(y.x, y.y));
+        mma_split(main[n], cross[n], a1, tf_b(y.z, y.w));
       }
     }
   }
+}
+__device__ __forceinline__ float* dn_y(const DnStepParams& p, int h, int64_t row) { return p.wy + ((size_t)h * p.pre_rows + row) * 128; }
+__device__ __forceinline__ float* dn_w(const DnStepParams& p, int h, int64_t row) { return p.wy + (size_t)p.Hv * p.pre_rows * 128 + ((size_t)h * p.pre_rows + row) * 64; }
+
+// What a chunk needs before its state is known. A CTA takes one chunk of one key head: K K^T and Q K^T once, then for each of
+// the value heads that read this key head A, T, W, U (in place of V), Y, and (Gamma, ratio(C, .)) in place of (decay, beta).
+// T by blocks of 16: the diagonal ones by substitution (a lane per column, in registers), the rest block row by block row.
+// grid (chunks, Hk, n_seq), block 512.
+constexpr size_t DN_WY_SMEM = sizeof(float) * (2 * DN_C * DN_P16 + DN_C * DN_P8 + 4 * DN_C * DN_P4 + 4 * DN_C);
+__global__ void __launch_bounds__(512, 1) dn_wy_kernel(DnStepParams p) {
+  const SeqDesc sq = p.seqs[blockIdx.z];
+  const int hk = blockIdx.y, c0 = blockIdx.x * DN_C, n = min(DN_C, sq.n - c0);
+  if (n <= 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, w8 = warp & 7;
+  const int64_t row0 = sq.row0 + c0;
+  extern __shared__ __align__(16) float dn_smem[];
+  float* Ks = dn_smem;                          // [64][P16]
+  float* Qs = Ks + DN_C * DN_P16;               // [64][P16]
+  float* Vs = Qs + DN_C * DN_P16;               // [64][P8]
+  float* KK = Vs + DN_C * DN_P8;                // [64][P4] each
+  float* QK = KK + DN_C * DN_P4;
+  float* Am = QK + DN_C * DN_P4;
+  float* Tm = Am + DN_C * DN_P4;                // lower blocks: T; upper blocks: scratch
+  float* Lg = Tm + DN_C * DN_P4;                // [64] cumulative log decay
+  float* Bt = Lg + DN_C;                        // [64] beta
+  float* Gm = Bt + DN_C;                        // [64] beta Gamma
+  pdl_wait();
+  pdl_launch();
+  for (int i = tid; i < DN_C * 64; i += 512) {
+    const int r = i >> 6, c = i & 63;           // 64 float4 per token: 32 of q, 32 of k
+    const float4 v = r < n ? __ldcg(reinterpret_cast<const float4*>(dn_pre_qk(p, hk, row0 + r) + 4 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>((c < 32 ? Qs : Ks) + r * DN_P16 + 4 * (c & 31)) = v;
+  }
   __syncthreads();
-  for (int idx = tid; idx < 32 * D; idx += 512) { const int j = idx >> 7, i = idx & 127; Sg[idx] = ST[j * DN_KP + i]; }
+  {
+    // lower triangles only: 20 tiles of 16 x 8 for each product, at most three to a warp
+    const int mt = w8 < 3 ? 3 : w8 < 5 ? 2 : w8 < 7 ? 1 : 0, nt0 = w8 == 1 || w8 == 4 ? 3 : w8 == 2 ? 6 : w8 == 6 ? 2 : 0, nts = w8 == 0 || w8 == 1 || w8 == 3 || w8 == 4 ? 3 : 2;
+    float m[3][4], x[3][4];
+    rows_by_rows<3>((warp >= 8 ? Qs : Ks) + mt * 16 * DN_P16, Ks + nt0 * 8 * DN_P16, g, t, m, x, nts);
+    float* out = (warp >= 8 ? QK : KK) + (mt * 16 + g) * DN_P4 + nt0 * 8 + 2 * t;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      if (i < nts) {
+        *reinterpret_cast<float2*>(out + 8 * i) = make_float2(m[i][0] + x[i][0], m[i][1] + x[i][1]);
+        *reinterpret_cast<float2*>(out + 8 * DN_P4 + 8 * i) = make_float2(m[i][2] + x[i][2], m[i][3] + x[i][3]);
+      }
+    }
+  }
+  for (int h = hk; h < p.Hv; h += p.Hk) {
+    if (warp == 0) {                            // cumulative log decay of the chunk: two tokens per lane
+      const int t0 = 2 * lane, t1 = t0 + 1;
+      float2 e0 = make_float2(1.f, 0.f), e1 = e0;
+      if (t0 < n) e0 = __ldcg(reinterpret_cast<const float2*>(dn_pre_gb(p, h, row0 + t0)));
+      if (t1 < n) e1 = __ldcg(reinterpret_cast<const float2*>(dn_pre_gb(p, h, row0 + t1)));
+      const float l0 = fmaxf(logf(e0.x), -87.f), l1 = fmaxf(logf(e1.x), -87.f);
+      float run = l0 + l1;                      // inclusive scan over the lanes' pair sums
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += up; }
+      const float total = __shfl_sync(0xffffffffu, run, 31), la = run - l1;
+      Lg[t0] = la; Lg[t1] = run; Bt[t0] = e0.y; Bt[t1] = e1.y; Gm[t0] = e0.y * expf(la); Gm[t1] = e1.y * expf(run);
+      if (t0 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t0)) = make_float2(expf(la), expf(total - la));
+      if (t1 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t1)) = make_float2(expf(run), expf(total - run));
+    }
+    for (int i = tid; i < DN_C * 32; i += 512) {
+      const int r = i >> 5, c = i & 31;
+      const float4 v = r < n ? __ldcg(reinterpret_cast<const float4*>(dn_pre_v(p, h, row0 + r) + 4 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(Vs + r * DN_P8 + 4 * c) = v;
+    }
+    __syncthreads();
+    for (int i = tid; i < DN_C * DN_C; i += 512) {
+      const int r = i >> 6, c = i & 63;
+      const float ratio = c <= r ? expf(Lg[r] - Lg[c]) : 0.f;
+      Am[r * DN_P4 + c] = c < r ? Bt[r] * ratio * KK[r * DN_P4 + c] : 0.f;
+      if (r < n) dn_w(p, h, row0 + r)[c] = c <= r ? ratio * QK[r * DN_P4 + c] : 0.f;
+    }
+    __syncthreads();
+    if (warp < 4 && lane < 16) {                // diagonal blocks of T: column `lane` of block `warp`
+      const float* a = Am + 16 * warp * (DN_P4 + 1);
+      float* o = Tm + 16 * warp * (DN_P4 + 1) + lane;
+      float x[16];
+#pragma unroll
+      for (int r = 0; r < 16; r++) {
+        float v = r == lane ? 1.f : 0.f;
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+          if (c < r) v -= a[r * DN_P4 + c] * x[c];
+        x[r] = v;
+        o[r * DN_P4] = v;
+      }
+    }
+    __syncthreads();
+    for (int lv = 1; lv < 4; lv++) {            // T_ba = -T_bb sum_{a <= c < b} A_bc T_ca for b = a + lv; the sums wait in block (a, b)
+      for (int i = tid; i < (4 - lv) * 256; i += 512) {
+        const int a = i >> 8, b = a + lv, r = (i >> 4) & 15, c = i & 15;
+        const float* ar = Am + (16 * b + r) * DN_P4 + 16 * a;
+        const float* tc = Tm + 16 * a * DN_P4 + 16 * a + c;
+        float s = 0.f;
+        for (int k = 0; k < 16 * lv; k++) s = fmaf(ar[k], tc[k * DN_P4], s);
+        Tm[(16 * a + r) * DN_P4 + 16 * b + c] = s;
+      }
+      __syncthreads();
+      for (int i = tid; i < (4 - lv) * 256; i += 512) {
+        const int a = i >> 8, b = a + lv, r = (i >> 4) & 15, c = i & 15;
+        const float* tr = Tm + (16 * b + r) * DN_P4 + 16 * b;
+        const float* xc = Tm + 16 * a * DN_P4 + 16 * b + c;
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; k++) s = fmaf(tr[k], xc[k * DN_P4], s);
+        Tm[(16 * b + r) * DN_P4 + 16 * a + c] = -s;
+      }
+      __syncthreads();
+    }
+    {
+      // U (first eight warps) and Y: all 64 rows x 16 columns per warp, contraction up to the diagonal block
+      const bool second = warp >= 8;
+      const float* B = second ? Ks : Vs;
+      const int bp = second ? DN_P16 : DN_P8;
+      const float* sc = second ? Gm : Bt;
+      float m[4][2][4], x[4][2][4];
+#pragma unroll
+      for (int a = 0; a < 32; a++) { (&m[0][0][0])[a] = 0.f; (&x[0][0][0])[a] = 0.f; }
+#pragma unroll
+      for (int k8 = 0; k8 < 8; k8++) {
+        const int ka = k8 * 8 + t, kb = ka + 4;
+        const float sa = sc[ka], sb = sc[kb];
+        TfB b[2];
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) b[nt] = tf_b(B[ka * bp + w8 * 16 + nt * 8 + g], B[kb * bp + w8 * 16 + nt * 8 + g]);
+#pragma unroll
+        for (int mt = 0; mt < 4; mt++) {
+          if (mt >= (k8 >> 1)) {
+            const float* tr = Tm + (mt * 16 + g) * DN_P4;
+            const TfA a = tf_a(tr[ka] * sa, tr[8 * DN_P4 + ka] * sa, tr[kb] * sb, tr[8 * DN_P4 + kb] * sb);
+#pragma unroll
+            for (int nt = 0; nt < 2; nt++) mma_split(m[mt][nt], x[mt][nt], a, b[nt]);
+          }
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < 4; mt++)
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+          for (int hh = 0; hh < 2; hh++) {
+            const int r = mt * 16 + g + 8 * hh;
+            if (r < n) *reinterpret_cast<float2*>((second ? dn_y(p, h, row0 + r) : dn_pre_v(p, h, row0 + r)) + w8 * 16 + nt * 8 + 2 * t) = make_float2(m[mt][nt][2 * hh] + x[mt][nt][2 * hh], m[mt][nt][2 * hh + 1] + x[mt][nt][2 * hh + 1]);
+          }
+    }
+    __syncthreads();                            // V, A and T are free for the next head
+  }
+}
+
+// The walk over the chunks. A CTA owns 32 of a head's 128 state rows: kept as f32 in the registers of the warps that update
+// them, with a copy in shared memory for the products that read them. Per chunk two phases: warps 0..7 form D while warps
+// 8..15 form Gamma Q S^T; then warps 0..7 update the state while warps 8..15 add W D and write the outputs. What a phase has
+// read is refilled for the next chunk by asynchronous copies under the other phase. grid (Hv * 4, n_seq), block 512.
+constexpr size_t DN_CHUNK_SMEM = sizeof(float) * (2 * DN_C * DN_P16 + DN_C * DN_P8 + DN_C * DN_P4 + DN_C * DN_PU + 32 * DN_P16 + DN_C * DN_PD + 4 * DN_C);
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool live) {   // zeros when not live
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__global__ void __launch_bounds__(512, 1) dn_chunk_kernel(DnStepParams p) {
+  constexpr int D = 128, RB = 4;
+  const int h = blockIdx.x / RB, rb = blockIdx.x % RB, hk = h % p.Hk;
+  const SeqDesc sq = p.seqs[blockIdx.y];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, w8 = warp & 7;
+  const bool second = warp >= 8;
+  extern __shared__ __align__(16) float dn_smem[];
+  float* Ys = dn_smem;                          // [64][P16]
+  float* Qs = Ys + DN_C * DN_P16;               // [64][P16]
+  float* Ks = Qs + DN_C * DN_P16;               // [64][P8]
+  float* Ws = Ks + DN_C * DN_P8;                // [64][P4]
+  float* Us = Ws + DN_C * DN_P4;                // [64][PU]
+  float* ST = Us + DN_C * DN_PU;                // [32][P16] the state rows
+  float* Ds = ST + 32 * DN_P16;                 // [64][PD]
+  float* gam = Ds + DN_C * DN_PD;               // [2][64][2] (Gamma_t, ratio(C, t)) of this chunk and the next
+  float* Sg = p.state + (size_t)sq.slot * p.state_slot_stride + (size_t)h * D * D + (size_t)(rb * 32) * D;
+  // the state block does not depend on the producer kernel
+  float s[2][2][4];                             // warps 0..7: rows 16 mt + g (+ 8), columns 16 w8 + 8 nt + 2t (+ 1)
+  for (int i = tid; i < 32 * 32; i += 512) *reinterpret_cast<float4*>(ST + (i >> 5) * DN_P16 + 4 * (i & 31)) = *reinterpret_cast<const float4*>(Sg + 4 * i);
+  if (!second) {
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+      for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+          const float2 v = *reinterpret_cast<const float2*>(Sg + (size_t)(16 * mt + g + 8 * hh) * D + 16 * w8 + 8 * nt + 2 * t);
+          s[mt][nt][2 * hh] = v.x; s[mt][nt][2 * hh + 1] = v.y;
+        }
+  }
+  const float oscale = 1.0f / sqrtf((float)D);
+  pdl_wait();
+  pdl_launch();
+  const float *pqk = dn_pre_qk(p, hk, sq.row0), *pu = dn_pre_v(p, h, sq.row0) + rb * 32, *pg = dn_pre_gb(p, h, sq.row0), *py = dn_y(p, h, sq.row0), *pw = dn_w(p, h, sq.row0);
+  auto load_first = [&](int c0, int buf) {      // what phase 1 reads (and the factors)
+    for (int i = tid; i < DN_C * 32; i += 512) {
+      const int r = i >> 5, c = 4 * (i & 31);
+      const bool live = c0 + r < sq.n;
+      const int64_t row = live ? c0 + r : 0;
+      cp_async16(Ys + r * DN_P16 + c, py + row * 128 + c, live);
+      cp_async16(Qs + r * DN_P16 + c, pqk + row * 256 + c, live);
+    }
+    { const int r = tid >> 3, c = 4 * (tid & 7); const bool live = c0 + r < sq.n; cp_async16(Us + r * DN_PU + c, pu + (live ? (int64_t)(c0 + r) * 128 : 0) + c, live); }
+    if (tid < 64) {
+      const bool live = c0 + tid < sq.n;
+      const float2 v = live ? __ldcg(reinterpret_cast<const float2*>(pg + (int64_t)(c0 + tid) * 2)) : make_float2(0.f, 0.f);
+      *reinterpret_cast<float2*>(gam + buf * 128 + 2 * tid) = v;
+    }
+  };
+  auto load_second = [&](int c0) {              // what phase 2 reads
+    for (int i = tid; i < DN_C * 32; i += 512) {
+      const int r = i >> 5, c = 4 * (i & 31);
+      const bool live = c0 + r < sq.n;
+      cp_async16(Ks + r * DN_P8 + c, pqk + (live ? (int64_t)(c0 + r) * 256 : 0) + 128 + c, live);
+    }
+    for (int i = tid; i < DN_C * 16; i += 512) {
+      const int r = i >> 4, c = 4 * (i & 15);
+      const bool live = c0 + r < sq.n;
+      cp_async16(Ws + r * DN_P4 + c, pw + (live ? (int64_t)(c0 + r) * 64 : 0) + c, live);
+    }
+  };
+  load_first(0, 0);
+  cp_async_wait_all();
+  __syncthreads();
+  load_second(0);
+  const int mt4 = w8 & 3, nh = w8 >> 2;         // 16-token tile and 16-column half of the products with 64 x 32 results
+  int buf = 0;
+  for (int c0 = 0; c0 < sq.n; c0 += DN_C, buf ^= 1) {
+    const int n = min(DN_C, sq.n - c0);
+    const float* gm = gam + buf * 128;
+    float o[2][4];
+    {
+      float m[2][4], x[2][4];
+      rows_by_rows<2>((second ? Qs : Ys) + mt4 * 16 * DN_P16, ST + nh * 16 * DN_P16, g, t, m, x);
+#pragma unroll
+      for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+          const int r = mt4 * 16 + g + 8 * hh, c = nh * 16 + 8 * nt + 2 * t;
+          const float v0 = m[nt][2 * hh] + x[nt][2 * hh], v1 = m[nt][2 * hh + 1] + x[nt][2 * hh + 1];
+          if (second) {
+            const float gr = gm[2 * r];
+            o[nt][2 * hh] = gr * v0; o[nt][2 * hh + 1] = gr * v1;
+          } else {
+            const float2 u = *reinterpret_cast<const float2*>(Us + r * DN_PU + c);
+            *reinterpret_cast<float2*>(Ds + r * DN_PD + c) = make_float2(u.x - v0, u.y - v1);
+          }
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();                            // D is there, this chunk's K and W have landed, Y, Q and U are free
+    if (c0 + DN_C < sq.n) load_first(c0 + DN_C, buf ^ 1);
+    if (second) {
+      float x[2][4];
+#pragma unroll
+      for (int i = 0; i < 8; i++) (&x[0][0])[i] = 0.f;
+      for (int k8 = 0; k8 < 2 * (mt4 + 1); k8++) {
+        const int ka = 8 * k8 + t, kb = ka + 4;
+        const float* w = Ws + (mt4 * 16 + g) * DN_P4;
+        const TfA a = tf_a(w[ka], w[8 * DN_P4 + ka], w[kb], w[8 * DN_P4 + kb]);
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) mma_split(o[nt], x[nt], a, tf_b(Ds[ka * DN_PD + nh * 16 + 8 * nt + g], Ds[kb * DN_PD + nh * 16 + 8 * nt + g]));
+      }
+#pragma unroll
+      for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++) {
+          const int r = mt4 * 16 + g + 8 * hh;
+          if (r < n) *reinterpret_cast<float2*>(p.o_raw + (size_t)(sq.row0 + c0 + r) * (p.Hv * D) + h * D + rb * 32 + nh * 16 + 8 * nt + 2 * t) =
+              make_float2((o[nt][2 * hh] + x[nt][2 * hh]) * oscale, (o[nt][2 * hh + 1] + x[nt][2 * hh + 1]) * oscale);
+        }
+    } else {
+      const float gc = gm[2 * (n - 1)];
+      float x[2][2][4];
+#pragma unroll
+      for (int i = 0; i < 16; i++) { (&s[0][0][0])[i] *= gc; (&x[0][0][0])[i] = 0.f; }
+#pragma unroll 2
+      for (int k8 = 0; k8 < 8; k8++) {
+        const int ka = 8 * k8 + t, kb = ka + 4;
+        const float ca = gm[2 * ka + 1], cb = gm[2 * kb + 1];
+        TfB b[2];
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++) b[nt] = tf_b(Ks[ka * DN_P8 + 16 * w8 + 8 * nt + g], Ks[kb * DN_P8 + 16 * w8 + 8 * nt + g]);
+#pragma unroll
+        for (int mt = 0; mt < 2; mt++) {
+          const float *da = Ds + ka * DN_PD + 16 * mt + g, *db = Ds + kb * DN_PD + 16 * mt + g;
+          const TfA a = tf_a(da[0] * ca, da[8] * ca, db[0] * cb, db[8] * cb);
+#pragma unroll
+          for (int nt = 0; nt < 2; nt++) mma_split(s[mt][nt], x[mt][nt], a, b[nt]);
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+          for (int hh = 0; hh < 2; hh++) {
+            float* sv = &s[mt][nt][2 * hh];
+            sv[0] += x[mt][nt][2 * hh]; sv[1] += x[mt][nt][2 * hh + 1];
+            *reinterpret_cast<float2*>(ST + (16 * mt + g + 8 * hh) * DN_P16 + 16 * w8 + 8 * nt + 2 * t) = make_float2(sv[0], sv[1]);
+          }
+    }
+    cp_async_wait_all();
+    __syncthreads();                            // the state is there, the next Y, Q and U have landed, K, W and D are free
+    if (c0 + DN_C < sq.n) load_second(c0 + DN_C);
+  }
+  if (!second) {
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+      for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+        for (int hh = 0; hh < 2; hh++)
+          *reinterpret_cast<float2*>(Sg + (size_t)(16 * mt + g + 8 * hh) * D + 16 * w8 + 8 * nt + 2 * t) = make_float2(s[mt][nt][2 * hh], s[mt][nt][2 * hh + 1]);
+  }
   // the ring keeps the last positions' conv inputs (written here, after every read of the old ring by the pre-pass)
   if (tid < 128) {
-    const int hk = h % p.Hk, qk = p.Hk * D;
+    const int qk = p.Hk * D;
     const int ch_q = hk * D + tid, ch_k = qk + hk * D + tid, ch_v = 2 * qk + h * D + rb * 32 + (tid & 31);
     float* ring = p.ring + (size_t)sq.slot * p.ring_slot_stride + (size_t)blockIdx.x * (DN_RING * DN_RING_W);
     for (int i = max(0, sq.n - DN_RING); i < sq.n; i++) {
@@ -1446,49 +1571,43 @@ __global__ void __launch_bounds__(512, 1) dn_chunk_kernel(DnStepParams p) {
   }
 }
 
-// gated RMSNorm of one token's head: sums of squares grouped as the step kernel groups them (eight rows
-// per warp in order, four warps per row block, four row blocks)
-__global__ void __launch_bounds__(128) dn_post_kernel(DnStepParams p, int M) {
-  const int D = 128, row = blockIdx.x, h = blockIdx.y, j = threadIdx.x;
-  __shared__ float sq[128], wss[16], tot_sm;
+// gated RMSNorm of a token's heads, a warp per (row, head), four of its 128 outputs per lane. grid ceil(M * Hv / 8), block 256.
+__global__ void __launch_bounds__(256) dn_post_kernel(DnStepParams p, int M) {
+  constexpr int D = 128;
+  const int w = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int row = w / p.Hv, h = w - row * p.Hv;
+  if (row >= M) return;
+  const float4 z = *reinterpret_cast<const float4*>(p.proj + (size_t)row * p.ldp + 2 * p.Hk * D + p.Hv * D + h * D + 4 * lane);   // written three kernels back
+  const float4 nw = *reinterpret_cast<const float4*>(p.norm_w + 4 * lane);
   pdl_wait();
   pdl_launch();
-  const float ov = p.o_raw[(size_t)row * (p.Hv * D) + h * D + j];
-  sq[j] = ov * ov;
-  __syncthreads();
-  if (j < 16) {
-    float ss = 0.f;
-    for (int r = 0; r < 8; r++) ss += sq[j * 8 + r];
-    wss[j] = ss;
-  }
-  __syncthreads();
-  if (j == 0) {
-    float tot = 0.f;
-    for (int rb = 0; rb < 4; rb++) tot += wss[4 * rb] + wss[4 * rb + 1] + wss[4 * rb + 2] + wss[4 * rb + 3];
-    tot_sm = tot;
-  }
-  __syncthreads();
-  const float nsc = 1.0f / sqrtf(tot_sm / (float)D + p.eps);
-  const float zz = p.proj[(size_t)row * p.ldp + 2 * p.Hk * D + p.Hv * D + h * D + j];
-  p.y16[(size_t)row * (p.Hv * D) + h * D + j] = __float2half_rn(ov * nsc * p.norm_w[j] * sigmoid_acc(zz));
+  const float4 o = __ldcg(reinterpret_cast<const float4*>(p.o_raw + (size_t)row * (p.Hv * D) + h * D + 4 * lane));
+  const float sc = 1.0f / sqrtf(warp_sum((o.x * o.x + o.y * o.y) + (o.z * o.z + o.w * o.w)) / (float)D + p.eps);
+  const uint2 v = make_uint2(pack_half2(o.x * sc * nw.x * sigmoid_acc(z.x), o.y * sc * nw.y * sigmoid_acc(z.y)), pack_half2(o.z * sc * nw.z * sigmoid_acc(z.z), o.w * sc * nw.w * sigmoid_acc(z.w)));
+  *reinterpret_cast<uint2*>(p.y16 + (size_t)row * (p.Hv * D) + h * D + 4 * lane) = v;
 }
 
-int launch_dn_scan(const DnStepParams& p, int M, int max_n, bool pdl, cudaStream_t st) {
+int launch_dn_scan(const DnStepParams& p, int M, int max_n, int* n_launches, bool pdl, cudaStream_t st) {
   if (p.D != 128 || p.conv != 4) { set_error("dn_scan: head dim must be 128 and conv kernel 4"); return EINVAL_; }
   if (p.mid != nullptr || p.pre == nullptr || p.o_raw == nullptr) { set_error("dn_scan: not available for speculative passes"); return EINVAL_; }
   if (p.ab == nullptr || p.H % 128 != 0 || (size_t)DN_AB_ROWS * p.H * 2 > 200 * 1024) { set_error("dn_scan: row length must be a multiple of 128 (at most 6400)"); return EINVAL_; }
   const int ab_smem = DN_AB_ROWS * p.H * 2;
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(dn_ab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  B200_TRY(launch_k(dn_ab_kernel, dim3((M + DN_AB_ROWS - 1) / DN_AB_ROWS), dim3(256), ab_smem, pdl, st, p, M));
-  B200_TRY(launch_k(dn_pre_kernel, dim3(p.Hk + p.Hv, p.n_seq, (max_n + DN_PRE_TOKENS - 1) / DN_PRE_TOKENS), dim3(128), 0, true, st, p));
+  B200_TRY(launch_k(dn_ab_kernel, dim3((M + DN_AB_ROWS - 1) / DN_AB_ROWS, DN_AB_CUT), dim3(256), ab_smem, pdl, st, p, M));
+  B200_TRY(launch_k(dn_pre_kernel, dim3(2 * p.Hk + p.Hv, p.n_seq, (max_n + DN_PRE_TOKENS - 1) / DN_PRE_TOKENS), dim3(256), 0, true, st, p));
+  *n_launches = 4;
   if (max_n >= DN_CHUNK_FROM) {
     // long sequences: the recurrence in chunks of 64 tokens
+    if (p.wy == nullptr) { set_error("dn_scan: no buffer for the chunked form"); return EINVAL_; }
+    B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(dn_wy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_WY_SMEM));
     B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(dn_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DN_CHUNK_SMEM));
+    B200_TRY(launch_k(dn_wy_kernel, dim3((max_n + DN_C - 1) / DN_C, p.Hk, p.n_seq), dim3(512), DN_WY_SMEM, true, st, p));
     B200_TRY(launch_k(dn_chunk_kernel, dim3(p.Hv * 4, p.n_seq), dim3(512), DN_CHUNK_SMEM, true, st, p));
+    *n_launches = 5;
   } else {
     B200_TRY(launch_k(dn_scan_kernel, dim3(p.Hv * 4, p.n_seq), dim3(128), 0, true, st, p));
   }
-  return launch_k(dn_post_kernel, dim3(M, p.Hv), dim3(128), 0, true, st, p, M);
+  return launch_k(dn_post_kernel, dim3((M * p.Hv + 7) / 8), dim3(256), 0, true, st, p, M);
 }
 
 int launch_dn_step(const DnStepParams& p, bool pdl, cudaStream_t st) {

@@ -75,6 +75,7 @@ struct DnStepParams {
   // many-token form (launch_dn_scan): state-independent inputs of the scan for every row, and its raw outputs
   float* pre;                                // [Hk][pre_rows][256] q | k, [Hv][pre_rows][128] v, [Hv][pre_rows][2] decay | beta
   int64_t pre_rows;
+  float* wy;                                 // chunked form: [Hv][pre_rows][128] Y, then [Hv][pre_rows][64] W
   float* o_raw;                              // [M][Hv*D]
   float* ab;                                 // [M][2*Hv] alpha | beta projections of every row
   int H, Hk, Hv, D, conv;
@@ -84,9 +85,9 @@ struct DnStepParams {
 constexpr int DN_RING = 8;      // positions kept per ring
 constexpr int DN_RING_W = 288;  // conv inputs per CTA: q 128 | k 128 | v 32
 int launch_dn_step(const DnStepParams& p, bool pdl, cudaStream_t st);
-// four launches: alpha / beta projections of all rows, the rest of the state-independent part, the scan, the gated
-// norm (max_n = longest sequence)
-int launch_dn_scan(const DnStepParams& p, int M, int max_n, bool pdl, cudaStream_t st);
+// alpha / beta projections of all rows, the rest of the state-independent part, the recurrence (token by token, or in chunks
+// as two launches), the gated norm (max_n = longest sequence)
+int launch_dn_scan(const DnStepParams& p, int M, int max_n, int* n_launches, bool pdl, cudaStream_t st);
 
 struct AttnParams {
   const float* proj; int64_t ldp;            // [M][ldp]: per head (q | gate) x Hq, then k, then v
