@@ -409,12 +409,14 @@ int32_t b200_qgemm(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
   if (!host_w || !host_x || !host_y || rows <= 0 || mrows <= 0) { set_error("qgemm: bad argument"); return EINVAL_; }
   Scratch sc; DTensor t; __half* x16 = nullptr; float* y = nullptr; int* err = nullptr;
   B200_TRY(stage_projection(sc, type, host_w, rows, k, host_x, mrows, &t, &x16, &y, &err));
-  alignas(64) unsigned char tmap[128];
-  B200_TRY(make_x_tensor_map(x16, mrows, (int)k, tile_rows, tmap));
-  QGemmParams p{};
-  p.w = t.data; p.one.expert = 0; p.one.x_row0 = 0; p.one.count = mrows; p.one.y_row0 = 0; p.max_problems = 1; p.max_count = mrows;
-  p.stride = t.stride; p.K = (int)k; p.N = (int)rows; p.y = y; p.ldy = rows; p.err = err;
-  B200_TRY(launch_qgemm(type, GEMM_STORE, tile_rows, p, tmap, false, 0));
+  if (tile_rows != 64 && tile_rows != 128 && tile_rows != 256) { set_error("qgemm: activation tile must be 64, 128 or 256 rows"); return EINVAL_; }
+  if (!wgemm_type(type) || (type == T_Q8_0 && tile_rows != 64)) { set_error("qgemm: weight type has no tensor-core projection kernel (Q4_K, Q5_K, Q6_K; Q8_0 with 64-row tiles)"); return EINVAL_; }
+  WGemmMaps maps{};
+  B200_TRY(make_wmap(type, t.data, rows, t.stride, 128, &maps.w));
+  B200_TRY(make_rows_map(x16, mrows, (int)k, 64, &maps.x));
+  WGemmParams p{};
+  p.one = GemmProblem{0, 0, mrows, 0}; p.n_problems = 1; p.max_count = mrows; p.K = (int)k; p.N = (int)rows; p.ksplit = 1; p.y = y; p.ldy = rows; p.err = err;
+  B200_TRY(launch_wgemm(type, WG_STORE, tile_rows, p, maps, false, 0));
   return finish_projection("qgemm", y, err, (int64_t)mrows * rows, host_y);
 }
 

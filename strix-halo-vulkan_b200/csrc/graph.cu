@@ -88,16 +88,9 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   B200_TRY(dalloc(&logits, (size_t)LR * c.vocab));
   { B200_TRY(dalloc(&dn_pre, (size_t)MR * ((size_t)c.dn_heads_k * 256 + (size_t)c.dn_heads_v * 130))); B200_TRY(dalloc(&dn_wy, (size_t)MR * c.dn_heads_v * 192, false)); B200_TRY(dalloc(&dn_oraw, (size_t)MR * vw)); B200_TRY(dalloc(&dn_ab, (size_t)MR * 2 * c.dn_heads_v)); }
   { std::vector<float> one(64, 1.f); B200_TRY(dalloc(&ones, one.size())); B200_CUDA(cudaMemcpy(ones, one.data(), one.size() * sizeof(float), cudaMemcpyHostToDevice)); }
-  B200_TRY(dalloc(&xperm16, (size_t)MR * used * H)); B200_TRY(dalloc(&gprob, (size_t)c.n_expert)); B200_TRY(dalloc(&n_expert_dev, 1));
-  B200_CUDA(cudaMemcpy(n_expert_dev, &c.n_expert, sizeof(int), cudaMemcpyHostToDevice));
-  for (int i = 0; i < 3; i++) {
-    const int tn = 64 << i;
-    B200_TRY(make_x_tensor_map(xperm16, (int64_t)MR * used, H, tn, tm_xperm[i]));
-    B200_TRY(make_x_tensor_map(act16, (int64_t)MR * slots1, c.ffn_expert, tn, tm_act[i]));
-    B200_TRY(make_x_tensor_map(xn16, MR, H, tn, tm_xn[i]));
-    B200_TRY(make_x_tensor_map(y16, MR, vw, tn, tm_y16[i]));
-    B200_TRY(make_x_tensor_map(ctx16, MR, qw, tn, tm_ctx[i]));
-  }
+  B200_TRY(dalloc(&xperm16, (size_t)MR * slots1 * H)); B200_TRY(dalloc(&gprob, (size_t)c.n_expert + 1));
+  B200_TRY(make_rows_map(xperm16, (int64_t)MR * slots1, H, 64, &tx_xperm));
+  if (c.ffn_expert % 64 == 0) B200_TRY(make_rows_map(act16, (int64_t)MR * slots1, c.ffn_expert, 64, &tx_act));
   const size_t stage_bytes = ((size_t)MR + 31) / 32 * 32 * (4 * sizeof(int32_t) + sizeof(SeqDesc));
   B200_TRY(dalloc(&stage_dev, stage_bytes)); B200_TRY(dalloc(&next_ids, (size_t)MR));
   B200_TRY(dalloc(&hist_len, 1));
@@ -178,16 +171,20 @@ int Graph::entry_cols(int M, bool stream) const {
 }
 int Graph::make_weight_maps() {
   wmaps.resize(m->layers.size());
-  auto map = [](const DTensor& w, int box, TMap* out) { return w.ok() && tgemm_type(w.type) ? make_w_tensor_map(w.type, w.data, w.rows, w.stride, box, out) : (int)OK; };
+  auto narrow = [](const DTensor& w, TMap* out) { return w.ok() && qlist_type(w.type) ? make_w_tensor_map(w.type, w.data, w.rows, w.stride, 16, out) : (int)OK; };
+  auto wide = [](const DTensor& w, int box, WMap* out) { return w.ok() && wgemm_type(w.type) ? make_wmap(w.type, w.data, w.rows, w.stride, box, out) : (int)OK; };
   for (size_t l = 0; l < m->layers.size(); l++) {
     const LayerW& L = m->layers[l];
     LayerMaps& W = wmaps[l];
-    B200_TRY(map(L.gate_exps, 16, &W.gate)); B200_TRY(map(L.up_exps, 16, &W.up)); B200_TRY(map(L.down_exps, 16, &W.down));
-    B200_TRY(map(L.gate_sh, 16, &W.gate_sh)); B200_TRY(map(L.up_sh, 16, &W.up_sh)); B200_TRY(map(L.down_sh, 16, &W.down_sh));
-    B200_TRY(map(L.qkv, 128, &W.qkv)); B200_TRY(map(L.z, 128, &W.z)); B200_TRY(map(L.ssm_out, 128, &W.out));
-    B200_TRY(map(L.q, 128, &W.q)); B200_TRY(map(L.k, 128, &W.k)); B200_TRY(map(L.o, 128, &W.o));
+    B200_TRY(narrow(L.gate_exps, &W.gate)); B200_TRY(narrow(L.up_exps, &W.up)); B200_TRY(narrow(L.down_exps, &W.down));
+    B200_TRY(narrow(L.gate_sh, &W.gate_sh)); B200_TRY(narrow(L.up_sh, &W.up_sh)); B200_TRY(narrow(L.down_sh, &W.down_sh));
+    B200_TRY(wide(L.gate_exps, 64, &W.wgate)); B200_TRY(wide(L.up_exps, 64, &W.wup)); B200_TRY(wide(L.down_exps, 128, &W.wdown));
+    B200_TRY(wide(L.gate_sh, 64, &W.wgate_sh)); B200_TRY(wide(L.up_sh, 64, &W.wup_sh)); B200_TRY(wide(L.down_sh, 128, &W.wdown_sh));
+    B200_TRY(wide(L.qkv, 128, &W.qkv)); B200_TRY(wide(L.z, 128, &W.z)); B200_TRY(wide(L.ssm_out, 128, &W.out));
+    B200_TRY(wide(L.q, 128, &W.q)); B200_TRY(wide(L.k, 128, &W.k)); B200_TRY(wide(L.v, 128, &W.v)); B200_TRY(wide(L.o, 128, &W.o));
+    B200_TRY(wide(L.router, 128, &W.router));
   }
-  return OK;
+  return wide(m->output, 128, &head_map);
 }
 
 int Graph::max_entries_for(int M, bool stream) const {
@@ -223,7 +220,8 @@ bool Graph::experts_stream(const LayerW& L, int M) const {
          c.ffn_expert % 256 == 0 && qlist_fits(c.n_embd, c.ffn_expert, max_entries) && qlist_fits(c.ffn_expert, c.n_embd, max_entries);
 }
 static bool pass_moe_gemm(const b200_config& c, const LayerW& L, int M, int H) {
-  return pass_uses_gemm(M, H) && (int64_t)M * c.n_expert_used >= 32 * (int64_t)c.n_expert && L.gate_exps.type == L.gate_sh.type && L.down_exps.type == L.down_sh.type;
+  return pass_uses_gemm(M, H) && (int64_t)M * c.n_expert_used >= 32 * (int64_t)c.n_expert && L.gate_exps.type == L.gate_sh.type && L.down_exps.type == L.down_sh.type &&
+         c.ffn_expert % 256 == 0 && c.n_embd % 128 == 0 && c.n_expert <= 1024;
 }
 
 // Which weight matrices a pass of M rows multiplies as fp16-rounded values (the tensor-core kernels, the
@@ -324,21 +322,34 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     resid_parts = std::min(tgemm_ksplit(K, H, M, tgemm_cols(M)), slots1);
     return tdense(w.type, wm, H, nullptr, 0, K, xm, sxm, down, H, resid_parts);
   };
-  // passes of 16 rows and more run their dense projections on the tensor cores
+  // passes of 16 rows and more run their dense projections on the tensor cores; one whose tiles would cover under a third
+  // of the SMs stays on exact weights
   const bool use_gemm = pass_uses_gemm(M, H);
-  // tile height per projection: as tall as the pass allows, shrunk while the launch would leave SMs idle
-  // a projection whose tiles would cover under a third of the SMs stays on the column-tiled kernel
-  auto gemm = [&](const DTensor& w, int K, int N, const __half* x, const unsigned char (*tmaps)[128], float* y, int64_t ldy, int epi) {
-    const int tn = gemm_tile_rows(M, N);
-    if (tn == 0) {
+  auto gemm = [&](const DTensor& w, const WMap& wm, int K, int N, const __half* x, const TMap& xm, float* y, int64_t ldy) {
+    if (gemm_tile_rows(M, N) == 0) {
       QGemvParams q = base(w, K, N, x, K);
       q.y = y; q.ldy = ldy;
-      return launch_qgemv(w.type, PRO_F16, epi == GEMM_RESID ? EPI_RESID : EPI_STORE, false, false, q, 0, pdl(), st);
+      return launch_qgemv(w.type, PRO_F16, EPI_STORE, false, false, q, 0, pdl(), st);
     }
-    const unsigned char* tmap = tmaps[tn == 64 ? 0 : tn == 128 ? 1 : 2];
-    QGemmParams g{};
-    g.w = w.data; g.one = GemmProblem{0, 0, M, 0}; g.max_problems = 1; g.max_count = M; g.stride = w.stride; g.K = K; g.N = N; g.y = y; g.ldy = ldy; g.err = err_flag;
-    return launch_qgemm(w.type, epi, tn, g, tmap, pdl(), st);
+    WGemmMaps maps{};
+    maps.w = wm; maps.x = xm;
+    WGemmParams g{};
+    g.one = GemmProblem{0, 0, M, 0}; g.n_problems = 1; g.max_count = M; g.K = K; g.N = N; g.ksplit = 1; g.y = y; g.ldy = ldy; g.err = err_flag;
+    return launch_wgemm(w.type, WG_STORE, wgemm_cols(M, N), g, maps, pdl(), st);
+  };
+  // an output projection: its planes wait in `down` for the row kernel after it, which adds them to the residual
+  auto gemm_resid = [&](const DTensor& w, const WMap& wm, int K, const __half* x, const TMap& xm) {
+    if (gemm_tile_rows(M, H) == 0) {
+      QGemvParams q = base(w, K, H, x, K);
+      q.y = hc; q.ldy = H;
+      return launch_qgemv(w.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st);
+    }
+    WGemmMaps maps{};
+    maps.w = wm; maps.x = xm;
+    WGemmParams g{};
+    resid_parts = std::min(wgemm_ksplit(M, H, K), slots1);
+    g.one = GemmProblem{0, 0, M, 0}; g.n_problems = 1; g.max_count = M; g.K = K; g.N = H; g.ksplit = resid_parts; g.y = down; g.ldy = H; g.plane = (int64_t)M * H; g.err = err_flag;
+    return launch_wgemm(w.type, WG_STORE, wgemm_cols(M, H), g, maps, pdl(), st);
   };
   const int l0 = f.draft ? c.n_layer : 0, l1 = f.draft ? c.n_layer + 1 : c.n_layer;
   if (f.draft) {
@@ -366,11 +377,11 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       p.w[1] = L.z.data; p.seg_end[0] = cw; p.seg_end[1] = cw + vw; p.nseg = 2;
       p.y = proj; p.ldy = proj_ld;
       if (dense_tg(L.qkv.type, M, cw) && dense_tg(L.z.type, M, vw) && cw % 128 == 0) {
-        B200_TRY(tdense(L.qkv.type, wmaps[l].qkv, cw, &wmaps[l].z, vw, H, tx_xn, ts_xn, proj, proj_ld, 1));
+        B200_TRY(tdense(L.qkv.type, wmaps[l].qkv.m[0], cw, &wmaps[l].z.m[0], vw, H, tx_xn, ts_xn, proj, proj_ld, 1));
       } else if (use_gemm) {
-        B200_TRY(gemm(L.qkv, H, cw, xn16, tm_xn, proj, proj_ld, GEMM_STORE));
-        if (dense_tg(L.z.type, M, vw)) B200_TRY(tdense(L.z.type, wmaps[l].z, vw, nullptr, 0, H, tx_xn, ts_xn, proj + cw, proj_ld, 1));
-        else B200_TRY(gemm(L.z, H, vw, xn16, tm_xn, proj + cw, proj_ld, GEMM_STORE));
+        B200_TRY(gemm(L.qkv, wmaps[l].qkv, H, cw, xn16, tx_xn[2], proj, proj_ld));
+        if (dense_tg(L.z.type, M, vw)) B200_TRY(tdense(L.z.type, wmaps[l].z.m[0], vw, nullptr, 0, H, tx_xn, ts_xn, proj + cw, proj_ld, 1));
+        else B200_TRY(gemm(L.z, wmaps[l].z, H, vw, xn16, tx_xn[2], proj + cw, proj_ld));
       } else {
         const int pro = normed(p, L.attn_norm, xn16);  // the DeltaNet step reads the fp16 rows for alpha / beta
         B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
@@ -393,8 +404,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       QGemvParams q = base(L.ssm_out, vw, H, y16, vw);
       q.y = hc; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(vw, H); }
-      if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16, sx_y, ts_y16));
-      else if (use_gemm) B200_TRY(gemm(L.ssm_out, vw, H, y16, tm_y16, hc, H, GEMM_RESID));
+      if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out.m[0], vw, y16, tx_y16, sx_y, ts_y16));
+      else if (use_gemm) B200_TRY(gemm_resid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16[2]));
       else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
     } else {
       const int ai = attn_index[l];
@@ -405,12 +416,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       bool xn_ready = false;
       int s0 = 0;
       if (dense_tg(L.q.type, M, 2 * qw) && dense_tg(L.k.type, M, kvw) && L.k.type == L.q.type && 2 * qw % 128 == 0) {
-        B200_TRY(tdense(L.q.type, wmaps[l].q, 2 * qw, &wmaps[l].k, kvw, H, tx_xn, ts_xn, proj, proj_ld, 1));
+        B200_TRY(tdense(L.q.type, wmaps[l].q.m[0], 2 * qw, &wmaps[l].k.m[0], kvw, H, tx_xn, ts_xn, proj, proj_ld, 1));
         off = 2 * qw + kvw; s0 = 2;
       }
       for (int s = s0; s < 3 && use_gemm; s++) {
-        if (s == 1 && dense_tg(L.k.type, M, kvw)) B200_TRY(tdense(L.k.type, wmaps[l].k, kvw, nullptr, 0, H, tx_xn, ts_xn, proj + off, proj_ld, 1));
-        else B200_TRY(gemm(*seg[s], H, rows[s], xn16, tm_xn, proj + off, proj_ld, GEMM_STORE));
+        if (s == 1 && dense_tg(L.k.type, M, kvw)) B200_TRY(tdense(L.k.type, wmaps[l].k.m[0], kvw, nullptr, 0, H, tx_xn, ts_xn, proj + off, proj_ld, 1));
+        else B200_TRY(gemm(*seg[s], s == 0 ? wmaps[l].q : s == 1 ? wmaps[l].k : wmaps[l].v, H, rows[s], xn16, tx_xn[2], proj + off, proj_ld));
         off += rows[s];
       }
       for (int s = s0; s < 3 && !use_gemm;) {
@@ -452,8 +463,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       QGemvParams q = base(L.o, qw, H, ctx16, qw);
       q.y = hc; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(qw, H); }
-      if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o, qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
-      else if (use_gemm) B200_TRY(gemm(L.o, qw, H, ctx16, tm_ctx, hc, H, GEMM_RESID));
+      if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o.m[0], qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
+      else if (use_gemm) B200_TRY(gemm_resid(L.o, wmaps[l].o, qw, ctx16, tx_ctx[2]));
       else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
     }
     if (!fused) {
@@ -483,12 +494,15 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (use_gemm && M >= ROUTER_MMA_FROM && L.router.type == T_Q8_0) {
       // many rows: the router logits are one more tensor-core GEMM (the reference's prefill router is an fp16
       // GEMM too: llm_gemm MODE 2 + llm_moe_route), selection and work list in a kernel of their own
-      QGemmParams g{};
-      g.w = L.router.data; g.one = GemmProblem{0, 0, M, 0}; g.max_problems = 1; g.max_count = M; g.stride = L.router.stride;
-      g.K = H; g.N = c.n_expert; g.y = r_logits; g.ldy = c.n_expert; g.err = err_flag;
       // up to a few hundred rows the four 128-expert tiles leave the device idle: column-tiled mma instead
       if (M < 256 && router_mma_fits(r)) { B200_TRY(launch_router_mma(r, pdl(), st)); }
-      else B200_TRY(launch_qgemm(T_Q8_0, GEMM_STORE, 64, g, tm_xn[0], pdl(), st));
+      else {
+        WGemmMaps maps{};
+        maps.w = wmaps[l].router; maps.x = tx_xn[2];
+        WGemmParams g{};
+        g.one = GemmProblem{0, 0, M, 0}; g.n_problems = 1; g.max_count = M; g.K = H; g.N = c.n_expert; g.ksplit = 1; g.y = r_logits; g.ldy = c.n_expert; g.err = err_flag;
+        B200_TRY(launch_wgemm(T_Q8_0, WG_STORE, 64, g, maps, pdl(), st));
+      }
       B200_TRY(launch_route_rows(r, pdl(), st));
     } else {
       B200_TRY(launch_router(r, pdl(), st));
@@ -536,26 +550,20 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       B200_TRY(launch_ep_combine(e, M * slots1 + (Mg - M) * used, pdl(), st));
       down_rows = reinterpret_cast<float*>(ep_arena + ep.off_down);
     } else if (moe_gemm) {
-      const int avg = M * used / c.n_expert, tne = avg <= 40 ? 64 : 128, tie = tne == 64 ? 0 : 1;
-      B200_TRY(launch_moe_gather(xn16, cols, M * used, slots1, H, xperm16, pdl(), st));
-      QGemmParams g{};
-      g.problems = reinterpret_cast<const GemmProblem*>(gprob); g.n_problems = n_expert_dev; g.max_problems = c.n_expert; g.max_count = M;
-      g.w = L.gate_exps.data; g.w2 = L.up_exps.data; g.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride; g.stride = L.gate_exps.stride;
+      // every expert's rows side by side, the shared expert's (all rows) last: one launch each for gate/up and down
+      B200_TRY(launch_moe_gather(xn16, cols, M * slots1, slots1, H, xperm16, pdl(), st));
+      const LayerMaps& W = wmaps[l];
+      WGemmMaps mg{};
+      mg.w = W.wgate; mg.w2 = W.wup; mg.ws = W.wgate_sh; mg.ws2 = W.wup_sh; mg.x = tx_xperm;
+      WGemmParams g{};
+      g.problems = reinterpret_cast<const GemmProblem*>(gprob); g.n_problems = c.n_expert + 1; g.max_count = M * slots1; g.ksplit = 1;
       g.K = H; g.N = c.ffn_expert; g.y16 = act16; g.ldy = c.ffn_expert; g.err = err_flag;
-      B200_TRY(launch_qgemm(L.gate_exps.type, GEMM_SWIGLU, tne, g, tm_xperm[tie], pdl(), st));
-      QGemmParams sh{};  // the shared expert: every row, outputs after the routed pairs
-      sh.one = GemmProblem{0, 0, M, M * used}; sh.max_problems = 1; sh.max_count = M; sh.w = L.gate_sh.data; sh.w2 = L.up_sh.data; sh.stride = L.gate_sh.stride;
-      sh.K = H; sh.N = c.ffn_expert; sh.y16 = act16; sh.ldy = c.ffn_expert; sh.err = err_flag;
-      B200_TRY(launch_qgemm(L.gate_sh.type, GEMM_SWIGLU, 64, sh, tm_xn[0], pdl(), st));  // few weight tiles: short activation tiles fill more SMs
-      QGemmParams d{};   // down projections: sorted rows in, pair rows out (cols maps sorted row -> pair)
-      d.problems = g.problems; d.n_problems = n_expert_dev; d.max_problems = c.n_expert; d.max_count = M;
-      d.w = L.down_exps.data; d.expert_stride = (int64_t)H * L.down_exps.stride; d.stride = L.down_exps.stride;
-      d.K = c.ffn_expert; d.N = H; d.y = down; d.ldy = H; d.y_rows = cols; d.err = err_flag;
-      B200_TRY(launch_qgemm(L.down_exps.type, GEMM_STORE, tne, d, tm_act[tie], pdl(), st));
-      QGemmParams ds{};
-      ds.one = GemmProblem{0, M * used, M, M * used}; ds.max_problems = 1; ds.max_count = M; ds.w = L.down_sh.data; ds.stride = L.down_sh.stride;
-      ds.K = c.ffn_expert; ds.N = H; ds.y = down; ds.ldy = H; ds.y_rows = cols; ds.err = err_flag;
-      B200_TRY(launch_qgemm(L.down_sh.type, GEMM_STORE, 64, ds, tm_act[0], pdl(), st));
+      B200_TRY(launch_wgemm(L.gate_exps.type, WG_SWIGLU, 128, g, mg, pdl(), st));
+      WGemmMaps md{};
+      md.w = W.wdown; md.ws = W.wdown_sh; md.x = tx_act;
+      WGemmParams d = g;   // sorted rows in, pair rows out (cols maps sorted row -> pair)
+      d.K = c.ffn_expert; d.N = H; d.y = down; d.ldy = H; d.y_rows = cols;
+      B200_TRY(launch_wgemm(L.down_exps.type, WG_STORE, 128, d, md, pdl(), st));
     } else if (moe_stream) {
       B200_TRY(stream_experts(xn16, sx_xn, entry_cols(M, true)));
     } else {
@@ -623,7 +631,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     p.M = n_logit_rows; p.xcols = std::min(n_logit_rows, QG_MAXCOLS); p.row_ids = logit_rows;
     p.y = logits; p.ldy = N;
     if (use_gemm && n_logit_rows == M) {
-      B200_TRY(gemm(m->output, H, N, xn16, tm_xn, logits, N, GEMM_STORE));
+      B200_TRY(gemm(m->output, head_map, H, N, xn16, tx_xn[2], logits, N));
     } else {
       const int pro = head_reads_xn ? (int)PRO_F16 : normed(p, nrm, nullptr);
       B200_TRY(launch_qgemv(m->output.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));

@@ -35,19 +35,21 @@ struct Graph {
   // reads one and writes the other. h is the one the last pass finished in.
   float *hbuf[2] = {nullptr, nullptr}, *h = nullptr, *proj = nullptr, *attn_partial = nullptr, *down = nullptr, *logits = nullptr, *e_buf = nullptr, *hs_buf = nullptr;
   __half *xn16 = nullptr, *q16 = nullptr, *ctx16 = nullptr, *act16 = nullptr, *y16 = nullptr, *xcat16 = nullptr;
-  // TMA tensor maps of the fp16 activation buffers for the many-row GEMM, per tile height 64 / 128 / 256
-  alignas(64) unsigned char tm_xn[3][128], tm_y16[3][128], tm_ctx[3][128], tm_xperm[3][128], tm_act[3][128];
   float *dn_pre = nullptr, *dn_wy = nullptr, *dn_oraw = nullptr, *dn_ab = nullptr;   // many-token DeltaNet: scan inputs (q | k per key head, v and decay | beta per value head), raw outputs [rows][Hv*D]
   int pass_max_n = 1;                            // longest sequence of the pass being enqueued
   float* ones = nullptr;       // [8] weights 1.0 (the combine of pre-weighted partial rows)
-  __half* xperm16 = nullptr;   // [rows * used][H]: activation rows in expert-sorted order
-  // exact tensor-core projections (tgemm.cuh): maps of every weight matrix and of the activation rows, sub-block sums
-  struct LayerMaps { TMap gate, up, down, gate_sh, up_sh, down_sh, qkv, z, out, q, k, o; };
+  __half* xperm16 = nullptr;   // [rows * (used + 1)][H]: activation rows in expert-sorted order, the shared expert's last
+  // tensor maps of every weight matrix and of the activation rows (tgemm, qlist, wgemm), sub-block sums of the rows
+  struct LayerMaps {
+    TMap gate, up, down, gate_sh, up_sh, down_sh;                 // boxes of 16 rows (qlist)
+    WMap wgate, wup, wdown, wgate_sh, wup_sh, wdown_sh, qkv, z, out, q, k, v, o, router;   // boxes of 64 (gate, up) and 128 rows
+  };
   std::vector<LayerMaps> wmaps;
+  WMap head_map{};
+  TMap tx_xperm{}, tx_act{};   // expert-sorted rows and their activations, boxes of 64 rows
   TMap tx_xn[3], ts_xn[3], tx_y16[3], ts_y16[3], tx_ctx[3], ts_ctx[3];   // activation rows and their sums, boxes of 16 / 32 / 64 rows
   __half *sx_xn = nullptr, *sx_act = nullptr, *sx_y = nullptr, *sx_ctx = nullptr, *sx_ep = nullptr;
-  int4* gprob = nullptr;       // [n_expert] GEMM problem per expert
-  int* n_expert_dev = nullptr;
+  int4* gprob = nullptr;       // [n_expert + 1] GEMM problem per expert, the shared expert's last
   float* ss_part = nullptr;   // [rows][SS_LD] partial sums of squares of the residual rows
   float *r_logits = nullptr, *topk_w = nullptr, *margin = nullptr;
   int32_t *topk = nullptr, *ids_dev = nullptr, *next_ids = nullptr, *history = nullptr;

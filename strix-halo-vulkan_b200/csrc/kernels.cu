@@ -278,7 +278,7 @@ __device__ void build_work_list(const RouterParams& p, int* counts, int* offs, i
       if (eoff[e] + i < p.max_entries) p.entries[eoff[e] + i] = make_int4(e, offs[e] + c, min(EC, counts[e] - c), 0);
   }
   // one GEMM problem per expert for the tensor-core expert kernels: rows [offs, offs + count) of the expert-sorted order
-  if (p.gprob != nullptr) for (int e = tid; e < nE; e += 256) p.gprob[e] = make_int4(e, offs[e], counts[e], offs[e]);
+  if (p.gprob != nullptr) for (int e = tid; e <= nE; e += 256) p.gprob[e] = e < nE ? make_int4(e, offs[e], counts[e], offs[e]) : make_int4(-1, offs[nE], M, offs[nE]);
   const int nshr = sh_hi - sh_lo, nsh = (nshr + EC - 1) / EC;
   for (int i = tid; i < nsh; i += 256)
     if (eoff[nE] + i < p.max_entries) p.entries[eoff[nE] + i] = make_int4(-1, offs[nE] + EC * i, min(EC, nshr - EC * i), 0);

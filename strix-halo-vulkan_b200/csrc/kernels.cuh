@@ -2,7 +2,7 @@
 #pragma once
 #include "common.cuh"
 #include "qgemv.cuh"
-#include "qgemm.cuh"
+#include "wgemm.cuh"
 #include "tgemm.cuh"
 #include "qlist.cuh"
 

@@ -19,7 +19,7 @@ struct RouterParams {
   float* margin;       // [M] optional: (p_k - p_{k+1}) / p_k
   int4* entries; int* n_entries; int* cols;   // expert work list for the grouped kernels
   int* ticket;         // [1 + ceil(M / 8)]: all rows, then one per group of eight rows
-  int4* gprob;         // optional [nE]: {expert, first sorted row, rows, first sorted row} per expert (GemmProblem)
+  int4* gprob;         // optional [nE + 1]: {expert, first sorted row, rows, first sorted row} per expert (GemmProblem), the shared expert last
   int max_entries;
   int defer;           // 1: stop after the logits; the expert kernel that follows selects the experts itself
   int ecols;           // columns per work-list entry (8, or 4 for passes of some tens of rows; 0 means 8)
