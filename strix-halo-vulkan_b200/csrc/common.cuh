@@ -150,6 +150,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
+// One lane of a converged warp, the same one every time. Code under it may hold its addresses and descriptors in uniform registers;
+// under `lane == 0` the compiler cannot tell that one lane runs, and each tcgen05 or TMA instruction costs a loop over the active lanes
+// (measured: eight tcgen05.mma of N 128 and their commits 929 cycles so, 636 under elect.sync).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xffffffff;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(p));
+  return p != 0;
+}
+
 // D = A(16x16, row) * B(16x8, col) + C, fp16 inputs, f32 accumulate.
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(

@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
   // ---- the copy side walks the chunks (unit, super-block, j) ahead of the arithmetic ----
   int f_left = n_units * nb * 4, f_unit = u0 + warp, f_sb = 0, f_j = 0, f_slot = 0, f_row = 0;
   const void *fa = nullptr, *fb = nullptr;
-  auto fetch = [&]() {   // lane 0
+  auto fetch = [&](bool reused) {   // the whole warp keeps the position, one lane asks
     if (f_left == 0) return;
     f_left--;
     if (f_sb == 0 && f_j == 0) {
@@ -114,13 +114,15 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
       fa = ex >= 0 ? &maps.w : &maps.ws;
       fb = !PAIR ? fa : ex >= 0 ? &maps.w2 : &maps.ws2;
     }
-    mbar_expect_tx(&bars[warp][f_slot], Cf::BYTES);
-    tma_box(ring + f_slot * Cf::BYTES, (f_j & 1) ? fb : fa, f_sb * Cf::BLK, f_row + (PAIR ? f_j >> 1 : f_j) * 16, &bars[warp][f_slot]);
+    if (elect_one()) {
+      if (reused) fence_proxy_async();
+      mbar_expect_tx(&bars[warp][f_slot], Cf::BYTES);
+      tma_box(ring + f_slot * Cf::BYTES, (f_j & 1) ? fb : fa, f_sb * Cf::BLK, f_row + (PAIR ? f_j >> 1 : f_j) * 16, &bars[warp][f_slot]);
+    }
     if (++f_j == 4) { f_j = 0; if (++f_sb == nb) { f_sb = 0; f_unit += Cf::WARPS; } }
     f_slot = f_slot + 1 == SLOTS ? 0 : f_slot + 1;
   };
-  if (lane == 0)
-    for (int i = 0; i < SLOTS; i++) fetch();
+  for (int i = 0; i < SLOTS; i++) fetch(false);
 
   // mma row g is row 2g of a chunk, mma row g + 8 row 2g + 1: at a pitch of 144 or 176 bytes the eight-byte reads of four
   // neighbouring g then fall on distinct banks
@@ -227,7 +229,7 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
           }
         }
         __syncwarp();   // every lane has read the chunk
-        if (lane == 0) { fence_proxy_async(); fetch(); }
+        fetch(true);
         if (++slot == SLOTS) { slot = 0; phase ^= 1; }
       }
     }

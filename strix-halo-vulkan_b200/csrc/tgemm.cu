@@ -134,10 +134,11 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
   const long long U = (long long)coltiles * tiles * p.ksplit;
   const int u0 = (int)(blockIdx.x * U / gridDim.x), u1 = (int)((blockIdx.x + 1) * U / gridDim.x);
   uint32_t early = 0;
-  if (warp == 0 && lane == 0) {
+  if (warp == 0) {
     for (int u = u0; u < u1 && early < (uint32_t)NS; u++) {
       const Unit t = unit_at(u);
-      for (int b = 0; b < t.nsb && early < (uint32_t)NS; b++, early++) load_raw(t, t.sb0 + b, early);
+      for (int b = 0; b < t.nsb && early < (uint32_t)NS; b++, early++)
+        if (elect_one()) load_raw(t, t.sb0 + b, early);
     }
   }
   pdl_wait();
@@ -145,50 +146,50 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
 
   if (warp == 0) {
     // ---- loads --------------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int u = u0; u < u1 && !failed; u++) {
-        const Unit t = unit_at(u);
-        for (int b = 0; b < t.nsb; b++, it++) {
-          const int s = it % NS;
-          if (it >= early) {
-            if (!mbar_wait(&empty[s], ((it / NS) & 1) ^ 1)) { give_up(); break; }
-            load_raw(t, t.sb0 + b, s);
-          }
+    uint32_t it = 0;
+    for (int u = u0; u < u1 && !failed; u++) {
+      const Unit t = unit_at(u);
+      for (int b = 0; b < t.nsb; b++, it++) {
+        const int s = it % NS;
+        if (it >= early && !mbar_wait(&empty[s], ((it / NS) & 1) ^ 1)) { give_up(); break; }
+        __syncwarp();
+        if (elect_one()) {
+          if (it >= early) load_raw(t, t.sb0 + b, s);
           load_x(t, t.sb0 + b, s);
         }
+        __syncwarp();
       }
-      // a CTA that gave up leaves only once its copies have landed
-      if (failed)
-        for (uint32_t k = it > (uint32_t)NS ? it - NS : 0; k < it; k++) mbar_wait(&full[k % NS], (k / NS) & 1);
     }
+    // a CTA that gave up leaves only once its copies have landed
+    if (failed)
+      for (uint32_t k = it > (uint32_t)NS ? it - NS : 0; k < it; k++) mbar_wait(&full[k % NS], (k / NS) & 1);
   } else if (warp == 1) {
     // ---- tensor core --------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t it = 0, hx = 0, cx = 0;
-      bool ok = true;
-      for (int u = u0; u < u1 && ok && !failed; u++) {
-        const Unit t = unit_at(u);
-        const uint32_t id = idesc_n((t.cnt + 15) & ~15);
-        for (int b = 0; b < t.nsb && ok; b++, it++, cx++) {
-          const int s = it % NS, cs = cx & 1;
-          const uint32_t acc = tm + TG_ACC + cs * 2 * NMAX;
-          if (!mbar_wait(&full[s], (it / NS) & 1) || !mbar_wait(&c_empty[cs], ((cx >> 1) & 1) ^ 1)) { give_up(); ok = false; break; }
-          const uint32_t bt = smem_addr(smem + (size_t)s * STAGE);
+    uint32_t it = 0, hx = 0, cx = 0;
+    bool ok = true;
+    for (int u = u0; u < u1 && ok && !failed; u++) {
+      const Unit t = unit_at(u);
+      const uint32_t id = idesc_n((t.cnt + 15) & ~15);
+      for (int b = 0; b < t.nsb && ok; b++, it++, cx++) {
+        const int s = it % NS, cs = cx & 1;
+        const uint32_t acc = tm + TG_ACC + cs * 2 * NMAX;
+        if (!mbar_wait(&full[s], (it / NS) & 1) || !mbar_wait(&c_empty[cs], ((cx >> 1) & 1) ^ 1)) { give_up(); ok = false; break; }
+        const uint32_t bt = smem_addr(smem + (size_t)s * STAGE);
 #pragma unroll
-          for (int h = 0; h < 2; h++, hx++) {
-            const int as = hx % TG_NA;
-            if (!mbar_wait(&a_full[as], (hx / TG_NA) & 1)) { give_up(); ok = false; break; }
-            fence_after();
+        for (int h = 0; h < 2; h++, hx++) {
+          const int as = hx % TG_NA;
+          if (!mbar_wait(&a_full[as], (hx / TG_NA) & 1)) { give_up(); ok = false; break; }
+          fence_after();
+          __syncwarp();
+          if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < 8; k++)
               mma_ts(acc, tm + as * TG_ASLOT + 8 * k, desc_sw128(bt + (2 * h + (k >> 2)) * (NMAX * 128)) + 2 * (k & 3), id, (h | k) != 0);
             if (h == 1) mma_ts(acc + NMAX, tm + TG_MIN + (it & 1) * 8, desc_sw128(bt + 4 * (NMAX * 128)), id, 0);
             commit(&a_empty[as]);
+            if (h == 1) { commit(&empty[s]); commit(&c_full[cs]); }
           }
-          if (!ok) break;
-          commit(&empty[s]);
-          commit(&c_full[cs]);
+          __syncwarp();
         }
       }
     }

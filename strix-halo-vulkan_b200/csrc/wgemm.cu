@@ -241,15 +241,16 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
 
   if (warp == 0) {
     // ---- weights --------------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
-        const Item t = item(idx);
-        const int row = (t.pr.expert > 0 ? t.pr.expert * p.N : 0) + t.nt * TROWS;
-        const WMap &wa = t.pr.expert >= 0 ? maps.w : maps.ws, &wb = t.pr.expert >= 0 ? maps.w2 : maps.ws2;
-        for (int b = 0; b < t.nsb; b++, it++) {
-          const int s = it % NR, sb = t.sb0 + b;
-          if (!mbar_wait(&r_empty[s], ((it / NR) & 1) ^ 1)) { give_up(); break; }
+    uint32_t it = 0;
+    for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
+      const Item t = item(idx);
+      const int row = (t.pr.expert > 0 ? t.pr.expert * p.N : 0) + t.nt * TROWS;
+      const WMap &wa = t.pr.expert >= 0 ? maps.w : maps.ws, &wb = t.pr.expert >= 0 ? maps.w2 : maps.ws2;
+      for (int b = 0; b < t.nsb; b++, it++) {
+        const int s = it % NR, sb = t.sb0 + b;
+        if (!mbar_wait(&r_empty[s], ((it / NR) & 1) ^ 1)) { give_up(); break; }
+        __syncwarp();
+        if (elect_one()) {
           mbar_expect_tx(&r_full[s], RAW);
 #pragma unroll
           for (int h = 0; h < (PAIR ? 2 : 1); h++) {
@@ -262,52 +263,59 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
             else { box(0, 128, 0, sb * 256); box(0, 128, 16384, sb * 256 + 128); box(1, 16, 32768, p.K + sb * 16); }
           }
         }
+        __syncwarp();
       }
-      if (failed)                                    // leave only once the copies in flight have landed
-        for (uint32_t k = it > (uint32_t)NR ? it - NR : 0; k < it; k++) mbar_wait(&r_full[k % NR], (k / NR) & 1);
     }
+    if (failed)                                      // leave only once the copies in flight have landed
+      for (uint32_t k = it > (uint32_t)NR ? it - NR : 0; k < it; k++) mbar_wait(&r_full[k % NR], (k / NR) & 1);
   } else if (warp == WG_XW) {
     // ---- activation rows ------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t it = 0;
-      for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
-        const Item t = item(idx);
-        const int boxes = (min(NT, t.pr.count - t.tt * NT) + 63) / 64, row = t.pr.x_row0 + t.tt * NT;
-        for (int c = 0; c < 4 * t.nsb; c++, it++) {
-          const int s = it % NX;
-          if (!mbar_wait(&x_empty[s], ((it / NX) & 1) ^ 1)) { give_up(); break; }
+    uint32_t it = 0;
+    for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
+      const Item t = item(idx);
+      const int boxes = (min(NT, t.pr.count - t.tt * NT) + 63) / 64, row = t.pr.x_row0 + t.tt * NT;
+      for (int c = 0; c < 4 * t.nsb; c++, it++) {
+        const int s = it % NX;
+        if (!mbar_wait(&x_empty[s], ((it / NX) & 1) ^ 1)) { give_up(); break; }
+        __syncwarp();
+        if (elect_one()) {
           mbar_expect_tx(&x_full[s], boxes * 8192);
           for (int b = 0; b < boxes; b++) tma_box(x0 + s * XST + b * 8192, reinterpret_cast<const CUtensorMap*>(&maps.x), t.sb0 * 256 + c * 64, row + 64 * b, &x_full[s]);
         }
+        __syncwarp();
       }
-      if (failed)
-        for (uint32_t k = it > (uint32_t)NX ? it - NX : 0; k < it; k++) mbar_wait(&x_full[k % NX], (k / NX) & 1);
     }
+    if (failed)
+      for (uint32_t k = it > (uint32_t)NX ? it - NX : 0; k < it; k++) mbar_wait(&x_full[k % NX], (k / NX) & 1);
   } else if (warp == 1) {
     // ---- tensor core ------------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t hx = 0, xi = 0, ci = 0;
-      const uint32_t id = idesc_n(NT);
-      bool ok = true;
-      for (int idx = blockIdx.x; idx < total && ok && !failed; idx += gridDim.x, ci++) {
-        const Item t = item(idx);
-        const uint32_t acc = tm + WG_ACC + (ci % NACC) * NT;
-        if (!mbar_wait(&c_empty[ci % NACC], ((ci / NACC) & 1) ^ 1)) { give_up(); break; }
-        for (int h = 0; h < 2 * t.nsb && ok; h++, hx++) {
-          const int as = hx % WG_NA;
-          if (!mbar_wait(&a_full[as], (hx / WG_NA) & 1)) { give_up(); ok = false; break; }
-          for (int c = 0; c < 2; c++, xi++) {
-            const int xs = xi % NX;
-            if (!mbar_wait(&x_full[xs], (xi / NX) & 1)) { give_up(); ok = false; break; }
-            fence_after();
+    uint32_t hx = 0, xi = 0, ci = 0;
+    bool ok = true;
+    for (int idx = blockIdx.x; idx < total && ok && !failed; idx += gridDim.x, ci++) {
+      const Item t = item(idx);
+      const int cols = min(NT, t.pr.count - t.tt * NT);
+      const uint32_t id = idesc_n((cols + 15) & ~15);
+      const uint32_t acc = tm + WG_ACC + (ci % NACC) * NT;
+      if (!mbar_wait(&c_empty[ci % NACC], ((ci / NACC) & 1) ^ 1)) { give_up(); break; }
+      for (int h = 0; h < 2 * t.nsb && ok; h++, hx++) {
+        const int as = hx % WG_NA;
+        if (!mbar_wait(&a_full[as], (hx / WG_NA) & 1)) { give_up(); ok = false; break; }
+#pragma unroll
+        for (int c = 0; c < 2; c++, xi++) {
+          const int xs = xi % NX;
+          if (!mbar_wait(&x_full[xs], (xi / NX) & 1)) { give_up(); ok = false; break; }
+          fence_after();
+          __syncwarp();
+          if (elect_one()) {
             const uint64_t bd = desc_sw128(smem_addr(x0 + xs * XST));
 #pragma unroll
             for (int k = 0; k < 4; k++) mma_ts(acc, tm + as * WG_ASLOT + 32 * c + 8 * k, bd + 2 * k, id, (h | c | k) != 0);
             commit(&x_empty[xs]);
+            if (c == 1) commit(&a_empty[as]);
+            if (c == 1 && h == 2 * t.nsb - 1) commit(&c_full[ci % NACC]);
           }
-          commit(&a_empty[as]);
+          __syncwarp();
         }
-        if (ok) commit(&c_full[ci % NACC]);
       }
     }
   } else if (warp < WG_EP0) {
