@@ -159,6 +159,9 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
+// The wait of a converged warp: every lane polls, and all get the same answer.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
 // D = A(16x16, row) * B(16x8, col) + C, fp16 inputs, f32 accumulate.
 __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(

@@ -108,6 +108,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
 
   const int nb = p.K / 256, tiles = (p.N + TG_TILE - 1) / TG_TILE, coltiles = (p.M + NMAX - 1) / NMAX;
   auto give_up = [&]() { if (p.err != nullptr) atomicExch(p.err, 1); failed = 1; };
+  auto stopped = [&]() { return __any_sync(0xffffffffu, failed); };
   auto unit_at = [&](int u) {
     Unit t;
     t.ks = u % p.ksplit;
@@ -147,12 +148,11 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
   if (warp == 0) {
     // ---- loads --------------------------------------------------------------------------------
     uint32_t it = 0;
-    for (int u = u0; u < u1 && !failed; u++) {
+    for (int u = u0; u < u1 && !stopped(); u++) {
       const Unit t = unit_at(u);
       for (int b = 0; b < t.nsb; b++, it++) {
         const int s = it % NS;
-        if (it >= early && !mbar_wait(&empty[s], ((it / NS) & 1) ^ 1)) { give_up(); break; }
-        __syncwarp();
+        if (it >= early && !warp_wait(&empty[s], ((it / NS) & 1) ^ 1)) { give_up(); break; }
         if (elect_one()) {
           if (it >= early) load_raw(t, t.sb0 + b, s);
           load_x(t, t.sb0 + b, s);
@@ -167,20 +167,19 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
     // ---- tensor core --------------------------------------------------------------------------
     uint32_t it = 0, hx = 0, cx = 0;
     bool ok = true;
-    for (int u = u0; u < u1 && ok && !failed; u++) {
+    for (int u = u0; u < u1 && ok && !stopped(); u++) {
       const Unit t = unit_at(u);
       const uint32_t id = idesc_n((t.cnt + 15) & ~15);
       for (int b = 0; b < t.nsb && ok; b++, it++, cx++) {
         const int s = it % NS, cs = cx & 1;
         const uint32_t acc = tm + TG_ACC + cs * 2 * NMAX;
-        if (!mbar_wait(&full[s], (it / NS) & 1) || !mbar_wait(&c_empty[cs], ((cx >> 1) & 1) ^ 1)) { give_up(); ok = false; break; }
+        if (!warp_wait(&full[s], (it / NS) & 1) || !warp_wait(&c_empty[cs], ((cx >> 1) & 1) ^ 1)) { give_up(); ok = false; break; }
         const uint32_t bt = smem_addr(smem + (size_t)s * STAGE);
 #pragma unroll
         for (int h = 0; h < 2; h++, hx++) {
           const int as = hx % TG_NA;
-          if (!mbar_wait(&a_full[as], (hx / TG_NA) & 1)) { give_up(); ok = false; break; }
+          if (!warp_wait(&a_full[as], (hx / TG_NA) & 1)) { give_up(); ok = false; break; }
           fence_after();
-          __syncwarp();
           if (elect_one()) {
 #pragma unroll
             for (int k = 0; k < 8; k++)
@@ -199,13 +198,13 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16);
     uint32_t it = 0;
     bool ok = true;
-    for (int u = u0; u < u1 && ok && !failed; u++) {
+    for (int u = u0; u < u1 && ok && !stopped(); u++) {
       const Unit t = unit_at(u);
       for (int b = 0; b < t.nsb; b++, it++) {
         const int s = it % NS;
         const uint32_t hx = 2 * it + half;
         const int as = hx % TG_NA;
-        if (!mbar_wait(&full[s], (it / NS) & 1)) { give_up(); ok = false; break; }
+        if (!warp_wait(&full[s], (it / NS) & 1)) { give_up(); ok = false; break; }
         const uint8_t* blk = smem + (size_t)s * STAGE + RAW + row * BLK;
         const uint4 hdr = lds128(blk);
         uint4 qv[4];
@@ -224,7 +223,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
         const uint32_t m01 = hadd2_u(__byte_perm(mn, 0x64646464u, 0x4140), h2c(-1024.f)), m23 = hadd2_u(__byte_perm(mn, 0x64646464u, 0x4342), h2c(-1024.f));
         uint32_t out[32];
         dequant_group<TYPE>(qv[0], qv[1], fifth, 2 * half, sc, 0, out);
-        if (!mbar_wait(&a_empty[as], ((hx / TG_NA) & 1) ^ 1)) { give_up(); ok = false; break; }
+        if (!warp_wait(&a_empty[as], ((hx / TG_NA) & 1) ^ 1)) { give_up(); ok = false; break; }
         fence_after();
         tmem_st32(lane_base + as * TG_ASLOT, out);
         const uint32_t mcol = lane_base + TG_MIN + (it & 1) * 8 + 2 * half;
@@ -245,14 +244,14 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16) + TG_ACC;
     uint32_t it = 0;
     bool ok = true;
-    for (int u = u0; u < u1 && ok && !failed; u++) {
+    for (int u = u0; u < u1 && ok && !stopped(); u++) {
       const Unit t = unit_at(u);
       float acc[NMAX];
 #pragma unroll
       for (int c = 0; c < NMAX; c++) acc[c] = 0.f;
       for (int b = 0; b < t.nsb; b++, it++) {
         const int cs = it & 1;
-        if (!mbar_wait(&d_full[it % TG_ND], (it / TG_ND) & 1) || !mbar_wait(&c_full[cs], (it >> 1) & 1)) { give_up(); ok = false; break; }
+        if (!warp_wait(&d_full[it % TG_ND], (it / TG_ND) & 1) || !warp_wait(&c_full[cs], (it >> 1) & 1)) { give_up(); ok = false; break; }
         fence_after();
         const float2 dm = dd[it % TG_ND][row];
 #pragma unroll

@@ -2,7 +2,7 @@
 //
 // A CTA of twenty warps walks items of 128 weight rows (or 64 gate + 64 up rows) x NT activation rows:
 //   warp 0        TMA boxes of the rows' quant blocks, one super-block per ring stage;
-//   warp 18       TMA boxes of the activation rows, 64 elements per ring stage, only as many rows as the problem has;
+//   warp 18       TMA boxes of the activation rows, 128 elements per ring stage (64 for NT 256), only as many rows as the problem has;
 //   warps 2..13   three groups of four: a group turns half a super-block of the 128 rows (a thread per row) into fp16 and puts
 //                 it into tensor memory with tcgen05.st; the groups take the halves in turn;
 //   warp 1        one thread issues eight tcgen05.mma (M 128, N NT, K 16) per half, A from tensor memory, B from shared memory;
@@ -35,8 +35,9 @@ constexpr int WG_NA = 4, WG_ASLOT = 64, WG_ACC = 256;   // tensor memory: four h
 
 template <int TYPE> __host__ __device__ constexpr int wg_raw() { return WG_TILE * (TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : TYPE == T_Q6_K ? 224 : 272); }
 template <int TYPE> __host__ __device__ constexpr int wg_nr() { return TYPE == T_Q4_K || TYPE == T_Q5_K ? 4 : 3; }
-template <int TYPE, int NT> __host__ __device__ constexpr int wg_nx() {   // activation stages in what the raw stages leave
-  return (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128) < 16 ? (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128) : 16;
+template <int NT> __host__ __device__ constexpr int wg_xc() { return NT == 256 ? 1 : 2; }   // chunks of 64 elements per activation stage
+template <int TYPE, int NT> __host__ __device__ constexpr int wg_nx() {                     // activation stages in what the raw stages leave
+  return (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) < 8 ? (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) : 8;
 }
 
 __device__ __forceinline__ uint32_t h2c(float v) {
@@ -166,19 +167,25 @@ template <> struct HalfBlock<T_Q8_0> {           // planes: int8 quants in two 1
   }
 };
 
-struct Item { GemmProblem pr; int nt, tt, sb0, nsb, ks; };
+__device__ __forceinline__ bool bar_and(int id, int threads, bool v) {
+  uint32_t r;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbarrier.cta.red.and.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}" : "=r"(r) : "r"((uint32_t)v), "r"(id), "r"(threads) : "memory");
+  return r != 0;
+}
+
+struct Item { int expert, cnt, x_row, y_row, nt, ks; };
 
 template <int TYPE, int NT, int EPI>
 __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_constant__ WGemmMaps maps, const WGemmParams p) {
   constexpr bool PAIR = EPI == WG_SWIGLU;
   constexpr int TROWS = PAIR ? 64 : 128;             // output rows of a tile
-  constexpr int NR = wg_nr<TYPE>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XST = NT * 128, NACC = NT == 256 ? 1 : 2;
+  constexpr int NR = wg_nr<TYPE>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC, NACC = NT == 256 ? 1 : 2;
   static_assert(NX >= 2, "two activation stages at least");
   extern __shared__ uint8_t wg_smem[];
   uint8_t* raw0 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wg_smem) + 1023) & ~(uintptr_t)1023);
   uint8_t* x0 = raw0 + NR * RAW;
   __shared__ __align__(8) uint64_t r_full[NR], r_empty[NR], x_full[NX], x_empty[NX], a_full[WG_NA], a_empty[WG_NA], c_full[NACC], c_empty[NACC];
-  __shared__ float ex[PAIR ? 2 * 64 * 33 : 1];
+  __shared__ float ex[PAIR ? 2 * 128 * 17 : 1];
   __shared__ int stile[WG_MAXPROB + 1];              // activation tiles before each problem (exclusive scan)
   __shared__ uint32_t tmem_sm;
   __shared__ volatile int failed;
@@ -221,35 +228,39 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
   }
   __syncthreads();
   const int total = stile[n_prob] * p.ksplit * n_tiles;
-  auto item = [&](int idx) {
-    Item t;
-    const int v = idx / n_tiles, tile = v / p.ksplit;
-    t.nt = idx - v * n_tiles; t.ks = v - tile * p.ksplit;
-    int lo = 0, hi = n_prob - 1;                     // the last problem whose first tile is not after `tile`
-    while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (stile[mid] <= tile) lo = mid; else hi = mid - 1; }
-    if (p.problems != nullptr) {
-      const int4 q = *reinterpret_cast<const int4*>(p.problems + lo);
-      t.pr = GemmProblem{q.x, q.y, q.z, q.w};
-    } else {
-      t.pr = p.one;
+  // A warp works its CTA's next 32 items out at once, one per lane, and takes them by shuffles.
+  Item mine{};
+  auto item = [&](int n) {
+    if ((n & 31) == 0) {
+      const int64_t idx = blockIdx.x + (int64_t)(n + lane) * gridDim.x;
+      if (idx < total) {
+        const int v = (int)idx / n_tiles, tile = v / p.ksplit;
+        int lo = 0, hi = n_prob - 1;                 // the last problem whose first tile is not after `tile`
+        while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (stile[mid] <= tile) lo = mid; else hi = mid - 1; }
+        const GemmProblem pr = p.problems != nullptr ? p.problems[lo] : p.one;
+        const int c0 = (tile - stile[lo]) * NT;
+        mine = Item{pr.expert, min(NT, pr.count - c0), pr.x_row0 + c0, pr.y_row0 + c0, (int)idx - v * n_tiles, v - tile * p.ksplit};
+      }
     }
-    t.tt = tile - stile[lo];
-    t.sb0 = t.ks * nb / p.ksplit; t.nsb = (t.ks + 1) * nb / p.ksplit - t.sb0;
-    return t;
+    const int l = n & 31;
+    auto from = [&](int v) { return __shfl_sync(0xffffffffu, v, l); };
+    return Item{from(mine.expert), from(mine.cnt), from(mine.x_row), from(mine.y_row), from(mine.nt), from(mine.ks)};
   };
+  const int n_items = blockIdx.x < total ? (total - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  auto sb_begin = [&](int ks) { return ks * nb / p.ksplit; };
   auto give_up = [&]() { if (p.err != nullptr) atomicExch(p.err, 1); failed = 1; };
+  auto stopped = [&]() { return __any_sync(0xffffffffu, failed); };
 
   if (warp == 0) {
     // ---- weights --------------------------------------------------------------------------------
     uint32_t it = 0;
-    for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
-      const Item t = item(idx);
-      const int row = (t.pr.expert > 0 ? t.pr.expert * p.N : 0) + t.nt * TROWS;
-      const WMap &wa = t.pr.expert >= 0 ? maps.w : maps.ws, &wb = t.pr.expert >= 0 ? maps.w2 : maps.ws2;
-      for (int b = 0; b < t.nsb; b++, it++) {
-        const int s = it % NR, sb = t.sb0 + b;
-        if (!mbar_wait(&r_empty[s], ((it / NR) & 1) ^ 1)) { give_up(); break; }
-        __syncwarp();
+    for (int n = 0; n < n_items && !stopped(); n++) {
+      const Item t = item(n);
+      const int row = (t.expert > 0 ? t.expert * p.N : 0) + t.nt * TROWS, sb1 = sb_begin(t.ks + 1);
+      const WMap &wa = t.expert >= 0 ? maps.w : maps.ws, &wb = t.expert >= 0 ? maps.w2 : maps.ws2;
+      for (int sb = sb_begin(t.ks); sb < sb1; sb++, it++) {
+        const int s = it % NR;
+        if (!warp_wait(&r_empty[s], ((it / NR) & 1) ^ 1)) { give_up(); break; }
         if (elect_one()) {
           mbar_expect_tx(&r_full[s], RAW);
 #pragma unroll
@@ -271,16 +282,17 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
   } else if (warp == WG_XW) {
     // ---- activation rows ------------------------------------------------------------------------
     uint32_t it = 0;
-    for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x) {
-      const Item t = item(idx);
-      const int boxes = (min(NT, t.pr.count - t.tt * NT) + 63) / 64, row = t.pr.x_row0 + t.tt * NT;
-      for (int c = 0; c < 4 * t.nsb; c++, it++) {
+    for (int n = 0; n < n_items && !stopped(); n++) {
+      const Item t = item(n);
+      const int boxes = (t.cnt + 63) / 64, c1 = 4 * sb_begin(t.ks + 1);
+      for (int c = 4 * sb_begin(t.ks); c < c1; c += XC, it++) {
         const int s = it % NX;
-        if (!mbar_wait(&x_empty[s], ((it / NX) & 1) ^ 1)) { give_up(); break; }
-        __syncwarp();
+        if (!warp_wait(&x_empty[s], ((it / NX) & 1) ^ 1)) { give_up(); break; }
         if (elect_one()) {
-          mbar_expect_tx(&x_full[s], boxes * 8192);
-          for (int b = 0; b < boxes; b++) tma_box(x0 + s * XST + b * 8192, reinterpret_cast<const CUtensorMap*>(&maps.x), t.sb0 * 256 + c * 64, row + 64 * b, &x_full[s]);
+          mbar_expect_tx(&x_full[s], boxes * 8192 * XC);
+#pragma unroll
+          for (int k = 0; k < XC; k++)
+            for (int b = 0; b < boxes; b++) tma_box(x0 + s * XST + k * (NT * 128) + b * 8192, reinterpret_cast<const CUtensorMap*>(&maps.x), (c + k) * 64, t.x_row + 64 * b, &x_full[s]);
         }
         __syncwarp();
       }
@@ -291,28 +303,29 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
     // ---- tensor core ------------------------------------------------------------------------------
     uint32_t hx = 0, xi = 0, ci = 0;
     bool ok = true;
-    for (int idx = blockIdx.x; idx < total && ok && !failed; idx += gridDim.x, ci++) {
-      const Item t = item(idx);
-      const int cols = min(NT, t.pr.count - t.tt * NT);
-      const uint32_t id = idesc_n((cols + 15) & ~15);
+    for (int n = 0; n < n_items && ok && !stopped(); n++, ci++) {
+      const Item t = item(n);
+      const int n_half = 2 * (sb_begin(t.ks + 1) - sb_begin(t.ks));
+      const uint32_t id = idesc_n((t.cnt + 15) & ~15);
       const uint32_t acc = tm + WG_ACC + (ci % NACC) * NT;
-      if (!mbar_wait(&c_empty[ci % NACC], ((ci / NACC) & 1) ^ 1)) { give_up(); break; }
-      for (int h = 0; h < 2 * t.nsb && ok; h++, hx++) {
+      if (!warp_wait(&c_empty[ci % NACC], ((ci / NACC) & 1) ^ 1)) { give_up(); break; }
+      for (int h = 0; h < n_half && ok; h++, hx++) {
         const int as = hx % WG_NA;
-        if (!mbar_wait(&a_full[as], (hx / WG_NA) & 1)) { give_up(); ok = false; break; }
 #pragma unroll
-        for (int c = 0; c < 2; c++, xi++) {
+        for (int c = 0; c < 2; c += XC, xi++) {
+          // even lanes wait for the weights, odd ones for the activations: one latency of a ready barrier instead of two
           const int xs = xi % NX;
-          if (!mbar_wait(&x_full[xs], (xi / NX) & 1)) { give_up(); ok = false; break; }
+          const bool wa = c == 0 && (lane & 1) == 0;
+          ok = __all_sync(0xffffffffu, mbar_wait(wa ? &a_full[as] : &x_full[xs], wa ? (hx / WG_NA) & 1 : (xi / NX) & 1));
+          if (!ok) { give_up(); break; }
           fence_after();
-          __syncwarp();
           if (elect_one()) {
             const uint64_t bd = desc_sw128(smem_addr(x0 + xs * XST));
 #pragma unroll
-            for (int k = 0; k < 4; k++) mma_ts(acc, tm + as * WG_ASLOT + 32 * c + 8 * k, bd + 2 * k, id, (h | c | k) != 0);
+            for (int k = 0; k < 4 * XC; k++) mma_ts(acc, tm + as * WG_ASLOT + 32 * c + 8 * k, bd + (k >> 2) * (NT * 8) + 2 * (k & 3), id, (h | c | k) != 0);
             commit(&x_empty[xs]);
-            if (c == 1) commit(&a_empty[as]);
-            if (c == 1 && h == 2 * t.nsb - 1) commit(&c_full[ci % NACC]);
+            if (c + XC == 2) commit(&a_empty[as]);
+            if (c + XC == 2 && h == n_half - 1) commit(&c_full[ci % NACC]);
           }
           __syncwarp();
         }
@@ -324,21 +337,22 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16);
     uint32_t it0 = 0, hx0 = 0;                       // super-blocks and halves before this item
     bool ok = true;
-    for (int idx = blockIdx.x; idx < total && ok && !failed; idx += gridDim.x) {
-      const Item t = item(idx);
-      for (uint32_t hx = hx0 + (grp + WG_GROUPS - hx0 % WG_GROUPS) % WG_GROUPS; hx < hx0 + 2 * t.nsb; hx += WG_GROUPS) {
+    for (int n = 0; n < n_items && ok && !stopped(); n++) {
+      const Item t = item(n);
+      const int sb0 = sb_begin(t.ks), nsb = sb_begin(t.ks + 1) - sb0;
+      for (uint32_t hx = hx0 + (grp + WG_GROUPS - hx0 % WG_GROUPS) % WG_GROUPS; hx < hx0 + 2 * nsb; hx += WG_GROUPS) {
         const int b = (hx - hx0) >> 1, half = (hx - hx0) & 1, as = hx % WG_NA;
         const uint32_t it = it0 + b;
         const int s = it % NR;
-        if (!mbar_wait(&r_full[s], (it / NR) & 1)) { give_up(); ok = false; break; }
+        if (!warp_wait(&r_full[s], (it / NR) & 1)) { give_up(); ok = false; break; }
         HalfBlock<TYPE> v;
-        v.load(raw0 + s * RAW, row, half, (nb * 208 + (t.sb0 + b) * 2) & 15);
+        v.load(raw0 + s * RAW, row, half, (nb * 208 + (sb0 + b) * 2) & 15);
         __syncwarp();
         if (lane == 0) arrive(&r_empty[s]);
         bool waited = false;
         v.form(half, [&](int sub, const uint32_t (&out)[16]) {
           if (!waited) {
-            ok = mbar_wait(&a_empty[as], ((hx / WG_NA) & 1) ^ 1);
+            ok = warp_wait(&a_empty[as], ((hx / WG_NA) & 1) ^ 1);
             fence_after();
             waited = true;
           }
@@ -350,7 +364,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
         __syncwarp();
         if (lane == 0) arrive(&a_full[as]);
       }
-      it0 += t.nsb; hx0 += 2 * t.nsb;
+      it0 += nsb; hx0 += 2 * nsb;
     }
   } else if (warp < WG_XW) {
     // ---- epilogue -----------------------------------------------------------------------------------
@@ -358,38 +372,50 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16) + WG_ACC;
     uint32_t ci = 0;
     int exb = 0;
-    for (int idx = blockIdx.x; idx < total && !failed; idx += gridDim.x, ci++) {
-      const Item t = item(idx);
-      if (!mbar_wait(&c_full[ci % NACC], (ci / NACC) & 1)) { give_up(); break; }
+    for (int n = 0; n < n_items; n++, ci++) {
+      const Item t = item(n);
+      const int cnt = t.cnt;
+      // output row of column c0 + lane, fetched by the lanes side by side ahead of its use and handed round by shuffles
+      auto row_of = [&](int c0) {
+        const int r = t.y_row + min(c0 + lane, cnt - 1);
+        return p.y_rows != nullptr ? __ldg(p.y_rows + r) : r;
+      };
+      int next_row = row_of(0);
+      bool ok = warp_wait(&c_full[ci % NACC], (ci / NACC) & 1);
+      if (!ok) give_up();
+      if constexpr (PAIR) ok = bar_and(1, 128, ok);   // the four warps meet again below: all leave or none
+      if (!ok) break;
       fence_after();
-      const int cnt = min(NT, t.pr.count - t.tt * NT);
 #pragma unroll 1
       for (int c0 = 0; c0 < cnt; c0 += 32) {
-        // output row of column c0 + lane, fetched by the lanes side by side and handed round by shuffles
-        int my_row = t.pr.y_row0 + t.tt * NT + min(c0 + lane, cnt - 1);
-        if (p.y_rows != nullptr) my_row = __ldg(p.y_rows + my_row);
+        const int my_row = next_row;
         uint32_t v[32];
         tmem_ld16(lane_base + (ci % NACC) * NT + c0, *reinterpret_cast<uint32_t (*)[16]>(v));
         tmem_ld16(lane_base + (ci % NACC) * NT + c0 + 16, *reinterpret_cast<uint32_t (*)[16]>(v + 16));
         tmem_ld_wait();
+        if (c0 + 32 < cnt) {
+          next_row = row_of(c0 + 32);
+        } else {                                     // the accumulator is free for the item after the next
+          fence_before();
+          __syncwarp();
+          if (lane == 0) arrive(&c_empty[ci % NACC]);
+        }
         const int live = min(32, cnt - c0);
         if constexpr (PAIR) {
-          // SwiGLU (shaders/llm_moe_gemv.comp:777-781): the warps of the up rows hand their values to those of the gate rows
-          float* e = ex + exb * (64 * 33) + ((q & 1) * 32 + lane) * 33;
+          // SwiGLU (shaders/llm_moe_gemv.comp:777-781): the gate rows' warps take the first 16 columns and get the up values,
+          // the up rows' warps take the others and get the gates
+          const int up = q >> 1, r = (q & 1) * 32 + lane, orow = t.nt * 64 + r;
+          float* e = ex + exb * (128 * 17);
           exb ^= 1;
-          if (q >= 2) {
 #pragma unroll
-            for (int i = 0; i < 32; i++) e[i] = __uint_as_float(v[i]);
-          }
+          for (int i = 0; i < 16; i++) e[((up ^ 1) * 64 + r) * 17 + i] = __uint_as_float(up ? v[i] : v[16 + i]);
           asm volatile("bar.sync 1, 128;" ::: "memory");
-          if (q < 2) {
-            const int orow = t.nt * 64 + q * 32 + lane;
 #pragma unroll
-            for (int i = 0; i < 32; i++) {
-              const int yr = __shfl_sync(0xffffffffu, my_row, i);
-              const float gv = __uint_as_float(v[i]);
-              if (i < live && orow < p.N) p.y16[(int64_t)yr * p.ldy + orow] = __float2half_rn(gv * sigmoid_acc(gv) * e[i]);
-            }
+          for (int i = 0; i < 16; i++) {
+            const float o = e[(up * 64 + r) * 17 + i], own = __uint_as_float(up ? v[16 + i] : v[i]);
+            const float gv = up ? o : own, uv = up ? own : o;
+            const int yr = __shfl_sync(0xffffffffu, my_row, up * 16 + i);
+            if (up * 16 + i < live && orow < p.N) p.y16[(int64_t)yr * p.ldy + orow] = __float2half_rn(gv * sigmoid_acc(gv) * uv);
           }
         } else {
           const int orow = t.nt * 128 + q * 32 + lane;
@@ -401,9 +427,6 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
           }
         }
       }
-      fence_before();
-      __syncwarp();
-      if (lane == 0) arrive(&c_empty[ci % NACC]);
     }
   }
   fence_before();
@@ -414,7 +437,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
 template <int TYPE, int NT, int EPI>
 int launch_t(const WGemmParams& p, const WGemmMaps& maps, bool pdl, cudaStream_t st) {
   auto kernel = wgemm_kernel<TYPE, NT, EPI>;
-  constexpr int smem = wg_nr<TYPE>() * wg_raw<TYPE>() + wg_nx<TYPE, NT>() * NT * 128 + 1024;
+  constexpr int smem = wg_nr<TYPE>() * wg_raw<TYPE>() + wg_nx<TYPE, NT>() * NT * 128 * wg_xc<NT>() + 1024;
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int sms = sm_count_current();
   if (sms <= 0) return ECUDA;
