@@ -139,6 +139,11 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst_smem, const void* src, u
                : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tma_box_2d(void* dst_smem, const void* map, int c0, int c1, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)),
+               "l"(map), "r"(c0), "r"(c1), "r"((uint32_t)__cvta_generic_to_shared(bar))
+               : "memory");
+}
 // Bounded wait: returns false if the phase did not complete within the limit.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22)) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(bar);

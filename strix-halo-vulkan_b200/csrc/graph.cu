@@ -77,7 +77,7 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
     else dn_index[l] = n_dn++;
   }
   max_entries = std::max(max_entries_for(MR, false), max_entries_for(std::min(MR, 128), false));
-  B200_TRY(dalloc(&hbuf[0], (size_t)MR * H)); B200_TRY(dalloc(&hbuf[1], (size_t)MR * H)); h = hbuf[0]; B200_TRY(dalloc(&proj, (size_t)MR * proj_ld));
+  B200_TRY(dalloc(&h, (size_t)MR * H)); B200_TRY(dalloc(&proj, (size_t)MR * proj_ld));
   B200_TRY(dalloc(&xn16, (size_t)MR * H)); B200_TRY(dalloc(&q16, (size_t)MR * qw)); B200_TRY(dalloc(&ctx16, (size_t)MR * qw));
   B200_TRY(dalloc(&attn_partial, (size_t)attn_rows * c.n_head * nsplit * (hd + 2)));
   B200_TRY(dalloc(&r_logits, (size_t)MR * c.n_expert));
@@ -87,7 +87,6 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   B200_TRY(dalloc(&act16, (size_t)MR * slots1 * c.ffn_expert)); B200_TRY(dalloc(&down, (size_t)MR * slots1 * H));
   B200_TRY(dalloc(&logits, (size_t)LR * c.vocab));
   { B200_TRY(dalloc(&dn_pre, (size_t)MR * ((size_t)c.dn_heads_k * 256 + (size_t)c.dn_heads_v * 130))); B200_TRY(dalloc(&dn_wy, (size_t)MR * c.dn_heads_v * 192, false)); B200_TRY(dalloc(&dn_oraw, (size_t)MR * vw)); B200_TRY(dalloc(&dn_ab, (size_t)MR * 2 * c.dn_heads_v)); }
-  { std::vector<float> one(64, 1.f); B200_TRY(dalloc(&ones, one.size())); B200_CUDA(cudaMemcpy(ones, one.data(), one.size() * sizeof(float), cudaMemcpyHostToDevice)); }
   B200_TRY(dalloc(&xperm16, (size_t)MR * slots1 * H)); B200_TRY(dalloc(&gprob, (size_t)c.n_expert + 1));
   B200_TRY(make_rows_map(xperm16, (int64_t)MR * slots1, H, 64, &tx_xperm));
   if (c.ffn_expert % 64 == 0) B200_TRY(make_rows_map(act16, (int64_t)MR * slots1, c.ffn_expert, 64, &tx_act));
@@ -204,19 +203,16 @@ static int gemm_tile_rows(int M, int N) {
 // Router logits of passes of this many rows and more come from the column-tiled mma kernel (Q8_0 weights as
 // fp16(d * q), the reference's many-row router arithmetic: llm_gemm MODE 2), below it from per-row dot products
 constexpr int ROUTER_MMA_FROM = 16;
-// Fused passes (at most 8 rows) of this many rows and more finish the MoE block's rows in one row kernel; with fewer
-// rows every CTA of the next projection forms them while it stages (each staged row costs every CTA a trip to L2)
-constexpr int COMBINE_ROWS_FROM = 4;
-static bool pass_uses_gemm(int M, int H) { return !(M <= QG_FUSED_ROWS && H <= QG_COMBINE_MAX_K) && M >= 16; }
+static bool pass_uses_gemm(int M, int H) { return !(M <= QG_FUSED_ROWS && H <= QG_FUSED_MAX_K) && M >= 16; }
 // Dense projections of passes above the fused ones that keep their weights exact - all of them below 16 rows, above that
 // those whose tiles would not fill the device as a GEMM - run on the tensor cores all the same where the type has the kernel
 bool Graph::dense_tg(uint32_t type, int M, int N) const {
-  return !(M <= QG_FUSED_ROWS && m->c.n_embd <= QG_COMBINE_MAX_K) && tgemm_type(type) && !(M >= 16 && gemm_tile_rows(M, N) != 0);
+  return !(M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K) && tgemm_type(type) && !(M >= 16 && gemm_tile_rows(M, N) != 0);
 }
 // The experts of passes above the fused ones: warps that stream the weights (qlist.cu), where its types and shapes allow
 bool Graph::experts_stream(const LayerW& L, int M) const {
   const b200_config& c = m->c;
-  return !(M <= QG_FUSED_ROWS && c.n_embd <= QG_COMBINE_MAX_K) && qlist_type(L.gate_exps.type) && qlist_type(L.down_exps.type) && L.down_exps.type == L.down_sh.type &&
+  return !(M <= QG_FUSED_ROWS && c.n_embd <= QG_FUSED_MAX_K) && qlist_type(L.gate_exps.type) && qlist_type(L.down_exps.type) && L.down_exps.type == L.down_sh.type &&
          c.ffn_expert % 256 == 0 && qlist_fits(c.n_embd, c.ffn_expert, max_entries) && qlist_fits(c.ffn_expert, c.n_embd, max_entries);
 }
 static bool pass_moe_gemm(const b200_config& c, const LayerW& L, int M, int H) {
@@ -257,19 +253,10 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   const int H = c.n_embd, D = c.dn_head_dim, qk = c.dn_heads_k * D, vw = c.dn_heads_v * D, cw = 2 * qk + vw;
   const int hd = c.head_dim, qw = c.n_head * hd, kvw = c.n_head_kv * hd, used = c.n_expert_used, slots1 = used + 1;
   const int xcols = std::min(M, QG_MAXCOLS);
-  const bool fused = M <= QG_FUSED_ROWS && H <= QG_COMBINE_MAX_K;
+  const bool fused = M <= QG_FUSED_ROWS && H <= QG_FUSED_MAX_K;
   // expert-parallel MoE block: plain decode passes only (every rank runs the same number of rows at the same time)
   const bool epx = ep_on && ep_ready && !f.draft && !f.spec && n_seq == M;
   const int Mg = epx ? M * ep.world : M;   // rows of all ranks
-  float* hc = hbuf[0];      // residual rows of this pass
-  bool pending = false;     // fused passes: the MoE output of the last layer is not in hc yet; the next
-                            // projection of the residual folds it in while staging and writes the other buffer
-  int trace_layer = -1;     // layer whose post-MoE residual is still to be traced
-  bool xn_valid = false;    // fused passes of 2..8 rows: a row kernel finished the MoE block and left the next
-                            // layer's normalised fp16 rows in xn16 (reading (used + 1) x M expert rows in every
-                            // CTA's staging costs more than that one launch)
-  int comb_used = used;     // what the pending combine adds: comb_used + 1 rows of `down` with weights comb_w
-  const float* comb_w = topk_w;
   launches = 0;
   bool first = true;
   int ss_n = 1;  // partial sums of squares the current residual rows carry
@@ -284,26 +271,14 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   };
   // a projection of the normalised residual: fused passes normalise while staging, others read xn16
   auto normed = [&](QGemvParams& p, const DTensor& gamma, __half* xn_copy) {
-    if (!fused || xn_valid) return (int)PRO_F16;
-    p.hsrc = hc; p.gamma = (const float*)gamma.data; p.xn_out = xn_copy;
-    if (!pending) { p.ss_in = ss_part; p.ss_n = ss_n; return (int)PRO_NORM; }
-    p.down = down; p.topk_w = comb_w; p.used = comb_used; p.h_out = hc == hbuf[0] ? hbuf[1] : hbuf[0];
-    return (int)PRO_COMBINE;
-  };
-  // after a PRO_COMBINE launch the rows live in the other buffer
-  auto combined = [&](int pro) {
-    if (pro != PRO_COMBINE) return OK;
-    hc = hc == hbuf[0] ? hbuf[1] : hbuf[0]; pending = false;
-    if (o.trace && trace_layer >= 0) {
-      B200_CUDA(cudaMemcpyAsync(tr_out + (size_t)trace_layer * MR * H, hc, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st));
-      first = true; trace_layer = -1;
-    }
-    return OK;
+    if (!fused) return (int)PRO_F16;
+    p.hsrc = h; p.gamma = (const float*)gamma.data; p.xn_out = xn_copy; p.ss_in = ss_part; p.ss_n = ss_n;
+    return (int)PRO_NORM;
   };
   auto row_tail = [&](int mode, const DTensor& gamma) {
     TailParams t{};
-    t.mode = mode; t.h = hc; t.gamma = (const float*)gamma.data; t.xn = xn16; t.down = down; t.topk_w = fused ? comb_w : topk_w;
-    t.used = fused ? comb_used : used; t.H = H; t.M = M; t.eps = c.eps; t.sx = fused ? nullptr : sx_xn;
+    t.mode = mode; t.h = h; t.gamma = (const float*)gamma.data; t.xn = xn16; t.down = down; t.topk_w = topk_w;
+    t.used = used; t.H = H; t.M = M; t.eps = c.eps; t.sx = sx_xn;
     return t;
   };
   // exact tensor-core projection of the pass's rows: up to two matrices of one type side by side, outputs at pitch ldy; cut > 1
@@ -341,7 +316,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   auto gemm_resid = [&](const DTensor& w, const WMap& wm, int K, const __half* x, const TMap& xm) {
     if (gemm_tile_rows(M, H) == 0) {
       QGemvParams q = base(w, K, H, x, K);
-      q.y = hc; q.ldy = H;
+      q.y = h; q.ldy = H;
       return launch_qgemv(w.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st);
     }
     WGemmMaps maps{};
@@ -359,13 +334,13 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     B200_TRY(launch_embed(ep, st)); pdl();
     B200_TRY(launch_concat_norm(e_buf, hs_buf, (const float*)L.enorm.data, (const float*)L.hnorm.data, c.eps, H, M, xcat16, pdl(), st));
     QGemvParams p = base(L.eh_proj, 2 * H, H, xcat16, 2 * H);
-    p.y = hc; p.ldy = H;
+    p.y = h; p.ldy = H;
     if (fused) { p.ss_out = ss_part; ss_n = qgemv_groups(2 * H, H); }
     B200_TRY(launch_qgemv(L.eh_proj.type, PRO_F16, EPI_STORE, false, false, p, 0, pdl(), st));
     if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.attn_norm), pdl(), st));
   } else {
     const LayerW& L0 = m->layers[0];
-    EmbedParams ep{m->token_embd, ids_dev, hc, M, H, fused ? nullptr : (const float*)L0.attn_norm.data, xn16, c.eps, fused ? ss_part : nullptr, fused ? nullptr : sx_xn};
+    EmbedParams ep{m->token_embd, ids_dev, h, M, H, fused ? nullptr : (const float*)L0.attn_norm.data, xn16, c.eps, fused ? ss_part : nullptr, fused ? nullptr : sx_xn};
     B200_TRY(launch_embed(ep, st)); pdl();
     ss_n = 1;
   }
@@ -385,7 +360,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       } else {
         const int pro = normed(p, L.attn_norm, xn16);  // the DeltaNet step reads the fp16 rows for alpha / beta
         B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
-        B200_TRY(combined(pro));
       }
       DnStepParams d{};
       d.proj = proj; d.ldp = proj_ld; d.xn = xn16; d.alpha_w = (const float*)L.alpha.data; d.beta_w = (const float*)L.beta.data;
@@ -402,7 +376,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         B200_TRY(launch_dn_step(d, pdl(), st));
       }
       QGemvParams q = base(L.ssm_out, vw, H, y16, vw);
-      q.y = hc; q.ldy = H;
+      q.y = h; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(vw, H); }
       if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out.m[0], vw, y16, tx_y16, sx_y, ts_y16));
       else if (use_gemm) B200_TRY(gemm_resid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16[2]));
@@ -413,7 +387,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       const DTensor* seg[3] = {&L.q, &L.k, &L.v};
       const int rows[3] = {2 * qw, kvw, kvw};
       int off = 0;
-      bool xn_ready = false;
       int s0 = 0;
       if (dense_tg(L.q.type, M, 2 * qw) && dense_tg(L.k.type, M, kvw) && L.k.type == L.q.type && 2 * qw % 128 == 0) {
         B200_TRY(tdense(L.q.type, wmaps[l].q.m[0], 2 * qw, &wmaps[l].k.m[0], kvw, H, tx_xn, ts_xn, proj, proj_ld, 1));
@@ -432,10 +405,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         for (int i = s; i < e; i++) { p.w[i - s] = seg[i]->data; n += rows[i]; p.seg_end[i - s] = n; }
         p.nseg = e - s; p.N = n;
         p.y = proj + off; p.ldy = proj_ld;
-        // the launch that folds the MoE output in also leaves the fp16 rows for the launches after it
-        const int pro = normed(p, L.attn_norm, pending ? xn16 : nullptr);
-        if (xn_ready) { B200_TRY(launch_qgemv(seg[s]->type, PRO_F16, EPI_STORE, false, false, p, 0, pdl(), st)); }
-        else { B200_TRY(launch_qgemv(seg[s]->type, pro, EPI_STORE, false, false, p, 0, pdl(), st)); xn_ready = pro == PRO_COMBINE; B200_TRY(combined(pro)); }
+        const int pro = normed(p, L.attn_norm, nullptr);
+        B200_TRY(launch_qgemv(seg[s]->type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
         off += n; s = e;
       }
       AttnParams a{};
@@ -461,7 +432,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         B200_TRY(launch_attn_merge(a, pdl(), st));
       }
       QGemvParams q = base(L.o, qw, H, ctx16, qw);
-      q.y = hc; q.ldy = H;
+      q.y = h; q.ldy = H;
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(qw, H); }
       if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o.m[0], qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
       else if (use_gemm) B200_TRY(gemm_resid(L.o, wmaps[l].o, qw, ctx16, tx_ctx[2]));
@@ -473,12 +444,11 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       resid_parts = 0;
       B200_TRY(launch_row_tail(t, pdl(), st));
     }
-    if (o.trace) { B200_CUDA(cudaMemcpyAsync(tr_mid + (size_t)l * MR * H, hc, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st)); first = true; }
+    if (o.trace) { B200_CUDA(cudaMemcpyAsync(tr_mid + (size_t)l * MR * H, h, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st)); first = true; }
     // MoE block
-    xn_valid = false;  // the router leaves its own normalised rows in xn16
     RouterParams r{};
     r.xn = xn16; r.router = L.router; r.sh_gate = (const float*)L.sh_gate_inp.data;
-    if (fused) { r.h = hc; r.gamma = (const float*)L.ffn_norm.data; r.ss_in = ss_part; r.ss_n = ss_n; r.eps = c.eps; r.xn_out = xn16; }
+    if (fused) { r.h = h; r.gamma = (const float*)L.ffn_norm.data; r.ss_in = ss_part; r.ss_n = ss_n; r.eps = c.eps; r.xn_out = xn16; }
     r.M = M; r.H = H; r.nE = c.n_expert; r.used = used; r.logits = r_logits; r.probs = nullptr; r.topk = topk; r.topk_w = topk_w;
     r.tl = tl(); r.margin = margin; r.entries = entries; r.n_entries = n_entries; r.cols = cols; r.ticket = r_ticket; r.max_entries = max_entries;
     // passes of at most 8 rows: the router stops after its logits and every row is routed, computed and combined on
@@ -486,7 +456,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     // decode and verify passes equal their rows stepped alone: llm/graph_batch_test.go:36, llm/spec_slots_test.go:199)
     const bool moe_gemm = pass_moe_gemm(c, L, M, H) && !epx;
     const bool moe_stream = !moe_gemm && experts_stream(L, M);
-    r.defer = fused && !epx; r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
+    r.defer = fused && !epx && L.down_exps.type == L.down_sh.type && moe_down_fits(L.down_exps.type, c.ffn_expert, H, used); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
     if (epx) { r.entries = nullptr; r.gprob = nullptr; }   // routing only: the work list comes from the gathered routing
     // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted
     // rows (below that the column-tiled kernel, which streams each expert's weights in whole tiles, is faster)
@@ -518,7 +488,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       d.entries = entries; d.n_entries = n_entries; d.cols = cols; d.x_div = 1; d.K = c.ffn_expert; d.N = H; d.x = act16; d.sx = sx_act; d.y = down; d.ldy = H; d.err = err_flag;
       return launch_qlist(L.down_exps.type, QL_STORE, cols_, d, QListMaps{W.down, W.down, W.down_sh, W.down_sh}, pdl(), st);
     };
-    comb_used = used; comb_w = topk_w;
     float* down_rows = down;   // where the pairs of this rank's rows land
     if (epx) {
       // dispatch -> work list over my experts -> gate/up -> down (stores to the rows' owners) -> barrier
@@ -573,44 +542,28 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     p.y16 = act16; p.ldy = c.ffn_expert;
     p.route_here = r.defer; p.route = r;
     B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, r.defer ? M * slots1 : ne, pdl(), st));
-    QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
-    q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
-    q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M, false));
-    q.y = down; q.ldy = H;
-    if (r.defer && L.down_exps.type == L.down_sh.type && slots1 <= 16) {
-      // per row: the routing weights are applied inside the down projection, which leaves a few partial rows
-      // (one per CTA of a tile) for the next projection to add, instead of used + 1 expert rows
-      MoeDown1Params d1{};
-      d1.w = L.down_exps.data; d1.ws = L.down_sh.data; d1.expert_stride = (int64_t)H * L.down_exps.stride; d1.stride = L.down_exps.stride;
-      d1.K = c.ffn_expert; d1.N = H; d1.used = used; d1.topk = topk; d1.topk_w = topk_w; d1.act = act16; d1.part = down;
-      d1.split = moe_down1_split(used, c.ffn_expert); d1.err = err_flag; d1.tl = tl();
-      B200_TRY(launch_moe_down1(L.down_exps.type, d1, M, pdl(), st));
-      comb_used = d1.split - 1; comb_w = ones;
+    if (r.defer) {
+      MoeDownParams d{};
+      d.K = c.ffn_expert; d.N = H; d.used = used; d.topk = topk; d.topk_w = topk_w; d.act = act16; d.h = h; d.ss_out = ss_part; d.err = err_flag; d.tl = tl();
+      ss_n = H / 16;
+      B200_TRY(launch_moe_down(L.down_exps.type, d, MoeDownMaps{wmaps[l].down, wmaps[l].down_sh}, M, pdl(), st));
     } else {
+      QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
+      q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
+      q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M, false));
+      q.y = down; q.ldy = H;
       B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, ne, pdl(), st));
     }
     }
-    if (r.defer && M >= COMBINE_ROWS_FROM) {
-      // the rows are finished once, by the arithmetic the next projection's staging would use (same sums in the
-      // same order, so the rows are the single-row pass's bit for bit), and the consumers read fp16 rows
-      const DTensor& next_norm = f.draft ? L.head_norm : (l + 1 < c.n_layer ? m->layers[l + 1].attn_norm : m->output_norm);
-      QGemvParams cp{};
-      cp.K = H; cp.M = M; cp.xcols = 1; cp.hsrc = hc; cp.gamma = (const float*)next_norm.data; cp.xn_out = xn16; cp.eps = c.eps;
-      cp.down = down; cp.topk_w = comb_w; cp.used = comb_used; cp.h_out = hc == hbuf[0] ? hbuf[1] : hbuf[0];
-      B200_TRY(launch_combine_rows(cp, pdl(), st));
-      hc = cp.h_out;
-      xn_valid = true;
-    } else if (r.defer) pending = true;
-    else {
+    if (!r.defer) {
       const DTensor& next_norm = f.draft ? L.head_norm : (l + 1 < c.n_layer ? m->layers[l + 1].attn_norm : m->output_norm);
       TailParams tp = row_tail(2, next_norm);
-      tp.down = down_rows;
+      tp.down = down_rows; tp.ss_out = fused ? ss_part : nullptr;
+      ss_n = 1;
       B200_TRY(launch_row_tail(tp, pdl(), st));
-      xn_valid = fused;
     }
     if (o.trace) {
-      if (pending) trace_layer = l;
-      else B200_CUDA(cudaMemcpyAsync(tr_out + (size_t)l * MR * H, hc, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st));
+      B200_CUDA(cudaMemcpyAsync(tr_out + (size_t)l * MR * H, h, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st));
       B200_CUDA(cudaMemcpyAsync(tr_topk + (size_t)l * MR * used, topk, (size_t)M * used * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
       B200_CUDA(cudaMemcpyAsync(tr_w + (size_t)l * MR * slots1, topk_w, (size_t)M * slots1 * sizeof(float), cudaMemcpyDeviceToDevice, st));
       B200_CUDA(cudaMemcpyAsync(tr_margin + (size_t)l * MR, margin, (size_t)M * sizeof(float), cudaMemcpyDeviceToDevice, st));
@@ -618,13 +571,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     }
   }
   const DTensor& nrm = f.draft ? m->layers[c.n_layer].head_norm : m->output_norm;
-  bool head_reads_xn = false;
-  if (pending && n_logit_rows != M) {
-    // the head stages only some of the rows (or none): finish every row in place first
-    B200_TRY(launch_row_tail(row_tail(2, nrm), pdl(), st));
-    pending = false; head_reads_xn = true;
-    if (o.trace && trace_layer >= 0) { B200_CUDA(cudaMemcpyAsync(tr_out + (size_t)trace_layer * MR * H, hc, (size_t)M * H * sizeof(float), cudaMemcpyDeviceToDevice, st)); first = true; trace_layer = -1; }
-  }
   if (n_logit_rows > 0) {
     const int N = f.draft && draft_vocab > 0 ? draft_vocab : c.vocab;
     QGemvParams p = base(m->output, H, N, xn16, H);
@@ -633,16 +579,14 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (use_gemm && n_logit_rows == M) {
       B200_TRY(gemm(m->output, head_map, H, N, xn16, tx_xn[2], logits, N));
     } else {
-      const int pro = head_reads_xn ? (int)PRO_F16 : normed(p, nrm, nullptr);
+      const int pro = normed(p, nrm, nullptr);
       B200_TRY(launch_qgemv(m->output.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
-      B200_TRY(combined(pro));
     }
     if (f.greedy) {
       B200_TRY(launch_argmax(logits, n_logit_rows, N, next_ids, pdl(), st));
       B200_TRY(launch_advance(ids_dev, next_ids, row_pos, seqs, M, history, hist_len, st)); launches++;
     }
   }
-  h = hc;
   last_launches = launches;
   return OK;
 }
@@ -723,10 +667,8 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) { set_error(std::string("graph instantiate: ") + cudaGetErrorString(e)); return ECUDA; }
       it = decode_graphs.emplace(gkey, exec).first;
-      decode_h[gkey] = h;
     }
     B200_CUDA(cudaGraphLaunch(it->second, st));
-    h = decode_h[gkey];
   } else {
     B200_TRY(upload_stage(M));
     B200_TRY(enqueue_pass(M, n_seq, n_lr, f));
@@ -743,7 +685,7 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   stats.host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host_t0).count();
   stats.last_rows = M; stats.last_launches = last_launches; stats.last_device_ms = ms;
   // rows of fused passes select their experts inside the expert kernel: one stream per row and slot
-  if (M <= QG_FUSED_ROWS && m->c.n_embd <= QG_COMBINE_MAX_K && !f.draft && !(ep_on && ep_ready && n_seq == M)) single_row_layers += (int64_t)M * m->c.n_layer;
+  if (M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !f.draft && !(ep_on && ep_ready && n_seq == M)) single_row_layers += (int64_t)M * m->c.n_layer;
   return OK;
 }
 
@@ -861,7 +803,7 @@ int Graph::generate_greedy(const int32_t* slots_in, const int32_t* first, int n,
   B200_CUDA(cudaEventElapsedTime(&last_ms, ev0, ev1));
   stats.passes += steps; stats.rows += (int64_t)steps * n; stats.launches += (int64_t)steps * last_launches; stats.device_ms += last_ms;
   stats.last_rows = n; stats.last_launches = last_launches; stats.last_device_ms = last_ms / steps;
-  if (n <= QG_FUSED_ROWS && m->c.n_embd <= QG_COMBINE_MAX_K && !(ep_on && ep_ready)) single_row_layers += (int64_t)steps * n * m->c.n_layer;
+  if (n <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !(ep_on && ep_ready)) single_row_layers += (int64_t)steps * n * m->c.n_layer;
   memcpy(out, ids_host, (size_t)steps * n * sizeof(int32_t));
   for (int i = 0; i < n; i++) past[slots[i]] += steps;
   spec_n = 0;

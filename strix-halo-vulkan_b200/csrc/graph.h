@@ -31,13 +31,10 @@ struct Graph {
   int n_dn = 0, n_attn = 0;
   std::vector<int> dn_index, attn_index;  // layer -> index among its kind (draft layer = last attention)
   // activations
-  // the residual stream alternates between two buffers: the kernel that folds the MoE output into it
-  // reads one and writes the other. h is the one the last pass finished in.
-  float *hbuf[2] = {nullptr, nullptr}, *h = nullptr, *proj = nullptr, *attn_partial = nullptr, *down = nullptr, *logits = nullptr, *e_buf = nullptr, *hs_buf = nullptr;
+  float *h = nullptr, *proj = nullptr, *attn_partial = nullptr, *down = nullptr, *logits = nullptr, *e_buf = nullptr, *hs_buf = nullptr;
   __half *xn16 = nullptr, *q16 = nullptr, *ctx16 = nullptr, *act16 = nullptr, *y16 = nullptr, *xcat16 = nullptr;
   float *dn_pre = nullptr, *dn_wy = nullptr, *dn_oraw = nullptr, *dn_ab = nullptr;   // many-token DeltaNet: scan inputs (q | k per key head, v and decay | beta per value head), raw outputs [rows][Hv*D]
   int pass_max_n = 1;                            // longest sequence of the pass being enqueued
-  float* ones = nullptr;       // [8] weights 1.0 (the combine of pre-weighted partial rows)
   __half* xperm16 = nullptr;   // [rows * (used + 1)][H]: activation rows in expert-sorted order, the shared expert's last
   // tensor maps of every weight matrix and of the activation rows (tgemm, qlist, wgemm), sub-block sums of the rows
   struct LayerMaps {
@@ -87,7 +84,6 @@ struct Graph {
   int last_rows = 0;
   // replay
   std::map<int, cudaGraphExec_t> decode_graphs, greedy_graphs;
-  std::map<int, float*> decode_h;  // residual buffer a replayed decode graph of M rows finishes in
   long long* timeline = nullptr;  // [launch][8] phase timestamps when B200_TIMELINE is set
   int timeline_cap = 0;
   int launches = 0, last_launches = 0, draft_vocab = 0, draft_vocab_default = 0, resid_off = 0;

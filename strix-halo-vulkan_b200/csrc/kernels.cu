@@ -310,6 +310,7 @@ int launch_ep_worklist(const RouterParams& p, bool pdl, cudaStream_t st) {
 
 __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
   __shared__ int is_last;
+  __shared__ float2 cand[8][32];
   __shared__ int counts[1025], offs[1025], eoff[1025];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H, M = p.M;
   const int row = blockIdx.x * RT_ROWS + warp;  // of the nE + 1 outputs; the last is the shared-expert gate
@@ -427,8 +428,8 @@ __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
   {
     const int n = blockIdx.y * 8 + warp;
     if (n < M) {
-      if (nE <= 512) route_token<16>(p, n, lane);
-      else route_token<32>(p, n, lane);
+      if (nE <= 512) route_token<16>(p, n, lane, true, cand[warp]);
+      else route_token<32>(p, n, lane, true, cand[warp]);
     }
   }
   __threadfence();
@@ -530,6 +531,7 @@ int launch_router_mma(const RouterParams& p, bool pdl, cudaStream_t st) {
 // CTA builds the work list. grid ceil(M / 8), block 256.
 __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
   __shared__ int is_last;
+  __shared__ float2 cand[8][32];
   __shared__ int counts[1025], offs[1025], eoff[1025];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H;
   pdl_wait();
@@ -547,8 +549,8 @@ __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
     }
     acc = warp_sum(acc);
     if (lane == 0) p.topk_w[(size_t)n * (p.used + 1) + p.used] = sigmoid_acc(acc);
-    if (p.nE <= 512) route_token<16>(p, n, lane);
-    else route_token<32>(p, n, lane);
+    if (p.nE <= 512) route_token<16>(p, n, lane, true, cand[warp]);
+    else route_token<32>(p, n, lane, true, cand[warp]);
   }
   __threadfence();
   __syncthreads();
@@ -614,29 +616,11 @@ __global__ void __launch_bounds__(QG_THREADS) row_tail_kernel(TailParams tp) {
       *reinterpret_cast<float4*>(hrow + k) = v;
     }
   }
-  row_rmsnorm_f16(hrow, tp.gamma, tp.eps, tp.H, tp.xn + (size_t)n * tp.H, scratch, tp.sx != nullptr ? tp.sx + (size_t)n * (tp.H / 256 * TG_SX) : nullptr);
+  row_rmsnorm_f16(hrow, tp.gamma, tp.eps, tp.H, tp.xn + (size_t)n * tp.H, scratch, tp.sx != nullptr ? tp.sx + (size_t)n * (tp.H / 256 * TG_SX) : nullptr,
+                  tp.ss_out != nullptr ? tp.ss_out + (size_t)n * SS_LD : nullptr);
 }
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st) {
   return launch_k(row_tail_kernel, dim3(tp.M), dim3(QG_THREADS), 0, pdl, st, tp);
-}
-
-// The MoE block's rows of a fused pass finished once instead of in every consumer CTA's staging: row n = residual +
-// the expert partial rows, then the next RMSNorm, by the very function the projection kernels stage with (so the
-// values are the ones a single-row pass forms in its next projection, bit for bit). grid M, block QG_THREADS.
-__global__ void __launch_bounds__(QG_THREADS) combine_rows_kernel(QGemvParams p) {
-  __shared__ __align__(16) uint8_t xs[2 * QG_COMBINE_MAX_K + 16 * (QG_COMBINE_MAX_K / 64) + 128];
-  __shared__ __align__(16) __half sxs[2 * (QG_COMBINE_MAX_K / 32)];
-  __shared__ float scratch[4 * QG_WARPS];
-  __shared__ int xrows[1];
-  pdl_wait();
-  pdl_launch();
-  if (threadIdx.x == 0) xrows[0] = blockIdx.x;
-  __syncthreads();
-  stage_x_combine(p, xs, sxs, scratch, 1, xrows, qg_xstride(p.K), true);
-}
-int launch_combine_rows(const QGemvParams& p, bool pdl, cudaStream_t st) {
-  if (p.K > QG_COMBINE_MAX_K || p.K % 256 || p.used < 0 || p.used > 32 || p.h_out == nullptr || p.h_out == p.hsrc || p.xn_out == nullptr) { set_error("combine_rows: outside its limits"); return EINVAL_; }
-  return launch_k(combine_rows_kernel, dim3(p.M), dim3(QG_THREADS), 0, pdl, st, p);
 }
 
 // Draft seed input: xcat[n] = fp16(rms(embd[n], enorm)) | fp16(rms(h_prev[n], hnorm))  (llm/mtp.go:352-384)

@@ -38,14 +38,11 @@ int launch_embed(const EmbedParams& p, cudaStream_t st);
 
 // K-quant projections; `pdl` marks the launch as a programmatic dependent of the previous kernel.
 int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st);
-// passes of at most QG_FUSED_ROWS rows: per row, every selected expert's down projection with the routing weights applied,
-// left as a few partial rows for the next projection to add
-int launch_moe_down1(uint32_t type, const MoeDown1Params& p, int rows, bool pdl, cudaStream_t st);
-int moe_down1_split(int used, int K);
+// passes of at most QG_FUSED_ROWS rows: per row, the selected experts' down projections, weighted, with the shared expert added to the residual
+bool moe_down_fits(uint32_t type, int K, int N, int used);
+int launch_moe_down(uint32_t type, const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st);
 int qgemv_groups(int K, int N);
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st);
-// rows of a fused pass: residual + expert partial rows + next RMSNorm, once per row (hsrc, down, topk_w, used, gamma, h_out, xn_out)
-int launch_combine_rows(const QGemvParams& p, bool pdl, cudaStream_t st);
 int launch_concat_norm(const float* e, const float* hs, const float* enorm, const float* hnorm, float eps, int H, int M, __half* xcat, bool pdl, cudaStream_t st);
 
 int launch_router(const RouterParams& p, bool pdl, cudaStream_t st);

@@ -22,8 +22,8 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
   // grid that fits at once needs no second round. Three per SM only for the expert kernels and the Q6_K ones (the head's long walk): elsewhere the register cap costs more than
   // the extra warps give, and every CTA of a projection reads the same activation rows out of L2 - the more
   // CTAs ask at once the longer each waits. Persistent CTAs share the device between the y / z slices.
-  const size_t fixed = qg_fixed_smem(p.K, p.xcols, DUAL), stage = qg_stage_bytes(p.K, p.stride, DUAL);
-  const size_t budgets[4] = {0, 220 * 1024, 110 * 1024, 72 * 1024};
+  const size_t fixed = qg_fixed_smem(p.K, p.xcols, DUAL), stage = qg_stage_bytes(p.K, qg_pitch(TYPE, p.stride), DUAL);
+  const size_t budgets[4] = {0, QG_SMEM_MAX, 110 * 1024, 72 * 1024};
   if (fixed + stage > budgets[1]) { set_error("qgemv: row length too large for shared memory"); return ECAPACITY; }
   int occ = 1, rounds = 1, gx = 1, ns = 1;
   dim3 grid;
@@ -53,7 +53,7 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
     grid = dim3(gx, ny, nz);
   }
   const size_t smem = fixed + (size_t)ns * stage;
-  B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(220 * 1024 + 4096)));
+  B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QG_SMEM_MAX));
   QGemvParams pp = p;
   pp.nstage = ns;
   cudaLaunchConfig_t cfg = {};
@@ -70,7 +70,6 @@ template <int TYPE>
 static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st) {
   if (!grouped && !dual) {
     if (pro == PRO_NORM && epi == EPI_STORE) return launch_one<TYPE, PRO_NORM, EPI_STORE, false, false>(p, 0, pdl, st);
-    if (pro == PRO_COMBINE && epi == EPI_STORE) return launch_one<TYPE, PRO_COMBINE, EPI_STORE, false, false>(p, 0, pdl, st);
     if (pro == PRO_F16 && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, false>(p, 0, pdl, st);
     if (pro == PRO_F16 && epi == EPI_RESID) return launch_one<TYPE, PRO_F16, EPI_RESID, false, false>(p, 0, pdl, st);
   } else if (grouped && pro == PRO_F16) {
@@ -89,45 +88,33 @@ int qgemv_groups(int K, int N) {
   return ((N + 15) / 16 + tpc - 1) / tpc;
 }
 
-// CTAs per tile so that every warp has one (slot, super-block) unit, at most 4
-int moe_down1_split(int used, int K) {
-  const int units = (used + 1) * (K / 256);
-  return std::max(1, std::min(4, (units + QG_WARPS - 1) / QG_WARPS));
-}
-
 template <int TYPE>
-static int launch_md(const MoeDown1Params& p, int rows, bool pdl, cudaStream_t st) {
-  auto kernel = moe_down1_kernel<TYPE>;
-  const int slots1 = p.used + 1, cl = p.split;
-  const size_t smem = md_smem(p.K, (slots1 + cl - 1) / cl, p.stride);
-  if (smem > 200 * 1024) { set_error("moe_down1: tiles too large for shared memory"); return ECAPACITY; }
+static int launch_md(const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st) {
+  auto kernel = moe_down_kernel<TYPE>;
+  const int units = (p.used + 1) * (p.K / 256), rounds = (units + MD_MAXWARPS - 1) / MD_MAXWARPS, warps = (units + rounds - 1) / rounds;
+  const size_t smem = (size_t)warps * (md_raw<TYPE>() + MD_X) + (size_t)units * 16 * sizeof(float);
+  if (smem > 200 * 1024) { set_error("moe_down: too many slots for shared memory"); return ECAPACITY; }
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(((p.N + 15) / 16) * cl, rows); cfg.blockDim = dim3(QG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = dim3(p.N / 16, rows); cfg.blockDim = dim3(warps * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
   return OK;
 }
 
-int launch_moe_down1(uint32_t type, const MoeDown1Params& p, int rows, bool pdl, cudaStream_t st) {
-  if (p.K % 256 != 0 || p.K <= 0 || p.used + 1 > MD_MAXSLOTS || p.split < 1 || p.split > 4 || p.part == nullptr || rows < 1 || rows > QG_FUSED_ROWS) { set_error("moe_down1: shape outside kernel limits"); return EINVAL_; }
-  switch (type) {
-    case T_Q4_K: return launch_md<T_Q4_K>(p, rows, pdl, st);
-    case T_Q5_K: return launch_md<T_Q5_K>(p, rows, pdl, st);
-    case T_Q6_K: return launch_md<T_Q6_K>(p, rows, pdl, st);
-  }
-  set_error("moe_down1: weight type has no fused projection kernel (Q4_K, Q5_K, Q6_K only)");
-  return EINVAL_;
+bool moe_down_fits(uint32_t type, int K, int N, int used) { return (type == T_Q4_K || type == T_Q5_K) && K % 256 == 0 && N % 16 == 0 && N / 16 <= SS_LD && used < 32 && (used + 1) * (K / 256) <= 512; }
+int launch_moe_down(uint32_t type, const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st) {
+  if (!moe_down_fits(type, p.K, p.N, p.used) || rows < 1) { set_error("moe_down: shape outside kernel limits (Q4_K, Q5_K)"); return EINVAL_; }
+  return type == T_Q4_K ? launch_md<T_Q4_K>(p, maps, rows, pdl, st) : launch_md<T_Q5_K>(p, maps, rows, pdl, st);
 }
 
 int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st) {
   if (p.K % 256 != 0 || p.K <= 0) { set_error("qgemv: row length must be a multiple of 256"); return EINVAL_; }
   if (p.xcols < 1 || p.xcols > QG_MAXCOLS) { set_error("qgemv: xcols out of range"); return EINVAL_; }
   if (p.ss_out != nullptr && qgemv_groups(p.K, p.N) > SS_LD) { set_error("qgemv: more tile groups than partial-sum slots"); return ECAPACITY; }
-  if (pro == PRO_COMBINE && (p.K > QG_COMBINE_MAX_K || p.used < 0 || p.used > 32 || p.M > QG_MAXCOLS || p.h_out == nullptr || p.h_out == p.hsrc)) { set_error("qgemv: combine prologue outside its limits"); return EINVAL_; }
   if (pro == PRO_NORM && (p.ss_n < 1 || p.ss_n > SS_LD)) { set_error("qgemv: bad partial-sum count"); return EINVAL_; }
   switch (type) {
     case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, max_entries, pdl, st);

@@ -31,11 +31,11 @@ namespace b200 {
 constexpr int QG_WARPS = 8;
 constexpr int QG_THREADS = QG_WARPS * 32;
 constexpr int QG_MAXCOLS = 8;
-constexpr int QG_FUSED_ROWS = 8;  // passes of at most this many rows fold norms and the MoE combine into the staging of the consumers
+constexpr int QG_FUSED_ROWS = 8;       // passes of at most this many rows fold norms into the staging of the consumers
+constexpr int QG_FUSED_MAX_K = 2048;   // ... of residual rows up to this long
 
 enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2 };
-enum { PRO_F16 = 0, PRO_NORM = 1, PRO_COMBINE = 2 };
-constexpr int QG_COMBINE_MAX_K = 2048;  // PRO_COMBINE keeps a row's values in registers: 8 per thread
+enum { PRO_F16 = 0, PRO_NORM = 1 };
 constexpr int SS_LD = 512;  // partial sums of squares kept per activation row
 
 struct QGemvParams {
@@ -76,16 +76,7 @@ struct QGemvParams {
   const float* ss_in;
   int ss_n;
   float eps;
-  __half* xn_out;            // PRO_NORM / PRO_COMBINE: optional copy of the normalised rows, [.][K], written by CTA 0
-  // PRO_COMBINE: the rows are the residual `hsrc` plus the MoE block's output that the expert down
-  // projection left per slot: v = h + (sum_s down[row][s] * topk_w[row][s] in slot order, then the gated
-  // shared expert) (reference: llm/moe.go:347-357, 403-406). Every CTA forms the rows it needs and their
-  // sums of squares itself; CTA 0 also writes them to `h_out`, which must not alias `hsrc` (other CTAs
-  // are still reading it).
-  const float* down;         // [.][used+1][K]
-  const float* topk_w;       // [.][used+1]
-  int used;
-  float* h_out;              // [.][K]
+  __half* xn_out;            // PRO_NORM: optional copy of the normalised rows, [.][K], written by CTA 0
   float* ss_out;             // STORE / RESID: optional partial sums of squares of the rows written, [.][SS_LD], part = tile group
   // epilogue
   float* y;                  // STORE / RESID: float [.][ldy]
@@ -99,7 +90,9 @@ __host__ __device__ inline int qg_xstride(int K) {
   return base + pad;
 }
 constexpr int QG_MAX_STAGES = 8;
-// bytes of one pipeline stage: the tiles one CTA works on per iteration, copied whole
+constexpr size_t QG_SMEM_MAX = 222 * 1024;   // dynamic shared memory of a CTA that has its SM alone
+// pitch of a weight row in shared memory (see mma_row), and bytes of one pipeline stage: the tiles one CTA works on per iteration
+__host__ __device__ inline int64_t qg_pitch(uint32_t type, int64_t stride) { return type == T_Q6_K ? stride : stride + 16; }
 __host__ __device__ inline size_t qg_stage_bytes(int K, int64_t stride, bool dual) {
   const int nb = K / 256;
   const int wpt = nb >= 8 ? 8 : nb >= 4 ? 4 : nb >= 2 ? 2 : 1;
@@ -120,99 +113,97 @@ __device__ __forceinline__ int xs_off(int k) {
   return 2 * ((k & ~3) | p) + 16 * (k >> 6);
 }
 
-struct Frag8 {  // A registers of the 8 mmas one 16-byte quad feeds, for one row
-  uint32_t lo02[4], lo13[4], hi02[4], hi13[4];
-};
-
-constexpr uint32_t H2_1024 = 0x64006400u;
+__device__ __forceinline__ uint4 ld_s128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_s64(uint32_t a) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
+  return v;
+}
 
 __device__ __forceinline__ uint32_t half2_const(float v) {
   __half2 h = __float2half2_rn(v);
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// ---- Q4_K ---------------------------------------------------------------------------
-// Block: d, dmin (fp16), 12 bytes of packed 6-bit (scale, min), 128 bytes of nibbles
-// (reference: gguf/dequant.go:238-276). Thread t of a quad takes 16-byte quads t and t+4:
-// groups t>>1 and (t>>1)+2, i.e. sub-blocks {2th, 2th+1} and {4+2th, 5+2th}.
-struct Q4KRow {
-  uint4 hdr, qa, qb;
-};
-
-__device__ __forceinline__ void q4k_issue(Q4KRow& r, const uint8_t* blk, int t) {
-  r.hdr = lds128(blk);
-  r.qa = lds128(blk + 16 + 16 * t);
-  r.qb = lds128(blk + 16 + 16 * (t + 4));
+// ---- Q4_K, Q5_K -------------------------------------------------------------------------
+// Block: d, dmin (fp16), 12 bytes of packed 6-bit (scale, min), for Q5_K 32 bytes of fifth bits, 128 bytes of nibbles
+// (reference: gguf/dequant.go:238-318); 32 bytes of nibbles hold two sub-blocks, the even one low. Thread t of a quad takes
+// bytes 8t .. 8t + 7 of each such group, so that one mma step lies within one sub-block.
+// Quants enter the tensor core as they are: four or five bits in the low end of a half are the subnormal q * 2^-24, exactly,
+// so a pair of weights costs one mask and no conversion, no multiply; the sub-block scale is applied to the f32 result of
+// the sub-block's two mma steps, the 2^24 (and the 16 of a high nibble left in place) with the block scale.
+// lo: sub-block 2G, hi: 2G + 1; of a word's four bytes the pairs are (0, 2) and (1, 3).
+template <int TYPE>
+__device__ __forceinline__ void unpack_word(uint32_t w, uint32_t fifth, int G, uint32_t& l02, uint32_t& l13, uint32_t& h02, uint32_t& h13) {
+  if constexpr (TYPE == T_Q4_K) {
+    const uint32_t w8 = w >> 8;
+    l02 = w & 0x000F000Fu; h02 = w & 0x00F000F0u; l13 = w8 & 0x000F000Fu; h13 = w8 & 0x00F000F0u;
+  } else {   // fifth bits: bit 2G of a byte belongs to its low nibble, bit 2G + 1 to the high one
+    const uint32_t f = fifth >> (2 * G);
+    const uint32_t lo = (w & 0x0F0F0F0Fu) | ((f << 4) & 0x10101010u), hi = ((w >> 4) & 0x0F0F0F0Fu) | ((f << 3) & 0x10101010u);
+    l02 = lo & 0x00FF00FFu; l13 = (lo >> 8) & 0x00FF00FFu; h02 = hi & 0x00FF00FFu; h13 = (hi >> 8) & 0x00FF00FFu;
+  }
+}
+// D = A B, no accumulator in
+__device__ __forceinline__ void mma16816_z(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+// scales (bytes 2 pair, 2 pair + 1 of a word) of a low- and a high-nibble sub-block as f32
+template <int TYPE>
+__device__ __forceinline__ void sub_scales(uint32_t four, int pair, float (&s)[2]) {
+  const uint32_t h2 = hadd2_u(__byte_perm(four, 0x64646464u, pair ? 0x4342 : 0x4140), half2_const(-1024.f));
+  s[0] = h2f_lo(h2);
+  s[1] = h2f_hi(TYPE == T_Q4_K ? hmul2_u(h2, half2_const(0.0625f)) : h2);
 }
 
-// (scale, min) byte pairs of the thread's two groups: *_a for quad a, *_b for quad b.
-__device__ __forceinline__ void k4_scales(const uint4& hdr, int th, uint32_t& sc_a, uint32_t& m_a, uint32_t& sc_b, uint32_t& m_b) {
-  int sel = th * 16;
-  uint32_t s0 = (hdr.y >> sel) & 0xFFFFu, s1 = (hdr.z >> sel) & 0xFFFFu, s2 = (hdr.w >> sel) & 0xFFFFu;
-  sc_a = s0 & 0x3F3Fu;
-  m_a = s1 & 0x3F3Fu;
-  sc_b = (s2 & 0x0F0Fu) | ((s0 >> 2) & 0x3030u);
-  m_b = ((s2 >> 4) & 0x0F0Fu) | ((s1 >> 2) & 0x3030u);
-}
+// two bytes (b0, b1) of each pair picked by sel -> half2(b0, b1), exact
+__device__ __forceinline__ uint32_t mins_half2(uint32_t four, uint32_t sel) { return hadd2_u(__byte_perm(four, 0x64646464u, sel), half2_const(-1024.f)); }
 
-// two bytes (b0, b1) -> half2(b0, b1), exact
-__device__ __forceinline__ uint32_t bytes_to_half2(uint32_t two_bytes) {
-  uint32_t magic = __byte_perm(two_bytes, 0x64646464u, 0x4140);  // (b0, 0x64, b1, 0x64)
-  return hadd2_u(magic, half2_const(-1024.f));
-}
-
-struct ScaleConst {  // per (row, group): constants turning magic halves into sc*q
-  uint32_t sl, ol, sh, oh;
-};
-__device__ __forceinline__ ScaleConst make_scale_const(uint32_t sc_pair_bytes) {
-  uint32_t sc2 = bytes_to_half2(sc_pair_bytes);     // (sc_even, sc_odd)
-  uint32_t se = __byte_perm(sc2, 0, 0x1010);        // (sc_even, sc_even)
-  uint32_t so = __byte_perm(sc2, 0, 0x3232);        // (sc_odd, sc_odd)
-  ScaleConst c;
-  c.sl = se;
-  c.ol = hmul2_u(se, half2_const(-1024.f));         // <= 64512, exact
-  c.sh = hmul2_u(so, half2_const(0.0625f));
-  c.oh = hmul2_u(so, half2_const(-64.f));
-  return c;
-}
-
-// One 32-bit word of nibbles (bytes b0..b3): low nibbles belong to the even sub-block,
-// high nibbles to the odd one. Pairs come out as (b0,b2) and (b1,b3).
-__device__ __forceinline__ void q4_unpack_word(uint32_t w, const ScaleConst& c, uint32_t& lo02, uint32_t& lo13, uint32_t& hi02, uint32_t& hi13) {
-  uint32_t w8 = w >> 8;
-  lo02 = hfma2_u(lop3_or_and(w, 0x000F000Fu, H2_1024), c.sl, c.ol);    // (1024+q)*sc - 1024*sc
-  hi02 = hfma2_u(lop3_or_and(w, 0x00F000F0u, H2_1024), c.sh, c.oh);    // (1024+16q)*sc/16 - 64*sc
-  lo13 = hfma2_u(lop3_or_and(w8, 0x000F000Fu, H2_1024), c.sl, c.ol);
-  hi13 = hfma2_u(lop3_or_and(w8, 0x00F000F0u, H2_1024), c.sh, c.oh);
-}
-
-// ---- Q5_K ---------------------------------------------------------------------------
-// Q4_K plus a 32-byte plane of fifth bits at offset 16; nibbles start at 48
-// (reference: gguf/dequant.go:282-318). Bit s of qh[l] belongs to sub-block s.
-struct Q5KRow {
-  uint4 hdr, qh, qa, qb;
-};
-__device__ __forceinline__ void q5k_issue(Q5KRow& r, const uint8_t* blk, int t) {
-  r.hdr = lds128(blk);
-  r.qh = lds128(blk + 16 + 16 * (t & 1));
-  r.qa = lds128(blk + 48 + 16 * t);
-  r.qb = lds128(blk + 48 + 16 * (t + 4));
-}
-// s_even = 2*group. v5 bytes = nibble | bit<<4, then (b0,b2) / (b1,b3) pairs as magic halves.
-__device__ __forceinline__ void q5_unpack_word(uint32_t w, uint32_t qh, int s_even, const ScaleConst& c, uint32_t& lo02, uint32_t& lo13,
-                                               uint32_t& hi02, uint32_t& hi13) {
-  // bit s of every byte -> bit 4 of that byte: rotate right by (s - 4) mod 32
-  uint32_t rl = __funnelshift_r(qh, qh, (s_even - 4) & 31);
-  uint32_t rh = __funnelshift_r(qh, qh, (s_even - 3) & 31);
-  uint32_t lo = lop3_or_andb(w & 0x0F0F0F0Fu, rl, 0x10101010u);
-  uint32_t hi = lop3_or_andb((w >> 4) & 0x0F0F0F0Fu, rh, 0x10101010u);
-  uint32_t neg = c.ol;  // -1024*sc_even
-  lo02 = hfma2_u(__byte_perm(lo, 0x64646464u, 0x4240), c.sl, neg);
-  lo13 = hfma2_u(__byte_perm(lo, 0x64646464u, 0x4341), c.sl, neg);
-  // odd sub-block: constants (sc_odd, -1024*sc_odd) = (16*sh, 16*oh)
-  uint32_t so = hmul2_u(c.sh, half2_const(16.f)), oo = hmul2_u(c.oh, half2_const(16.f));
-  hi02 = hfma2_u(__byte_perm(hi, 0x64646464u, 0x4240), so, oo);
-  hi13 = hfma2_u(__byte_perm(hi, 0x64646464u, 0x4341), so, oo);
+// One super-block of the rows of mma rows g (at smem address ra) and g + 8 (rb), added to acc (C layout: [0], [1] row g, columns
+// 2t, 2t + 1; [2], [3] row g + 8). x: this lane's column of the staged activations at the super-block (xs_off layout); sx0, sx1:
+// its pairs of sub-block sums 2 (t / 2), + 1 and 4 + these, hi parts for even t and lo parts for odd t.
+template <int TYPE>
+__device__ __forceinline__ void k45_accumulate(float (&acc)[4], uint32_t ra, uint32_t rb, const uint8_t* x, uint32_t sx0, uint32_t sx1, int t) {
+  constexpr int QOFF = TYPE == T_Q4_K ? 16 : 48;
+  const uint4 h0 = ld_s128(ra), h1 = ld_s128(rb);
+  // 6-bit scales of the two rows, four sub-blocks to a word (gguf/dequant.go:238-243)
+  const uint32_t scl[2][2] = {{h0.y & 0x3F3F3F3Fu, (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u)}, {h1.y & 0x3F3F3F3Fu, (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u)}};
+  uint2 f0 = make_uint2(0, 0), f1 = f0;
+  if constexpr (TYPE == T_Q5_K) { f0 = ld_s64(ra + 16 + 8 * t); f1 = ld_s64(rb + 16 + 8 * t); }
+  float a[4] = {0.f, 0.f, 0.f, 0.f};   // sub-block scale x (q . x), without d
+#pragma unroll
+  for (int G = 0; G < 4; G++) {
+    const uint2 q0 = ld_s64(ra + QOFF + 32 * G + 8 * t), q1 = ld_s64(rb + QOFF + 32 * G + 8 * t);
+    uint32_t al[2][4], ah[2][4];
+    unpack_word<TYPE>(q0.x, f0.x, G, al[0][0], al[0][2], ah[0][0], ah[0][2]);
+    unpack_word<TYPE>(q1.x, f1.x, G, al[0][1], al[0][3], ah[0][1], ah[0][3]);
+    unpack_word<TYPE>(q0.y, f0.y, G, al[1][0], al[1][2], ah[1][0], ah[1][2]);
+    unpack_word<TYPE>(q1.y, f1.y, G, al[1][1], al[1][3], ah[1][1], ah[1][3]);
+    float s0[2], s1[2];
+    sub_scales<TYPE>(scl[0][G >> 1], G & 1, s0);
+    sub_scales<TYPE>(scl[1][G >> 1], G & 1, s1);
+    const uint4 xl = *reinterpret_cast<const uint4*>(x + 144 * G + 16 * t), xh = *reinterpret_cast<const uint4*>(x + 144 * G + 64 + 16 * t);
+    float C[4], D[4];
+    mma16816_z(C, al[0], xl.x, xl.y); mma16816(C, al[1], xl.z, xl.w);
+    mma16816_z(D, ah[0], xh.x, xh.y); mma16816(D, ah[1], xh.z, xh.w);
+    a[0] = fmaf(s0[0], C[0], a[0]); a[1] = fmaf(s0[0], C[1], a[1]); a[2] = fmaf(s1[0], C[2], a[2]); a[3] = fmaf(s1[0], C[3], a[3]);
+    a[0] = fmaf(s0[1], D[0], a[0]); a[1] = fmaf(s0[1], D[1], a[1]); a[2] = fmaf(s1[1], D[2], a[2]); a[3] = fmaf(s1[1], D[3], a[3]);
+  }
+  // min term: one mma over the eight sub-block sums, then the block scales
+  const uint32_t sel = 0x4040u | (2 * (t >> 1)) | ((2 * (t >> 1) + 1) << 8);
+  const uint32_t am[4] = {mins_half2(h0.z & 0x3F3F3F3Fu, sel), mins_half2(h1.z & 0x3F3F3F3Fu, sel), mins_half2(((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u), sel),
+                          mins_half2(((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u), sel)};
+  float Cm[4];
+  mma16816_z(Cm, am, sx0, sx1);
+  const float d0 = h2f_lo(h0.x) * 16777216.f, n0 = h2f_hi(h0.x), d1 = h2f_lo(h1.x) * 16777216.f, n1 = h2f_hi(h1.x);
+  acc[0] = fmaf(-n0, Cm[0], fmaf(d0, a[0], acc[0])); acc[1] = fmaf(-n0, Cm[1], fmaf(d0, a[1], acc[1]));
+  acc[2] = fmaf(-n1, Cm[2], fmaf(d1, a[2], acc[2])); acc[3] = fmaf(-n1, Cm[3], fmaf(d1, a[3], acc[3]));
 }
 
 // ---- Q6_K (row planes, see DTensor) ---------------------------------------------------
@@ -280,94 +271,52 @@ __device__ __forceinline__ void quad_mmas(float (&C)[4], const uint8_t* xrow, bo
   }
 }
 
-template <int TYPE>
-struct RowRegs;
-template <> struct RowRegs<T_Q4_K> { using type = Q4KRow; };
-template <> struct RowRegs<T_Q5_K> { using type = Q5KRow; };
-template <> struct RowRegs<T_Q6_K> { using type = Q6KRow; };
-
-template <int TYPE>
-__device__ __forceinline__ void issue_row(typename RowRegs<TYPE>::type& r, const uint8_t* row, int nb, int blk, int t) {
-  if constexpr (TYPE == T_Q4_K) q4k_issue(r, row + (size_t)blk * 144, t);
-  else if constexpr (TYPE == T_Q5_K) q5k_issue(r, row + (size_t)blk * 176, t);
-  else q6k_issue(r, row, nb, blk, t);
-}
-
-// Accumulates one super-block of rows (g, g+8) into acc (C layout: [0],[1] row g cols 2t,2t+1;
-// [2],[3] row g+8).
-template <int TYPE>
-__device__ __forceinline__ void block_accumulate(float (&acc)[4], const typename RowRegs<TYPE>::type& r0, const typename RowRegs<TYPE>::type& r1,
-                                                 const uint8_t* xrow, const __half* sxrow, bool live, int blk, int t) {
+// One super-block of rows g and g + 8 into acc (C layout as in k45_accumulate)
+__device__ __forceinline__ void q6_accumulate(float (&acc)[4], const Q6KRow& r0, const Q6KRow& r1, const uint8_t* xrow, bool live, int blk, int t) {
   const int th = t >> 1, hb = t & 1;
   float C[4] = {0.f, 0.f, 0.f, 0.f}, C2[4] = {0.f, 0.f, 0.f, 0.f};
-  if constexpr (TYPE == T_Q4_K || TYPE == T_Q5_K) {
-    uint32_t sca0, ma0, scb0, mb0, sca1, ma1, scb1, mb1;
-    k4_scales(r0.hdr, th, sca0, ma0, scb0, mb0);
-    k4_scales(r1.hdr, th, sca1, ma1, scb1, mb1);
-    const ScaleConst ca0 = make_scale_const(sca0), cb0 = make_scale_const(scb0);
-    const ScaleConst ca1 = make_scale_const(sca1), cb1 = make_scale_const(scb1);
-    const int ka = blk * 256 + 64 * th + 16 * hb, kb = ka + 128;
-    if constexpr (TYPE == T_Q4_K) {
-      quad_mmas(C, xrow, live, ka, 32, r0.qa, r1.qa,
-                [&](int, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q4_unpack_word(w, ca0, a, b, c, d); },
-                [&](int, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q4_unpack_word(w, ca1, a, b, c, d); });
-      quad_mmas(C2, xrow, live, kb, 32, r0.qb, r1.qb,
-                [&](int, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q4_unpack_word(w, cb0, a, b, c, d); },
-                [&](int, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q4_unpack_word(w, cb1, a, b, c, d); });
-    } else {
-      const uint32_t h0[4] = {r0.qh.x, r0.qh.y, r0.qh.z, r0.qh.w}, h1[4] = {r1.qh.x, r1.qh.y, r1.qh.z, r1.qh.w};
-      const int sa = 2 * th, sb = 4 + 2 * th;
-      quad_mmas(C, xrow, live, ka, 32, r0.qa, r1.qa,
-                [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q5_unpack_word(w, h0[i], sa, ca0, a, b, c, d); },
-                [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q5_unpack_word(w, h1[i], sa, ca1, a, b, c, d); });
-      quad_mmas(C2, xrow, live, kb, 32, r0.qb, r1.qb,
-                [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q5_unpack_word(w, h0[i], sb, cb0, a, b, c, d); },
-                [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q5_unpack_word(w, h1[i], sb, cb1, a, b, c, d); });
-    }
-    // min term: one mma over the 8 sub-block sums; even t carries the hi parts, odd t the lo parts
-    float Cm[4] = {0.f, 0.f, 0.f, 0.f};
-    uint32_t am[4] = {bytes_to_half2(ma0), bytes_to_half2(ma1), bytes_to_half2(mb0), bytes_to_half2(mb1)};
-    uint32_t b0 = 0, b1 = 0;
-    if (live) {
-      const __half* p = sxrow + blk * 8;  // sxrow: this column's hi plane (even t) or lo plane (odd t)
-      b0 = *reinterpret_cast<const uint32_t*>(p + 2 * th);
-      b1 = *reinterpret_cast<const uint32_t*>(p + 4 + 2 * th);
-    }
-    mma16816(Cm, am, b0, b1);
+  // unit a = t: hf 0, lh = th, l0 = 16*hb; unit b = t+4: hf 1
+  const int sia = hb + 2 * th, sib = 8 + hb + 2 * th;  // scale index of the low-nibble quarter; high is +4
+  auto sc2 = [](int s) { return half2_const((float)s); };
+  const uint32_t sla0 = sc2(q6_scale(r0.sc, sia)), sha0 = sc2(q6_scale(r0.sc, sia + 4));
+  const uint32_t slb0 = sc2(q6_scale(r0.sc, sib)), shb0 = sc2(q6_scale(r0.sc, sib + 4));
+  const uint32_t sla1 = sc2(q6_scale(r1.sc, sia)), sha1 = sc2(q6_scale(r1.sc, sia + 4));
+  const uint32_t slb1 = sc2(q6_scale(r1.sc, sib)), shb1 = sc2(q6_scale(r1.sc, sib + 4));
+  const uint32_t ha0[4] = {r0.qha.x, r0.qha.y, r0.qha.z, r0.qha.w}, hb0[4] = {r0.qhb.x, r0.qhb.y, r0.qhb.z, r0.qhb.w};
+  const uint32_t ha1[4] = {r1.qha.x, r1.qha.y, r1.qha.z, r1.qha.w}, hb1[4] = {r1.qhb.x, r1.qhb.y, r1.qhb.z, r1.qhb.w};
+  const int ka = blk * 256 + 32 * th + 16 * hb, kb = ka + 128;
+  quad_mmas(C, xrow, live, ka, 64, r0.qla, r1.qla,
+            [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, ha0[i], th, sla0, sha0, a, b, c, d); },
+            [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, ha1[i], th, sla1, sha1, a, b, c, d); });
+  quad_mmas(C2, xrow, live, kb, 64, r0.qlb, r1.qlb,
+            [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, hb0[i], th, slb0, shb0, a, b, c, d); },
+            [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, hb1[i], th, slb1, shb1, a, b, c, d); });
 #pragma unroll
-    for (int i = 0; i < 4; i++) C[i] += C2[i];
-    const float d0 = h2f_lo(r0.hdr.x), dm0 = h2f_hi(r0.hdr.x), d1 = h2f_lo(r1.hdr.x), dm1 = h2f_hi(r1.hdr.x);
-    acc[0] = fmaf(-dm0, Cm[0], fmaf(d0, C[0], acc[0]));
-    acc[1] = fmaf(-dm0, Cm[1], fmaf(d0, C[1], acc[1]));
-    acc[2] = fmaf(-dm1, Cm[2], fmaf(d1, C[2], acc[2]));
-    acc[3] = fmaf(-dm1, Cm[3], fmaf(d1, C[3], acc[3]));
-  } else {  // Q6_K
-    // unit a = t: hf 0, lh = th, l0 = 16*hb; unit b = t+4: hf 1
-    const int sia = hb + 2 * th, sib = 8 + hb + 2 * th;  // scale index of the low-nibble quarter; high is +4
-    auto sc2 = [](int s) { return half2_const((float)s); };
-    const uint32_t sla0 = sc2(q6_scale(r0.sc, sia)), sha0 = sc2(q6_scale(r0.sc, sia + 4));
-    const uint32_t slb0 = sc2(q6_scale(r0.sc, sib)), shb0 = sc2(q6_scale(r0.sc, sib + 4));
-    const uint32_t sla1 = sc2(q6_scale(r1.sc, sia)), sha1 = sc2(q6_scale(r1.sc, sia + 4));
-    const uint32_t slb1 = sc2(q6_scale(r1.sc, sib)), shb1 = sc2(q6_scale(r1.sc, sib + 4));
-    const uint32_t ha0[4] = {r0.qha.x, r0.qha.y, r0.qha.z, r0.qha.w}, hb0[4] = {r0.qhb.x, r0.qhb.y, r0.qhb.z, r0.qhb.w};
-    const uint32_t ha1[4] = {r1.qha.x, r1.qha.y, r1.qha.z, r1.qha.w}, hb1[4] = {r1.qhb.x, r1.qhb.y, r1.qhb.z, r1.qhb.w};
-    const int ka = blk * 256 + 32 * th + 16 * hb, kb = ka + 128;
-    quad_mmas(C, xrow, live, ka, 64, r0.qla, r1.qla,
-              [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, ha0[i], th, sla0, sha0, a, b, c, d); },
-              [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, ha1[i], th, sla1, sha1, a, b, c, d); });
-    quad_mmas(C2, xrow, live, kb, 64, r0.qlb, r1.qlb,
-              [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, hb0[i], th, slb0, shb0, a, b, c, d); },
-              [&](int i, uint32_t w, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) { q6_unpack_word(w, hb1[i], th, slb1, shb1, a, b, c, d); });
-#pragma unroll
-    for (int i = 0; i < 4; i++) C[i] += C2[i];
-    const float d0 = __half2float(__ushort_as_half((unsigned short)r0.d)), d1 = __half2float(__ushort_as_half((unsigned short)r1.d));
-    acc[0] = fmaf(d0, C[0], acc[0]);
-    acc[1] = fmaf(d0, C[1], acc[1]);
-    acc[2] = fmaf(d1, C[2], acc[2]);
-    acc[3] = fmaf(d1, C[3], acc[3]);
-  }
+  for (int i = 0; i < 4; i++) C[i] += C2[i];
+  const float d0 = __half2float(__ushort_as_half((unsigned short)r0.d)), d1 = __half2float(__ushort_as_half((unsigned short)r1.d));
+  acc[0] = fmaf(d0, C[0], acc[0]);
+  acc[1] = fmaf(d0, C[1], acc[1]);
+  acc[2] = fmaf(d1, C[2], acc[2]);
+  acc[3] = fmaf(d1, C[3], acc[3]);
 }
 
+// The tile row that mma row g (second = false) or g + 8 stands for. Q4_K and Q5_K rows are read in eight-byte pieces at a pitch of
+// their length + 16: with mma row g on row 2g, g + 8 on 2g + 1, the reads of a warp fall on distinct banks.
+template <int TYPE> __device__ __forceinline__ int mma_row(int g, bool second) { return TYPE == T_Q6_K ? g + (second ? 8 : 0) : 2 * g + (second ? 1 : 0); }
+template <int TYPE>
+__device__ __forceinline__ void block_accumulate(float (&acc)[4], const uint8_t* row0, const uint8_t* row1, const uint8_t* xrow, const __half* sxrow, bool live, int nb, int blk, int t) {
+  if constexpr (TYPE == T_Q6_K) {
+    Q6KRow a0, a1;
+    q6k_issue(a0, row0, nb, blk, t);
+    q6k_issue(a1, row1, nb, blk, t);
+    q6_accumulate(acc, a0, a1, xrow, live, blk, t);
+  } else {   // a column past the last repeats the first: its results are not stored
+    constexpr int BLK = TYPE == T_Q4_K ? 144 : 176;
+    const __half* sp = sxrow + blk * 8 + 2 * (t >> 1);
+    k45_accumulate<TYPE>(acc, (uint32_t)__cvta_generic_to_shared(row0 + (size_t)blk * BLK), (uint32_t)__cvta_generic_to_shared(row1 + (size_t)blk * BLK), xrow + 576 * blk,
+                         *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
+  }
+}
 
 // ---- row-level helpers -------------------------------------------------------------------
 // Executed by one whole CTA (QG_THREADS threads) for one activation row: the row kernels of passes of
@@ -375,7 +324,7 @@ __device__ __forceinline__ void block_accumulate(float (&acc)[4], const typename
 
 // xn[k] = fp16(h[k] * gamma[k] / sqrt(mean(h^2) + eps))   (reference: llm/hc.go:176-190)
 // and, when asked, the sums of the rounded values over every 32 of them (the eight threads of a sub-block are neighbours)
-__device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gamma, float eps, int H, __half* xn, float* scratch, __half* sx = nullptr) {
+__device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gamma, float eps, int H, __half* xn, float* scratch, __half* sx = nullptr, float* ss_out = nullptr) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   float s = 0.f;
   for (int k = tid * 4; k < H; k += QG_THREADS * 4) {
@@ -389,6 +338,7 @@ __device__ __forceinline__ void row_rmsnorm_f16(const float* h, const float* gam
   float tot = 0.f;
 #pragma unroll
   for (int w = 0; w < QG_WARPS; w++) tot += scratch[w];
+  if (ss_out != nullptr && tid == 0) *ss_out = tot;
   const float scale = 1.0f / sqrtf(tot / (float)H + eps);
   for (int k = tid * 4; k < H; k += QG_THREADS * 4) {
     float4 v = *reinterpret_cast<const float4*>(h + k);
@@ -437,36 +387,29 @@ struct TailParams {
   int n_parts;
   int64_t part_plane;
   __half* sx;           // optional: sub-block sums of the normalised rows, [M][H / 256][TG_SX]
+  float* ss_out;        // optional: [M][SS_LD] sum of squares of the row, as one part
 };
 
 // ---- activation staging ------------------------------------------------------------------
-// Copies `ncols` fp16 activation rows into shared memory in the permuted, padded layout the
-// B fragments are read in, and forms the per-sub-block sums (fp16 hi + lo planes) of the min
-// term. sxs layout: [plane(2)][xcols][K/32] halves.
-// sub-block sums of the staged fp16 values, as fp16 hi + lo planes
-__device__ __forceinline__ void stage_sx(int K, int xcols, const uint8_t* xs, __half* sxs, int ncols, int xstride) {
-  const int nsub = K / 32;
-  for (int i = threadIdx.x; i < ncols * nsub; i += QG_THREADS) {
-    const int c = i / nsub, s = i - c * nsub;
-    const uint8_t* src = xs + (size_t)c * xstride + 64 * s + 16 * (s >> 1);
-    float sum = 0.f;
+// Activation rows go to shared memory as fp16 in the permuted, padded layout the B fragments are read in, with the sums of every
+// 32 of them (fp16 hi + lo planes, [plane(2)][xcols][K/32] halves) for the min term. The threads that hold a sub-block are
+// neighbours and add it up by shuffles: (x0 + x1) + (x2 + x3) per four elements, then a tree over the eight fours, whoever stages.
+__device__ __forceinline__ float sum4_h2(uint32_t x02, uint32_t x13) { return (h2f_lo(x02) + h2f_lo(x13)) + (h2f_hi(x02) + h2f_hi(x13)); }
+template <int LANES>   // that share a sub-block: 8 of four elements each, or 4 of eight
+__device__ __forceinline__ void put_sx(float sum, __half* sx_hi, __half* sx_lo, int sub) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t mask = ((1u << LANES) - 1) << (lane & ~(LANES - 1));
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      uint4 v = *reinterpret_cast<const uint4*>(src + 16 * j);
-      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int q = 0; q < 4; q++) sum += h2f_lo(w[q]) + h2f_hi(w[q]);
-    }
-    __half hi = __float2half_rn(sum);
-    __half lo = __float2half_rn(sum - __half2float(hi));
-    sxs[(size_t)c * nsub + s] = hi;
-    sxs[(size_t)(xcols + c) * nsub + s] = lo;
+  for (int o = 1; o < LANES; o <<= 1) sum += __shfl_xor_sync(mask, sum, o);
+  if ((lane & (LANES - 1)) == 0) {
+    const __half hi = __float2half_rn(sum);
+    sx_hi[sub] = hi;
+    sx_lo[sub] = __float2half_rn(sum - __half2float(hi));
   }
-  __syncthreads();
 }
 
-// one fp16 row into the permuted layout, by threads t of nt
-__device__ __forceinline__ void copy_x_row(const __half* src, int K, uint8_t* dst, int t, int nt) {
+// one fp16 row into the permuted layout, by threads t of nt (nt a multiple of 8, t and the thread's lane alike in their low bits)
+__device__ __forceinline__ void copy_x_row(const __half* src, int K, uint8_t* dst, __half* sx_hi, __half* sx_lo, int t, int nt) {
   // every CTA reads the same row: each starts at another 128-byte line so the L2 slices are not all asked for
   // the same line at the same moment
   t = (t + 8 * (int)((blockIdx.x + blockIdx.y) % (unsigned)(nt / 8))) % nt;
@@ -476,15 +419,14 @@ __device__ __forceinline__ void copy_x_row(const __half* src, int K, uint8_t* ds
     o.x = __byte_perm(v.x, v.y, 0x5410); o.y = __byte_perm(v.x, v.y, 0x7632);
     o.z = __byte_perm(v.z, v.w, 0x5410); o.w = __byte_perm(v.z, v.w, 0x7632);
     *reinterpret_cast<uint4*>(dst + 2 * k + 16 * (k >> 6)) = o;
+    put_sx<4>(sum4_h2(o.x, o.y) + sum4_h2(o.z, o.w), sx_hi, sx_lo, k >> 5);
   }
 }
-__device__ __forceinline__ void stage_x_f16(const __half* x, int64_t ldx, int K, int xcols, uint8_t* xs, __half* sxs, int ncols, const int* xrows,
-                                            int xstride, bool copied = false) {
-  if (!copied) {
-    for (int c = 0; c < ncols; c++) copy_x_row(x + (int64_t)xrows[c] * ldx, K, xs + (size_t)c * xstride, threadIdx.x, QG_THREADS);
-    __syncthreads();
-  }
-  stage_sx(K, xcols, xs, sxs, ncols, xstride);
+__device__ __forceinline__ void stage_x_f16(const __half* x, int64_t ldx, int K, int xcols, uint8_t* xs, __half* sxs, int ncols, const int* xrows, int xstride) {
+  const int nsub = K / 32;
+  for (int c = 0; c < ncols; c++)
+    copy_x_row(x + (int64_t)xrows[c] * ldx, K, xs + (size_t)c * xstride, sxs + (size_t)c * nsub, sxs + (size_t)(xcols + c) * nsub, threadIdx.x, QG_THREADS);
+  __syncthreads();
 }
 
 // 1 / sqrt(mean(h^2) + eps) of row `row` from the partial sums its producer left, by one warp
@@ -532,97 +474,10 @@ __device__ __forceinline__ void stage_x_norm(const QGemvParams& p, uint8_t* xs, 
         __half2 n0 = __floats2half2_rn(v0, v1), n1 = __floats2half2_rn(v2, v3);
         *reinterpret_cast<uint2*>(p.xn_out + row * K + k) = make_uint2(*reinterpret_cast<uint32_t*>(&n0), *reinterpret_cast<uint32_t*>(&n1));
       }
+      put_sx<8>(sum4_h2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b)), sxs + (size_t)c * (K / 32), sxs + (size_t)(p.xcols + c) * (K / 32), k >> 5);
     }
   }
   __syncthreads();
-  stage_sx(K, p.xcols, xs, sxs, ncols, xstride);
-}
-
-// The MoE combine and the RMSNorm that follows it, fused into the staging: columns go four at a time,
-// a thread keeping its 8 values of each in registers between the sum of squares and the scaling.
-__device__ __forceinline__ void stage_x_combine(const QGemvParams& p, uint8_t* xs, __half* sxs, float* scratch, int ncols, const int* xrows,
-                                                int xstride, bool writer, const float4* pre_gam = nullptr, const float4* pre_h = nullptr) {
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K = p.K, slots1 = p.used + 1;
-  // Element index of this thread, rotated per CTA (every CTA reads the same rows: they should not all ask for the
-  // same line at the same moment). The rotation moves whole warps, and the warps' sums of squares are added in the
-  // order of the elements, not of the warps: every CTA, whatever its index and whatever the launch's grid, forms the
-  // same sums in the same order, so a row's normalised values do not depend on which CTA computes them.
-  const int rot = (int)((blockIdx.x + blockIdx.y) & 7);
-  const int et = (tid + 32 * rot) & (QG_THREADS - 1);
-  const int ewarp = (warp + rot) & (QG_WARPS - 1);   // the warp-sized group of elements this warp holds
-  // the norm weights are fetched with the first loads, not after the reduction
-  float4 gam[2];
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const int k = et * 4 + i * QG_THREADS * 4;
-    gam[i] = pre_gam != nullptr ? pre_gam[i] : k < K ? *reinterpret_cast<const float4*>(p.gamma + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  for (int c0 = 0; c0 < ncols; c0 += 4) {
-    float4 v[4][2];
-    float sq[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int cc = 0; cc < 4; cc++) {
-      const int c = c0 + cc < ncols ? c0 + cc : ncols - 1;
-      const int64_t row = xrows[c];
-      const float* hrow = p.hsrc + row * K;
-      const float* dn = p.down + row * slots1 * K;
-      const float* w = p.topk_w + row * slots1;   // read by every thread alongside its rows (one trip to L2, not two)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int k = et * 4 + i * QG_THREADS * 4;
-        v[cc][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (k < K && c0 + cc < ncols) {
-          const float4 hv = pre_h != nullptr ? pre_h[i] : __ldcg(reinterpret_cast<const float4*>(hrow + k));
-          const float4 sh = __ldcg(reinterpret_cast<const float4*>(dn + (size_t)p.used * K + k));
-          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 5
-          for (int s = 0; s < p.used; s++) {
-            const float4 d = __ldcg(reinterpret_cast<const float4*>(dn + (size_t)s * K + k));
-            const float wk = __ldcg(w + s);
-            acc.x += d.x * wk; acc.y += d.y * wk; acc.z += d.z * wk; acc.w += d.w * wk;
-          }
-          const float sg = __ldcg(w + p.used);
-          float4 r;
-          r.x = hv.x + (acc.x + sh.x * sg); r.y = hv.y + (acc.y + sh.y * sg); r.z = hv.z + (acc.z + sh.z * sg); r.w = hv.w + (acc.w + sh.w * sg);
-          v[cc][i] = r;
-          sq[cc] += (r.x * r.x + r.y * r.y) + (r.z * r.z + r.w * r.w);
-          if (writer) *reinterpret_cast<float4*>(p.h_out + row * K + k) = r;
-        }
-      }
-    }
-#pragma unroll
-    for (int cc = 0; cc < 4; cc++) {
-      sq[cc] = warp_sum(sq[cc]);
-      if (lane == 0) scratch[ewarp * 4 + cc] = sq[cc];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int cc = 0; cc < 4; cc++) {
-      if (c0 + cc >= ncols) break;
-      float t2 = 0.f;
-#pragma unroll
-      for (int w2 = 0; w2 < QG_WARPS; w2++) t2 += scratch[w2 * 4 + cc];
-      const float scale = 1.0f / sqrtf(t2 / (float)K + p.eps);
-      uint8_t* dst = xs + (size_t)(c0 + cc) * xstride;
-      const int64_t row = xrows[c0 + cc];
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int k = et * 4 + i * QG_THREADS * 4;
-        if (k < K) {
-          const float4 g = gam[i];
-          const float v0 = v[cc][i].x * scale * g.x, v1 = v[cc][i].y * scale * g.y, v2 = v[cc][i].z * scale * g.z, v3 = v[cc][i].w * scale * g.w;
-          __half2 a = __floats2half2_rn(v0, v2), b = __floats2half2_rn(v1, v3);  // stored order [x0,x2,x1,x3]
-          *reinterpret_cast<uint2*>(dst + 2 * k + 16 * (k >> 6)) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
-          if (writer && p.xn_out != nullptr) {
-            __half2 n0 = __floats2half2_rn(v0, v1), n1 = __floats2half2_rn(v2, v3);
-            *reinterpret_cast<uint2*>(p.xn_out + row * K + k) = make_uint2(*reinterpret_cast<uint32_t*>(&n0), *reinterpret_cast<uint32_t*>(&n1));
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  stage_sx(K, p.xcols, xs, sxs, ncols, xstride);
 }
 
 // ---- the kernel ----------------------------------------------------------------------------
@@ -646,13 +501,14 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   __half* sxs = reinterpret_cast<__half*>(smem + (size_t)p.xcols * xstride);
   float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sxs) + (((size_t)p.xcols * (K / 32) * 2 * sizeof(__half) + 15) & ~(size_t)15));
   uint8_t* stages = smem + qg_fixed_smem(K, p.xcols, DUAL);
-  const size_t tile_bytes = (size_t)16 * p.stride;
+  const size_t pitch = (size_t)qg_pitch(TYPE, p.stride), tile_bytes = 16 * pitch;
   const size_t stage_bytes = (size_t)tpc * tile_bytes * (DUAL ? 2 : 1);
   const int NS = p.nstage;
   __shared__ float scratch[4 * QG_WARPS];
   __shared__ float ssq[2][QG_WARPS][8];
   __shared__ int col_rows[QG_MAXCOLS], xrows[QG_MAXCOLS];
   __shared__ int route_expert, route_topk[32];
+  __shared__ float2 cand[32];
   __shared__ __align__(8) uint64_t full_bar[QG_MAX_STAGES];
 
   const int tiles = (p.N + 15) / 16;
@@ -687,12 +543,12 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       active = row < p.route.M;
       if (warp == 0) {
         if (active) {
-          const int ex = p.route.nE <= 512 ? route_token<16>(p.route, row, lane, writer, slot, route_topk) : route_token<32>(p.route, row, lane, writer, slot, route_topk);
+          const int ex = p.route.nE <= 512 ? route_token<16>(p.route, row, lane, writer, cand, slot, route_topk) : route_token<32>(p.route, row, lane, writer, cand, slot, route_topk);
           if (lane == 0) route_expert = slot < used ? ex : -1;
         }
       } else if constexpr (PRO == PRO_F16) {
         // meanwhile the other warps stage the row's activations (they do not depend on the routing)
-        if (active) copy_x_row(p.x + (int64_t)row * p.ldx, K, xs, tid - 32, QG_THREADS - 32);
+        if (active) copy_x_row(p.x + (int64_t)row * p.ldx, K, xs, sxs, sxs + (size_t)p.xcols * (K / 32), tid - 32, QG_THREADS - 32);
       }
       x_copied = PRO == PRO_F16;  // for every thread alike: the barrier below covers the copy
       __syncthreads();
@@ -722,18 +578,21 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     col_off = (int)blockIdx.z * QG_MAXCOLS;
     n_units = own_units();
   }
-  // thread 0 is the producer: one bulk copy per tile (and per tensor when DUAL)
+  // warp 0 is the producer: one bulk copy per tile row, or per tile where rows lie as in memory
   auto issue_group = [&](int grp, int s, const uint8_t* ga, const uint8_t* gb) {
-    uint32_t total = 0;
-    for (int l = 0; l < tpc; l++) {
-      const int tile = grp * tpc + l;
-      if (tile < tiles) total += (uint32_t)(min(16, p.N - tile * 16) * p.stride) * (DUAL ? 2 : 1);
+    if (lane == 0) {
+      uint32_t total = 0;
+      for (int l = 0; l < tpc; l++) {
+        const int tile = grp * tpc + l;
+        if (tile < tiles) total += (uint32_t)(min(16, p.N - tile * 16) * p.stride) * (DUAL ? 2 : 1);
+      }
+      mbar_expect_tx(&full_bar[s], total);
     }
-    mbar_expect_tx(&full_bar[s], total);
+    __syncwarp();
     for (int l = 0; l < tpc; l++) {
       const int tile = grp * tpc + l;
       if (tile >= tiles) continue;
-      const uint32_t bytes = (uint32_t)(min(16, p.N - tile * 16) * p.stride);
+      const int nrows = min(16, p.N - tile * 16);
       const uint8_t *base = ga, *base2 = gb;
       int seg_r0 = 0;
       if constexpr (!GROUPED) {
@@ -744,8 +603,16 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
         if constexpr (DUAL) base2 = p.w2[sg];
       }
       uint8_t* dst = stages + (size_t)s * stage_bytes + (size_t)l * tile_bytes * (DUAL ? 2 : 1);
-      bulk_copy_g2s(dst, base + (size_t)(tile * 16 - seg_r0) * p.stride, bytes, &full_bar[s]);
-      if constexpr (DUAL) bulk_copy_g2s(dst + tile_bytes, base2 + (size_t)(tile * 16 - seg_r0) * p.stride, bytes, &full_bar[s]);
+      const int64_t off = (int64_t)(tile * 16 - seg_r0) * p.stride;
+      if constexpr (TYPE == T_Q6_K) {
+        if (lane == 0) {
+          bulk_copy_g2s(dst, base + off, (uint32_t)(nrows * p.stride), &full_bar[s]);
+          if constexpr (DUAL) bulk_copy_g2s(dst + tile_bytes, base2 + off, (uint32_t)(nrows * p.stride), &full_bar[s]);
+        }
+      } else {
+        const int r = lane & 15;
+        if (r < nrows && lane < (DUAL ? 32 : 16)) bulk_copy_g2s(dst + (lane >> 4) * tile_bytes + r * pitch, (lane < 16 ? base : base2) + off + r * p.stride, (uint32_t)p.stride, &full_bar[s]);
+      }
     }
   };
   // unit j of this CTA goes to ring stage j % NS
@@ -762,24 +629,8 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       issue_group((int)blockIdx.x + j * (int)gridDim.x, j % NS, wa, wb);
     }
   };
-  if (tid == 0)
+  if (warp == 0)
     for (int k = 0; k < NS && k < n_units; k++) issue_unit(k);
-  // Single-row combine: the norm weights and the residual row (final four kernels back) are fetched before the
-  // wait, so that only the partial rows of the down projection are asked of L2 once it is over.
-  float4 pre_g[2], pre_h[2];
-  bool pre = false;
-  if constexpr (PRO == PRO_COMBINE) {
-    if (p.M == 1) {
-      pre = true;
-      const int et = (tid + 32 * (int)((blockIdx.x + blockIdx.y) & 7)) & (QG_THREADS - 1);   // as in stage_x_combine
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int k = et * 4 + i * QG_THREADS * 4;
-        pre_g[i] = k < K ? *reinterpret_cast<const float4*>(p.gamma + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        pre_h[i] = k < K ? __ldcg(reinterpret_cast<const float4*>(p.hsrc + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-    }
-  }
   if constexpr (!GROUPED) pdl_wait();
   pdl_launch();
   tl_mark(p.tl, 1);
@@ -798,9 +649,8 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       xrows[tid] = GROUPED ? id / p.x_div : id;
     }
     __syncthreads();
-    if constexpr (PRO == PRO_COMBINE) stage_x_combine(p, xs, sxs, scratch, ncols, xrows, xstride, blockIdx.x == 0 && blockIdx.y == 0, pre ? pre_g : nullptr, pre ? pre_h : nullptr);
-    else if constexpr (PRO == PRO_NORM) stage_x_norm(p, xs, sxs, scratch, ncols, xrows, xstride, p.xn_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0);
-    else stage_x_f16(p.x, p.ldx, K, p.xcols, xs, sxs, ncols, xrows, xstride, x_copied);
+    if constexpr (PRO == PRO_NORM) stage_x_norm(p, xs, sxs, scratch, ncols, xrows, xstride, p.xn_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0);
+    else if (!x_copied) stage_x_f16(p.x, p.ldx, K, p.xcols, xs, sxs, ncols, xrows, xstride);
     live = g < ncols;
     xrow = xs + (size_t)(live ? g : 0) * xstride;
     sxrow = sxs + (size_t)((t & 1) * p.xcols + (live ? g : 0)) * (K / 32);
@@ -832,35 +682,27 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
     const int tile = grp * tpc + lt;
     if (tile < tiles) {
-      int r0 = g, r1 = g + 8;
       const int nrows = min(16, p.N - tile * 16);
-      if (r0 >= nrows) r0 = nrows - 1;
-      if (r1 >= nrows) r1 = nrows - 1;
       const uint8_t* tb = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes * (DUAL ? 2 : 1);
+      const uint8_t *row0 = tb + min(mma_row<TYPE>(g, false), nrows - 1) * pitch, *row1 = tb + min(mma_row<TYPE>(g, true), nrows - 1) * pitch;
       for (int blk = kslice; blk < nb; blk += wpt) {
-        typename RowRegs<TYPE>::type a0, a1;
-        issue_row<TYPE>(a0, tb + (size_t)r0 * p.stride, nb, blk, t);
-        issue_row<TYPE>(a1, tb + (size_t)r1 * p.stride, nb, blk, t);
-        block_accumulate<TYPE>(acc, a0, a1, xrow, sxrow, live, blk, t);
-        if constexpr (DUAL) {
-          issue_row<TYPE>(a0, tb + tile_bytes + (size_t)r0 * p.stride, nb, blk, t);
-          issue_row<TYPE>(a1, tb + tile_bytes + (size_t)r1 * p.stride, nb, blk, t);
-          block_accumulate<TYPE>(acc2, a0, a1, xrow, sxrow, live, blk, t);
-        }
+        block_accumulate<TYPE>(acc, row0, row1, xrow, sxrow, live, nb, blk, t);
+        if constexpr (DUAL) block_accumulate<TYPE>(acc2, row0 + tile_bytes, row1 + tile_bytes, xrow, sxrow, live, nb, blk, t);
       }
     }
     // cross-warp reduction in warp order, double-buffered so one barrier per group suffices
     float* myred = red + (size_t)buf * RED + (size_t)warp * 128;
-    myred[g * 8 + 2 * t] = acc[0]; myred[g * 8 + 2 * t + 1] = acc[1];
-    myred[(g + 8) * 8 + 2 * t] = acc[2]; myred[(g + 8) * 8 + 2 * t + 1] = acc[3];
+    const int m0 = mma_row<TYPE>(g, false) * 8 + 2 * t, m1 = mma_row<TYPE>(g, true) * 8 + 2 * t;
+    *reinterpret_cast<float2*>(myred + m0) = make_float2(acc[0], acc[1]);
+    *reinterpret_cast<float2*>(myred + m1) = make_float2(acc[2], acc[3]);
     if constexpr (DUAL) {
       float* r2 = myred + QG_WARPS * 128;
-      r2[g * 8 + 2 * t] = acc2[0]; r2[g * 8 + 2 * t + 1] = acc2[1];
-      r2[(g + 8) * 8 + 2 * t] = acc2[2]; r2[(g + 8) * 8 + 2 * t + 1] = acc2[3];
+      *reinterpret_cast<float2*>(r2 + m0) = make_float2(acc2[0], acc2[1]);
+      *reinterpret_cast<float2*>(r2 + m1) = make_float2(acc2[2], acc2[3]);
     }
     __syncthreads();
     // every warp is done with stage s: refill it with the unit NS iterations ahead
-    if (tid == 0 && it + NS < n_units) { fence_proxy_async(); issue_unit(it + NS); }
+    if (warp == 0 && it + NS < n_units) { fence_proxy_async(); issue_unit(it + NS); }
     const float* rb = red + (size_t)buf * RED;
     float sq = 0.f;  // this thread's column is tid & 7 in every iteration
     for (int i = tid; i < tpc * 128; i += QG_THREADS) {
@@ -901,107 +743,90 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
 }
 
 // -----------------------------------------------------------------------------------------
-// Expert down projections of a single-row pass with the routing weights applied: part[r][row] =
-// sum over the slots s of CTA r of w_s * (W_down[e_s][row] . act[s]) (reference: llm/moe.go:347-357,
-// 403-406; shaders/llm_moe_combine.comp:48-63). The consumer then adds `split` partial rows instead of
-// used + 1 expert rows. `split` CTAs share a tile (one (slot, super-block) unit per warp); the weighted
-// sums are added in warp order. grid N / 16 * split, block QG_THREADS.
+// The MoE block's end of a pass that routes per row: expert down projections, routing weights, shared expert and residual in one
+// kernel, h[row][i] += sum_s w_s * (W_down[e_s][i] . act[s]) + sigmoid(gate) * shared (reference: llm/moe.go:347-357, 403-406;
+// shaders/llm_moe_combine.comp:48-63), with the sum of squares of each tile's rows for the norm that follows.
+// A CTA owns 16 rows of h of one row of the pass; each of its warps takes a (slot, super-block) unit alone - fetches the 16 x 256
+// weights as one TMA box, stages the 256 activations itself - and the units' sums are added in slot order at the end. One round of
+// latency instead of a chain: the form before (8 warps, CTA-wide staging, three partial rows that every CTA of the next projection
+// added up again) took 8 us plus 3 us more of that projection's staging. grid (N / 16, rows), block 32 * warps.
 // -----------------------------------------------------------------------------------------
-struct MoeDown1Params {
-  const uint8_t* w;         // routed down weights [nE][N][K]
-  const uint8_t* ws;        // shared expert
-  int64_t expert_stride, stride;
+struct MoeDownParams {
   int K, N, used;
   const int32_t* topk;      // [rows][used]
   const float* topk_w;      // [rows][used + 1]
   const __half* act;        // [rows][used + 1][K]
-  float* part;              // [rows][split][N] weighted partial sums, one row per CTA of a tile; blockIdx.y is the row
-  int split;                // CTAs per tile (1..4)
+  float* h;                 // [rows][N]
+  float* ss_out;            // [rows][SS_LD] sums of squares, part = tile
   int* err;
   Timeline tl;
 };
-constexpr int MD_MAXSLOTS = 16;
-
-// shared memory of a CTA that holds `maxloc` slots
-__host__ __device__ inline size_t md_smem(int K, int maxloc, int64_t stride) {
-  size_t xs = (size_t)maxloc * qg_xstride(K);
-  size_t sx = (((size_t)maxloc * (K / 32) * 2 * sizeof(__half)) + 15) & ~(size_t)15;
-  return ((xs + sx + 127) & ~(size_t)127) + (size_t)maxloc * 16 * (size_t)stride;
-}
+struct MoeDownMaps { TMap w, ws; };   // boxes of 16 rows (make_w_tensor_map)
+constexpr int MD_MAXWARPS = 24;
+template <int TYPE> __host__ __device__ constexpr int md_raw() { return 16 * (TYPE == T_Q4_K ? 144 : 176); }
+constexpr int MD_X = 4 * 144 + 32;     // one super-block of a staged row, its eight sums as hi | lo
 
 template <int TYPE>
-__global__ void __launch_bounds__(QG_THREADS) moe_down1_kernel(const MoeDown1Params p) {
-  // `split` CTAs share one 16-row tile: CTA r of them takes the slots s = r, r + split, ... and leaves its
-  // weighted sum as partial row r; the next projection adds the partial rows to the residual while staging
-  const int CL = p.split, rank = blockIdx.x % CL;
+__global__ void __launch_bounds__(MD_MAXWARPS * 32) moe_down_kernel(const __grid_constant__ MoeDownMaps maps, const MoeDownParams p) {
+  constexpr int BLK = TYPE == T_Q4_K ? 144 : 176;
   extern __shared__ __align__(128) uint8_t smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int K = p.K, nb = K / 256, slots1 = p.used + 1, xstride = qg_xstride(K);
-  const int nloc = (slots1 - rank + CL - 1) / CL;   // slots of this CTA
-  const int maxloc = (slots1 + CL - 1) / CL;
-  uint8_t* xs = smem;
-  __half* sxs = reinterpret_cast<__half*>(smem + (size_t)maxloc * xstride);
-  uint8_t* tiles = smem + (((size_t)maxloc * xstride + ((((size_t)maxloc * (K / 32) * 2 * sizeof(__half)) + 15) & ~(size_t)15) + 127) & ~(size_t)127);
-  const size_t tile_bytes = (size_t)16 * p.stride;
-  __shared__ float red[QG_WARPS][16], wgt[MD_MAXSLOTS];
-  __shared__ int expert[MD_MAXSLOTS];
-  __shared__ __align__(8) uint64_t bar;
+  __shared__ __align__(8) uint64_t bars[MD_MAXWARPS];
+  __shared__ float wgt[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, warps = blockDim.x >> 5;
+  const int nb = p.K / 256, slots1 = p.used + 1, units = slots1 * nb, tile = blockIdx.x, row = blockIdx.y;
+  uint8_t* raw = smem + warp * md_raw<TYPE>();
+  uint8_t* xs = smem + warps * md_raw<TYPE>() + warp * MD_X;
+  __half* sx = reinterpret_cast<__half*>(xs + 4 * 144);
+  float* yv = reinterpret_cast<float*>(smem + warps * (md_raw<TYPE>() + MD_X));   // [units][16]
   tl_mark(p.tl, 0);
-  if (tid == 0) { mbar_init(&bar, 1); mbar_fence_init(); }
+  if (lane == 0) { mbar_init(&bars[warp], 1); mbar_fence_init(); }
+  __syncwarp();
   pdl_wait();   // the selection and the activations come from the kernel before
   pdl_launch();
   tl_mark(p.tl, 1);
-  const int prow = blockIdx.y;   // row of the pass: each row is finished exactly as a single-row pass finishes its own
-  const int32_t* topk = p.topk + (size_t)prow * p.used;
-  const float* topk_w = p.topk_w + (size_t)prow * slots1;
-  const __half* act = p.act + (size_t)prow * slots1 * K;
-  if (tid < nloc) {
-    const int s = rank + tid * CL;
-    expert[tid] = s < p.used ? __ldcg(topk + s) : -1;
-    wgt[tid] = __ldcg(topk_w + s);
-  }
-  __syncthreads();
-  const int tile = blockIdx.x / CL, nrows = min(16, p.N - tile * 16);
-  if (tid == 0 && nloc > 0) {
-    mbar_expect_tx(&bar, (uint32_t)(nloc * nrows * p.stride));
-    for (int i = 0; i < nloc; i++) {
-      const uint8_t* base = expert[i] >= 0 ? p.w + (size_t)expert[i] * p.expert_stride : p.ws;
-      bulk_copy_g2s(tiles + (size_t)i * tile_bytes, base + (size_t)tile * 16 * p.stride, (uint32_t)(nrows * p.stride), &bar);
+  float hv = 0.f;
+  if (tid < 16) hv = __ldcg(p.h + (size_t)row * p.N + tile * 16 + tid);
+  if (tid < slots1) wgt[tid] = __ldcg(p.topk_w + (size_t)row * slots1 + tid);
+  int phase = 0;
+  for (int u = warp; u < units; u += warps, phase ^= 1) {
+    const int s = u / nb, blk = u - s * nb;
+    const int e = s < p.used ? __ldcg(p.topk + (size_t)row * p.used + s) : -1;
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.act + ((size_t)row * slots1 + s) * p.K + blk * 256 + 8 * lane));
+    if (elect_one()) {
+      if (u != warp) fence_proxy_async();
+      mbar_expect_tx(&bars[warp], md_raw<TYPE>());
+      tma_box_2d(raw, e >= 0 ? &maps.w : &maps.ws, blk * BLK, (e >= 0 ? e * p.N : 0) + tile * 16, &bars[warp]);
     }
-  }
-  for (int i = 0; i < nloc; i++) copy_x_row(act + (size_t)(rank + i * CL) * K, K, xs + (size_t)i * xstride, tid, QG_THREADS);
-  __syncthreads();
-  stage_sx(K, maxloc, xs, sxs, nloc, xstride);
-  tl_mark(p.tl, 2);
-  bool ok = true;
-  if (nloc > 0 && !mbar_wait(&bar, 0)) {
-    if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report, contribute nothing
-    ok = false;
+    const uint4 o = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
+    *reinterpret_cast<uint4*>(xs + 16 * lane + 16 * (lane >> 3)) = o;
+    put_sx<4>(sum4_h2(o.x, o.y) + sum4_h2(o.z, o.w), sx, sx + 8, lane >> 2);
+    __syncwarp();
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    if (warp_wait(&bars[warp], phase)) {
+      const uint32_t ra = (uint32_t)__cvta_generic_to_shared(raw) + 2 * g * BLK;
+      const __half* sp = sx + ((t & 1) ? 8 : 0) + 2 * (t >> 1);
+      k45_accumulate<TYPE>(acc, ra, ra + BLK, xs, *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
+    } else if (lane == 0 && p.err != nullptr) {
+      atomicExch(p.err, 1);   // a copy never landed: report, the results are void
+    }
+    if (t == 0) *reinterpret_cast<float2*>(yv + u * 16 + 2 * g) = make_float2(acc[0], acc[2]);   // every column holds the one activation row
+    __syncwarp();
   }
   tl_mark(p.tl, 3);
-  int r0 = g, r1 = g + 8;
-  if (r0 >= nrows) r0 = nrows - 1;
-  if (r1 >= nrows) r1 = nrows - 1;
-  const bool live = g == 0;  // the single activation row sits in column 0 of the mma's N axis
-  float tot0 = 0.f, tot1 = 0.f;
-  for (int u = warp; ok && u < nloc * nb; u += QG_WARPS) {
-    const int i = u / nb, blk = u - i * nb;
-    const uint8_t* tb = tiles + (size_t)i * tile_bytes;
-    typename RowRegs<TYPE>::type a0, a1;
-    issue_row<TYPE>(a0, tb + (size_t)r0 * p.stride, nb, blk, t);
-    issue_row<TYPE>(a1, tb + (size_t)r1 * p.stride, nb, blk, t);
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    block_accumulate<TYPE>(acc, a0, a1, xs + (size_t)i * xstride, sxs + (size_t)((t & 1) * maxloc + i) * (K / 32), live, blk, t);
-    tot0 = fmaf(wgt[i], acc[0], tot0);   // column 0: rows g and g + 8 on the lanes with t == 0
-    tot1 = fmaf(wgt[i], acc[2], tot1);
-  }
-  if (t == 0) { red[warp][g] = tot0; red[warp][g + 8] = tot1; }
   __syncthreads();
-  if (tid < nrows) {
-    float v = 0.f;
+  if (tid < 16) {
+    float acc = 0.f, y = 0.f;
+    for (int s = 0; s < slots1; s++) {
+      y = 0.f;
+      for (int b = 0; b < nb; b++) y += yv[(s * nb + b) * 16 + tid];
+      if (s < p.used) acc = fmaf(wgt[s], y, acc);
+    }
+    const float r = hv + fmaf(wgt[p.used], y, acc);
+    p.h[(size_t)row * p.N + tile * 16 + tid] = r;
+    float sq = r * r;
 #pragma unroll
-    for (int w = 0; w < QG_WARPS; w++) v += red[w][tid];
-    p.part[((size_t)prow * CL + rank) * p.N + (size_t)tile * 16 + tid] = v;
+    for (int o = 1; o < 16; o <<= 1) sq += __shfl_xor_sync(0xffffu, sq, o);
+    if (tid == 0) p.ss_out[(size_t)row * SS_LD + tile] = sq;
   }
   tl_mark(p.tl, 4);
 }

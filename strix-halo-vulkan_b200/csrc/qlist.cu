@@ -24,49 +24,10 @@ template <int TYPE, int NC> struct QlCfg {
   static constexpr int SLOTS = 216 * 1024 / WARPS / BYTES < 8 ? 216 * 1024 / WARPS / BYTES : 8;
 };
 
-__device__ __forceinline__ uint4 ld_s(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-  return v;
-}
 __device__ __forceinline__ void tma_box(uint32_t dst, const void* tm, int c0, int c1, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(tm), "r"(c0), "r"(c1),
                "r"((uint32_t)__cvta_generic_to_shared(bar))
                : "memory");
-}
-
-// Quants enter the tensor core as they are: four or five bits in the low end of a half are the subnormal q * 2^-24, exactly,
-// so a pair of weights costs one mask and no conversion, no multiply; the sub-block scale is applied to the f32 result of
-// the sub-block's two mma steps, the 2^24 (and the 16 of a high nibble left in place) with the block scale.
-// lo: sub-block 2G, hi: 2G + 1; of a word's four bytes the pairs are (0, 2) and (1, 3).
-template <int TYPE>
-__device__ __forceinline__ void unpack_word(uint32_t w, uint32_t fifth, int G, uint32_t& l02, uint32_t& l13, uint32_t& h02, uint32_t& h13) {
-  if constexpr (TYPE == T_Q4_K) {
-    const uint32_t w8 = w >> 8;
-    l02 = w & 0x000F000Fu; h02 = w & 0x00F000F0u; l13 = w8 & 0x000F000Fu; h13 = w8 & 0x00F000F0u;
-  } else {   // fifth bits: bit 2G of a byte belongs to its low nibble, bit 2G + 1 to the high one
-    const uint32_t f = fifth >> (2 * G);
-    const uint32_t lo = (w & 0x0F0F0F0Fu) | ((f << 4) & 0x10101010u), hi = ((w >> 4) & 0x0F0F0F0Fu) | ((f << 3) & 0x10101010u);
-    l02 = lo & 0x00FF00FFu; l13 = (lo >> 8) & 0x00FF00FFu; h02 = hi & 0x00FF00FFu; h13 = (hi >> 8) & 0x00FF00FFu;
-  }
-}
-// D = A B, no accumulator in
-__device__ __forceinline__ void mma16816_z(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-// scales (bytes 2 pair, 2 pair + 1 of a word) of a low- and a high-nibble sub-block as f32
-template <int TYPE>
-__device__ __forceinline__ void sub_scales(uint32_t four, int pair, float (&s)[2]) {
-  const uint32_t h2 = hadd2_u(__byte_perm(four, 0x64646464u, pair ? 0x4342 : 0x4140), half2_const(-1024.f));
-  s[0] = h2f_lo(h2);
-  s[1] = h2f_hi(TYPE == T_Q4_K ? hmul2_u(h2, half2_const(0.0625f)) : h2);
-}
-__device__ __forceinline__ uint2 ld_s64(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-  return v;
 }
 
 template <int TYPE, int NC, int EPI>
@@ -169,7 +130,7 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
           return;
         }
         const uint32_t base = ring + slot * Cf::BYTES + row_off;
-        const uint4 h0 = ld_s(base), h1 = ld_s(base + Cf::BLK);
+        const uint4 h0 = ld_s128(base), h1 = ld_s128(base + Cf::BLK);
         // 6-bit scales of the two rows, four sub-blocks to a word (gguf/dequant.go:238-243)
         const uint32_t scl[2][2] = {{h0.y & 0x3F3F3F3Fu, (h0.w & 0x0F0F0F0Fu) | ((h0.y >> 2) & 0x30303030u)}, {h1.y & 0x3F3F3F3Fu, (h1.w & 0x0F0F0F0Fu) | ((h1.y >> 2) & 0x30303030u)}};
         float sum[NC][4];   // sub-block scale x (q . x), without d

@@ -43,9 +43,9 @@ static int scratch_for_current_device(StaticScratch* out) {
 // Shared memory the projection kernel needs for m staged rows of length k plus one stage of weight
 // tiles; the launch is refused when it exceeds what an SM offers (the same sum launch_qgemv checks).
 static size_t static_smem_need(uint32_t type, int64_t k, int m) {
-  return qg_fixed_smem((int)k, m, false) + qg_stage_bytes((int)k, device_row_stride(type, k), false);
+  return qg_fixed_smem((int)k, m, false) + qg_stage_bytes((int)k, qg_pitch(type, device_row_stride(type, k)), false);
 }
-constexpr size_t STATIC_SMEM_BUDGET = 220 * 1024;
+constexpr size_t STATIC_SMEM_BUDGET = QG_SMEM_MAX;
 
 int qgemv_static(uint32_t type, const void* dev_w, int64_t rows, int64_t k, const float* dev_x, int32_t m, float* dev_y) {
   if (!dev_w || !dev_x || !dev_y) { set_error("qgemv_static: null pointer"); return EINVAL_; }
