@@ -2,6 +2,7 @@
 // layers() loop (llm/graph.go:2330-2466) with a plain pre-norm residual stream in place of
 // its hyper-connection mixers.
 #include "graph.h"
+#include "moerow.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -254,6 +255,10 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   const int hd = c.head_dim, qw = c.n_head * hd, kvw = c.n_head_kv * hd, used = c.n_expert_used, slots1 = used + 1;
   const int xcols = std::min(M, QG_MAXCOLS);
   const bool fused = M <= QG_FUSED_ROWS && H <= QG_FUSED_MAX_K;
+  auto rows_moe = [&](const LayerW& L) {
+    return L.gate_exps.type == L.up_exps.type && L.gate_exps.type == L.gate_sh.type && L.gate_sh.type == L.up_sh.type && L.down_exps.type == L.down_sh.type &&
+           moe_rows_fit(L.gate_exps.type, L.down_exps.type, H, c.ffn_expert, c.n_expert, used);
+  };
   // expert-parallel MoE block: plain decode passes only (every rank runs the same number of rows at the same time)
   const bool epx = ep_on && ep_ready && !f.draft && !f.spec && n_seq == M;
   const int Mg = epx ? M * ep.world : M;   // rows of all ranks
@@ -304,7 +309,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (gemm_tile_rows(M, N) == 0) {
       QGemvParams q = base(w, K, N, x, K);
       q.y = y; q.ldy = ldy;
-      return launch_qgemv(w.type, PRO_F16, EPI_STORE, false, false, q, 0, pdl(), st);
+      return launch_qgemv(w.type, PRO_F16, EPI_STORE, false, false, q, pdl(), st);
     }
     WGemmMaps maps{};
     maps.w = wm; maps.x = xm;
@@ -317,7 +322,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (gemm_tile_rows(M, H) == 0) {
       QGemvParams q = base(w, K, H, x, K);
       q.y = h; q.ldy = H;
-      return launch_qgemv(w.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st);
+      return launch_qgemv(w.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st);
     }
     WGemmMaps maps{};
     maps.w = wm; maps.x = xm;
@@ -336,7 +341,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     QGemvParams p = base(L.eh_proj, 2 * H, H, xcat16, 2 * H);
     p.y = h; p.ldy = H;
     if (fused) { p.ss_out = ss_part; ss_n = qgemv_groups(2 * H, H); }
-    B200_TRY(launch_qgemv(L.eh_proj.type, PRO_F16, EPI_STORE, false, false, p, 0, pdl(), st));
+    B200_TRY(launch_qgemv(L.eh_proj.type, PRO_F16, EPI_STORE, false, false, p, pdl(), st));
     if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.attn_norm), pdl(), st));
   } else {
     const LayerW& L0 = m->layers[0];
@@ -359,7 +364,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         else B200_TRY(gemm(L.z, wmaps[l].z, H, vw, xn16, tx_xn[2], proj + cw, proj_ld));
       } else {
         const int pro = normed(p, L.attn_norm, xn16);  // the DeltaNet step reads the fp16 rows for alpha / beta
-        B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
+        B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, pdl(), st));
       }
       DnStepParams d{};
       d.proj = proj; d.ldp = proj_ld; d.xn = xn16; d.alpha_w = (const float*)L.alpha.data; d.beta_w = (const float*)L.beta.data;
@@ -380,7 +385,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(vw, H); }
       if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out.m[0], vw, y16, tx_y16, sx_y, ts_y16));
       else if (use_gemm) B200_TRY(gemm_resid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16[2]));
-      else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
+      else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));
     } else {
       const int ai = attn_index[l];
       // fused q|k|v projection; tensors of one type share a launch
@@ -406,7 +411,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         p.nseg = e - s; p.N = n;
         p.y = proj + off; p.ldy = proj_ld;
         const int pro = normed(p, L.attn_norm, nullptr);
-        B200_TRY(launch_qgemv(seg[s]->type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
+        B200_TRY(launch_qgemv(seg[s]->type, pro, EPI_STORE, false, false, p, pdl(), st));
         off += n; s = e;
       }
       AttnParams a{};
@@ -436,7 +441,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(qw, H); }
       if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o.m[0], qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
       else if (use_gemm) B200_TRY(gemm_resid(L.o, wmaps[l].o, qw, ctx16, tx_ctx[2]));
-      else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, 0, pdl(), st));
+      else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));
     }
     if (!fused) {
       TailParams t = row_tail(1, L.ffn_norm);
@@ -456,7 +461,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     // decode and verify passes equal their rows stepped alone: llm/graph_batch_test.go:36, llm/spec_slots_test.go:199)
     const bool moe_gemm = pass_moe_gemm(c, L, M, H) && !epx;
     const bool moe_stream = !moe_gemm && experts_stream(L, M);
-    r.defer = fused && !epx && L.down_exps.type == L.down_sh.type && moe_down_fits(L.down_exps.type, c.ffn_expert, H, used); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
+    r.defer = fused && !epx && rows_moe(L); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
     if (epx) { r.entries = nullptr; r.gprob = nullptr; }   // routing only: the work list comes from the gathered routing
     // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted
     // rows (below that the column-tiled kernel, which streams each expert's weights in whole tiles, is faster)
@@ -477,7 +482,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     } else {
       B200_TRY(launch_router(r, pdl(), st));
     }
-    const int ne = max_entries_for(Mg, moe_stream);
     // the two expert launches of a work list: activation rows x (ids / x_div), outputs by pair id
     auto stream_experts = [&](const __half* x, const __half* sx, int cols_) {
       const LayerMaps& W = wmaps[l];
@@ -508,12 +512,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
       p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = ecx; p.M = Mg;
       p.y16 = act16; p.ldy = c.ffn_expert;
-      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, ne, pdl(), st));
+      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, pdl(), st));
       QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
       q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
       q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = ecx; q.M = Mg;
       q.y = down; q.ldy = H;     // local: rows by pair id; the combine kernel carries them to the rows' owners
-      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, ne, pdl(), st));
+      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, pdl(), st));
       }
       e.y_local = down; e.cols = cols; e.n_pairs = ep_epoch + 2; e.pairs_per_rank = M * slots1;
       B200_TRY(launch_ep_combine(e, M * slots1 + (Mg - M) * used, pdl(), st));
@@ -535,25 +539,27 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       B200_TRY(launch_wgemm(L.down_exps.type, WG_STORE, 128, d, md, pdl(), st));
     } else if (moe_stream) {
       B200_TRY(stream_experts(xn16, sx_xn, entry_cols(M, true)));
-    } else {
-    QGemvParams p = base(L.gate_exps, H, c.ffn_expert, xn16, H);
-    p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
-    p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = r.defer ? 1 : std::min(xcols, entry_cols(M, false));
-    p.y16 = act16; p.ldy = c.ffn_expert;
-    p.route_here = r.defer; p.route = r;
-    B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, r.defer ? M * slots1 : ne, pdl(), st));
-    if (r.defer) {
+    } else if (r.defer) {
+      const LayerMaps& W = wmaps[l];
+      MoeGateParams p{};
+      p.route = r; p.K = H; p.N = c.ffn_expert; p.M = M; p.x = xn16; p.act = act16; p.err = err_flag; p.tl = tl();
+      p.down = L.down_exps.data; p.down_sh = L.down_sh.data; p.down_bytes = (int64_t)H * L.down_exps.stride;
+      B200_TRY(launch_moe_gate(L.gate_exps.type, p, MoeGateMaps{W.gate, W.up, W.gate_sh, W.up_sh}, pdl(), st));
       MoeDownParams d{};
       d.K = c.ffn_expert; d.N = H; d.used = used; d.topk = topk; d.topk_w = topk_w; d.act = act16; d.h = h; d.ss_out = ss_part; d.err = err_flag; d.tl = tl();
       ss_n = H / 16;
-      B200_TRY(launch_moe_down(L.down_exps.type, d, MoeDownMaps{wmaps[l].down, wmaps[l].down_sh}, M, pdl(), st));
+      B200_TRY(launch_moe_down(L.down_exps.type, d, MoeDownMaps{W.down, W.down_sh}, M, pdl(), st));
     } else {
+      QGemvParams p = base(L.gate_exps, H, c.ffn_expert, xn16, H);
+      p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
+      p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = std::min(xcols, entry_cols(M, false));
+      p.y16 = act16; p.ldy = c.ffn_expert;
+      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, pdl(), st));
       QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
       q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
       q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M, false));
       q.y = down; q.ldy = H;
-      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, ne, pdl(), st));
-    }
+      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, pdl(), st));
     }
     if (!r.defer) {
       const DTensor& next_norm = f.draft ? L.head_norm : (l + 1 < c.n_layer ? m->layers[l + 1].attn_norm : m->output_norm);
@@ -580,7 +586,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       B200_TRY(gemm(m->output, head_map, H, N, xn16, tx_xn[2], logits, N));
     } else {
       const int pro = normed(p, nrm, nullptr);
-      B200_TRY(launch_qgemv(m->output.type, pro, EPI_STORE, false, false, p, 0, pdl(), st));
+      B200_TRY(launch_qgemv(m->output.type, pro, EPI_STORE, false, false, p, pdl(), st));
     }
     if (f.greedy) {
       B200_TRY(launch_argmax(logits, n_logit_rows, N, next_ids, pdl(), st));

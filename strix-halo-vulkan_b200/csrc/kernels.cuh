@@ -37,10 +37,7 @@ struct EmbedParams {
 int launch_embed(const EmbedParams& p, cudaStream_t st);
 
 // K-quant projections; `pdl` marks the launch as a programmatic dependent of the previous kernel.
-int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st);
-// passes of at most QG_FUSED_ROWS rows: per row, the selected experts' down projections, weighted, with the shared expert added to the residual
-bool moe_down_fits(uint32_t type, int K, int N, int used);
-int launch_moe_down(uint32_t type, const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st);
+int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st);
 int qgemv_groups(int K, int N);
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st);
 int launch_concat_norm(const float* e, const float* hs, const float* enorm, const float* hnorm, float eps, int H, int M, __half* xcat, bool pdl, cudaStream_t st);

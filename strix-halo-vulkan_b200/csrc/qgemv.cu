@@ -4,10 +4,9 @@
 
 namespace b200 {
 
-// max_entries: grid.y of a launch whose CTAs route for themselves (one per row and slot). Launches over a work list
-// ignore it: their grid is the device's resident CTAs, which share the list evenly whatever its length.
+// The grid of a launch over a work list is the device's resident CTAs, which share the list evenly whatever its length.
 template <int TYPE, int PRO, int EPI, bool DUAL, bool GROUPED>
-static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st) {
+static int launch_one(const QGemvParams& p, bool pdl, cudaStream_t st) {
   auto kernel = qgemv_kernel<TYPE, PRO, EPI, DUAL, GROUPED>;
   const int g_sm_count = sm_count_current();
   if (g_sm_count <= 0) return ECUDA;
@@ -16,7 +15,7 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
   const int tpc = QG_WARPS / wpt;
   const int tiles = (p.N + 15) / 16;
   const int groups = (tiles + tpc - 1) / tpc;
-  const int ny = GROUPED ? max_entries : 1, nz = GROUPED ? 1 : (p.M + QG_MAXCOLS - 1) / QG_MAXCOLS;
+  const int nz = GROUPED ? 1 : (p.M + QG_MAXCOLS - 1) / QG_MAXCOLS;
   // As many CTAs per SM (up to three: 80 registers per thread) as still leave each a ring of two stages, or of
   // one when it has a single group to walk: more resident warps hide the dequantisation's latencies, and a
   // grid that fits at once needs no second round. Three per SM only for the expert kernels and the Q6_K ones (the head's long walk): elsewhere the register cap costs more than
@@ -27,7 +26,7 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
   if (fixed + stage > budgets[1]) { set_error("qgemv: row length too large for shared memory"); return ECAPACITY; }
   int occ = 1, rounds = 1, gx = 1, ns = 1;
   dim3 grid;
-  if (GROUPED && !p.route_here) {
+  if (GROUPED) {
     // A work list: persistent CTAs, each with an equal contiguous share of the list's (entry, group) units. The
     // walk is bound by the instructions that turn quants into fragments, so the resident warps count for more than
     // the ring's depth: three CTAs per SM with a single stage beat two with two stages when three fit.
@@ -37,8 +36,8 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
     grid = dim3(g_sm_count * occ, 1, 1);
   } else {
     for (int o = 3; o >= 1; o--) {
-      if (o == 3 && !GROUPED && TYPE != T_Q6_K) continue;  // the other plain kernels are compiled for two CTAs per SM
-      int cap = g_sm_count * o / (ny * nz);
+      if (o == 3 && TYPE != T_Q6_K) continue;  // the other plain kernels are compiled for two CTAs per SM
+      int cap = g_sm_count * o / nz;
       if (cap < 1) cap = 1;
       // every CTA walks the same number of groups (a ragged last round leaves most SMs idle)
       rounds = (groups + cap - 1) / cap;
@@ -50,7 +49,7 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
     if (ns > QG_MAX_STAGES) ns = QG_MAX_STAGES;
     if (ns > rounds) ns = rounds;
     if (ns < 1) ns = 1;
-    grid = dim3(gx, ny, nz);
+    grid = dim3(gx, 1, nz);
   }
   const size_t smem = fixed + (size_t)ns * stage;
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QG_SMEM_MAX));
@@ -67,14 +66,14 @@ static int launch_one(const QGemvParams& p, int max_entries, bool pdl, cudaStrea
 }
 
 template <int TYPE>
-static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st) {
+static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st) {
   if (!grouped && !dual) {
-    if (pro == PRO_NORM && epi == EPI_STORE) return launch_one<TYPE, PRO_NORM, EPI_STORE, false, false>(p, 0, pdl, st);
-    if (pro == PRO_F16 && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, false>(p, 0, pdl, st);
-    if (pro == PRO_F16 && epi == EPI_RESID) return launch_one<TYPE, PRO_F16, EPI_RESID, false, false>(p, 0, pdl, st);
+    if (pro == PRO_NORM && epi == EPI_STORE) return launch_one<TYPE, PRO_NORM, EPI_STORE, false, false>(p, pdl, st);
+    if (pro == PRO_F16 && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, false>(p, pdl, st);
+    if (pro == PRO_F16 && epi == EPI_RESID) return launch_one<TYPE, PRO_F16, EPI_RESID, false, false>(p, pdl, st);
   } else if (grouped && pro == PRO_F16) {
-    if (dual && epi == EPI_SWIGLU) return launch_one<TYPE, PRO_F16, EPI_SWIGLU, true, true>(p, max_entries, pdl, st);
-    if (!dual && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, true>(p, max_entries, pdl, st);
+    if (dual && epi == EPI_SWIGLU) return launch_one<TYPE, PRO_F16, EPI_SWIGLU, true, true>(p, pdl, st);
+    if (!dual && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, true>(p, pdl, st);
   }
   set_error("qgemv: this prologue / epilogue combination is not built");
   return EINVAL_;
@@ -88,38 +87,15 @@ int qgemv_groups(int K, int N) {
   return ((N + 15) / 16 + tpc - 1) / tpc;
 }
 
-template <int TYPE>
-static int launch_md(const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st) {
-  auto kernel = moe_down_kernel<TYPE>;
-  const int units = (p.used + 1) * (p.K / 256), rounds = (units + MD_MAXWARPS - 1) / MD_MAXWARPS, warps = (units + rounds - 1) / rounds;
-  const size_t smem = (size_t)warps * (md_raw<TYPE>() + MD_X) + (size_t)units * 16 * sizeof(float);
-  if (smem > 200 * 1024) { set_error("moe_down: too many slots for shared memory"); return ECAPACITY; }
-  B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.N / 16, rows); cfg.blockDim = dim3(warps * 32); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, p));
-  return OK;
-}
-
-bool moe_down_fits(uint32_t type, int K, int N, int used) { return (type == T_Q4_K || type == T_Q5_K) && K % 256 == 0 && N % 16 == 0 && N / 16 <= SS_LD && used < 32 && (used + 1) * (K / 256) <= 512; }
-int launch_moe_down(uint32_t type, const MoeDownParams& p, const MoeDownMaps& maps, int rows, bool pdl, cudaStream_t st) {
-  if (!moe_down_fits(type, p.K, p.N, p.used) || rows < 1) { set_error("moe_down: shape outside kernel limits (Q4_K, Q5_K)"); return EINVAL_; }
-  return type == T_Q4_K ? launch_md<T_Q4_K>(p, maps, rows, pdl, st) : launch_md<T_Q5_K>(p, maps, rows, pdl, st);
-}
-
-int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, int max_entries, bool pdl, cudaStream_t st) {
+int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st) {
   if (p.K % 256 != 0 || p.K <= 0) { set_error("qgemv: row length must be a multiple of 256"); return EINVAL_; }
   if (p.xcols < 1 || p.xcols > QG_MAXCOLS) { set_error("qgemv: xcols out of range"); return EINVAL_; }
   if (p.ss_out != nullptr && qgemv_groups(p.K, p.N) > SS_LD) { set_error("qgemv: more tile groups than partial-sum slots"); return ECAPACITY; }
   if (pro == PRO_NORM && (p.ss_n < 1 || p.ss_n > SS_LD)) { set_error("qgemv: bad partial-sum count"); return EINVAL_; }
   switch (type) {
-    case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, max_entries, pdl, st);
-    case T_Q5_K: return launch_type<T_Q5_K>(pro, epi, dual, grouped, p, max_entries, pdl, st);
-    case T_Q6_K: return launch_type<T_Q6_K>(pro, epi, dual, grouped, p, max_entries, pdl, st);
+    case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, pdl, st);
+    case T_Q5_K: return launch_type<T_Q5_K>(pro, epi, dual, grouped, p, pdl, st);
+    case T_Q6_K: return launch_type<T_Q6_K>(pro, epi, dual, grouped, p, pdl, st);
   }
   set_error("qgemv: weight type has no fused projection kernel (Q4_K, Q5_K, Q6_K only)");
   return EINVAL_;

@@ -54,11 +54,6 @@ struct QGemvParams {
   const uint8_t* ws;         // shared expert weights (grouped mode)
   const uint8_t* ws2;
   int x_div;                 // grouped: x row = cols[c] / x_div
-  // grouped, passes of at most QG_FUSED_ROWS rows: the router kernel stopped after the logits (route.defer); every
-  // CTA selects the experts of its row itself (one warp, a few hundred instructions) instead of waiting for a last
-  // router CTA to do it, and the first CTA of a row leaves the row's selection for the kernels after it
-  int route_here;
-  RouterParams route;
   // plain mode columns: rows [ztile*8, ztile*8+8) of M
   int M;
   int xcols;                 // columns the shared-memory layout is sized for (1..8)
@@ -481,9 +476,8 @@ __device__ __forceinline__ void stage_x_norm(const QGemvParams& p, uint8_t* xs, 
 }
 
 // ---- the kernel ----------------------------------------------------------------------------
-// grid.x: persistent CTAs walking the row-tile groups; grid.y: (row, slot) of a grouped launch that
-// routes for itself, else 0; grid.z: column tile of 8 activation rows (plain mode). A grouped launch over
-// a work list is one row of CTAs that share the list's (entry, group) units evenly.
+// grid.x: persistent CTAs walking the row-tile groups; grid.z: column tile of 8 activation rows (plain mode).
+// A grouped launch over a work list is one row of CTAs that share the list's (entry, group) units evenly.
 //
 // Weights reach the SM as whole tiles (16 consecutive rows are one contiguous run of the
 // checkpoint's own blocks) through cp.async.bulk into a ring of shared-memory stages, each
@@ -507,8 +501,6 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   __shared__ float scratch[4 * QG_WARPS];
   __shared__ float ssq[2][QG_WARPS][8];
   __shared__ int col_rows[QG_MAXCOLS], xrows[QG_MAXCOLS];
-  __shared__ int route_expert, route_topk[32];
-  __shared__ float2 cand[32];
   __shared__ __align__(8) uint64_t full_bar[QG_MAX_STAGES];
 
   const int tiles = (p.N + 15) / 16;
@@ -522,61 +514,22 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   }
   __syncthreads();
 
-  // What this CTA walks is a sequence of units, each one row-tile group of one weight matrix. Plain launches and
-  // launches that route for themselves take the groups blockIdx.x, blockIdx.x + gridDim.x, ... of the one matrix they
+  // What this CTA walks is a sequence of units, each one row-tile group of one weight matrix. Plain launches take the groups blockIdx.x, blockIdx.x + gridDim.x, ... of the one matrix they
   // are given. Launches over a work list cut the whole list, entries * groups units, into one contiguous run per CTA:
   // every CTA gets the same share whatever the list's length (known only on the device), a run stages the activation
   // rows of an entry once, and the weight ring runs ahead across the entries' boundaries.
-  const uint8_t *wa = nullptr, *wb = nullptr;
   int ncols = 0, col_off = 0, n_units = 0;
   long long u0 = 0;
-  bool active = true, x_copied = false;
-  bool flat = false;
-  auto own_units = [&]() { return (int)blockIdx.x < ngroups ? (ngroups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0; };
   if constexpr (GROUPED) {
-    pdl_wait();  // the entries (or the logits) are written by the router kernel
-    if (p.route_here) {
-      // blockIdx.y = row * (used + 1) + slot: every row of the pass is routed and computed on its own, exactly as a
-      // single-row pass would do it, so a pass of several rows gives each row the single-row result bit for bit
-      const int used = p.route.used, slots1 = used + 1, y = blockIdx.y, row = y / slots1, slot = y - row * slots1;
-      const bool writer = blockIdx.x == 0 && slot == 0;
-      active = row < p.route.M;
-      if (warp == 0) {
-        if (active) {
-          const int ex = p.route.nE <= 512 ? route_token<16>(p.route, row, lane, writer, cand, slot, route_topk) : route_token<32>(p.route, row, lane, writer, cand, slot, route_topk);
-          if (lane == 0) route_expert = slot < used ? ex : -1;
-        }
-      } else if constexpr (PRO == PRO_F16) {
-        // meanwhile the other warps stage the row's activations (they do not depend on the routing)
-        if (active) copy_x_row(p.x + (int64_t)row * p.ldx, K, xs, sxs, sxs + (size_t)p.xcols * (K / 32), tid - 32, QG_THREADS - 32);
-      }
-      x_copied = PRO == PRO_F16;  // for every thread alike: the barrier below covers the copy
-      __syncthreads();
-      if (writer && p.route.entries != nullptr) {  // the row's part of the work list: one entry per slot, the shared expert last
-        if (tid < used) { p.route.entries[row * slots1 + tid] = make_int4(route_topk[tid], row * slots1 + tid, 1, 0); p.route.cols[row * slots1 + tid] = row * slots1 + tid; }
-        if (tid == used) {
-          p.route.entries[row * slots1 + used] = make_int4(-1, row * slots1 + used, 1, 0); p.route.cols[row * slots1 + used] = row * slots1 + used;
-          if (row == 0) *p.route.n_entries = p.route.M * slots1;
-        }
-      }
-      if (active) {
-        const int ex = route_expert;
-        col_off = y; ncols = 1;
-        wa = ex >= 0 ? p.w[0] + (size_t)ex * p.expert_stride : p.ws;
-        if constexpr (DUAL) wb = ex >= 0 ? p.w2[0] + (size_t)ex * p.expert_stride : p.ws2;
-        n_units = own_units();
-      }
-    } else {
-      flat = true;
-      const long long U = (long long)*p.n_entries * ngroups, C = (long long)gridDim.x * gridDim.y, c = (long long)blockIdx.y * gridDim.x + blockIdx.x;
-      u0 = c * U / C;
-      n_units = (int)((c + 1) * U / C - u0);
-    }
+    pdl_wait();  // the entries are written by the router kernel
+    const long long U = (long long)*p.n_entries * ngroups, c = blockIdx.x;
+    u0 = c * U / gridDim.x;
+    n_units = (int)((c + 1) * U / gridDim.x - u0);
   } else {
     ncols = p.M - (int)blockIdx.z * QG_MAXCOLS;
     if (ncols > QG_MAXCOLS) ncols = QG_MAXCOLS;
     col_off = (int)blockIdx.z * QG_MAXCOLS;
-    n_units = own_units();
+    n_units = (int)blockIdx.x < ngroups ? (ngroups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   }
   // warp 0 is the producer: one bulk copy per tile row, or per tile where rows lie as in memory
   auto issue_group = [&](int grp, int s, const uint8_t* ga, const uint8_t* gb) {
@@ -617,7 +570,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   };
   // unit j of this CTA goes to ring stage j % NS
   auto issue_unit = [&](int j) {
-    if (flat) {
+    if constexpr (GROUPED) {
       const long long u = u0 + j;
       const int en = (int)(u / ngroups), grp = (int)(u - (long long)en * ngroups);
       const int ex = p.entries[en].x;
@@ -626,7 +579,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       if constexpr (DUAL) gb = ex >= 0 ? p.w2[0] + (size_t)ex * p.expert_stride : p.ws2;
       issue_group(grp, j % NS, ga, gb);
     } else {
-      issue_group((int)blockIdx.x + j * (int)gridDim.x, j % NS, wa, wb);
+      issue_group((int)blockIdx.x + j * (int)gridDim.x, j % NS, nullptr, nullptr);
     }
   };
   if (warp == 0)
@@ -643,24 +596,24 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     if (tid < QG_MAXCOLS) {
       const int c = tid < ncols ? tid : 0;
       int id;
-      if constexpr (GROUPED) id = p.route_here ? col_off + c : p.cols[col_off + c];
+      if constexpr (GROUPED) id = p.cols[col_off + c];
       else id = p.row_ids ? p.row_ids[col_off + c] : col_off + c;
       col_rows[tid] = id;
       xrows[tid] = GROUPED ? id / p.x_div : id;
     }
     __syncthreads();
     if constexpr (PRO == PRO_NORM) stage_x_norm(p, xs, sxs, scratch, ncols, xrows, xstride, p.xn_out != nullptr && blockIdx.x == 0 && blockIdx.y == 0);
-    else if (!x_copied) stage_x_f16(p.x, p.ldx, K, p.xcols, xs, sxs, ncols, xrows, xstride);
+    else stage_x_f16(p.x, p.ldx, K, p.xcols, xs, sxs, ncols, xrows, xstride);
     live = g < ncols;
     xrow = xs + (size_t)(live ? g : 0) * xstride;
     sxrow = sxs + (size_t)((t & 1) * p.xcols + (live ? g : 0)) * (K / 32);
   };
-  if (active && !flat) { stage_rows(); tl_mark(p.tl, 2); }
+  if constexpr (!GROUPED) { stage_rows(); tl_mark(p.tl, 2); }
 
   int cur = -1, buf = 0;
   for (int it = 0; it < n_units; it++) {
     int grp;
-    if (flat) {
+    if constexpr (GROUPED) {
       const long long u = u0 + it;
       const int en = (int)(u / ngroups);
       grp = (int)(u - (long long)en * ngroups);
@@ -738,95 +691,6 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       }
     }
     buf ^= 1;
-  }
-  tl_mark(p.tl, 4);
-}
-
-// -----------------------------------------------------------------------------------------
-// The MoE block's end of a pass that routes per row: expert down projections, routing weights, shared expert and residual in one
-// kernel, h[row][i] += sum_s w_s * (W_down[e_s][i] . act[s]) + sigmoid(gate) * shared (reference: llm/moe.go:347-357, 403-406;
-// shaders/llm_moe_combine.comp:48-63), with the sum of squares of each tile's rows for the norm that follows.
-// A CTA owns 16 rows of h of one row of the pass; each of its warps takes a (slot, super-block) unit alone - fetches the 16 x 256
-// weights as one TMA box, stages the 256 activations itself - and the units' sums are added in slot order at the end. One round of
-// latency instead of a chain: the form before (8 warps, CTA-wide staging, three partial rows that every CTA of the next projection
-// added up again) took 8 us plus 3 us more of that projection's staging. grid (N / 16, rows), block 32 * warps.
-// -----------------------------------------------------------------------------------------
-struct MoeDownParams {
-  int K, N, used;
-  const int32_t* topk;      // [rows][used]
-  const float* topk_w;      // [rows][used + 1]
-  const __half* act;        // [rows][used + 1][K]
-  float* h;                 // [rows][N]
-  float* ss_out;            // [rows][SS_LD] sums of squares, part = tile
-  int* err;
-  Timeline tl;
-};
-struct MoeDownMaps { TMap w, ws; };   // boxes of 16 rows (make_w_tensor_map)
-constexpr int MD_MAXWARPS = 24;
-template <int TYPE> __host__ __device__ constexpr int md_raw() { return 16 * (TYPE == T_Q4_K ? 144 : 176); }
-constexpr int MD_X = 4 * 144 + 32;     // one super-block of a staged row, its eight sums as hi | lo
-
-template <int TYPE>
-__global__ void __launch_bounds__(MD_MAXWARPS * 32) moe_down_kernel(const __grid_constant__ MoeDownMaps maps, const MoeDownParams p) {
-  constexpr int BLK = TYPE == T_Q4_K ? 144 : 176;
-  extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ __align__(8) uint64_t bars[MD_MAXWARPS];
-  __shared__ float wgt[32];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, warps = blockDim.x >> 5;
-  const int nb = p.K / 256, slots1 = p.used + 1, units = slots1 * nb, tile = blockIdx.x, row = blockIdx.y;
-  uint8_t* raw = smem + warp * md_raw<TYPE>();
-  uint8_t* xs = smem + warps * md_raw<TYPE>() + warp * MD_X;
-  __half* sx = reinterpret_cast<__half*>(xs + 4 * 144);
-  float* yv = reinterpret_cast<float*>(smem + warps * (md_raw<TYPE>() + MD_X));   // [units][16]
-  tl_mark(p.tl, 0);
-  if (lane == 0) { mbar_init(&bars[warp], 1); mbar_fence_init(); }
-  __syncwarp();
-  pdl_wait();   // the selection and the activations come from the kernel before
-  pdl_launch();
-  tl_mark(p.tl, 1);
-  float hv = 0.f;
-  if (tid < 16) hv = __ldcg(p.h + (size_t)row * p.N + tile * 16 + tid);
-  if (tid < slots1) wgt[tid] = __ldcg(p.topk_w + (size_t)row * slots1 + tid);
-  int phase = 0;
-  for (int u = warp; u < units; u += warps, phase ^= 1) {
-    const int s = u / nb, blk = u - s * nb;
-    const int e = s < p.used ? __ldcg(p.topk + (size_t)row * p.used + s) : -1;
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.act + ((size_t)row * slots1 + s) * p.K + blk * 256 + 8 * lane));
-    if (elect_one()) {
-      if (u != warp) fence_proxy_async();
-      mbar_expect_tx(&bars[warp], md_raw<TYPE>());
-      tma_box_2d(raw, e >= 0 ? &maps.w : &maps.ws, blk * BLK, (e >= 0 ? e * p.N : 0) + tile * 16, &bars[warp]);
-    }
-    const uint4 o = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
-    *reinterpret_cast<uint4*>(xs + 16 * lane + 16 * (lane >> 3)) = o;
-    put_sx<4>(sum4_h2(o.x, o.y) + sum4_h2(o.z, o.w), sx, sx + 8, lane >> 2);
-    __syncwarp();
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    if (warp_wait(&bars[warp], phase)) {
-      const uint32_t ra = (uint32_t)__cvta_generic_to_shared(raw) + 2 * g * BLK;
-      const __half* sp = sx + ((t & 1) ? 8 : 0) + 2 * (t >> 1);
-      k45_accumulate<TYPE>(acc, ra, ra + BLK, xs, *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
-    } else if (lane == 0 && p.err != nullptr) {
-      atomicExch(p.err, 1);   // a copy never landed: report, the results are void
-    }
-    if (t == 0) *reinterpret_cast<float2*>(yv + u * 16 + 2 * g) = make_float2(acc[0], acc[2]);   // every column holds the one activation row
-    __syncwarp();
-  }
-  tl_mark(p.tl, 3);
-  __syncthreads();
-  if (tid < 16) {
-    float acc = 0.f, y = 0.f;
-    for (int s = 0; s < slots1; s++) {
-      y = 0.f;
-      for (int b = 0; b < nb; b++) y += yv[(s * nb + b) * 16 + tid];
-      if (s < p.used) acc = fmaf(wgt[s], y, acc);
-    }
-    const float r = hv + fmaf(wgt[p.used], y, acc);
-    p.h[(size_t)row * p.N + tile * 16 + tid] = r;
-    float sq = r * r;
-#pragma unroll
-    for (int o = 1; o < 16; o <<= 1) sq += __shfl_xor_sync(0xffffu, sq, o);
-    if (tid == 0) p.ss_out[(size_t)row * SS_LD + tile] = sq;
   }
   tl_mark(p.tl, 4);
 }

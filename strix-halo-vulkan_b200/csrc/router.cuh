@@ -35,7 +35,7 @@ struct RouterParams {
 // softmax + top-k + weights of one token by one warp; a lane owns experts lane + 32*i in registers
 // (reference: llm/moe.go:219-282, 426-443; shaders/llm_moe_route_decode.comp:84-213)
 template <int NPL>
-__device__ __forceinline__ int route_token(const RouterParams& p, int n, int lane, bool write, float2 (&cand)[32], int want_slot = -1, int* sm_topk = nullptr) {
+__device__ __forceinline__ int route_token(const RouterParams& p, int n, int lane, bool write, float2 (&cand)[32], int want_slot = -1) {
   int wanted = -1;
   const int nE = p.nE, used = p.used;
   float pv[NPL];
@@ -92,7 +92,6 @@ __device__ __forceinline__ int route_token(const RouterParams& p, int n, int lan
         rank += o > v || (o == v && j < lane);
       }
       if (lane >= n_cand) rank = 64;
-      if (sm_topk != nullptr && rank < used) sm_topk[rank] = idx;
       const uint32_t hit = __ballot_sync(0xffffffffu, rank == want_slot);
       const int wanted = __shfl_sync(0xffffffffu, idx, hit != 0 ? __ffs((int)hit) - 1 : 0);
       if (write) {
@@ -142,13 +141,96 @@ __device__ __forceinline__ int route_token(const RouterParams& p, int n, int lan
       for (int i = 0; i < NPL; i++) if (i == (widx >> 5)) pv[i] = -1.f;
     }
     if (k == want_slot) wanted = widx;
-    if (lane == k) { myw = wv; if (write) p.topk[(size_t)n * used + k] = widx; if (sm_topk != nullptr) sm_topk[k] = widx; }
+    if (lane == k) { myw = wv; if (write) p.topk[(size_t)n * used + k] = widx; }
     wsum += wv; last_p = wv;
   }
   // normalise the weights (llm/moe.go:256-282)
   if (wsum < 6.103515625e-5f) wsum = 6.103515625e-5f;
   if (write && lane < used) p.topk_w[(size_t)n * (used + 1) + lane] = myw / wsum;
   return wanted;
+}
+
+// The same selection by a CTA of 256 threads with VPT experts each, of one row whose logits an earlier kernel left; returns the expert
+// of slot want_slot (in every thread). In one warp the chain of instructions is what costs (3.6 us for 512 experts); spread over
+// eight it is three barriers and about as many hundred instructions.
+struct RouteSmem { float mx[8], sum[8], gmax[32]; float2 cand[32]; int n_cand, expert; };
+template <int VPT>
+__device__ __forceinline__ int route_row_cta(const RouterParams& p, int n, const float (&l)[VPT], bool write, int want_slot, RouteSmem& sm) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, used = p.used;
+  float m = l[0];
+#pragma unroll
+  for (int i = 1; i < VPT; i++) m = fmaxf(m, l[i]);
+  int key = __float_as_int(m);                       // order of the floats as signed integers
+  key ^= (key >> 31) & 0x7fffffff;
+  key = __reduce_max_sync(0xffffffffu, key);
+  if (lane == 0) sm.mx[warp] = __int_as_float(key ^ ((key >> 31) & 0x7fffffff));
+  if (tid == 0) sm.n_cand = 0;
+  __syncthreads();
+  m = sm.mx[0];
+#pragma unroll
+  for (int w = 1; w < 8; w++) m = fmaxf(m, sm.mx[w]);
+  float ev[VPT], s = 0.f, gm = -1.f;
+#pragma unroll
+  for (int i = 0; i < VPT; i++) {
+    const bool live = tid + 256 * i < p.nE;
+    ev[i] = live ? expf(l[i] - m) : -1.f;
+    s += live ? ev[i] : 0.f;
+    gm = fmaxf(gm, ev[i]);
+  }
+  s = warp_sum(s);
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+  if (lane == 0) sm.sum[warp] = s;
+  if ((lane & 7) == 0) sm.gmax[tid >> 3] = gm;
+  __syncthreads();
+  s = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; w++) s += sm.sum[w];
+  const float inv = 1.0f / s;
+  // bound: the (used + 1)-th largest of the 32 groups' maxima
+  const float g = sm.gmax[lane];
+  int above = 0;
+#pragma unroll 8
+  for (int j = 0; j < 32; j++) { const float o = sm.gmax[j]; above += o > g || (o == g && j < lane); }
+  const uint32_t at = __ballot_sync(0xffffffffu, above == used);
+  const float be = __shfl_sync(0xffffffffu, g, at != 0 ? __ffs((int)at) - 1 : 0), bound = at != 0 && be >= 0.f ? be * inv : -1.f;
+#pragma unroll
+  for (int i = 0; i < VPT; i++) {
+    const float pv = ev[i] * inv;
+    if (ev[i] >= 0.f && pv >= bound) {
+      const int c = atomicAdd(&sm.n_cand, 1);
+      if (c < 32) sm.cand[c] = make_float2(pv, __int_as_float(tid + 256 * i));
+    }
+  }
+  __syncthreads();
+  const int nc = sm.n_cand;
+  if (nc > 32 || nc <= used) {   // many equal values (or none comparable): the one-warp form
+    if (warp == 0) {
+      const int ex = p.nE <= 512 ? route_token<16>(p, n, lane, write, sm.cand, want_slot) : route_token<32>(p, n, lane, write, sm.cand, want_slot);
+      if (lane == 0) sm.expert = ex;
+    }
+    __syncthreads();
+    return sm.expert;
+  }
+  const float v = lane < nc ? sm.cand[lane].x : -1.f;
+  const int idx = lane < nc ? __float_as_int(sm.cand[lane].y) : 0x7fffffff;
+  int rank = lane < nc ? 0 : 64;
+  for (int j = 0; j < nc; j++) { const float2 o = sm.cand[j]; rank += o.x > v || (o.x == v && __float_as_int(o.y) < idx); }
+  const uint32_t hit = __ballot_sync(0xffffffffu, rank == want_slot);
+  if (write && warp == 0) {
+    if (rank < used) p.topk[(size_t)n * used + rank] = idx;
+    // the weights, added in slot order (llm/moe.go:256-282): lane k takes the value of rank k
+    float mine = 0.f, wsum = 0.f, last = 0.f, next = 0.f;
+    for (int k = 0; k <= used; k++) {
+      const float x = __shfl_sync(0xffffffffu, v, __ffs((int)__ballot_sync(0xffffffffu, rank == k)) - 1);
+      if (k == lane) mine = x;
+      if (k < used) { wsum += x; last = x; } else next = x;
+    }
+    if (lane == 0 && p.margin) p.margin[n] = last > 0.f ? (last - next) / last : 0.f;
+    if (wsum < 6.103515625e-5f) wsum = 6.103515625e-5f;
+    if (lane < used) p.topk_w[(size_t)n * (used + 1) + lane] = mine / wsum;
+  }
+  return __shfl_sync(0xffffffffu, idx, hit != 0 ? __ffs((int)hit) - 1 : 0);
 }
 
 #endif

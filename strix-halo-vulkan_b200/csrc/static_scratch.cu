@@ -69,7 +69,7 @@ int qgemv_static(uint32_t type, const void* dev_w, int64_t rows, int64_t k, cons
   QGemvParams p{};
   p.w[0] = (const uint8_t*)dev_w; p.seg_end[0] = (int)rows; p.nseg = 1; p.stride = device_row_stride(type, k);
   p.K = (int)k; p.N = (int)rows; p.M = m; p.xcols = m; p.x = sc.x16; p.ldx = k; p.y = dev_y; p.ldy = rows; p.x_div = 1; p.err = sc.err;
-  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, 0, false, 0));
+  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, false, 0));
   int herr = 0;
   B200_CUDA(cudaMemcpy(&herr, sc.err, sizeof(int), cudaMemcpyDeviceToHost));  // also waits for the work
   if (herr != 0) { set_error("qgemv_static: a bounded wait for the weight copies gave up; dev_y is not valid"); return ETIMEOUT; }
