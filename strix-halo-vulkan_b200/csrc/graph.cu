@@ -340,7 +340,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     B200_TRY(launch_concat_norm(e_buf, hs_buf, (const float*)L.enorm.data, (const float*)L.hnorm.data, c.eps, H, M, xcat16, pdl(), st));
     QGemvParams p = base(L.eh_proj, 2 * H, H, xcat16, 2 * H);
     p.y = h; p.ldy = H;
-    if (fused) { p.ss_out = ss_part; ss_n = qgemv_groups(2 * H, H); }
+    if (fused) { p.ss_out = ss_part; ss_n = (H + 15) / 16; }
     B200_TRY(launch_qgemv(L.eh_proj.type, PRO_F16, EPI_STORE, false, false, p, pdl(), st));
     if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.attn_norm), pdl(), st));
   } else {
@@ -382,7 +382,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       }
       QGemvParams q = base(L.ssm_out, vw, H, y16, vw);
       q.y = h; q.ldy = H;
-      if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(vw, H); }
+      if (fused) { q.ss_out = ss_part; ss_n = (H + 15) / 16; }
       if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out.m[0], vw, y16, tx_y16, sx_y, ts_y16));
       else if (use_gemm) B200_TRY(gemm_resid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16[2]));
       else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));
@@ -438,7 +438,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       }
       QGemvParams q = base(L.o, qw, H, ctx16, qw);
       q.y = h; q.ldy = H;
-      if (fused) { q.ss_out = ss_part; ss_n = qgemv_groups(qw, H); }
+      if (fused) { q.ss_out = ss_part; ss_n = (H + 15) / 16; }
       if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o.m[0], qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
       else if (use_gemm) B200_TRY(gemm_resid(L.o, wmaps[l].o, qw, ctx16, tx_ctx[2]));
       else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));

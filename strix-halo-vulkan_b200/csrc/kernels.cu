@@ -224,7 +224,7 @@ static int launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem
 // Router: ffn_norm + router GEMV (exact f32 dequant) + softmax + top-k + work list
 // (reference: llm/moe.go:219-282; shaders/llm_moe_router.comp, llm_moe_route_decode.comp)
 // =========================================================================================
-constexpr int RT_ROWS = 8;  // router rows per CTA: one per warp
+constexpr int RT_ROWS = 4;  // router rows per CTA: two warps to a row, half of its contraction each, so that 513 rows reach every SM
 
 // Expert work list of a pass from its routing, by one CTA of 256 threads: pair id = n*(used+1) + slot,
 // slot == used is the shared expert; entries of at most 8 columns per expert for the column-tiled kernels,
@@ -311,20 +311,22 @@ int launch_ep_worklist(const RouterParams& p, bool pdl, cudaStream_t st) {
 __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
   __shared__ int is_last;
   __shared__ float2 cand[8][32];
+  __shared__ float half_sum[8][8];
   __shared__ int counts[1025], offs[1025], eoff[1025];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H, M = p.M;
-  const int row = blockIdx.x * RT_ROWS + warp;  // of the nE + 1 outputs; the last is the shared-expert gate
+  const int row = blockIdx.x * RT_ROWS + (warp >> 1), half = warp & 1;  // of the nE + 1 outputs; the last is the shared-expert gate
+  const int k_lo = half * (H / 2), k_hi = half ? H : H / 2;
   tl_mark(p.tl, 0);
   const bool q8 = p.router.type == T_Q8_0 && H % 512 == 0 && H <= 4096;
   // the row's weights do not depend on the producer kernel: fetch them first
-  uint4 wq[8]; float wd[8];
+  uint4 wq[4]; float wd[4];
   if (row < p.nE && q8) {
     const uint8_t* wr = p.router.data + (size_t)row * p.router.stride;
     const int nb = H / 32;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const int k0 = lane * 16 + i * 512;
-      if (k0 < H) { wq[i] = ldg_stream(wr + k0); wd[i] = ld_f16(wr + nb * 32 + (k0 / 32) * 2); }
+    for (int i = 0; i < 4; i++) {
+      const int k0 = k_lo + lane * 16 + i * 512;
+      if (k0 < k_hi) { wq[i] = ldg_stream(wr + k0); wd[i] = ld_f16(wr + nb * 32 + (k0 / 32) * 2); }
     }
   }
   const bool staged = p.h != nullptr;
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
       const __half* x = staged ? rxs + (size_t)n * H : p.xn + (size_t)n * H;
       float acc = 0.f;
       if (row == p.nE) {
-        for (int k = lane * 8; k < H; k += 256) {
+        for (int k = k_lo + lane * 8; k < k_hi; k += 256) {
           uint4 xv = *reinterpret_cast<const uint4*>(x + k);
           const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
           float4 g0 = *reinterpret_cast<const float4*>(p.sh_gate + k), g1 = *reinterpret_cast<const float4*>(p.sh_gate + k + 4);
@@ -387,9 +389,9 @@ __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
         }
       } else if (q8) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int k0 = lane * 16 + i * 512;
-          if (k0 < H) {
+        for (int i = 0; i < 4; i++) {
+          const int k0 = k_lo + lane * 16 + i * 512;
+          if (k0 < k_hi) {
             uint4 xa = *reinterpret_cast<const uint4*>(x + k0), xb = *reinterpret_cast<const uint4*>(x + k0 + 8);
             const uint32_t xw[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
             const uint32_t w[4] = {wq[i].x, wq[i].y, wq[i].z, wq[i].w};
@@ -403,13 +405,19 @@ __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
         }
       } else {
         const uint8_t* wr = p.router.data + (size_t)row * p.router.stride;
-        for (int k = lane; k < H; k += 32) acc = fmaf(dequant_elem(p.router.type, wr, H, k), __half2float(x[k]), acc);
+        for (int k = k_lo + lane; k < k_hi; k += 32) acc = fmaf(dequant_elem(p.router.type, wr, H, k), __half2float(x[k]), acc);
       }
       acc = warp_sum(acc);
-      if (lane == 0) {
-        if (row == p.nE) p.topk_w[(size_t)n * (p.used + 1) + p.used] = sigmoid_acc(acc);
-        else p.logits[(size_t)n * p.nE + row] = acc;
-      }
+      if (lane == 0) half_sum[n - n_lo][warp] = acc;
+    }
+  }
+  __syncthreads();
+  if (tid < 8 * RT_ROWS) {
+    const int n = blockIdx.y * 8 + tid / RT_ROWS, w = tid % RT_ROWS, e = blockIdx.x * RT_ROWS + w;
+    if (n < M && e <= p.nE) {
+      const float v = half_sum[tid / RT_ROWS][2 * w] + half_sum[tid / RT_ROWS][2 * w + 1];
+      if (e == p.nE) p.topk_w[(size_t)n * (p.used + 1) + p.used] = sigmoid_acc(v);
+      else p.logits[(size_t)n * p.nE + e] = v;
     }
   }
   tl_mark(p.tl, 4);
@@ -568,7 +576,7 @@ int launch_route_rows(const RouterParams& p, bool pdl, cudaStream_t st) {
 }
 
 int launch_router(const RouterParams& p, bool pdl, cudaStream_t st) {
-  if (p.nE > 1024 || p.used > 32 || p.H % 8) { set_error("router: shape outside kernel limits"); return ECAPACITY; }
+  if (p.nE > 1024 || p.used > 32 || p.H % 16) { set_error("router: shape outside kernel limits"); return ECAPACITY; }
   int grid = (p.nE + 1 + RT_ROWS - 1) / RT_ROWS;
   size_t smem = 0;
   if (p.h != nullptr) {
@@ -652,9 +660,25 @@ __device__ __forceinline__ float softplus_ref(float x) {  // llm/deltanet.go:450
   return logf(1.0f + expf(x));
 }
 __device__ __forceinline__ float silu_acc(float x) { return x * sigmoid_acc(x); }
+// Sums of eight values over the warp's lanes, every lane getting all eight: halves of the values change hands at each of the first
+// three steps, so 17 shuffles instead of 40, and every sum is the one the plain butterfly from 16 down to 1 forms.
+__device__ __forceinline__ void warp_sum8(float (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  float a[4], b[2];
+  const bool h4 = lane & 16, h2 = lane & 8, h1 = lane & 4;
+#pragma unroll
+  for (int i = 0; i < 4; i++) a[i] = (h4 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, h4 ? v[i] : v[i + 4], 16);
+#pragma unroll
+  for (int i = 0; i < 2; i++) b[i] = (h2 ? a[i + 2] : a[i]) + __shfl_xor_sync(0xffffffffu, h2 ? a[i] : a[i + 2], 8);
+  float c = (h1 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h1 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+#pragma unroll
+  for (int r = 0; r < 8; r++) v[r] = __shfl_sync(0xffffffffu, c, 4 * r);   // row r sits in the lanes whose bits 4, 3, 2 spell it
+}
 
 // (Passes of 16 sequences and more use dn_head_kernel below instead.)
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128, 1) dn_step_kernel(DnStepParams p) {
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128, 5) dn_step_kernel(DnStepParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   const int D = 128, RB = 4;
   const int h = blockIdx.x / RB, rb = blockIdx.x % RB, hk = h % p.Hk;
@@ -761,22 +785,14 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128, 1) dn_step_kern
       s[r].x *= g; s[r].y *= g; s[r].z *= g; s[r].w *= g;
       kv[r] = s[r].x * k4.x + s[r].y * k4.y + s[r].z * k4.z + s[r].w * k4.w;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int r = 0; r < 8; r++) kv[r] += __shfl_xor_sync(0xffffffffu, kv[r], o);
-    }
+    warp_sum8(kv);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const float dj = (vs[warp * 8 + r] - kv[r]) * beta;
       s[r].x += dj * k4.x; s[r].y += dj * k4.y; s[r].z += dj * k4.z; s[r].w += dj * k4.w;
       oo[r] = s[r].x * q4.x + s[r].y * q4.y + s[r].z * q4.z + s[r].w * q4.w;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int r = 0; r < 8; r++) oo[r] += __shfl_xor_sync(0xffffffffu, oo[r], o);
-    }
+    warp_sum8(oo);
     // gated norm: sum of squares over the head's 128 outputs = four CTA partials, added in rank order
     float ov = oo[0] * oscale, ss = 0.f;
 #pragma unroll
@@ -906,22 +922,14 @@ __global__ void __launch_bounds__(512, 2) dn_head_kernel(DnStepParams p) {
       s[r].x *= g; s[r].y *= g; s[r].z *= g; s[r].w *= g;
       kv[r] = s[r].x * k4.x + s[r].y * k4.y + s[r].z * k4.z + s[r].w * k4.w;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int r = 0; r < 8; r++) kv[r] += __shfl_xor_sync(0xffffffffu, kv[r], o);
-    }
+    warp_sum8(kv);
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const float dj = (vs[j0 + r] - kv[r]) * beta;
       s[r].x += dj * k4.x; s[r].y += dj * k4.y; s[r].z += dj * k4.z; s[r].w += dj * k4.w;
       oo[r] = s[r].x * q4.x + s[r].y * q4.y + s[r].z * q4.z + s[r].w * q4.w;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-      for (int r = 0; r < 8; r++) oo[r] += __shfl_xor_sync(0xffffffffu, oo[r], o);
-    }
+    warp_sum8(oo);
     // gated norm: sum of squares over the head's 128 outputs, warp partials grouped by four as the row blocks were
     float ov = oo[0] * oscale, ss = 0.f;
 #pragma unroll

@@ -38,7 +38,6 @@ int launch_embed(const EmbedParams& p, cudaStream_t st);
 
 // K-quant projections; `pdl` marks the launch as a programmatic dependent of the previous kernel.
 int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st);
-int qgemv_groups(int K, int N);
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st);
 int launch_concat_norm(const float* e, const float* hs, const float* enorm, const float* hnorm, float eps, int H, int M, __half* xcat, bool pdl, cudaStream_t st);
 

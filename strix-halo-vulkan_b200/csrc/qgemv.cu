@@ -79,18 +79,10 @@ static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvPar
   return EINVAL_;
 }
 
-// tile groups a projection of N rows of length K is cut into (= partial sums of squares it leaves per row)
-int qgemv_groups(int K, int N) {
-  const int nb = K / 256;
-  const int wpt = nb >= 8 ? 8 : nb >= 4 ? 4 : nb >= 2 ? 2 : 1;
-  const int tpc = QG_WARPS / wpt;
-  return ((N + 15) / 16 + tpc - 1) / tpc;
-}
-
 int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st) {
   if (p.K % 256 != 0 || p.K <= 0) { set_error("qgemv: row length must be a multiple of 256"); return EINVAL_; }
   if (p.xcols < 1 || p.xcols > QG_MAXCOLS) { set_error("qgemv: xcols out of range"); return EINVAL_; }
-  if (p.ss_out != nullptr && qgemv_groups(p.K, p.N) > SS_LD) { set_error("qgemv: more tile groups than partial-sum slots"); return ECAPACITY; }
+  if (p.ss_out != nullptr && (p.N + 15) / 16 > SS_LD) { set_error("qgemv: more tiles than partial-sum slots"); return ECAPACITY; }
   if (pro == PRO_NORM && (p.ss_n < 1 || p.ss_n > SS_LD)) { set_error("qgemv: bad partial-sum count"); return EINVAL_; }
   switch (type) {
     case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, pdl, st);

@@ -72,7 +72,7 @@ struct QGemvParams {
   int ss_n;
   float eps;
   __half* xn_out;            // PRO_NORM: optional copy of the normalised rows, [.][K], written by CTA 0
-  float* ss_out;             // STORE / RESID: optional partial sums of squares of the rows written, [.][SS_LD], part = tile group
+  float* ss_out;             // STORE / RESID: optional partial sums of squares of the rows written, [.][SS_LD], part = tile of 16 rows
   // epilogue
   float* y;                  // STORE / RESID: float [.][ldy]
   int64_t ldy;
@@ -96,7 +96,7 @@ __host__ __device__ inline size_t qg_stage_bytes(int K, int64_t stride, bool dua
 __host__ __device__ inline size_t qg_fixed_smem(int K, int xcols, bool dual) {
   size_t xs = (size_t)xcols * qg_xstride(K);
   size_t sx = (size_t)xcols * (K / 32) * 2 * sizeof(__half);  // hi and lo planes
-  size_t red = (size_t)2 * QG_WARPS * 16 * 8 * sizeof(float) * (dual ? 2 : 1);  // double-buffered
+  size_t red = (size_t)2 * QG_WARPS * 16 * 8 * sizeof(float);  // partial sums: two units of eight columns, or one of a pair of matrices
   return ((xs + ((sx + 15) & ~(size_t)15) + red) + 127) & ~(size_t)127;
 }
 
@@ -490,7 +490,6 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   const int wpt = nb >= 8 ? 8 : nb >= 4 ? 4 : nb >= 2 ? 2 : 1;  // warps per tile (K-slices)
   const int tpc = QG_WARPS / wpt;                               // tiles per CTA and iteration
   const int xstride = qg_xstride(K);
-  constexpr int RED = QG_WARPS * 128 * (DUAL ? 2 : 1);          // floats per reduction buffer
   uint8_t* xs = smem;
   __half* sxs = reinterpret_cast<__half*>(smem + (size_t)p.xcols * xstride);
   float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sxs) + (((size_t)p.xcols * (K / 32) * 2 * sizeof(__half) + 15) & ~(size_t)15));
@@ -499,7 +498,6 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   const size_t stage_bytes = (size_t)tpc * tile_bytes * (DUAL ? 2 : 1);
   const int NS = p.nstage;
   __shared__ float scratch[4 * QG_WARPS];
-  __shared__ float ssq[2][QG_WARPS][8];
   __shared__ int col_rows[QG_MAXCOLS], xrows[QG_MAXCOLS];
   __shared__ __align__(8) uint64_t full_bar[QG_MAX_STAGES];
 
@@ -610,87 +608,83 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   };
   if constexpr (!GROUPED) { stage_rows(); tl_mark(p.tl, 2); }
 
-  int cur = -1, buf = 0;
-  for (int it = 0; it < n_units; it++) {
-    int grp;
+  // Units go through in chunks: every warp leaves its partial sums of a chunk's units, [unit][warp][column][row], one barrier, and
+  // the CTA adds them up in warp order. (A barrier per unit left the warps waiting for one another three times in a decode step's
+  // largest projection.) A chunk is what the ring and 8 KB of partial sums hold.
+  const int xc = GROUPED ? QG_MAXCOLS : p.xcols, chunk = GROUPED ? 1 : min(NS, 2 * QG_MAXCOLS / xc);
+  const size_t plane2 = QG_WARPS * 16 * QG_MAXCOLS;   // DUAL: the second matrix's sums
+  int cur = -1;
+  for (int it0 = 0; it0 < n_units; it0 += chunk) {
+    const int cnt = min(chunk, n_units - it0);
+    if (it0 > 0) __syncthreads();   // the sums before are read; GROUPED: every warp is done with the rows of the entry before
     if constexpr (GROUPED) {
-      const long long u = u0 + it;
-      const int en = (int)(u / ngroups);
-      grp = (int)(u - (long long)en * ngroups);
+      const int en = (int)((u0 + it0) / ngroups);
       if (en != cur) {
-        if (cur >= 0) __syncthreads();   // every warp is done with the rows and the row ids of the entry before
         const int4 e = p.entries[en];
         col_off = e.y; ncols = e.z; cur = en;
         stage_rows();
       }
-    } else {
-      grp = (int)blockIdx.x + it * (int)gridDim.x;
     }
-    const int s = it % NS;
-    if (!mbar_wait(&full_bar[s], (uint32_t)((it / NS) & 1))) {
-      if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report and leave
-      return;
-    }
-    if (it == 0) tl_mark(p.tl, 3);
-    float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
-    const int tile = grp * tpc + lt;
-    if (tile < tiles) {
-      const int nrows = min(16, p.N - tile * 16);
-      const uint8_t* tb = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes * (DUAL ? 2 : 1);
-      const uint8_t *row0 = tb + min(mma_row<TYPE>(g, false), nrows - 1) * pitch, *row1 = tb + min(mma_row<TYPE>(g, true), nrows - 1) * pitch;
-      for (int blk = kslice; blk < nb; blk += wpt) {
-        block_accumulate<TYPE>(acc, row0, row1, xrow, sxrow, live, nb, blk, t);
-        if constexpr (DUAL) block_accumulate<TYPE>(acc2, row0 + tile_bytes, row1 + tile_bytes, xrow, sxrow, live, nb, blk, t);
+    auto group_of = [&](int it) {
+      if constexpr (GROUPED) return (int)((u0 + it) % ngroups);
+      else return (int)blockIdx.x + it * (int)gridDim.x;
+    };
+    for (int u = 0; u < cnt; u++) {
+      const int it = it0 + u, s = it % NS;
+      if (!mbar_wait(&full_bar[s], (uint32_t)((it / NS) & 1))) {
+        if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report and leave
+        return;
       }
-    }
-    // cross-warp reduction in warp order, double-buffered so one barrier per group suffices
-    float* myred = red + (size_t)buf * RED + (size_t)warp * 128;
-    const int m0 = mma_row<TYPE>(g, false) * 8 + 2 * t, m1 = mma_row<TYPE>(g, true) * 8 + 2 * t;
-    *reinterpret_cast<float2*>(myred + m0) = make_float2(acc[0], acc[1]);
-    *reinterpret_cast<float2*>(myred + m1) = make_float2(acc[2], acc[3]);
-    if constexpr (DUAL) {
-      float* r2 = myred + QG_WARPS * 128;
-      *reinterpret_cast<float2*>(r2 + m0) = make_float2(acc2[0], acc2[1]);
-      *reinterpret_cast<float2*>(r2 + m1) = make_float2(acc2[2], acc2[3]);
+      if (it == 0) tl_mark(p.tl, 3);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
+      const int tile = group_of(it) * tpc + lt;
+      if (tile < tiles) {
+        const int nrows = min(16, p.N - tile * 16);
+        const uint8_t* tb = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes * (DUAL ? 2 : 1);
+        const uint8_t *row0 = tb + min(mma_row<TYPE>(g, false), nrows - 1) * pitch, *row1 = tb + min(mma_row<TYPE>(g, true), nrows - 1) * pitch;
+        for (int blk = kslice; blk < nb; blk += wpt) {
+          block_accumulate<TYPE>(acc, row0, row1, xrow, sxrow, live, nb, blk, t);
+          if constexpr (DUAL) block_accumulate<TYPE>(acc2, row0 + tile_bytes, row1 + tile_bytes, xrow, sxrow, live, nb, blk, t);
+        }
+      }
+      auto leave = [&](float* my, const float (&a)[4]) {
+        const int m0 = mma_row<TYPE>(g, false), m1 = mma_row<TYPE>(g, true);
+        if (2 * t < xc) { my[2 * t * 16 + m0] = a[0]; my[2 * t * 16 + m1] = a[2]; }
+        if (2 * t + 1 < xc) { my[(2 * t + 1) * 16 + m0] = a[1]; my[(2 * t + 1) * 16 + m1] = a[3]; }
+      };
+      leave(red + (size_t)(u * QG_WARPS + warp) * 16 * xc, acc);
+      if constexpr (DUAL) leave(red + plane2 + (size_t)(u * QG_WARPS + warp) * 16 * xc, acc2);
     }
     __syncthreads();
-    // every warp is done with stage s: refill it with the unit NS iterations ahead
-    if (warp == 0 && it + NS < n_units) { fence_proxy_async(); issue_unit(it + NS); }
-    const float* rb = red + (size_t)buf * RED;
-    float sq = 0.f;  // this thread's column is tid & 7 in every iteration
-    for (int i = tid; i < tpc * 128; i += QG_THREADS) {
-      const int l2 = i >> 7, rc = i & 127, r = rc >> 3, c = rc & 7;
-      const int grow = (grp * tpc + l2) * 16 + r;
-      if (grow >= p.N || c >= ncols) continue;
-      float v = 0.f, v2 = 0.f;
+    // every warp is done with these stages: refill them with the units NS iterations ahead
+    if (warp == 0)
+      for (int u = 0; u < cnt; u++)
+        if (it0 + u + NS < n_units) { fence_proxy_async(); issue_unit(it0 + u + NS); }
+    // sixteen threads per (unit, tile, column), one row each
+    const int r = tid & 15, sets = cnt * tpc, inv = 65535 / sets + 1;
+    for (int q = tid >> 4; q < sets * ncols; q += QG_THREADS / 16) {
+      const int c = (q * inv) >> 16, ul = q - c * sets, u = ul / tpc, l2 = ul - u * tpc;
+      const int tile = group_of(it0 + u) * tpc + l2, grow = tile * 16 + r;
+      const float* rb = red + ((size_t)(u * QG_WARPS + l2 * wpt) * xc + c) * 16 + r;
+      float v = 0.f, v2 = 0.f, sq = 0.f;
       for (int w = 0; w < wpt; w++) {
-        v += rb[(size_t)(l2 * wpt + w) * 128 + rc];
-        if constexpr (DUAL) v2 += rb[(size_t)(QG_WARPS + l2 * wpt + w) * 128 + rc];
+        v += rb[w * 16 * xc];
+        if constexpr (DUAL) v2 += rb[plane2 + w * 16 * xc];
       }
       const int64_t orow = (!GROUPED && p.row_ids != nullptr) ? col_off + c : col_rows[c];
-      if constexpr (EPI == EPI_STORE) { p.y[orow * p.ldy + grow] = v; sq += v * v; }
-      else if constexpr (EPI == EPI_RESID) { const float nv = p.y[orow * p.ldy + grow] + v; p.y[orow * p.ldy + grow] = nv; sq += nv * nv; }
-      else {  // SwiGLU of (gate, up) rounded to fp16 (reference: shaders/llm_moe_gemv.comp:777-781)
-        float sw = v * sigmoid_acc(v) * v2;
-        p.y16[orow * p.ldy + grow] = __float2half_rn(sw);
+      if (grow < p.N) {
+        if constexpr (EPI == EPI_STORE) { p.y[orow * p.ldy + grow] = v; sq = v * v; }
+        else if constexpr (EPI == EPI_RESID) { const float nv = p.y[orow * p.ldy + grow] + v; p.y[orow * p.ldy + grow] = nv; sq = nv * nv; }
+        else p.y16[orow * p.ldy + grow] = __float2half_rn(v * sigmoid_acc(v) * v2);  // SwiGLU of (gate, up) rounded to fp16 (reference: shaders/llm_moe_gemv.comp:777-781)
       }
-    }
-    if constexpr (EPI != EPI_SWIGLU && !GROUPED) {
-      if (p.ss_out != nullptr) {  // sum of squares of this group's rows per column, in a fixed order
-        sq += __shfl_xor_sync(0xffffffffu, sq, 8);
-        sq += __shfl_xor_sync(0xffffffffu, sq, 16);
-        if (lane < 8) ssq[buf][warp][lane] = sq;
-        __syncthreads();
-        if (tid < ncols) {
-          float t2 = 0.f;
+      if constexpr (EPI != EPI_SWIGLU && !GROUPED) {
+        if (p.ss_out != nullptr) {  // sum of squares of this tile's rows per column, in a fixed order
 #pragma unroll
-          for (int w = 0; w < QG_WARPS; w++) t2 += ssq[buf][w][tid];
-          const int64_t orow = p.row_ids != nullptr ? col_off + tid : col_rows[tid];
-          p.ss_out[orow * SS_LD + grp] = t2;
+          for (int o = 1; o < 16; o <<= 1) sq += __shfl_xor_sync(0xffffu << (lane & 16), sq, o);
+          if (r == 0 && tile < tiles) p.ss_out[orow * SS_LD + tile] = sq;
         }
       }
     }
-    buf ^= 1;
   }
   tl_mark(p.tl, 4);
 }
