@@ -400,7 +400,9 @@ int32_t b200_qgemv(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
   QGemvParams p{};
   p.w[0] = t.data; p.seg_end[0] = (int)rows; p.nseg = 1; p.stride = t.stride; p.K = (int)k; p.N = (int)rows; p.M = mrows; p.xcols = mrows < QG_MAXCOLS ? mrows : QG_MAXCOLS;
   p.x = x16; p.ldx = k; p.y = y; p.ldy = rows; p.x_div = 1; p.err = err;
-  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, false, 0));
+  QGemvMaps maps{};
+  B200_TRY(make_qgemv_map(type, t.data, rows, t.stride, &maps.w[0]));
+  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, maps, false, 0));
   return finish_projection("qgemv", y, err, (int64_t)mrows * rows, host_y);
 }
 

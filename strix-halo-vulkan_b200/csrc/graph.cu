@@ -173,9 +173,15 @@ int Graph::make_weight_maps() {
   wmaps.resize(m->layers.size());
   auto narrow = [](const DTensor& w, TMap* out) { return w.ok() && qlist_type(w.type) ? make_w_tensor_map(w.type, w.data, w.rows, w.stride, 16, out) : (int)OK; };
   auto wide = [](const DTensor& w, int box, WMap* out) { return w.ok() && wgemm_type(w.type) ? make_wmap(w.type, w.data, w.rows, w.stride, box, out) : (int)OK; };
+  auto boxed = [&](const DTensor& w) {
+    if (!w.ok()) return (int)OK;
+    return make_qgemv_map(w.type, w.data, w.rows, w.stride, &row_maps[w.data]);
+  };
+  B200_TRY(boxed(m->output));
   for (size_t l = 0; l < m->layers.size(); l++) {
     const LayerW& L = m->layers[l];
     LayerMaps& W = wmaps[l];
+    for (const DTensor* w : {&L.qkv, &L.z, &L.ssm_out, &L.q, &L.k, &L.v, &L.o, &L.eh_proj}) B200_TRY(boxed(*w));
     B200_TRY(narrow(L.gate_exps, &W.gate)); B200_TRY(narrow(L.up_exps, &W.up)); B200_TRY(narrow(L.down_exps, &W.down));
     B200_TRY(narrow(L.gate_sh, &W.gate_sh)); B200_TRY(narrow(L.up_sh, &W.up_sh)); B200_TRY(narrow(L.down_sh, &W.down_sh));
     B200_TRY(wide(L.gate_exps, 64, &W.wgate)); B200_TRY(wide(L.up_exps, 64, &W.wup)); B200_TRY(wide(L.down_exps, 128, &W.wdown));
@@ -274,6 +280,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     p.x = x; p.ldx = ldx; p.err = err_flag; p.tl = tl(); p.eps = c.eps;
     return p;
   };
+  // launches a plain projection; its segments' weights name their tensor maps
+  auto project = [&](uint32_t type, int pro, int epi, const QGemvParams& p) {
+    QGemvMaps maps{};
+    for (int i = 0; i < p.nseg; i++) maps.w[i] = row_maps.at(p.w[i]);
+    return launch_qgemv(type, pro, epi, false, false, p, maps, pdl(), st);
+  };
   // a projection of the normalised residual: fused passes normalise while staging, others read xn16
   auto normed = [&](QGemvParams& p, const DTensor& gamma, __half* xn_copy) {
     if (!fused) return (int)PRO_F16;
@@ -309,7 +321,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (gemm_tile_rows(M, N) == 0) {
       QGemvParams q = base(w, K, N, x, K);
       q.y = y; q.ldy = ldy;
-      return launch_qgemv(w.type, PRO_F16, EPI_STORE, false, false, q, pdl(), st);
+      return project(w.type, PRO_F16, EPI_STORE, q);
     }
     WGemmMaps maps{};
     maps.w = wm; maps.x = xm;
@@ -322,7 +334,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     if (gemm_tile_rows(M, H) == 0) {
       QGemvParams q = base(w, K, H, x, K);
       q.y = h; q.ldy = H;
-      return launch_qgemv(w.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st);
+      return project(w.type, PRO_F16, EPI_RESID, q);
     }
     WGemmMaps maps{};
     maps.w = wm; maps.x = xm;
@@ -341,7 +353,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     QGemvParams p = base(L.eh_proj, 2 * H, H, xcat16, 2 * H);
     p.y = h; p.ldy = H;
     if (fused) { p.ss_out = ss_part; ss_n = (H + 15) / 16; }
-    B200_TRY(launch_qgemv(L.eh_proj.type, PRO_F16, EPI_STORE, false, false, p, pdl(), st));
+    B200_TRY(project(L.eh_proj.type, PRO_F16, EPI_STORE, p));
     if (!fused) B200_TRY(launch_row_tail(row_tail(1, L.attn_norm), pdl(), st));
   } else {
     const LayerW& L0 = m->layers[0];
@@ -364,7 +376,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         else B200_TRY(gemm(L.z, wmaps[l].z, H, vw, xn16, tx_xn[2], proj + cw, proj_ld));
       } else {
         const int pro = normed(p, L.attn_norm, xn16);  // the DeltaNet step reads the fp16 rows for alpha / beta
-        B200_TRY(launch_qgemv(L.qkv.type, pro, EPI_STORE, false, false, p, pdl(), st));
+        B200_TRY(project(L.qkv.type, pro, EPI_STORE, p));
       }
       DnStepParams d{};
       d.proj = proj; d.ldp = proj_ld; d.xn = xn16; d.alpha_w = (const float*)L.alpha.data; d.beta_w = (const float*)L.beta.data;
@@ -385,7 +397,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       if (fused) { q.ss_out = ss_part; ss_n = (H + 15) / 16; }
       if (dense_tg(L.ssm_out.type, M, H) && vw % 256 == 0) B200_TRY(tresid(L.ssm_out, wmaps[l].out.m[0], vw, y16, tx_y16, sx_y, ts_y16));
       else if (use_gemm) B200_TRY(gemm_resid(L.ssm_out, wmaps[l].out, vw, y16, tx_y16[2]));
-      else B200_TRY(launch_qgemv(L.ssm_out.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));
+      else B200_TRY(project(L.ssm_out.type, PRO_F16, EPI_RESID, q));
     } else {
       const int ai = attn_index[l];
       // fused q|k|v projection; tensors of one type share a launch
@@ -411,7 +423,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
         p.nseg = e - s; p.N = n;
         p.y = proj + off; p.ldy = proj_ld;
         const int pro = normed(p, L.attn_norm, nullptr);
-        B200_TRY(launch_qgemv(seg[s]->type, pro, EPI_STORE, false, false, p, pdl(), st));
+        B200_TRY(project(seg[s]->type, pro, EPI_STORE, p));
         off += n; s = e;
       }
       AttnParams a{};
@@ -441,7 +453,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       if (fused) { q.ss_out = ss_part; ss_n = (H + 15) / 16; }
       if (dense_tg(L.o.type, M, H) && qw % 256 == 0) B200_TRY(tresid(L.o, wmaps[l].o.m[0], qw, ctx16, tx_ctx, sx_ctx, ts_ctx));
       else if (use_gemm) B200_TRY(gemm_resid(L.o, wmaps[l].o, qw, ctx16, tx_ctx[2]));
-      else B200_TRY(launch_qgemv(L.o.type, PRO_F16, EPI_RESID, false, false, q, pdl(), st));
+      else B200_TRY(project(L.o.type, PRO_F16, EPI_RESID, q));
     }
     if (!fused) {
       TailParams t = row_tail(1, L.ffn_norm);
@@ -512,12 +524,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
       p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = ecx; p.M = Mg;
       p.y16 = act16; p.ldy = c.ffn_expert;
-      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, pdl(), st));
+      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, QGemvMaps{}, pdl(), st));
       QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
       q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
       q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = ecx; q.M = Mg;
       q.y = down; q.ldy = H;     // local: rows by pair id; the combine kernel carries them to the rows' owners
-      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, pdl(), st));
+      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, QGemvMaps{}, pdl(), st));
       }
       e.y_local = down; e.cols = cols; e.n_pairs = ep_epoch + 2; e.pairs_per_rank = M * slots1;
       B200_TRY(launch_ep_combine(e, M * slots1 + (Mg - M) * used, pdl(), st));
@@ -544,6 +556,11 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       MoeGateParams p{};
       p.route = r; p.K = H; p.N = c.ffn_expert; p.M = M; p.x = xn16; p.act = act16; p.err = err_flag; p.tl = tl();
       p.down = L.down_exps.data; p.down_sh = L.down_sh.data; p.down_bytes = (int64_t)H * L.down_exps.stride;
+      if (l + 1 < l1) {
+        const LayerW& X = m->layers[l + 1];
+        for (const DTensor* w : {&X.qkv, &X.z, &X.ssm_out, &X.q, &X.k, &X.v, &X.o, &X.router})
+          if (w->ok() && p.n_ahead < 6) { p.ahead[p.n_ahead] = w->data; p.ahead_bytes[p.n_ahead++] = w->rows * w->stride; }
+      }
       B200_TRY(launch_moe_gate(L.gate_exps.type, p, MoeGateMaps{W.gate, W.up, W.gate_sh, W.up_sh}, pdl(), st));
       MoeDownParams d{};
       d.K = c.ffn_expert; d.N = H; d.used = used; d.topk = topk; d.topk_w = topk_w; d.act = act16; d.h = h; d.ss_out = ss_part; d.err = err_flag; d.tl = tl();
@@ -554,12 +571,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       p.w2[0] = L.up_exps.data; p.ws = L.gate_sh.data; p.ws2 = L.up_sh.data; p.expert_stride = (int64_t)c.ffn_expert * L.gate_exps.stride;
       p.entries = entries; p.n_entries = n_entries; p.cols = cols; p.x_div = slots1; p.xcols = std::min(xcols, entry_cols(M, false));
       p.y16 = act16; p.ldy = c.ffn_expert;
-      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, pdl(), st));
+      B200_TRY(launch_qgemv(L.gate_exps.type, PRO_F16, EPI_SWIGLU, true, true, p, QGemvMaps{}, pdl(), st));
       QGemvParams q = base(L.down_exps, c.ffn_expert, H, act16, c.ffn_expert);
       q.ws = L.down_sh.data; q.expert_stride = (int64_t)H * L.down_exps.stride;
       q.entries = entries; q.n_entries = n_entries; q.cols = cols; q.x_div = 1; q.xcols = std::min(xcols, entry_cols(M, false));
       q.y = down; q.ldy = H;
-      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, pdl(), st));
+      B200_TRY(launch_qgemv(L.down_exps.type, PRO_F16, EPI_STORE, false, true, q, QGemvMaps{}, pdl(), st));
     }
     if (!r.defer) {
       const DTensor& next_norm = f.draft ? L.head_norm : (l + 1 < c.n_layer ? m->layers[l + 1].attn_norm : m->output_norm);
@@ -586,7 +603,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       B200_TRY(gemm(m->output, head_map, H, N, xn16, tx_xn[2], logits, N));
     } else {
       const int pro = normed(p, nrm, nullptr);
-      B200_TRY(launch_qgemv(m->output.type, pro, EPI_STORE, false, false, p, pdl(), st));
+      B200_TRY(project(m->output.type, pro, EPI_STORE, p));
     }
     if (f.greedy) {
       B200_TRY(launch_argmax(logits, n_logit_rows, N, next_ids, pdl(), st));

@@ -42,6 +42,7 @@ struct Graph {
     WMap wgate, wup, wdown, wgate_sh, wup_sh, wdown_sh, qkv, z, out, q, k, v, o, router;   // boxes of 64 (gate, up) and 128 rows
   };
   std::vector<LayerMaps> wmaps;
+  std::map<const uint8_t*, TMap> row_maps;   // by weight: the maps of the projections of at most eight rows
   WMap head_map{};
   TMap tx_xperm{}, tx_act{};   // expert-sorted rows and their activations, boxes of 64 rows
   TMap tx_xn[3], ts_xn[3], tx_y16[3], ts_y16[3], tx_ctx[3], ts_ctx[3];   // activation rows and their sums, boxes of 16 / 32 / 64 rows

@@ -678,7 +678,10 @@ __device__ __forceinline__ void warp_sum8(float (&v)[8]) {
 }
 
 // (Passes of 16 sequences and more use dn_head_kernel below instead.)
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128, 5) dn_step_kernel(DnStepParams p) {
+// OCC: CTAs per SM it is compiled for. One or two sequences leave an SM two CTAs at most, and everything that is fetched before the
+// wait stays in registers; from three on, five to an SM keep a pass in one wave (18 us against 10 for five sequences).
+template <int OCC>
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(128, OCC) dn_step_kernel(DnStepParams p) {
   cg::cluster_group cluster = cg::this_cluster();
   const int D = 128, RB = 4;
   const int h = blockIdx.x / RB, rb = blockIdx.x % RB, hk = h % p.Hk;
@@ -1606,7 +1609,8 @@ int launch_dn_step(const DnStepParams& p, bool pdl, cudaStream_t st) {
   if (p.D != 128 || p.conv != 4) { set_error("dn_step: head dim must be 128 and conv kernel 4"); return EINVAL_; }
   // (passes of at most 8 sequences stay on dn_step_kernel: they give every row the single-row pass's bits)
   if (p.n_seq >= 16) return launch_k(dn_head_kernel, dim3(p.Hv, p.n_seq), dim3(512), 0, pdl, st, p);
-  return launch_k(dn_step_kernel, dim3(p.Hv * 4, p.n_seq), dim3(128), 0, pdl, st, p);
+  if (p.n_seq > 2) return launch_k(dn_step_kernel<5>, dim3(p.Hv * 4, p.n_seq), dim3(128), 0, pdl, st, p);
+  return launch_k(dn_step_kernel<1>, dim3(p.Hv * 4, p.n_seq), dim3(128), 0, pdl, st, p);
 }
 
 // =========================================================================================

@@ -37,7 +37,9 @@ struct EmbedParams {
 int launch_embed(const EmbedParams& p, cudaStream_t st);
 
 // K-quant projections; `pdl` marks the launch as a programmatic dependent of the previous kernel.
-int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st);
+int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, const QGemvMaps& maps, bool pdl, cudaStream_t st);
+// the tensor map a plain launch wants for a row segment of `type` (left alone for types that are copied by tile)
+int make_qgemv_map(uint32_t type, const uint8_t* w, int64_t rows, int64_t stride, TMap* out);
 int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st);
 int launch_concat_norm(const float* e, const float* hs, const float* enorm, const float* hnorm, float eps, int H, int M, __half* xcat, bool pdl, cudaStream_t st);
 

@@ -68,6 +68,12 @@ __global__ void __launch_bounds__(256, 3) moe_gate_kernel(const __grid_constant_
     const uint8_t* d = (ex >= 0 ? p.down + ex * p.down_bytes : p.down_sh) + blockIdx.x * share;
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(d), "r"((uint32_t)share) : "memory");
   }
+  // and of the next layer's dense weights: the chain of latencies leaves memory idle, and whoever needs them next finds them in L2
+  if (warp == 1 && lane < p.n_ahead) {
+    const int64_t n = (int64_t)gridDim.x * gridDim.y, c = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, units = p.ahead_bytes[lane] / 16;
+    const int64_t from = units * c / n, to = units * (c + 1) / n;
+    if (to > from) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.ahead[lane] + from * 16), "r"((uint32_t)((to - from) * 16)) : "memory");
+  }
   tl_mark(p.tl, 2);
   int phase = 0, buf = 0;
   const uint32_t ra = (uint32_t)__cvta_generic_to_shared(raw) + 2 * g * BLK;

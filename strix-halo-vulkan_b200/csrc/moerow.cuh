@@ -13,6 +13,9 @@ struct MoeGateParams {
   __half* act;              // [M][used + 1][N]
   const uint8_t *down, *down_sh;   // the down projection's weights, brought to L2 on the way: [expert][down_bytes]
   int64_t down_bytes;       // of one expert
+  const uint8_t* ahead[6];  // the next layer's dense weights, likewise
+  int64_t ahead_bytes[6];
+  int n_ahead;
   int* err;
   Timeline tl;
 };

@@ -6,7 +6,7 @@ namespace b200 {
 
 // The grid of a launch over a work list is the device's resident CTAs, which share the list evenly whatever its length.
 template <int TYPE, int PRO, int EPI, bool DUAL, bool GROUPED>
-static int launch_one(const QGemvParams& p, bool pdl, cudaStream_t st) {
+static int launch_one(const QGemvParams& p, const QGemvMaps& maps, bool pdl, cudaStream_t st) {
   auto kernel = qgemv_kernel<TYPE, PRO, EPI, DUAL, GROUPED>;
   const int g_sm_count = sm_count_current();
   if (g_sm_count <= 0) return ECUDA;
@@ -21,7 +21,7 @@ static int launch_one(const QGemvParams& p, bool pdl, cudaStream_t st) {
   // grid that fits at once needs no second round. Three per SM only for the expert kernels and the Q6_K ones (the head's long walk): elsewhere the register cap costs more than
   // the extra warps give, and every CTA of a projection reads the same activation rows out of L2 - the more
   // CTAs ask at once the longer each waits. Persistent CTAs share the device between the y / z slices.
-  const size_t fixed = qg_fixed_smem(p.K, p.xcols, DUAL), stage = qg_stage_bytes(p.K, qg_pitch(TYPE, p.stride), DUAL);
+  const size_t fixed = qg_fixed_smem(p.K, p.xcols, DUAL), stage = qg_stage_bytes(p.K, qg_pitch(TYPE, p.stride, GROUPED), DUAL);
   const size_t budgets[4] = {0, QG_SMEM_MAX, 110 * 1024, 72 * 1024};
   if (fixed + stage > budgets[1]) { set_error("qgemv: row length too large for shared memory"); return ECAPACITY; }
   int occ = 1, rounds = 1, gx = 1, ns = 1;
@@ -61,33 +61,37 @@ static int launch_one(const QGemvParams& p, bool pdl, cudaStream_t st) {
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = pdl ? 1 : 0;
-  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, pp));
+  B200_CUDA(cudaLaunchKernelEx(&cfg, kernel, maps, pp));
   return OK;
 }
 
 template <int TYPE>
-static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st) {
+static int launch_type(int pro, int epi, bool dual, bool grouped, const QGemvParams& p, const QGemvMaps& maps, bool pdl, cudaStream_t st) {
   if (!grouped && !dual) {
-    if (pro == PRO_NORM && epi == EPI_STORE) return launch_one<TYPE, PRO_NORM, EPI_STORE, false, false>(p, pdl, st);
-    if (pro == PRO_F16 && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, false>(p, pdl, st);
-    if (pro == PRO_F16 && epi == EPI_RESID) return launch_one<TYPE, PRO_F16, EPI_RESID, false, false>(p, pdl, st);
+    if (pro == PRO_NORM && epi == EPI_STORE) return launch_one<TYPE, PRO_NORM, EPI_STORE, false, false>(p, maps, pdl, st);
+    if (pro == PRO_F16 && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, false>(p, maps, pdl, st);
+    if (pro == PRO_F16 && epi == EPI_RESID) return launch_one<TYPE, PRO_F16, EPI_RESID, false, false>(p, maps, pdl, st);
   } else if (grouped && pro == PRO_F16) {
-    if (dual && epi == EPI_SWIGLU) return launch_one<TYPE, PRO_F16, EPI_SWIGLU, true, true>(p, pdl, st);
-    if (!dual && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, true>(p, pdl, st);
+    if (dual && epi == EPI_SWIGLU) return launch_one<TYPE, PRO_F16, EPI_SWIGLU, true, true>(p, maps, pdl, st);
+    if (!dual && epi == EPI_STORE) return launch_one<TYPE, PRO_F16, EPI_STORE, false, true>(p, maps, pdl, st);
   }
   set_error("qgemv: this prologue / epilogue combination is not built");
   return EINVAL_;
 }
 
-int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, bool pdl, cudaStream_t st) {
+int make_qgemv_map(uint32_t type, const uint8_t* w, int64_t rows, int64_t stride, TMap* out) { return qg_boxed(type, false) ? make_w_tensor_map(type, w, rows, stride, 16, out) : (int)OK; }
+
+int launch_qgemv(uint32_t type, int pro, int epi, bool dual, bool grouped, const QGemvParams& p, const QGemvMaps& maps, bool pdl, cudaStream_t st) {
   if (p.K % 256 != 0 || p.K <= 0) { set_error("qgemv: row length must be a multiple of 256"); return EINVAL_; }
   if (p.xcols < 1 || p.xcols > QG_MAXCOLS) { set_error("qgemv: xcols out of range"); return EINVAL_; }
   if (p.ss_out != nullptr && (p.N + 15) / 16 > SS_LD) { set_error("qgemv: more tiles than partial-sum slots"); return ECAPACITY; }
   if (pro == PRO_NORM && (p.ss_n < 1 || p.ss_n > SS_LD)) { set_error("qgemv: bad partial-sum count"); return EINVAL_; }
+  for (int i = 0; i + 1 < p.nseg; i++)
+    if (!grouped && p.seg_end[i] % 16 != 0) { set_error("qgemv: row segments end on whole tiles"); return EINVAL_; }
   switch (type) {
-    case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, pdl, st);
-    case T_Q5_K: return launch_type<T_Q5_K>(pro, epi, dual, grouped, p, pdl, st);
-    case T_Q6_K: return launch_type<T_Q6_K>(pro, epi, dual, grouped, p, pdl, st);
+    case T_Q4_K: return launch_type<T_Q4_K>(pro, epi, dual, grouped, p, maps, pdl, st);
+    case T_Q5_K: return launch_type<T_Q5_K>(pro, epi, dual, grouped, p, maps, pdl, st);
+    case T_Q6_K: return launch_type<T_Q6_K>(pro, epi, dual, grouped, p, maps, pdl, st);
   }
   set_error("qgemv: weight type has no fused projection kernel (Q4_K, Q5_K, Q6_K only)");
   return EINVAL_;

@@ -79,6 +79,11 @@ struct QGemvParams {
   __half* y16;               // SWIGLU: half [.][ldy]
 };
 
+// Q4_K and Q5_K, plain mode: tensor maps of the row segments, boxes of 16 rows x one super-block (make_w_tensor_map)
+struct QGemvMaps { TMap w[4]; };
+// whether a launch reads its weights through QGemvMaps
+__host__ __device__ constexpr bool qg_boxed(uint32_t type, bool grouped) { return !grouped && (type == T_Q4_K || type == T_Q5_K); }
+
 __host__ __device__ inline int qg_xstride(int K) {
   int base = 2 * K + 16 * (K / 64);
   int pad = (64 - base % 128 + 128) % 128;
@@ -87,7 +92,7 @@ __host__ __device__ inline int qg_xstride(int K) {
 constexpr int QG_MAX_STAGES = 8;
 constexpr size_t QG_SMEM_MAX = 222 * 1024;   // dynamic shared memory of a CTA that has its SM alone
 // pitch of a weight row in shared memory (see mma_row), and bytes of one pipeline stage: the tiles one CTA works on per iteration
-__host__ __device__ inline int64_t qg_pitch(uint32_t type, int64_t stride) { return type == T_Q6_K ? stride : stride + 16; }
+__host__ __device__ inline int64_t qg_pitch(uint32_t type, int64_t stride, bool grouped) { return type != T_Q6_K && grouped ? stride + 16 : stride; }
 __host__ __device__ inline size_t qg_stage_bytes(int K, int64_t stride, bool dual) {
   const int nb = K / 256;
   const int wpt = nb >= 8 ? 8 : nb >= 4 ? 4 : nb >= 2 ? 2 : 1;
@@ -295,9 +300,10 @@ __device__ __forceinline__ void q6_accumulate(float (&acc)[4], const Q6KRow& r0,
   acc[3] = fmaf(d1, C[3], acc[3]);
 }
 
-// The tile row that mma row g (second = false) or g + 8 stands for. Q4_K and Q5_K rows are read in eight-byte pieces at a pitch of
-// their length + 16: with mma row g on row 2g, g + 8 on 2g + 1, the reads of a warp fall on distinct banks.
+// The tile row that mma row g (second = false) or g + 8 stands for. Q4_K and Q5_K rows are read in eight-byte pieces at a pitch of a
+// block (144 or 176 bytes) or of the row's length + 16: with mma row g on row 2g, g + 8 on 2g + 1, a warp's reads fall on distinct banks.
 template <int TYPE> __device__ __forceinline__ int mma_row(int g, bool second) { return TYPE == T_Q6_K ? g + (second ? 8 : 0) : 2 * g + (second ? 1 : 0); }
+// row0, row1: the rows' blocks `blk` (Q4_K, Q5_K), or the rows (Q6_K, whose blocks are spread over planes)
 template <int TYPE>
 __device__ __forceinline__ void block_accumulate(float (&acc)[4], const uint8_t* row0, const uint8_t* row1, const uint8_t* xrow, const __half* sxrow, bool live, int nb, int blk, int t) {
   if constexpr (TYPE == T_Q6_K) {
@@ -306,10 +312,9 @@ __device__ __forceinline__ void block_accumulate(float (&acc)[4], const uint8_t*
     q6k_issue(a1, row1, nb, blk, t);
     q6_accumulate(acc, a0, a1, xrow, live, blk, t);
   } else {   // a column past the last repeats the first: its results are not stored
-    constexpr int BLK = TYPE == T_Q4_K ? 144 : 176;
     const __half* sp = sxrow + blk * 8 + 2 * (t >> 1);
-    k45_accumulate<TYPE>(acc, (uint32_t)__cvta_generic_to_shared(row0 + (size_t)blk * BLK), (uint32_t)__cvta_generic_to_shared(row1 + (size_t)blk * BLK), xrow + 576 * blk,
-                         *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
+    k45_accumulate<TYPE>(acc, (uint32_t)__cvta_generic_to_shared(row0), (uint32_t)__cvta_generic_to_shared(row1), xrow + 576 * blk, *reinterpret_cast<const uint32_t*>(sp),
+                         *reinterpret_cast<const uint32_t*>(sp + 4), t);
   }
 }
 
@@ -483,7 +488,7 @@ __device__ __forceinline__ void stage_x_norm(const QGemvParams& p, uint8_t* xs, 
 // checkpoint's own blocks) through cp.async.bulk into a ring of shared-memory stages, each
 // completing on its mbarrier, so many tiles are in flight per SM without holding registers.
 template <int TYPE, int PRO, int EPI, bool DUAL, bool GROUPED>
-__global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 2) qgemv_kernel(const QGemvParams p) {
+__global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 2) qgemv_kernel(const __grid_constant__ QGemvMaps maps, const QGemvParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int K = p.K, nb = K / 256;
@@ -494,23 +499,31 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   __half* sxs = reinterpret_cast<__half*>(smem + (size_t)p.xcols * xstride);
   float* red = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(sxs) + (((size_t)p.xcols * (K / 32) * 2 * sizeof(__half) + 15) & ~(size_t)15));
   uint8_t* stages = smem + qg_fixed_smem(K, p.xcols, DUAL);
-  const size_t pitch = (size_t)qg_pitch(TYPE, p.stride), tile_bytes = 16 * pitch;
+  constexpr bool BOXED = qg_boxed(TYPE, GROUPED);
+  constexpr int BLK = TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : 0;   // bytes of a super-block where a row's lie side by side
+  const size_t pitch = (size_t)qg_pitch(TYPE, p.stride, GROUPED), tile_bytes = 16 * pitch;
   const size_t stage_bytes = (size_t)tpc * tile_bytes * (DUAL ? 2 : 1);
   const int NS = p.nstage;
   __shared__ float scratch[4 * QG_WARPS];
   __shared__ int col_rows[QG_MAXCOLS], xrows[QG_MAXCOLS];
-  __shared__ __align__(8) uint64_t full_bar[QG_MAX_STAGES];
+  __shared__ __align__(8) uint64_t full_bar[BOXED ? QG_WARPS : 1][QG_MAX_STAGES];
 
   const int tiles = (p.N + 15) / 16;
   const int ngroups = (tiles + tpc - 1) / tpc;
   const int lt = warp / wpt, kslice = warp % wpt;
 
   tl_mark(p.tl, 0);
-  if (tid == 0) {
-    for (int s = 0; s < NS; s++) mbar_init(&full_bar[s], 1);
-    mbar_fence_init();
+  if constexpr (BOXED) {
+    if (lane < NS) mbar_init(&full_bar[warp][lane], 1);
+    if (lane == 0) mbar_fence_init();
+    __syncwarp();
+  } else {
+    if (tid == 0) {
+      for (int s = 0; s < NS; s++) mbar_init(&full_bar[0][s], 1);
+      mbar_fence_init();
+    }
+    __syncthreads();
   }
-  __syncthreads();
 
   // What this CTA walks is a sequence of units, each one row-tile group of one weight matrix. Plain launches take the groups blockIdx.x, blockIdx.x + gridDim.x, ... of the one matrix they
   // are given. Launches over a work list cut the whole list, entries * groups units, into one contiguous run per CTA:
@@ -529,7 +542,21 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     col_off = (int)blockIdx.z * QG_MAXCOLS;
     n_units = (int)blockIdx.x < ngroups ? (ngroups - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
   }
-  // warp 0 is the producer: one bulk copy per tile row, or per tile where rows lie as in memory
+  // BOXED: each warp brings its own super-blocks of its own tile, 16 x 256 weights to a box at a pitch of a block, and refills them
+  // alone. Else warp 0 is the producer: one bulk copy per tile row, or per tile where rows lie as in memory.
+  auto issue_boxes = [&](int it) {
+    const int tile = ((int)blockIdx.x + it * (int)gridDim.x) * tpc + lt, s = it % NS;
+    if (tile >= tiles || kslice >= nb) return;
+    if (elect_one()) {
+      int sg = 0;
+      while (sg + 1 < p.nseg && tile * 16 >= p.seg_end[sg]) sg++;
+      const int r = tile * 16 - (sg > 0 ? p.seg_end[sg - 1] : 0);
+      uint8_t* dst = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes;
+      mbar_expect_tx(&full_bar[BOXED ? warp : 0][s], (uint32_t)((nb - kslice + wpt - 1) / wpt * 16 * BLK));
+      for (int blk = kslice; blk < nb; blk += wpt) tma_box_2d(dst + blk * (16 * BLK), &maps.w[sg], blk * BLK, r, &full_bar[BOXED ? warp : 0][s]);
+    }
+    __syncwarp();
+  };
   auto issue_group = [&](int grp, int s, const uint8_t* ga, const uint8_t* gb) {
     if (lane == 0) {
       uint32_t total = 0;
@@ -537,7 +564,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
         const int tile = grp * tpc + l;
         if (tile < tiles) total += (uint32_t)(min(16, p.N - tile * 16) * p.stride) * (DUAL ? 2 : 1);
       }
-      mbar_expect_tx(&full_bar[s], total);
+      mbar_expect_tx(&full_bar[0][s], total);
     }
     __syncwarp();
     for (int l = 0; l < tpc; l++) {
@@ -557,12 +584,12 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       const int64_t off = (int64_t)(tile * 16 - seg_r0) * p.stride;
       if constexpr (TYPE == T_Q6_K) {
         if (lane == 0) {
-          bulk_copy_g2s(dst, base + off, (uint32_t)(nrows * p.stride), &full_bar[s]);
-          if constexpr (DUAL) bulk_copy_g2s(dst + tile_bytes, base2 + off, (uint32_t)(nrows * p.stride), &full_bar[s]);
+          bulk_copy_g2s(dst, base + off, (uint32_t)(nrows * p.stride), &full_bar[0][s]);
+          if constexpr (DUAL) bulk_copy_g2s(dst + tile_bytes, base2 + off, (uint32_t)(nrows * p.stride), &full_bar[0][s]);
         }
       } else {
         const int r = lane & 15;
-        if (r < nrows && lane < (DUAL ? 32 : 16)) bulk_copy_g2s(dst + (lane >> 4) * tile_bytes + r * pitch, (lane < 16 ? base : base2) + off + r * p.stride, (uint32_t)p.stride, &full_bar[s]);
+        if (r < nrows && lane < (DUAL ? 32 : 16)) bulk_copy_g2s(dst + (lane >> 4) * tile_bytes + r * pitch, (lane < 16 ? base : base2) + off + r * p.stride, (uint32_t)p.stride, &full_bar[0][s]);
       }
     }
   };
@@ -580,8 +607,11 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       issue_group((int)blockIdx.x + j * (int)gridDim.x, j % NS, nullptr, nullptr);
     }
   };
-  if (warp == 0)
+  if constexpr (BOXED) {
+    for (int k = 0; k < NS && k < n_units; k++) issue_boxes(k);
+  } else if (warp == 0) {
     for (int k = 0; k < NS && k < n_units; k++) issue_unit(k);
+  }
   if constexpr (!GROUPED) pdl_wait();
   pdl_launch();
   tl_mark(p.tl, 1);
@@ -631,20 +661,35 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     };
     for (int u = 0; u < cnt; u++) {
       const int it = it0 + u, s = it % NS;
-      if (!mbar_wait(&full_bar[s], (uint32_t)((it / NS) & 1))) {
-        if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report and leave
-        return;
-      }
-      if (it == 0) tl_mark(p.tl, 3);
-      float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
       const int tile = group_of(it) * tpc + lt;
-      if (tile < tiles) {
-        const int nrows = min(16, p.N - tile * 16);
-        const uint8_t* tb = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes * (DUAL ? 2 : 1);
-        const uint8_t *row0 = tb + min(mma_row<TYPE>(g, false), nrows - 1) * pitch, *row1 = tb + min(mma_row<TYPE>(g, true), nrows - 1) * pitch;
-        for (int blk = kslice; blk < nb; blk += wpt) {
-          block_accumulate<TYPE>(acc, row0, row1, xrow, sxrow, live, nb, blk, t);
-          if constexpr (DUAL) block_accumulate<TYPE>(acc2, row0 + tile_bytes, row1 + tile_bytes, xrow, sxrow, live, nb, blk, t);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
+      if constexpr (BOXED) {
+        if (tile < tiles && kslice < nb) {
+          if (!warp_wait(&full_bar[BOXED ? warp : 0][s], (uint32_t)((it / NS) & 1))) {   // a copy never landed: report, the results are void
+            if (p.err != nullptr && lane == 0) atomicExch(p.err, 1);
+          } else {
+            if (it == 0) tl_mark(p.tl, 3);
+            const uint8_t* row0 = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes + 2 * g * BLK;
+            for (int blk = kslice; blk < nb; blk += wpt) block_accumulate<TYPE>(acc, row0 + blk * (16 * BLK), row0 + blk * (16 * BLK) + BLK, xrow, sxrow, live, nb, blk, t);
+          }
+          __syncwarp();
+          if (it + NS < n_units) { fence_proxy_async(); issue_boxes(it + NS); }
+        }
+      } else {
+        if (!mbar_wait(&full_bar[0][s], (uint32_t)((it / NS) & 1))) {
+          if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report and leave
+          return;
+        }
+        if (it == 0) tl_mark(p.tl, 3);
+        if (tile < tiles) {
+          const int nrows = min(16, p.N - tile * 16);
+          const uint8_t* tb = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes * (DUAL ? 2 : 1);
+          const uint8_t *row0 = tb + min(mma_row<TYPE>(g, false), nrows - 1) * pitch, *row1 = tb + min(mma_row<TYPE>(g, true), nrows - 1) * pitch;
+          for (int blk = kslice; blk < nb; blk += wpt) {
+            const int off = blk * BLK;
+            block_accumulate<TYPE>(acc, row0 + off, row1 + off, xrow, sxrow, live, nb, blk, t);
+            if constexpr (DUAL) block_accumulate<TYPE>(acc2, row0 + tile_bytes + off, row1 + tile_bytes + off, xrow, sxrow, live, nb, blk, t);
+          }
         }
       }
       auto leave = [&](float* my, const float (&a)[4]) {
@@ -657,9 +702,11 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
     }
     __syncthreads();
     // every warp is done with these stages: refill them with the units NS iterations ahead
-    if (warp == 0)
-      for (int u = 0; u < cnt; u++)
-        if (it0 + u + NS < n_units) { fence_proxy_async(); issue_unit(it0 + u + NS); }
+    if constexpr (!BOXED) {
+      if (warp == 0)
+        for (int u = 0; u < cnt; u++)
+          if (it0 + u + NS < n_units) { fence_proxy_async(); issue_unit(it0 + u + NS); }
+    }
     // sixteen threads per (unit, tile, column), one row each
     const int r = tid & 15, sets = cnt * tpc, inv = 65535 / sets + 1;
     for (int q = tid >> 4; q < sets * ncols; q += QG_THREADS / 16) {

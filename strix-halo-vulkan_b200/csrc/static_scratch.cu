@@ -43,7 +43,7 @@ static int scratch_for_current_device(StaticScratch* out) {
 // Shared memory the projection kernel needs for m staged rows of length k plus one stage of weight
 // tiles; the launch is refused when it exceeds what an SM offers (the same sum launch_qgemv checks).
 static size_t static_smem_need(uint32_t type, int64_t k, int m) {
-  return qg_fixed_smem((int)k, m, false) + qg_stage_bytes((int)k, qg_pitch(type, device_row_stride(type, k)), false);
+  return qg_fixed_smem((int)k, m, false) + qg_stage_bytes((int)k, qg_pitch(type, device_row_stride(type, k), false), false);
 }
 constexpr size_t STATIC_SMEM_BUDGET = QG_SMEM_MAX;
 
@@ -69,7 +69,9 @@ int qgemv_static(uint32_t type, const void* dev_w, int64_t rows, int64_t k, cons
   QGemvParams p{};
   p.w[0] = (const uint8_t*)dev_w; p.seg_end[0] = (int)rows; p.nseg = 1; p.stride = device_row_stride(type, k);
   p.K = (int)k; p.N = (int)rows; p.M = m; p.xcols = m; p.x = sc.x16; p.ldx = k; p.y = dev_y; p.ldy = rows; p.x_div = 1; p.err = sc.err;
-  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, false, 0));
+  QGemvMaps maps{};
+  B200_TRY(make_qgemv_map(type, p.w[0], rows, p.stride, &maps.w[0]));
+  B200_TRY(launch_qgemv(type, PRO_F16, EPI_STORE, false, false, p, maps, false, 0));
   int herr = 0;
   B200_CUDA(cudaMemcpy(&herr, sc.err, sizeof(int), cudaMemcpyDeviceToHost));  // also waits for the work
   if (herr != 0) { set_error("qgemv_static: a bounded wait for the weight copies gave up; dev_y is not valid"); return ETIMEOUT; }
