@@ -15,6 +15,8 @@ namespace {
 template <int TYPE> __host__ __device__ constexpr int mr_blk() { return TYPE == T_Q4_K ? 144 : 176; }
 template <int TYPE> __host__ __device__ constexpr int mr_raw() { return 16 * mr_blk<TYPE>(); }
 
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) { asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory"); }
+
 int slices(int nb) { return nb >= 8 ? 8 : nb >= 4 ? 4 : nb >= 2 ? 2 : 1; }   // warps that share a tile's contraction
 
 // A CTA serves one (row, slot): blockIdx.y. Its eight warps share out tiles of 16 gate + 16 up rows, `slices` warps to a tile, one
@@ -62,18 +64,19 @@ __global__ void __launch_bounds__(256, 3) moe_gate_kernel(const __grid_constant_
   };
   const int step = tpc * gridDim.x, tile0 = blockIdx.x * tpc + lt;
   if (tile0 < tiles && bpt > 0) fetch(tile0, 0);
-  // this CTA's share of the slot's down weights on their way to L2 for the next kernel
-  if (tid == 0 && p.down != nullptr) {
-    const int64_t share = p.down_bytes / gridDim.x & ~(int64_t)15;
-    const uint8_t* d = (ex >= 0 ? p.down + ex * p.down_bytes : p.down_sh) + blockIdx.x * share;
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(d), "r"((uint32_t)share) : "memory");
-  }
-  // and of the next layer's dense weights: the chain of latencies leaves memory idle, and whoever needs them next finds them in L2
-  if (warp == 1 && lane < p.n_ahead) {
-    const int64_t n = (int64_t)gridDim.x * gridDim.y, c = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, units = p.ahead_bytes[lane] / 16;
-    const int64_t from = units * c / n, to = units * (c + 1) / n;
-    if (to > from) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.ahead[lane] + from * 16), "r"((uint32_t)((to - from) * 16)) : "memory");
-  }
+  // Once this CTA's first weights are here: its share of the slot's down weights, and of the next layer's dense weights, on their way
+  // to L2. The chain of latencies leaves memory idle, and the kernels that need them next find them there.
+  auto bring = [&]() {
+    if (warp == 0 && lane == 0) {
+      const int64_t share = p.down_bytes / gridDim.x & ~(int64_t)15;
+      prefetch_l2((ex >= 0 ? p.down + ex * p.down_bytes : p.down_sh) + blockIdx.x * share, (uint32_t)share);
+    }
+    if (warp == 1 && lane < p.n_ahead) {
+      const int64_t n = (int64_t)gridDim.x * gridDim.y, c = (int64_t)blockIdx.y * gridDim.x + blockIdx.x, units = p.ahead_bytes[lane] / 16;
+      const int64_t from = units * c / n, to = units * (c + 1) / n;
+      if (to > from) prefetch_l2(p.ahead[lane] + from * 16, (uint32_t)((to - from) * 16));
+    }
+  };
   tl_mark(p.tl, 2);
   int phase = 0, buf = 0;
   const uint32_t ra = (uint32_t)__cvta_generic_to_shared(raw) + 2 * g * BLK;
@@ -95,6 +98,7 @@ __global__ void __launch_bounds__(256, 3) moe_gate_kernel(const __grid_constant_
         if (more || tile + step < tiles) { fence_proxy_async(); fetch(more ? tile : tile + step, more ? b + 1 : 0); }
       }
     }
+    if (base == (int)blockIdx.x * tpc) bring();
     if (t == 0) {   // every column holds the one activation row
 #pragma unroll
       for (int m = 0; m < 2; m++) *reinterpret_cast<float2*>(&red[buf][m][warp][2 * g]) = make_float2(acc[m][0], acc[m][2]);
