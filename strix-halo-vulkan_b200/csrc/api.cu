@@ -60,6 +60,10 @@ struct HostPool {
     size_of[p] = want;
     return p;
   }
+  bool owns(const void* p) {
+    std::lock_guard<std::mutex> lock(mu);
+    return size_of.count(const_cast<void*>(p)) != 0;
+  }
   void release(void* p) {
     std::lock_guard<std::mutex> lock(mu);
     auto it = size_of.find(p);
@@ -171,6 +175,7 @@ int32_t b200_graph_set_outputs(b200_graph* g, float* logits, int64_t logit_float
   if (!g) { set_error("set_outputs: null argument"); return EINVAL_; }
   g->g.out_logits = logits; g->g.out_logits_cap = logits ? logit_floats : 0;
   g->g.out_resid = residual; g->g.out_resid_cap = residual ? residual_floats : 0;
+  g->g.out_logits_mapped = logits && host_pool().owns(logits); g->g.out_resid_mapped = residual && host_pool().owns(residual);
   return OK;
 }
 int32_t b200_graph_forward(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {

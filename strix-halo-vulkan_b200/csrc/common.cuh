@@ -85,6 +85,10 @@ struct Timeline {
 };
 
 #ifdef __CUDACC__
+// A kernel's error report. The word may lie in mapped host memory (a graph's does: no copy brings it back), so it is a plain store.
+__device__ __forceinline__ void report_error(int* err, int code = 1) {
+  if (err != nullptr) { *reinterpret_cast<volatile int*>(err) = code; __threadfence_system(); }
+}
 __device__ __forceinline__ void tl_mark(const Timeline& t, int phase, bool any_block = false) {
   if (t.buf != nullptr && threadIdx.x == 0 && (any_block || (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0))) {
     long long v;

@@ -28,7 +28,7 @@ __device__ bool wait_flag(const int* flag, int want, long long limit_ns, int* er
   const long long t0 = global_ns();
   for (;;) {
     if (ld_acquire_sys(flag) >= want) return true;
-    if (global_ns() - t0 > limit_ns) { atomicExch(err, 2); return false; }
+    if (global_ns() - t0 > limit_ns) { report_error(err, 2); return false; }
     __nanosleep(40);
   }
 }

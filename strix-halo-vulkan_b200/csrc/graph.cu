@@ -37,13 +37,14 @@ Graph::~Graph() {
   if (logits_host) cudaFreeHost(logits_host);
   if (resid_host) cudaFreeHost(resid_host);
   if (hidden_host) cudaFreeHost(hidden_host);
-  if (err_host) cudaFreeHost(err_host);
+  if (err_flag) cudaFreeHost(err_flag);
   if (ids_host) cudaFreeHost(ids_host);
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (st) cudaStreamDestroy(st);
 }
 
+constexpr size_t STAGE_HEAD = 64;   // PassOut in front of a pass's staged inputs
 int Graph::init(Model* model, const b200_graph_opts& opts) {
   m = model; o = opts;
   if (!m->finalized) { set_error("graph: model is not finalized"); return ESTATE; }
@@ -84,14 +85,14 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   B200_TRY(dalloc(&r_logits, (size_t)MR * c.n_expert));
   B200_TRY(dalloc(&topk, (size_t)MR * used)); B200_TRY(dalloc(&topk_w, (size_t)MR * slots1)); B200_TRY(dalloc(&margin, (size_t)MR));
   B200_TRY(dalloc(&entries, (size_t)max_entries)); B200_TRY(dalloc(&n_entries, 1)); B200_TRY(dalloc(&cols, (size_t)MR * slots1));
-  B200_TRY(dalloc(&r_ticket, (size_t)2 + MR / 8)); B200_TRY(dalloc(&err_flag, 1)); B200_TRY(dalloc(&ss_part, (size_t)MR * SS_LD)); B200_TRY(dalloc(&y16, (size_t)MR * vw));
+  B200_TRY(dalloc(&r_ticket, (size_t)2 + MR / 8)); B200_TRY(dalloc(&ss_part, (size_t)MR * SS_LD)); B200_TRY(dalloc(&y16, (size_t)MR * vw));
   B200_TRY(dalloc(&act16, (size_t)MR * slots1 * c.ffn_expert)); B200_TRY(dalloc(&down, (size_t)MR * slots1 * H));
   B200_TRY(dalloc(&logits, (size_t)LR * c.vocab));
   { B200_TRY(dalloc(&dn_pre, (size_t)MR * ((size_t)c.dn_heads_k * 256 + (size_t)c.dn_heads_v * 130))); B200_TRY(dalloc(&dn_wy, (size_t)MR * c.dn_heads_v * 192, false)); B200_TRY(dalloc(&dn_oraw, (size_t)MR * vw)); B200_TRY(dalloc(&dn_ab, (size_t)MR * 2 * c.dn_heads_v)); }
   B200_TRY(dalloc(&xperm16, (size_t)MR * slots1 * H)); B200_TRY(dalloc(&gprob, (size_t)c.n_expert + 1));
   B200_TRY(make_rows_map(xperm16, (int64_t)MR * slots1, H, 64, &tx_xperm));
   if (c.ffn_expert % 64 == 0) B200_TRY(make_rows_map(act16, (int64_t)MR * slots1, c.ffn_expert, 64, &tx_act));
-  const size_t stage_bytes = ((size_t)MR + 31) / 32 * 32 * (4 * sizeof(int32_t) + sizeof(SeqDesc));
+  const size_t stage_bytes = STAGE_HEAD + ((size_t)MR + 31) / 32 * 32 * (4 * sizeof(int32_t) + sizeof(SeqDesc));
   B200_TRY(dalloc(&stage_dev, stage_bytes)); B200_TRY(dalloc(&next_ids, (size_t)MR));
   B200_TRY(dalloc(&hist_len, 1));
   B200_TRY(dalloc(&distinct_dev, 1));
@@ -148,8 +149,8 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   resid_host_cap = (int64_t)std::min(MR, 16) * H;
   B200_CUDA(cudaMallocHost((void**)&resid_host, (size_t)resid_host_cap * sizeof(float)));
   B200_CUDA(cudaMallocHost((void**)&hidden_host, (size_t)H * sizeof(float)));
-  B200_CUDA(cudaMallocHost((void**)&err_host, sizeof(int)));
-  *err_host = 0;
+  B200_CUDA(cudaMallocHost((void**)&err_flag, sizeof(int)));   // kernels write it where the host reads it
+  *err_flag = 0;
   B200_CUDA(cudaMallocHost((void**)&ids_host, (size_t)MR * 4096 * sizeof(int32_t)));
   B200_TRY(dalloc(&history, (size_t)MR * 4096));
   if (o.trace) {
@@ -191,6 +192,12 @@ int Graph::make_weight_maps() {
     B200_TRY(wide(L.router, 128, &W.router));
   }
   return wide(m->output, 128, &head_map);
+}
+
+// Passes whose head stages residual rows (at most eight rows, norm fused into the projection) and whose last logits row is the pass's
+// last row leave their results through PassOut.
+bool Graph::direct_out(const PassFlags& f, int M, int n_logit_rows) const {
+  return M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && n_logit_rows > 0 && !f.greedy;
 }
 
 int Graph::max_entries_for(int M, bool stream) const {
@@ -599,6 +606,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     QGemvParams p = base(m->output, H, N, xn16, H);
     p.M = n_logit_rows; p.xcols = std::min(n_logit_rows, QG_MAXCOLS); p.row_ids = logit_rows;
     p.y = logits; p.ldy = N;
+    if (direct_out(f, M, n_logit_rows)) p.out = (const PassOut*)stage_dev;
     if (use_gemm && n_logit_rows == M) {
       B200_TRY(gemm(m->output, head_map, H, N, xn16, tx_xn[2], logits, N));
     } else {
@@ -619,12 +627,12 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
 // and a captured pass of M rows always finds them at the same addresses.
 void Graph::place_stage(int M) {
   const int P = (M + 31) / 32 * 32;
-  ids_dev = (int32_t*)stage_dev; row_slot = ids_dev + P; row_pos = ids_dev + 2 * P; logit_rows = ids_dev + 3 * P; seqs = (SeqDesc*)(ids_dev + 4 * P);
+  ids_dev = (int32_t*)(stage_dev + STAGE_HEAD); row_slot = ids_dev + P; row_pos = ids_dev + 2 * P; logit_rows = ids_dev + 3 * P; seqs = (SeqDesc*)(ids_dev + 4 * P);
 }
 
 static void fill_stage(uint8_t* stage, const int32_t* ids, const int* slots, const int* pos, int M, const std::vector<SeqDesc>& sq, const std::vector<int>& lrows) {
   const int P = (M + 31) / 32 * 32;
-  int32_t* s_ids = (int32_t*)stage; int* s_slot = s_ids + P; int* s_pos = s_ids + 2 * P; int* s_lr = s_ids + 3 * P;
+  int32_t* s_ids = (int32_t*)(stage + STAGE_HEAD); int* s_slot = s_ids + P; int* s_pos = s_ids + 2 * P; int* s_lr = s_ids + 3 * P;
   SeqDesc* s_sq = (SeqDesc*)(s_ids + 4 * P);
   for (int i = 0; i < M; i++) { s_ids[i] = ids[i]; s_slot[i] = slots[i]; s_pos[i] = pos[i]; }
   for (size_t i = 0; i < lrows.size(); i++) s_lr[i] = lrows[i];
@@ -634,7 +642,7 @@ static void fill_stage(uint8_t* stage, const int32_t* ids, const int* slots, con
 int Graph::upload_stage(int M) {
   place_stage(M);
   const size_t P = (size_t)(M + 31) / 32 * 32;
-  B200_CUDA(cudaMemcpyAsync(stage_dev, stage, P * (4 * sizeof(int32_t) + sizeof(SeqDesc)), cudaMemcpyHostToDevice, st));
+  B200_CUDA(cudaMemcpyAsync(stage_dev, stage, STAGE_HEAD + P * (4 * sizeof(int32_t) + sizeof(SeqDesc)), cudaMemcpyHostToDevice, st));
   return OK;
 }
 
@@ -672,6 +680,12 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   float *lg_dst = nullptr, *rs_dst = nullptr;
   B200_TRY(result_buffers((int64_t)n_lr * NV, f.want_residual ? (int64_t)(resid_off + M) * c.n_embd : 0, &lg_dst, &rs_dst));
   bool single = !f.spec && !f.draft && !o.trace && o.use_cuda_graph && n_seq == M && n_lr == M && !f.want_residual;
+  // The head of a pass of few rows writes logits and residual rows where the caller reads them, over the bus while it still computes
+  // the rest; each copy after it would cost its own trip. (Pageable output buffers get the copies.)
+  const bool direct = direct_out(f, M, n_lr);
+  const bool to_logits = direct && (out_logits == nullptr || out_logits_mapped);
+  const bool to_h = direct && (f.want_residual ? n_lr == M && (out_resid == nullptr || out_resid_mapped) : f.want_hidden);
+  *(PassOut*)stage = PassOut{to_logits ? lg_dst : logits, !to_h ? nullptr : f.want_residual ? rs_dst + (size_t)resid_off * c.n_embd : hidden_host, f.want_residual ? 0 : n_lr - 1, 0};
   B200_CUDA(cudaEventRecord(ev0, st));
   if (single) {
     const int gkey = M * 2 + (ep_on ? 1 : 0);
@@ -696,9 +710,11 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
     B200_TRY(upload_stage(M));
     B200_TRY(enqueue_pass(M, n_seq, n_lr, f));
   }
-  if (n_lr > 0) B200_CUDA(cudaMemcpyAsync(lg_dst, logits, (size_t)n_lr * NV * sizeof(float), cudaMemcpyDeviceToHost, st));
-  if (f.want_residual) B200_CUDA(cudaMemcpyAsync(rs_dst + (size_t)resid_off * c.n_embd, h, (size_t)M * c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
-  else if (f.want_hidden) B200_CUDA(cudaMemcpyAsync(hidden_host, h + (size_t)(M - 1) * c.n_embd, (size_t)c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
+  if (n_lr > 0 && !to_logits) B200_CUDA(cudaMemcpyAsync(lg_dst, logits, (size_t)n_lr * NV * sizeof(float), cudaMemcpyDeviceToHost, st));
+  if (!to_h) {
+    if (f.want_residual) B200_CUDA(cudaMemcpyAsync(rs_dst + (size_t)resid_off * c.n_embd, h, (size_t)M * c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
+    else if (f.want_hidden) B200_CUDA(cudaMemcpyAsync(hidden_host, h + (size_t)(M - 1) * c.n_embd, (size_t)c.n_embd * sizeof(float), cudaMemcpyDeviceToHost, st));
+  }
   B200_CUDA(cudaEventRecord(ev1, st));
   B200_TRY(finish_pass());
   last_rows = M;
@@ -712,16 +728,13 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   return OK;
 }
 
-// Reads the error word back with the pass's results. A bounded wait that gave up is reported once:
+// Waits for the pass and looks at its error word. A bounded wait that gave up is reported once:
 // the word is cleared so that the graph stays usable (what the slot held is the caller's to forget,
 // as the reference's scheduler does after a failed unit, backend/llm_sched.go:713-717).
 int Graph::finish_pass() {
-  B200_CUDA(cudaMemcpyAsync(err_host, err_flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   B200_CUDA(cudaStreamSynchronize(st));
-  if (*err_host != 0) {
-    *err_host = 0;
-    B200_CUDA(cudaMemsetAsync(err_flag, 0, sizeof(int), st));
-    B200_CUDA(cudaStreamSynchronize(st));
+  if (*reinterpret_cast<volatile int*>(err_flag) != 0) {
+    *err_flag = 0;
     set_error("a kernel gave up a bounded wait (a copy or a peer that never arrived); the pass's results are not valid");
     return ETIMEOUT;
   }

@@ -51,7 +51,7 @@ struct Graph {
   float* ss_part = nullptr;   // [rows][SS_LD] partial sums of squares of the residual rows
   float *r_logits = nullptr, *topk_w = nullptr, *margin = nullptr;
   int32_t *topk = nullptr, *ids_dev = nullptr, *next_ids = nullptr, *history = nullptr;
-  int *r_ticket = nullptr, *err_flag = nullptr, *err_host = nullptr, *n_entries = nullptr, *cols = nullptr, *row_slot = nullptr, *row_pos = nullptr, *logit_rows = nullptr, *hist_len = nullptr;
+  int *r_ticket = nullptr, *err_flag = nullptr, *n_entries = nullptr, *cols = nullptr, *row_slot = nullptr, *row_pos = nullptr, *logit_rows = nullptr, *hist_len = nullptr;
   int4* entries = nullptr;
   int64_t* distinct_dev = nullptr;     // experts streamed by the work lists built so far (device counter)
   int64_t single_row_layers = 0;       // (row, layer) pairs of fused passes, whose experts are selected inside the expert kernel
@@ -70,7 +70,7 @@ struct Graph {
   int dcur = 0;        // slot whose draft cache the draft calls read and write (MTPHead.UseSlot)
   // running totals over the passes this graph ran (the reference's GraphStats: llm/graph.go:527-589)
   b200_graph_stats stats{};
-  // host staging (pinned) and its image on the device: ids | slots | positions | logit rows | sequences, one copy per pass
+  // host staging (pinned) and its image on the device: PassOut | ids | slots | positions | logit rows | sequences, one copy per pass
   uint8_t *stage = nullptr, *stage_dev = nullptr;
   // results land in the graph's own pinned buffers (grown to what calls ask for: a pass may return hundreds of
   // megabytes of logits) or, for one call, where b200_graph_set_outputs points
@@ -78,6 +78,7 @@ struct Graph {
   int64_t logits_host_cap = 0, resid_host_cap = 0;
   float *out_logits = nullptr, *out_resid = nullptr;
   int64_t out_logits_cap = 0, out_resid_cap = 0;
+  bool out_logits_mapped = false, out_resid_mapped = false;   // blocks the device can write
   int32_t* ids_host = nullptr;
   // trace
   float *tr_mid = nullptr, *tr_out = nullptr, *tr_w = nullptr, *tr_margin = nullptr;
@@ -108,6 +109,7 @@ struct Graph {
   int entry_cols(int M, bool stream) const;
   int max_entries_for(int M, bool stream) const;
   bool dense_tg(uint32_t type, int M, int N) const;
+  bool direct_out(const PassFlags& f, int M, int n_logit_rows) const;
   bool experts_stream(const LayerW& L, int M) const;
   int make_weight_maps();
   uint32_t fp16_weight_mask(int M, int n_logit_rows) const;

@@ -1949,7 +1949,7 @@ __global__ void __launch_bounds__(256, 1) attn_ring_kernel(AttnParams p) {
     }
     issue(jv + 3);  // the keys two blocks ahead, into the slot the values just left
   }
-  if (lost && p.err != nullptr && lane == 0) atomicExch(p.err, 1);  // a copy never landed: report; the result is void
+  if (lost && lane == 0) report_error(p.err);  // a copy never landed: report; the result is void
   // row sums live as per-lane partials over the four t lanes
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
@@ -2121,7 +2121,7 @@ __global__ void __launch_bounds__(256, 1) attn_prefill_kernel(AttnParams p) {
     __syncthreads();                       // every warp is done with stage s
     if (warp == 0) { fence_proxy_async(); issue(k + 2); }
   }
-  if (lost && p.err != nullptr && lane == 0) atomicExch(p.err, 1);  // a copy never landed: report; the result is void
+  if (lost && lane == 0) report_error(p.err);  // a copy never landed: report; the result is void
   lA += __shfl_xor_sync(0xffffffffu, lA, 1); lA += __shfl_xor_sync(0xffffffffu, lA, 2);
   lB += __shfl_xor_sync(0xffffffffu, lB, 1); lB += __shfl_xor_sync(0xffffffffu, lB, 2);
   // out = O / l * sigmoid(gate) -> fp16 context rows (reference: shaders/llm_attn_combine.comp:100-102)
@@ -2324,7 +2324,7 @@ __global__ void wait_timeout_probe_kernel(int* err, uint32_t limit) {
     mbar_init(&bar, 1);
     mbar_fence_init();
     mbar_expect_tx(&bar, 16);
-    if (!mbar_wait(&bar, 0, limit)) atomicExch(err, 1);
+    if (!mbar_wait(&bar, 0, limit)) report_error(err);
   }
 }
 int launch_wait_timeout_probe(int* err, cudaStream_t st) {

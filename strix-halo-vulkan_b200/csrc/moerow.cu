@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(256, 3) moe_gate_kernel(const __grid_constant_
 #pragma unroll
         for (int m = 0; m < 2; m++) {
           if (warp_wait(&bars[warp][m], phase)) k45_accumulate<TYPE>(acc[m], ra + m * RAW, ra + m * RAW + BLK, xs + 576 * blk, s0, s1, t);
-          else if (lane == 0 && p.err != nullptr) atomicExch(p.err, 1);   // a copy never landed: report, the results are void
+          else if (lane == 0) report_error(p.err);   // a copy never landed: report, the results are void
         }
         __syncwarp();
         const bool more = b + 1 < bpt;
@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(MD_MAXWARPS * 32) moe_down_kernel(const __grid
       const uint32_t ra = (uint32_t)__cvta_generic_to_shared(smem + u * RAW) + 2 * g * BLK;
       const __half* sp = sx + ((t & 1) ? 8 : 0) + 2 * (t >> 1);
       k45_accumulate<TYPE>(acc, ra, ra + BLK, xs, *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
-    } else if (lane == 0 && p.err != nullptr) {
-      atomicExch(p.err, 1);   // a copy never landed: report, the results are void
+    } else if (lane == 0) {
+      report_error(p.err);   // a copy never landed: report, the results are void
     }
     if (t == 0) { yv[2 * g * ld + u] = w * acc[0]; yv[(2 * g + 1) * ld + u] = w * acc[2]; }   // every column holds the one activation row
   }

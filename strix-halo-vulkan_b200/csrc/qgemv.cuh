@@ -38,6 +38,10 @@ enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2 };
 enum { PRO_F16 = 0, PRO_NORM = 1 };
 constexpr int SS_LD = 512;  // partial sums of squares kept per activation row
 
+// Where a pass of few rows leaves its results, read on the device so that a replayed pass can change them: host memory the device can
+// write (or the graph's own device buffer), and the residual rows of the columns from h_first on (nullptr: not wanted).
+struct PassOut { float* logits; float* h; int h_first, pad; };
+
 struct QGemvParams {
   // weights: up to 4 row segments of one fused projection (same type and K)
   const uint8_t* w[4];
@@ -73,6 +77,7 @@ struct QGemvParams {
   float eps;
   __half* xn_out;            // PRO_NORM: optional copy of the normalised rows, [.][K], written by CTA 0
   float* ss_out;             // STORE / RESID: optional partial sums of squares of the rows written, [.][SS_LD], part = tile of 16 rows
+  const PassOut* out;        // the head of a pass of few rows: y and the residual copy come from here
   // epilogue
   float* y;                  // STORE / RESID: float [.][ldy]
   int64_t ldy;
@@ -441,6 +446,8 @@ __device__ __forceinline__ float scale_from_parts(const float* ss_in, int ss_n, 
 __device__ __forceinline__ void stage_x_norm(const QGemvParams& p, uint8_t* xs, __half* sxs, float* scratch, int ncols, const int* xrows, int xstride,
                                              bool write_xn) {
   const int warp = threadIdx.x >> 5, K = p.K;
+  float* hout = p.out != nullptr && blockIdx.x == 0 && blockIdx.z == 0 ? p.out->h : nullptr;
+  const int h_first = hout != nullptr ? p.out->h_first : 0;
   // element index of this thread, rotated by whole 128-byte lines per CTA (every CTA reads the same rows)
   const int tid = (threadIdx.x + 8 * (int)((blockIdx.x + blockIdx.y) & 31)) & (QG_THREADS - 1);
   // the residual values do not depend on the scale: fetch the first batch before reducing the partials
@@ -470,6 +477,7 @@ __device__ __forceinline__ void stage_x_norm(const QGemvParams& p, uint8_t* xs, 
       const float v0 = h.x * scale * g.x, v1 = h.y * scale * g.y, v2 = h.z * scale * g.z, v3 = h.w * scale * g.w;
       __half2 a = __floats2half2_rn(v0, v2), b = __floats2half2_rn(v1, v3);  // stored order [x0,x2,x1,x3]
       *reinterpret_cast<uint2*>(dst + 2 * k + 16 * (k >> 6)) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+      if (hout != nullptr && c >= h_first) *reinterpret_cast<float4*>(hout + (size_t)(c - h_first) * K + k) = h;
       if (write_xn) {
         __half2 n0 = __floats2half2_rn(v0, v1), n1 = __floats2half2_rn(v2, v3);
         *reinterpret_cast<uint2*>(p.xn_out + row * K + k) = make_uint2(*reinterpret_cast<uint32_t*>(&n0), *reinterpret_cast<uint32_t*>(&n1));
@@ -616,6 +624,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   pdl_launch();
   tl_mark(p.tl, 1);
 
+  float* const y = p.out != nullptr ? p.out->logits : p.y;
   bool live = false;
   const uint8_t* xrow = xs;
   const __half* sxrow = sxs;
@@ -666,7 +675,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       if constexpr (BOXED) {
         if (tile < tiles && kslice < nb) {
           if (!warp_wait(&full_bar[BOXED ? warp : 0][s], (uint32_t)((it / NS) & 1))) {   // a copy never landed: report, the results are void
-            if (p.err != nullptr && lane == 0) atomicExch(p.err, 1);
+            if (lane == 0) report_error(p.err);
           } else {
             if (it == 0) tl_mark(p.tl, 3);
             const uint8_t* row0 = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes + 2 * g * BLK;
@@ -677,7 +686,7 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
         }
       } else {
         if (!mbar_wait(&full_bar[0][s], (uint32_t)((it / NS) & 1))) {
-          if (p.err != nullptr && tid == 0) atomicExch(p.err, 1);  // a copy never landed: report and leave
+          if (tid == 0) report_error(p.err);  // a copy never landed: report and leave
           return;
         }
         if (it == 0) tl_mark(p.tl, 3);
@@ -720,8 +729,8 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       }
       const int64_t orow = (!GROUPED && p.row_ids != nullptr) ? col_off + c : col_rows[c];
       if (grow < p.N) {
-        if constexpr (EPI == EPI_STORE) { p.y[orow * p.ldy + grow] = v; sq = v * v; }
-        else if constexpr (EPI == EPI_RESID) { const float nv = p.y[orow * p.ldy + grow] + v; p.y[orow * p.ldy + grow] = nv; sq = nv * nv; }
+        if constexpr (EPI == EPI_STORE) { y[orow * p.ldy + grow] = v; sq = v * v; }
+        else if constexpr (EPI == EPI_RESID) { const float nv = y[orow * p.ldy + grow] + v; y[orow * p.ldy + grow] = nv; sq = nv * nv; }
         else p.y16[orow * p.ldy + grow] = __float2half_rn(v * sigmoid_acc(v) * v2);  // SwiGLU of (gate, up) rounded to fp16 (reference: shaders/llm_moe_gemv.comp:777-781)
       }
       if constexpr (EPI != EPI_SWIGLU && !GROUPED) {

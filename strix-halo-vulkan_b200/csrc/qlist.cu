@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         if (!warp_wait(&bars[warp][slot], phase)) {   // a copy never landed: report, the results are void
-          if (p.err != nullptr && lane == 0) atomicExch(p.err, 1);
+          if (lane == 0) report_error(p.err);
           for (int k = 1; k < SLOTS; k++) mbar_wait(&bars[warp][(slot + k) % SLOTS], phase ^ (slot + k >= SLOTS));   // leave with no copy in flight
           return;
         }

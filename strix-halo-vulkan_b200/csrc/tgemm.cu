@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
   const uint32_t tm = tmem_sm;
 
   const int nb = p.K / 256, tiles = (p.N + TG_TILE - 1) / TG_TILE, coltiles = (p.M + NMAX - 1) / NMAX;
-  auto give_up = [&]() { if (p.err != nullptr) atomicExch(p.err, 1); failed = 1; };
+  auto give_up = [&]() { report_error(p.err); failed = 1; };
   auto stopped = [&]() { return __any_sync(0xffffffffu, failed); };
   auto unit_at = [&](int u) {
     Unit t;

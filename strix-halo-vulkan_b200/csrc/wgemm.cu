@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
   };
   const int n_items = blockIdx.x < total ? (total - 1 - blockIdx.x) / gridDim.x + 1 : 0;
   auto sb_begin = [&](int ks) { return ks * nb / p.ksplit; };
-  auto give_up = [&]() { if (p.err != nullptr) atomicExch(p.err, 1); failed = 1; };
+  auto give_up = [&]() { report_error(p.err); failed = 1; };
   auto stopped = [&]() { return __any_sync(0xffffffffu, failed); };
 
   if (warp == 0) {
