@@ -2,6 +2,7 @@
 // layers() loop (llm/graph.go:2330-2466) with a plain pre-norm residual stream in place of
 // its hyper-connection mixers.
 #include "graph.h"
+#include "attn_tc.cuh"
 #include "moerow.cuh"
 
 #include <algorithm>
@@ -81,7 +82,8 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   max_entries = std::max(max_entries_for(MR, false), max_entries_for(std::min(MR, 128), false));
   B200_TRY(dalloc(&h, (size_t)MR * H)); B200_TRY(dalloc(&proj, (size_t)MR * proj_ld));
   B200_TRY(dalloc(&xn16, (size_t)MR * H)); B200_TRY(dalloc(&q16, (size_t)MR * qw)); B200_TRY(dalloc(&ctx16, (size_t)MR * qw));
-  B200_TRY(dalloc(&attn_partial, (size_t)attn_rows * c.n_head * nsplit * (hd + 2)));
+  attn_partial_floats = (int64_t)attn_rows * c.n_head * nsplit * (hd + 2);
+  B200_TRY(dalloc(&attn_partial, (size_t)attn_partial_floats));
   B200_TRY(dalloc(&r_logits, (size_t)MR * c.n_expert));
   B200_TRY(dalloc(&topk, (size_t)MR * used)); B200_TRY(dalloc(&topk_w, (size_t)MR * slots1)); B200_TRY(dalloc(&margin, (size_t)MR));
   B200_TRY(dalloc(&entries, (size_t)max_entries)); B200_TRY(dalloc(&n_entries, 1)); B200_TRY(dalloc(&cols, (size_t)MR * slots1));
@@ -143,6 +145,9 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
     B200_TRY(dalloc(&kcache[i], (size_t)o.slots * kv_slot_stride));
     B200_TRY(dalloc(&vcache[i], (size_t)o.slots * kv_slot_stride));
   }
+  attn_maps.resize(n_attn);
+  if (attn_tc_shape(c.n_head, c.n_head_kv, hd))
+    for (int i = 0; i < n_attn; i++) B200_TRY(make_attn_maps(q16, MR, c.n_head, kcache[i], vcache[i], (int64_t)o.slots * o.n_kv, c.n_head_kv, hd, &attn_maps[i]));
   past.assign(o.slots, 0); draft_past.assign(o.slots, 0);
   // host staging
   B200_CUDA(cudaMallocHost((void**)&stage, stage_bytes));
@@ -446,9 +451,11 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       a.one_row_per_seq = M == n_seq && !f.spec; a.err = err_flag; a.tl = tl();
       B200_TRY(launch_attn_pack(a, pdl(), st));
       a.tl = tl();
-      if (n_seq == 1 && !f.spec && attn_prefill_fits(a)) {
-        // many rows of one sequence: query tiles x key tiles, straight to the gated context rows
-        B200_TRY(launch_attn_prefill(a, pdl(), st));
+      if (n_seq == 1 && !f.spec && attn_tc_fits(a)) {
+        // many rows of one sequence: query tiles x key tiles, straight to the gated context rows where no cut is needed
+        B200_TRY(launch_attn_tc(a, attn_maps[ai], pass_last_pos, attn_partial_floats, pdl(), st));
+        a.tl = tl();
+        if (a.nsplit > 0) B200_TRY(launch_attn_merge(a, pdl(), st));
       } else {
         if (M > attn_rows) { set_error("pass of " + std::to_string(M) + " rows: the split attention buffers hold " + std::to_string(attn_rows)); return ECAPACITY; }
         B200_TRY(launch_attn_decode(a, pdl(), st));
@@ -673,7 +680,7 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   B200_CUDA(cudaSetDevice(m->device));
   const auto host_t0 = std::chrono::steady_clock::now();
   fill_stage(stage, ids, slots, pos, M, sq, lrows);
-  pass_max_n = 1;
+  pass_max_n = 1; pass_last_pos = sq.size() == 1 ? sq[0].pos0 + sq[0].n - 1 : 0;
   for (const SeqDesc& s : sq) pass_max_n = std::max(pass_max_n, s.n);
   const int n_lr = (int)lrows.size(), n_seq = (int)sq.size();
   const int NV = f.draft && draft_vocab > 0 ? draft_vocab : c.vocab;

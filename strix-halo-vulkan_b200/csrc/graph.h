@@ -5,6 +5,7 @@
 #include <map>
 #include <vector>
 
+#include "attn_tc.cuh"
 #include "ep.cuh"
 #include "kernels.cuh"
 #include "model.h"
@@ -60,6 +61,9 @@ struct Graph {
   int proj_ld = 0, max_entries = 0, nsplit = 0, split_cells = 0;
   // sequence state
   std::vector<float*> dn_state, dn_ring, dn_mid;   // per DeltaNet layer
+  std::vector<AttnTcMaps> attn_maps;               // per attention layer: query rows and its caches
+  int64_t attn_partial_floats = 0;
+  int pass_last_pos = 0;                           // passes of one sequence: position of the last row
   std::vector<__half*> kcache, vcache;             // per attention layer (+ draft)
   int64_t state_slot_stride = 0, ring_slot_stride = 0, kv_slot_stride = 0, mid_seq_stride = 0;
   std::vector<int> past, draft_past;

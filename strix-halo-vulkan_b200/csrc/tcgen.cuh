@@ -26,6 +26,16 @@ __device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t bdesc, u
   asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d), "r"(a), "l"(bdesc), "r"(idesc), "r"(accumulate)
                : "memory");
 }
+// D[tmem] (+)= A[smem desc] * B[smem desc], fp16 x fp16 -> f32
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void tma_box3(void* dst, const void* tm, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)), "l"(tm), "r"(c0),
+               "r"(c1), "r"(c2), "r"(smem_addr(bar))
+               : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t t, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(t),
@@ -50,10 +60,23 @@ __device__ __forceinline__ void tmem_ld16(uint32_t t, uint32_t (&r)[16]) {
                : "r"(t)
                : "memory");
 }
+__device__ __forceinline__ void tmem_ld32(uint32_t t, float (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]),
+        "=f"(r[14]), "=f"(r[15]), "=f"(r[16]), "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), "=f"(r[24]), "=f"(r[25]), "=f"(r[26]),
+        "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31])
+      : "r"(t)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // K-major tile of 128-byte rows under the 128-byte swizzle, groups of eight rows 1024 bytes apart
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t a) { return (uint64_t)((a >> 4) & 0x3FFF) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61); }
+// MN-major operand under the 128-byte swizzle: rows of 64 elements along M or N (128 bytes), one per K, in groups of eight 1024 bytes
+// apart; the next 64 elements along M or N are `chunk` bytes on
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t a, uint32_t chunk) { return (uint64_t)((a >> 4) & 0x3FFF) | ((uint64_t)(chunk >> 4) << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61); }
+constexpr uint32_t IDESC_B_MN = 1u << 16;   // B is MN-major
 // f32 accumulator, fp16 A and B, both K-major, M 128
 __device__ __forceinline__ uint32_t idesc_n(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | (8u << 24); }
 
@@ -61,6 +84,7 @@ __device__ __forceinline__ uint32_t idesc_n(int n) { return (1u << 4) | ((uint32
 #endif
 
 // 2-D tensor map of rows `stride` bytes apart; CUtensorMapDataType / CUtensorMapSwizzle as in cuda.h
+int encode_nd(CUtensorMapDataType type, const void* base, int rank, const int64_t* dims, const int64_t* strides, const int* box, CUtensorMapSwizzle swizzle, TMap* out);
 int encode_2d(CUtensorMapDataType type, const void* base, int64_t inner, int64_t rows, int64_t stride, int box_inner, int box_rows, CUtensorMapSwizzle swizzle, TMap* out);
 
 }  // namespace b200

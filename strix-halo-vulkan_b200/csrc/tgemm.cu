@@ -325,23 +325,29 @@ __global__ void __launch_bounds__(256) row_sums_kernel(const __half* x, int K, _
 typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                              CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-int encode_2d(CUtensorMapDataType type, const void* base, int64_t inner, int64_t rows, int64_t stride, int box_inner, int box_rows, CUtensorMapSwizzle swizzle, TMap* out) {
+int encode_nd(CUtensorMapDataType type, const void* base, int rank, const int64_t* dims_, const int64_t* strides_, const int* box_, CUtensorMapSwizzle swizzle, TMap* out) {
   static std::atomic<EncodeFn> encode{nullptr};
   EncodeFn fn = encode.load();
   if (fn == nullptr) {
     void* q = nullptr;
     cudaDriverEntryPointQueryResult res;
     B200_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &q, cudaEnableDefault, &res));
-    if (q == nullptr || res != cudaDriverEntryPointSuccess) { set_error("tgemm: the driver does not export cuTensorMapEncodeTiled"); return ECUDA; }
+    if (q == nullptr || res != cudaDriverEntryPointSuccess) { set_error("the driver does not export cuTensorMapEncodeTiled"); return ECUDA; }
     fn = (EncodeFn)q;
     encode.store(fn);
   }
-  const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)stride};
-  const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows}, estr[2] = {1, 1};
-  const CUresult r = fn(reinterpret_cast<CUtensorMap*>(out->b), type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+  cuuint64_t dims[3], strides[2];
+  cuuint32_t box[3], estr[3] = {1, 1, 1};
+  for (int i = 0; i < rank; i++) { dims[i] = (cuuint64_t)dims_[i]; box[i] = (cuuint32_t)box_[i]; if (i + 1 < rank) strides[i] = (cuuint64_t)strides_[i]; }
+  const CUresult r = fn(reinterpret_cast<CUtensorMap*>(out->b), type, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                         CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error("tgemm: cuTensorMapEncodeTiled failed with code " + std::to_string((int)r)); return ECUDA; }
+  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed with code " + std::to_string((int)r)); return ECUDA; }
   return OK;
+}
+int encode_2d(CUtensorMapDataType type, const void* base, int64_t inner, int64_t rows, int64_t stride, int box_inner, int box_rows, CUtensorMapSwizzle swizzle, TMap* out) {
+  const int64_t dims[2] = {inner, rows};
+  const int box[2] = {box_inner, box_rows};
+  return encode_nd(type, base, 2, dims, &stride, box, swizzle, out);
 }
 
 bool tgemm_type(uint32_t type) { return type == T_Q4_K || type == T_Q5_K; }
