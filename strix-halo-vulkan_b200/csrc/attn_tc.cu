@@ -233,24 +233,33 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
     if (ok && nt > 0 && warp_wait(&pv_done, (nt - 1) & 1)) {
       fence_after();
       const bool whole = p.nsplit == 0, live = r / G < rows;
-      const float inv = 1.0f / l;
       const float* gate = p.proj + (size_t)n * p.ldp + (size_t)head * 2 * HD + HD;
       __half* dst = p.ctx16 + (size_t)n * p.Hq * HD + (size_t)head * HD;
       float* part = p.partial + (((size_t)n * p.Hq + head) * p.nsplit + blockIdx.z) * (HD + 2);
+      // The gates are a row's own 128 bytes per 32 columns: asked for ahead of their use. O / l * sigmoid(gate)
+      // (reference: shaders/llm_attn_combine.comp:100-102) is one quotient, O / (l (1 + exp(-gate))).
+      float4 gn[8];
+      auto ask = [&](int j) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) gn[i] = *reinterpret_cast<const float4*>(gate + j + 4 * i);
+      };
+      if (whole && live) ask(0);
 #pragma unroll 1
       for (int j = 0; j < HD; j += 32) {
         float o[32];
         tmem_ld32(lanes + TO + j, o);
         tmem_ld_wait();
         if (!live) continue;
-        if (whole) {                                          // out = O / l * sigmoid(gate) (reference: shaders/llm_attn_combine.comp:100-102)
+        if (whole) {
+          float g[32];
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            const float4 g0 = *reinterpret_cast<const float4*>(gate + j + i), g1 = *reinterpret_cast<const float4*>(gate + j + i + 4);
-            *reinterpret_cast<uint4*>(dst + j + i) =
-                make_uint4(half2_of(o[i] * inv * sigmoid_acc(g0.x), o[i + 1] * inv * sigmoid_acc(g0.y)), half2_of(o[i + 2] * inv * sigmoid_acc(g0.z), o[i + 3] * inv * sigmoid_acc(g0.w)),
-                           half2_of(o[i + 4] * inv * sigmoid_acc(g1.x), o[i + 5] * inv * sigmoid_acc(g1.y)), half2_of(o[i + 6] * inv * sigmoid_acc(g1.z), o[i + 7] * inv * sigmoid_acc(g1.w)));
-          }
+          for (int i = 0; i < 8; i++) { g[4 * i] = gn[i].x; g[4 * i + 1] = gn[i].y; g[4 * i + 2] = gn[i].z; g[4 * i + 3] = gn[i].w; }
+          if (j + 32 < HD) ask(j + 32);
+#pragma unroll
+          for (int i = 0; i < 32; i++) o[i] = __fdividef(o[i], fmaf(l, __expf(fminf(-g[i], 80.f)), l));
+#pragma unroll
+          for (int i = 0; i < 32; i += 8)
+            *reinterpret_cast<uint4*>(dst + j + i) = make_uint4(half2_of(o[i], o[i + 1]), half2_of(o[i + 2], o[i + 3]), half2_of(o[i + 4], o[i + 5]), half2_of(o[i + 6], o[i + 7]));
         } else {
 #pragma unroll
           for (int i = 0; i < 32; i += 2) *reinterpret_cast<float2*>(part + j + i) = make_float2(o[i], o[i + 1]);

@@ -87,7 +87,7 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
   B200_TRY(dalloc(&r_logits, (size_t)MR * c.n_expert));
   B200_TRY(dalloc(&topk, (size_t)MR * used)); B200_TRY(dalloc(&topk_w, (size_t)MR * slots1)); B200_TRY(dalloc(&margin, (size_t)MR));
   B200_TRY(dalloc(&entries, (size_t)max_entries)); B200_TRY(dalloc(&n_entries, 1)); B200_TRY(dalloc(&cols, (size_t)MR * slots1));
-  B200_TRY(dalloc(&r_ticket, (size_t)2 + MR / 8)); B200_TRY(dalloc(&ss_part, (size_t)MR * SS_LD)); B200_TRY(dalloc(&y16, (size_t)MR * vw));
+  B200_TRY(dalloc(&r_ticket, 1)); B200_TRY(dalloc(&pair_counts, (size_t)c.n_expert)); B200_TRY(dalloc(&pair_pos, (size_t)MR * used)); B200_TRY(dalloc(&ss_part, (size_t)MR * SS_LD)); B200_TRY(dalloc(&y16, (size_t)MR * vw));
   B200_TRY(dalloc(&act16, (size_t)MR * slots1 * c.ffn_expert)); B200_TRY(dalloc(&down, (size_t)MR * slots1 * H));
   B200_TRY(dalloc(&logits, (size_t)LR * c.vocab));
   { B200_TRY(dalloc(&dn_pre, (size_t)MR * ((size_t)c.dn_heads_k * 256 + (size_t)c.dn_heads_v * 130))); B200_TRY(dalloc(&dn_wy, (size_t)MR * c.dn_heads_v * 192, false)); B200_TRY(dalloc(&dn_oraw, (size_t)MR * vw)); B200_TRY(dalloc(&dn_ab, (size_t)MR * 2 * c.dn_heads_v)); }
@@ -481,7 +481,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     r.xn = xn16; r.router = L.router; r.sh_gate = (const float*)L.sh_gate_inp.data;
     if (fused) { r.h = h; r.gamma = (const float*)L.ffn_norm.data; r.ss_in = ss_part; r.ss_n = ss_n; r.eps = c.eps; r.xn_out = xn16; }
     r.M = M; r.H = H; r.nE = c.n_expert; r.used = used; r.logits = r_logits; r.probs = nullptr; r.topk = topk; r.topk_w = topk_w;
-    r.tl = tl(); r.margin = margin; r.entries = entries; r.n_entries = n_entries; r.cols = cols; r.ticket = r_ticket; r.max_entries = max_entries;
+    r.tl = tl(); r.margin = margin; r.entries = entries; r.n_entries = n_entries; r.cols = cols; r.ticket = r_ticket; r.pair_counts = pair_counts; r.pair_pos = pair_pos; r.max_entries = max_entries;
     // passes of at most 8 rows: the router stops after its logits and every row is routed, computed and combined on
     // the single-row schedule, so each row's result is the single-row pass's, bit for bit (the reference's batched
     // decode and verify passes equal their rows stepped alone: llm/graph_batch_test.go:36, llm/spec_slots_test.go:199)
@@ -507,6 +507,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       B200_TRY(launch_route_rows(r, pdl(), st));
     } else {
       B200_TRY(launch_router(r, pdl(), st));
+      r.gate_done = 1;
+      if (!r.defer) B200_TRY(launch_route_rows(r, pdl(), st));
     }
     // the two expert launches of a work list: activation rows x (ids / x_div), outputs by pair id
     auto stream_experts = [&](const __half* x, const __half* sx, int cols_) {
@@ -525,7 +527,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       e.rows = M; e.xn = xn16; e.topk = topk;
       B200_TRY(launch_ep_dispatch(e, pdl(), st));
       RouterParams w = r;
-      w.M = Mg; w.topk = reinterpret_cast<int32_t*>(ep_arena + ep.off_topk); w.entries = entries; w.ecols = entry_cols(Mg, moe_stream);
+      w.M = Mg; w.pair_pos = nullptr; w.topk = reinterpret_cast<int32_t*>(ep_arena + ep.off_topk); w.entries = entries; w.ecols = entry_cols(Mg, moe_stream);
       w.e_lo = ep.rank * (c.n_expert / ep.world); w.e_hi = w.e_lo + c.n_expert / ep.world; w.sh_lo = ep.rank * M; w.sh_hi = w.sh_lo + M;
       w.n_pairs = ep_epoch + 2;
       B200_TRY(launch_ep_worklist(w, pdl(), st));
@@ -550,7 +552,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
       down_rows = reinterpret_cast<float*>(ep_arena + ep.off_down);
     } else if (moe_gemm) {
       // every expert's rows side by side, the shared expert's (all rows) last: one launch each for gate/up and down
-      B200_TRY(launch_moe_gather(xn16, cols, M * slots1, slots1, H, xperm16, pdl(), st));
+      B200_TRY(launch_moe_gather(xn16, r, xperm16, pdl(), st));
       const LayerMaps& W = wmaps[l];
       WGemmMaps mg{};
       mg.w = W.wgate; mg.w2 = W.wup; mg.ws = W.wgate_sh; mg.ws2 = W.wup_sh; mg.x = tx_xperm;

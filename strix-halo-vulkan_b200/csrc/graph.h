@@ -52,7 +52,7 @@ struct Graph {
   float* ss_part = nullptr;   // [rows][SS_LD] partial sums of squares of the residual rows
   float *r_logits = nullptr, *topk_w = nullptr, *margin = nullptr;
   int32_t *topk = nullptr, *ids_dev = nullptr, *next_ids = nullptr, *history = nullptr;
-  int *r_ticket = nullptr, *err_flag = nullptr, *n_entries = nullptr, *cols = nullptr, *row_slot = nullptr, *row_pos = nullptr, *logit_rows = nullptr, *hist_len = nullptr;
+  int *r_ticket = nullptr, *pair_counts = nullptr, *pair_pos = nullptr, *err_flag = nullptr, *n_entries = nullptr, *cols = nullptr, *row_slot = nullptr, *row_pos = nullptr, *logit_rows = nullptr, *hist_len = nullptr;
   int4* entries = nullptr;
   int64_t* distinct_dev = nullptr;     // experts streamed by the work lists built so far (device counter)
   int64_t single_row_layers = 0;       // (row, layer) pairs of fused passes, whose experts are selected inside the expert kernel

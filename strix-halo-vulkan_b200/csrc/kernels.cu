@@ -241,13 +241,19 @@ __device__ void build_work_list(const RouterParams& p, int* counts, int* offs, i
   }
   const int e_lo = p.e_hi > 0 ? p.e_lo : 0, e_hi = p.e_hi > 0 ? p.e_hi : nE;
   const int sh_lo = p.sh_hi > 0 ? p.sh_lo : 0, sh_hi = p.sh_hi > 0 ? p.sh_hi : M;
-  for (int i = tid; i <= nE; i += 256) counts[i] = 0;
-  __syncthreads();
-  for (int i = tid; i < M * used; i += 256) {
-    const int e = __ldcg(p.topk + i);
-    if (e >= e_lo && e < e_hi) atomicAdd(&counts[e], 1);
+  const bool counted = p.pair_pos != nullptr;   // the routing has counted the pairs and placed each among its expert's
+  for (int i = tid; i <= nE; i += 256) {
+    counts[i] = counted && i < nE ? __ldcg(p.pair_counts + i) : 0;
+    if (counted && i < nE) p.pair_counts[i] = 0;
   }
   __syncthreads();
+  if (!counted) {
+    for (int i = tid; i < M * used; i += 256) {
+      const int e = __ldcg(p.topk + i);
+      if (e >= e_lo && e < e_hi) atomicAdd(&counts[e], 1);
+    }
+    __syncthreads();
+  }
   if (p.distinct != nullptr) {   // experts this pass streams (what a step's byte count needs)
     int mine = 0;
     for (int e = tid; e < nE; e += 256) mine += counts[e] > 0;
@@ -283,14 +289,23 @@ __device__ void build_work_list(const RouterParams& p, int* counts, int* offs, i
   for (int i = tid; i < nsh; i += 256)
     if (eoff[nE] + i < p.max_entries) p.entries[eoff[nE] + i] = make_int4(-1, offs[nE] + EC * i, min(EC, nshr - EC * i), 0);
   if (tid == 0) { *p.n_entries = min(eoff[nE] + nsh, p.max_entries); if (p.n_pairs != nullptr) *p.n_pairs = offs[nE] + nshr; }
-  __syncthreads();
-  for (int i = tid; i <= nE; i += 256) counts[i] = 0;
-  __syncthreads();
-  for (int i = tid; i < M * used; i += 256) {
-    const int e = __ldcg(p.topk + i), n = i / used, k = i - n * used;
-    if (e < e_lo || e >= e_hi) continue;
-    const int pos = atomicAdd(&counts[e], 1);
-    p.cols[offs[e] + pos] = n * (used + 1) + k;
+  if (counted && p.gprob != nullptr) return;     // the gather kernel writes cols as it places the rows
+  if (counted) {
+#pragma unroll 4
+    for (int i = tid; i < M * used; i += 256) {
+      const int n = i / used;
+      p.cols[offs[__ldcg(p.topk + i)] + __ldcg(p.pair_pos + i)] = n * (used + 1) + i - n * used;
+    }
+  } else {
+    __syncthreads();
+    for (int i = tid; i <= nE; i += 256) counts[i] = 0;
+    __syncthreads();
+    for (int i = tid; i < M * used; i += 256) {
+      const int e = __ldcg(p.topk + i), n = i / used, k = i - n * used;
+      if (e < e_lo || e >= e_hi) continue;
+      const int pos = atomicAdd(&counts[e], 1);
+      p.cols[offs[e] + pos] = n * (used + 1) + k;
+    }
   }
   for (int n = tid; n < nshr; n += 256) p.cols[offs[nE] + n] = (sh_lo + n) * (used + 1) + used;
 }
@@ -308,11 +323,9 @@ int launch_ep_worklist(const RouterParams& p, bool pdl, cudaStream_t st) {
   return launch_k(ep_worklist_kernel, dim3(1), dim3(256), 0, pdl, st, p);
 }
 
+// Router logits by per-row dot products, and the shared expert's gate; weights exact. Selection is the next kernel's.
 __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
-  __shared__ int is_last;
-  __shared__ float2 cand[8][32];
   __shared__ float half_sum[8][8];
-  __shared__ int counts[1025], offs[1025], eoff[1025];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H, M = p.M;
   const int row = blockIdx.x * RT_ROWS + (warp >> 1), half = warp & 1;  // of the nE + 1 outputs; the last is the shared-expert gate
   const int k_lo = half * (H / 2), k_hi = half ? H : H / 2;
@@ -421,34 +434,6 @@ __global__ void __launch_bounds__(256) router_kernel(RouterParams p) {
     }
   }
   tl_mark(p.tl, 4);
-  if (p.defer) return;  // the expert kernel selects the experts itself
-  // Two levels of tickets: the last CTA of a row group (blockIdx.y) routes that group's eight rows, one
-  // per warp; the last group to finish builds the work list of the whole pass.
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = (atomicAdd(p.ticket + 1 + blockIdx.y, 1) == (int)gridDim.x - 1);
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  if (tid == 0) p.ticket[1 + blockIdx.y] = 0;
-  tl_mark(p.tl, 5, true);
-  const int nE = p.nE, used = p.used;
-  {
-    const int n = blockIdx.y * 8 + warp;
-    if (n < M) {
-      if (nE <= 512) route_token<16>(p, n, lane, true, cand[warp]);
-      else route_token<32>(p, n, lane, true, cand[warp]);
-    }
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) is_last = (atomicAdd(p.ticket, 1) == (int)gridDim.y - 1);
-  __syncthreads();
-  if (!is_last) return;
-  __threadfence();
-  if (tid == 0) *p.ticket = 0;
-  if (p.entries == nullptr) return;   // routing only (expert-parallel passes build their list from the gathered routing)
-  build_work_list(p, counts, offs, eoff);
 }
 
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
@@ -534,21 +519,26 @@ int launch_router_mma(const RouterParams& p, bool pdl, cudaStream_t st) {
   return launch_k(router_mma_kernel, dim3(p.nE / 16, (p.M + 63) / 64), dim3(256), 0, pdl, st, p);
 }
 
-// Routing of a many-row pass whose router logits came from the tensor-core GEMM: one warp per row
-// computes the shared-expert gate (f32 weights against the fp16 row) and selects the experts; the last
-// CTA builds the work list. grid ceil(M / 8), block 256.
+// Selection for every row of a pass from its logits, a CTA per row (route_row_cta), with the shared expert's gate (f32 weights
+// against the fp16 row) where the router has not left it. Every pair also takes its place among its expert's pairs, so that the last
+// CTA has only the experts to go over for the work list. (A warp per row, and one CTA that counted and placed all pairs, took 22 us
+// for 64 rows and 57 for 2048, most of it that CTA's walk over the pairs.) grid M, block 256.
+template <int VPT>
 __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
   __shared__ int is_last;
-  __shared__ float2 cand[8][32];
+  __shared__ RouteSmem rs;
+  __shared__ float gate[8];
   __shared__ int counts[1025], offs[1025], eoff[1025];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H, n = blockIdx.x, used = p.used;
   pdl_wait();
   pdl_launch();
-  const int n = blockIdx.x * 8 + warp;
-  if (n < p.M) {
+  float l[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; i++) l[i] = tid + 256 * i < p.nE ? __ldcg(p.logits + (size_t)n * p.nE + tid + 256 * i) : -INFINITY;
+  if (!p.gate_done) {
     const __half* x = p.xn + (size_t)n * H;
     float acc = 0.f;
-    for (int k = lane * 8; k < H; k += 256) {
+    for (int k = tid * 8; k < H; k += 2048) {
       uint4 xv = *reinterpret_cast<const uint4*>(x + k);
       const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
       float4 g0 = *reinterpret_cast<const float4*>(p.sh_gate + k), g1 = *reinterpret_cast<const float4*>(p.sh_gate + k + 4);
@@ -556,9 +546,14 @@ __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
       acc = fmaf(g1.x, h2f_lo(xw[2]), acc); acc = fmaf(g1.y, h2f_hi(xw[2]), acc); acc = fmaf(g1.z, h2f_lo(xw[3]), acc); acc = fmaf(g1.w, h2f_hi(xw[3]), acc);
     }
     acc = warp_sum(acc);
-    if (lane == 0) p.topk_w[(size_t)n * (p.used + 1) + p.used] = sigmoid_acc(acc);
-    if (p.nE <= 512) route_token<16>(p, n, lane, true, cand[warp]);
-    else route_token<32>(p, n, lane, true, cand[warp]);
+    if (lane == 0) gate[warp] = acc;   // read after the selection's barriers
+  }
+  route_row_cta<VPT>(p, n, l, true, -1, rs);
+  if (!p.gate_done && tid == 0) p.topk_w[(size_t)n * (used + 1) + used] = sigmoid_acc(((gate[0] + gate[1]) + (gate[2] + gate[3])) + ((gate[4] + gate[5]) + (gate[6] + gate[7])));
+  if (p.entries == nullptr) return;   // routing only (expert-parallel passes build their list from the gathered routing)
+  if (warp == 0 && p.M > 1) {
+    __syncwarp();                     // the row's experts were written by other lanes
+    if (lane < used) p.pair_pos[(size_t)n * used + lane] = atomicAdd(p.pair_counts + __ldcg(p.topk + (size_t)n * used + lane), 1);
   }
   __threadfence();
   __syncthreads();
@@ -567,12 +562,11 @@ __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
   if (!is_last) return;
   __threadfence();
   if (tid == 0) *p.ticket = 0;
-  if (p.entries == nullptr) return;   // routing only
   build_work_list(p, counts, offs, eoff);
 }
 int launch_route_rows(const RouterParams& p, bool pdl, cudaStream_t st) {
-  if (p.nE > 1024 || p.used > 32 || p.H % 8 || p.xn == nullptr) { set_error("route_rows: shape outside kernel limits"); return ECAPACITY; }
-  return launch_k(route_rows_kernel, dim3((p.M + 7) / 8), dim3(256), 0, pdl, st, p);
+  if (p.nE > 1024 || p.used > 32 || p.H % 8 || p.xn == nullptr || p.pair_pos == nullptr) { set_error("route_rows: shape outside kernel limits"); return ECAPACITY; }
+  return p.nE <= 512 ? launch_k(route_rows_kernel<2>, dim3(p.M), dim3(256), 0, pdl, st, p) : launch_k(route_rows_kernel<4>, dim3(p.M), dim3(256), 0, pdl, st, p);
 }
 
 int launch_router(const RouterParams& p, bool pdl, cudaStream_t st) {
@@ -590,16 +584,18 @@ int launch_router(const RouterParams& p, bool pdl, cudaStream_t st) {
 
 // Expert-sorted copy of the activation rows for the tensor-core expert kernels (the reference's
 // shaders/llm_moe_perm.comp): sorted row i holds the row of token cols[i] / (used + 1).
-__global__ void __launch_bounds__(256) moe_gather_kernel(const __half* xn, const int* cols, int slots1, int H, __half* xperm) {
+__global__ void __launch_bounds__(256) moe_gather_kernel(const __half* xn, RouterParams p, __half* xperm) {
   pdl_wait();
   pdl_launch();
-  const int i = blockIdx.x;
-  const uint4* src = reinterpret_cast<const uint4*>(xn + (size_t)(cols[i] / slots1) * H);
-  uint4* dst = reinterpret_cast<uint4*>(xperm + (size_t)i * H);
-  for (int k = threadIdx.x; k < H / 8; k += 256) dst[k] = __ldcg(src + k);
+  const int slots1 = p.used + 1, n = blockIdx.x / slots1, s = blockIdx.x - n * slots1;
+  const int i = s < p.used ? p.gprob[p.topk[n * p.used + s]].y + p.pair_pos[n * p.used + s] : p.gprob[p.nE].y + n;
+  if (threadIdx.x == 0) p.cols[i] = blockIdx.x;
+  const uint4* src = reinterpret_cast<const uint4*>(xn + (size_t)n * p.H);
+  uint4* dst = reinterpret_cast<uint4*>(xperm + (size_t)i * p.H);
+  for (int k = threadIdx.x; k < p.H / 8; k += 256) dst[k] = __ldcg(src + k);
 }
-int launch_moe_gather(const __half* xn, const int* cols, int pairs, int slots1, int H, __half* xperm, bool pdl, cudaStream_t st) {
-  return launch_k(moe_gather_kernel, dim3(pairs), dim3(256), 0, pdl, st, xn, cols, slots1, H, xperm);
+int launch_moe_gather(const __half* xn, const RouterParams& p, __half* xperm, bool pdl, cudaStream_t st) {
+  return launch_k(moe_gather_kernel, dim3(p.M * (p.used + 1)), dim3(256), 0, pdl, st, xn, p, xperm);
 }
 
 // Row kernels, one CTA per row, for passes of more than QG_FUSED_ROWS rows: RMSNorm, or MoE combine + RMSNorm.
@@ -983,15 +979,16 @@ __device__ __forceinline__ float* dn_pre_gb(const DnStepParams& p, int h, int64_
 constexpr int DN_PRE_TOKENS = 64;
 constexpr int DN_CHUNK_FROM = 64;   // sequences of this many tokens and more run the chunked recurrence, shorter ones the token-by-token scan
 
-// alpha / beta projections of all rows of a pass (llm/deltanet.go:305-318): out[row][o], o = head for alpha, Hv + head
-// beta. A CTA keeps 16 rows of the normalised input in shared memory and walks a quarter of the 2*Hv weight rows once for
-// all of them (a warp per pair of weight rows, lanes along K): the weights are read once per 16 tokens, and four CTAs per 16
-// rows fill the device where one each left a 200-row pass with 13 busy SMs (126 us, now 9).
-// grid (ceil(M / 16), 4), block 256, dynamic shared memory 16 * H halves.
-constexpr int DN_AB_ROWS = 16, DN_AB_CUT = 4;
+// alpha / beta projections of all rows of a pass (llm/deltanet.go:305-318): out[row][o], o = head for alpha, Hv + head for
+// beta. A CTA keeps 16 rows of the normalised input in shared memory and takes its share of the 2*Hv weight rows; a warp takes two of
+// them at a time, or, where the CTA has fewer pairs than warps, a slice of the contraction of two. Few rows are cut finely (12 CTAs
+// that each walked 16 weight rows left a 37-row pass waiting for 20 us), many coarsely, since every CTA reads its 16 rows.
+// grid (ceil(M / 16), cut), block 256, dynamic shared memory 16 * H halves.
+constexpr int DN_AB_ROWS = 16;
 __global__ void __launch_bounds__(256) dn_ab_kernel(DnStepParams p, int M) {
   extern __shared__ __align__(16) uint8_t dn_ab_smem[];
   __half* xs = reinterpret_cast<__half*>(dn_ab_smem);
+  __shared__ float part[8][33];
   const int H = p.H, r0 = blockIdx.x * DN_AB_ROWS, nr = min(DN_AB_ROWS, M - r0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_wait();
@@ -1002,30 +999,42 @@ __global__ void __launch_bounds__(256) dn_ab_kernel(DnStepParams p, int M) {
   }
   __syncthreads();
   auto row = [&](int o) { return o < p.Hv ? p.alpha_w + (size_t)o * H : p.beta_w + (size_t)(o - p.Hv) * H; };
-  const int n_out = 2 * p.Hv, per = (n_out + DN_AB_CUT - 1) / DN_AB_CUT, o_end = min(n_out, (int)(blockIdx.y + 1) * per);
-  for (int o = blockIdx.y * per + 2 * warp; o < o_end; o += 16) {
-    const bool two = o + 1 < o_end;
-    const float *wa = row(o), *wb = row(two ? o + 1 : o);
-    float acc[2][DN_AB_ROWS];
+  const int n_out = 2 * p.Hv, per = (n_out + gridDim.y - 1) / gridDim.y, o0 = blockIdx.y * per, o_end = min(n_out, o0 + per);
+  const int pairs = (per + 1) / 2, ks = pairs >= 8 ? 1 : pairs >= 4 ? 2 : pairs >= 2 ? 4 : 8;   // warps that share a pair of weight rows
+  const int kn = (H / 128 + ks - 1) / ks * 128, k0 = (warp % ks) * kn, k1 = min(H, k0 + kn);
+  for (int b = o0; b < o_end; b += 2 * (8 / ks)) {
+    const int o = b + 2 * (warp / ks);
+    const bool one = o < o_end, two = o + 1 < o_end;
+    const float *wa = row(one ? o : o0), *wb = row(two ? o + 1 : o0);
+    float acc[32];   // [weight row][row]
 #pragma unroll
-    for (int r = 0; r < DN_AB_ROWS; r++) { acc[0][r] = 0.f; acc[1][r] = 0.f; }
-    for (int k = lane * 4; k < H; k += 128) {
+    for (int r = 0; r < 32; r++) acc[r] = 0.f;
+    for (int k = k0 + lane * 4; k < k1; k += 128) {
       const float4 va = *reinterpret_cast<const float4*>(wa + k), vb = *reinterpret_cast<const float4*>(wb + k);
 #pragma unroll
       for (int r = 0; r < DN_AB_ROWS; r++) {
         const uint2 xv = *reinterpret_cast<const uint2*>(xs + (size_t)r * H + k);
         const float2 f01 = __half22float2(*reinterpret_cast<const __half2*>(&xv.x)), f23 = __half22float2(*reinterpret_cast<const __half2*>(&xv.y));
-        acc[0][r] = fmaf(va.w, f23.y, fmaf(va.z, f23.x, fmaf(va.y, f01.y, fmaf(va.x, f01.x, acc[0][r]))));
-        acc[1][r] = fmaf(vb.w, f23.y, fmaf(vb.z, f23.x, fmaf(vb.y, f01.y, fmaf(vb.x, f01.x, acc[1][r]))));
+        acc[r] = fmaf(va.w, f23.y, fmaf(va.z, f23.x, fmaf(va.y, f01.y, fmaf(va.x, f01.x, acc[r]))));
+        acc[16 + r] = fmaf(vb.w, f23.y, fmaf(vb.z, f23.x, fmaf(vb.y, f01.y, fmaf(vb.x, f01.x, acc[16 + r]))));
       }
     }
+    // sums over the lanes: halves of the values change hands at each step, lane i ends with value i
 #pragma unroll
-    for (int h = 0; h < 2; h++)
+    for (int s = 16; s > 0; s >>= 1) {
+      const bool up = lane & s;
 #pragma unroll
-      for (int r = 0; r < DN_AB_ROWS; r++) {
-        const float v = warp_sum(acc[h][r]);
-        if (lane == 0 && r < nr && (h == 0 || two)) p.ab[(size_t)(r0 + r) * n_out + o + h] = v;
-      }
+      for (int i = 0; i < s; i++) acc[i] = (up ? acc[i + s] : acc[i]) + __shfl_xor_sync(0xffffffffu, up ? acc[i] : acc[i + s], s);
+    }
+    part[warp][lane] = acc[0];
+    __syncthreads();
+    if (warp % ks == 0) {
+      float v = 0.f;
+      for (int w = 0; w < ks; w++) v += part[warp + w][lane];
+      const int r = lane & 15, h = lane >> 4;
+      if (r < nr && (h ? two : one)) p.ab[(size_t)(r0 + r) * n_out + o + h] = v;
+    }
+    __syncthreads();
   }
 }
 
@@ -1588,7 +1597,7 @@ int launch_dn_scan(const DnStepParams& p, int M, int max_n, int* n_launches, boo
   if (p.ab == nullptr || p.H % 128 != 0 || (size_t)DN_AB_ROWS * p.H * 2 > 200 * 1024) { set_error("dn_scan: row length must be a multiple of 128 (at most 6400)"); return EINVAL_; }
   const int ab_smem = DN_AB_ROWS * p.H * 2;
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(dn_ab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  B200_TRY(launch_k(dn_ab_kernel, dim3((M + DN_AB_ROWS - 1) / DN_AB_ROWS, DN_AB_CUT), dim3(256), ab_smem, pdl, st, p, M));
+  B200_TRY(launch_k(dn_ab_kernel, dim3((M + DN_AB_ROWS - 1) / DN_AB_ROWS, M <= 256 ? 16 : 8), dim3(256), ab_smem, pdl, st, p, M));
   B200_TRY(launch_k(dn_pre_kernel, dim3(2 * p.Hk + p.Hv, p.n_seq, (max_n + DN_PRE_TOKENS - 1) / DN_PRE_TOKENS), dim3(256), 0, true, st, p));
   *n_launches = 4;
   if (max_n >= DN_CHUNK_FROM) {

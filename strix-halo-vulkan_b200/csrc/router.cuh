@@ -18,10 +18,13 @@ struct RouterParams {
   float* topk_w;       // [M][used+1] (last = sigmoid(shared gate))
   float* margin;       // [M] optional: (p_k - p_{k+1}) / p_k
   int4* entries; int* n_entries; int* cols;   // expert work list for the grouped kernels
-  int* ticket;         // [1 + ceil(M / 8)]: all rows, then one per group of eight rows
+  int* ticket;         // rows routed so far (left zero)
+  int* pair_counts;    // [nE] pairs per expert, counted while the rows are routed (left zero)
+  int* pair_pos;       // [M][used] place of a pair among its expert's, in the order of the counting
+  int gate_done;       // the router kernel has left the shared expert's gate
   int4* gprob;         // optional [nE + 1]: {expert, first sorted row, rows, first sorted row} per expert (GemmProblem), the shared expert last
   int max_entries;
-  int defer;           // 1: stop after the logits; the expert kernel that follows selects the experts itself
+  int defer;           // the expert kernel that follows selects the experts itself
   int ecols;           // columns per work-list entry (8, or 4 for passes of some tens of rows; 0 means 8)
   // expert parallelism: the work list keeps the experts [e_lo, e_hi) only (e_hi == 0: all) and makes shared-expert
   // entries for the rows [sh_lo, sh_hi) only (sh_hi == 0: all rows)

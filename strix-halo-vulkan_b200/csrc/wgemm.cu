@@ -34,10 +34,11 @@ constexpr int WG_DQ0 = 2, WG_GROUPS = 3, WG_EP0 = 14, WG_XW = 18;
 constexpr int WG_NA = 4, WG_ASLOT = 64, WG_ACC = 256;   // tensor memory: four half-block operands of 64 columns, then the accumulators
 
 template <int TYPE> __host__ __device__ constexpr int wg_raw() { return WG_TILE * (TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : TYPE == T_Q6_K ? 224 : 272); }
-template <int TYPE> __host__ __device__ constexpr int wg_nr() { return TYPE == T_Q4_K || TYPE == T_Q5_K ? 4 : 3; }
+// stages of raw weights: 256 columns need the room for activations, whose 64 KB per super-block set the pace there (83 us against 76)
+template <int NT> __host__ __device__ constexpr int wg_nr() { return NT == 256 ? 2 : 3; }
 template <int NT> __host__ __device__ constexpr int wg_xc() { return NT == 256 ? 1 : 2; }   // chunks of 64 elements per activation stage
 template <int TYPE, int NT> __host__ __device__ constexpr int wg_nx() {                     // activation stages in what the raw stages leave
-  return (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) < 8 ? (200 * 1024 - wg_nr<TYPE>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) : 8;
+  return (204 * 1024 - wg_nr<NT>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) < 8 ? (204 * 1024 - wg_nr<NT>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) : 8;
 }
 
 __device__ __forceinline__ uint32_t h2c(float v) {
@@ -179,7 +180,7 @@ template <int TYPE, int NT, int EPI>
 __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_constant__ WGemmMaps maps, const WGemmParams p) {
   constexpr bool PAIR = EPI == WG_SWIGLU;
   constexpr int TROWS = PAIR ? 64 : 128;             // output rows of a tile
-  constexpr int NR = wg_nr<TYPE>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC, NACC = NT == 256 ? 1 : 2;
+  constexpr int NR = wg_nr<NT>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC, NACC = NT == 256 ? 1 : 2;
   static_assert(NX >= 2, "two activation stages at least");
   extern __shared__ uint8_t wg_smem[];
   uint8_t* raw0 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wg_smem) + 1023) & ~(uintptr_t)1023);
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
 template <int TYPE, int NT, int EPI>
 int launch_t(const WGemmParams& p, const WGemmMaps& maps, bool pdl, cudaStream_t st) {
   auto kernel = wgemm_kernel<TYPE, NT, EPI>;
-  constexpr int smem = wg_nr<TYPE>() * wg_raw<TYPE>() + wg_nx<TYPE, NT>() * NT * 128 * wg_xc<NT>() + 1024;
+  constexpr int smem = wg_nr<NT>() * wg_raw<TYPE>() + wg_nx<TYPE, NT>() * NT * 128 * wg_xc<NT>() + 1024;
   B200_ONCE_PER_DEVICE(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int sms = sm_count_current();
   if (sms <= 0) return ECUDA;
