@@ -1625,54 +1625,64 @@ int launch_dn_step(const DnStepParams& p, bool pdl, cudaStream_t st) {
 // =========================================================================================
 // Attention pre-pass: per-head RMSNorm of q and k, NeoX partial rotary from a host-built
 // table, fp16 K/V into the cache (reference: llm/attn.go:144-184, 510-586;
-// shaders/llm_attn_pack.comp). grid (Hq + 2*Hkv, M), block hd.
+// shaders/llm_attn_pack.comp). A warp per (row, head): the norm is a warp sum and the rotary partner comes from shared
+// memory of the warp's own (a CTA per head and two barriers took 66 us for 2048 rows). grid (ceil((Hq + 2 Hkv) / 4), M), block 128.
 // =========================================================================================
-__global__ void attn_pack_kernel(AttnParams p) {
-  const int hd = p.hd, d = threadIdx.x, n = blockIdx.y, which = blockIdx.x;
-  __shared__ float buf[256], red[8];
+template <int HD>
+__global__ void __launch_bounds__(128) attn_pack_kernel(AttnParams p) {
+  constexpr int V = HD / 32;                         // dims of a lane: lane * V ..
+  const int n = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, which = blockIdx.x * 4 + warp, d0 = lane * V;
+  __shared__ __align__(16) float buf[4][HD];
   tl_mark(p.tl, 0);
-  // what the producer kernel does not write (position, slot, norm weight, rotary entry) is fetched before waiting for it
-  const int pos = p.row_pos[n], slot = p.row_slot[n];
+  // what the producer kernel does not write (position, slot, norm weight, rotary entries) is fetched before waiting for it
+  const int pos = p.row_pos[n], slot = p.row_slot[n], half = p.rope_dims / 2;
   const float* gamma = which < p.Hq ? p.q_norm : which < p.Hq + p.Hkv ? p.k_norm : nullptr;
-  const float gamma_d = gamma != nullptr ? gamma[d] : 0.f;
-  const int half = p.rope_dims / 2;
-  float2 cs = make_float2(1.f, 0.f);
-  if (gamma != nullptr && d < p.rope_dims) cs = *reinterpret_cast<const float2*>(p.rope + ((size_t)(pos + p.rope_off) * half + (d < half ? d : d - half)) * 2);
+  float ga[V];
+  float2 cs[V];
+#pragma unroll
+  for (int i = 0; i < V; i++) {
+    const int d = d0 + i;
+    ga[i] = gamma != nullptr ? gamma[d] : 0.f;
+    cs[i] = gamma != nullptr && d < p.rope_dims ? *reinterpret_cast<const float2*>(p.rope + ((size_t)(pos + p.rope_off) * half + (d < half ? d : d - half)) * 2) : make_float2(1.f, 0.f);
+  }
   pdl_wait();
   pdl_launch();
   tl_mark(p.tl, 1);
-  const float* pr = p.proj + (size_t)n * p.ldp;
-  const int kv_off = p.Hq * 2 * hd;
-  float x;
-  if (which < p.Hq) x = pr[which * 2 * hd + d];
-  else if (which < p.Hq + p.Hkv) x = pr[kv_off + (which - p.Hq) * hd + d];
-  else x = pr[kv_off + p.Hkv * hd + (which - p.Hq - p.Hkv) * hd + d];
+  if (which >= p.Hq + 2 * p.Hkv) return;
+  const float* pr = p.proj + (size_t)n * p.ldp + (which < p.Hq ? which * 2 * HD : p.Hq * 2 * HD + (which - p.Hq) * HD);   // q | gate per head, then k, then v
+  float x[V];
+#pragma unroll
+  for (int i = 0; i < V; i += 4) *reinterpret_cast<float4*>(x + i) = *reinterpret_cast<const float4*>(pr + d0 + i);
   if (gamma != nullptr) {
-    float ss = warp_sum(x * x);
-    if ((d & 31) == 0) red[d >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-    for (int w = 0; w < hd / 32; w++) tot += red[w];
-    x = x * (1.0f / sqrtf(tot / (float)hd + p.eps)) * gamma_d;
-    buf[d] = x;
-    __syncthreads();
-    if (d < p.rope_dims) {
-      const int i = d < half ? d : d - half;
-      const float x0 = buf[i], x1 = buf[i + half];
-      x = d < half ? x0 * cs.x - x1 * cs.y : x0 * cs.y + x1 * cs.x;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < V; i++) ss += x[i] * x[i];
+    const float sc = 1.0f / sqrtf(warp_sum(ss) / (float)HD + p.eps);
+#pragma unroll
+    for (int i = 0; i < V; i++) { x[i] = x[i] * sc * ga[i]; buf[warp][d0 + i] = x[i]; }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      const int d = d0 + i;
+      if (d < p.rope_dims) x[i] = d < half ? x[i] * cs[i].x - buf[warp][d + half] * cs[i].y : buf[warp][d - half] * cs[i].y + x[i] * cs[i].x;
     }
   }
-  if (which < p.Hq) p.q16[((size_t)n * p.Hq + which) * hd + d] = __float2half_rn(x);
+  __half* dst;
+  if (which < p.Hq) dst = p.q16 + ((size_t)n * p.Hq + which) * HD;
   else {
     const bool isk = which < p.Hq + p.Hkv;
     const int kh = isk ? which - p.Hq : which - p.Hq - p.Hkv;
-    __half* c = (isk ? p.kcache : p.vcache) + (size_t)slot * p.slot_stride + ((size_t)pos * p.Hkv + kh) * hd;
-    c[d] = __float2half_rn(x);
+    dst = (isk ? p.kcache : p.vcache) + (size_t)slot * p.slot_stride + ((size_t)pos * p.Hkv + kh) * HD;
   }
+#pragma unroll
+  for (int i = 0; i < V; i += 4) *reinterpret_cast<uint2*>(dst + d0 + i) = make_uint2(pack_half2(x[i], x[i + 1]), pack_half2(x[i + 2], x[i + 3]));
 }
 int launch_attn_pack(const AttnParams& p, bool pdl, cudaStream_t st) {
-  if (p.hd > 256 || p.hd % 32) { set_error("attn_pack: head dim must be a multiple of 32, at most 256"); return EINVAL_; }
-  return launch_k(attn_pack_kernel, dim3(p.Hq + 2 * p.Hkv, p.M), dim3(p.hd), 0, pdl, st, p);
+  const dim3 grid((p.Hq + 2 * p.Hkv + 3) / 4, p.M);
+  if (p.hd == 256) return launch_k(attn_pack_kernel<256>, grid, dim3(128), 0, pdl, st, p);
+  if (p.hd == 128) return launch_k(attn_pack_kernel<128>, grid, dim3(128), 0, pdl, st, p);
+  set_error("attn_pack: head dim must be 128 or 256");
+  return EINVAL_;
 }
 
 // =========================================================================================

@@ -1,12 +1,12 @@
 // tcgen05 GEMM over K-quant weights rounded to fp16 (see wgemm.cuh).
 //
-// A CTA of twenty warps walks items of 128 weight rows (or 64 gate + 64 up rows) x NT activation rows:
+// A CTA of 19 or 23 warps walks items of 128 weight rows (or 64 gate + 64 up rows) x NT activation rows:
 //   warp 0        TMA boxes of the rows' quant blocks, one super-block per ring stage;
-//   warp 18       TMA boxes of the activation rows, 128 elements per ring stage (64 for NT 256), only as many rows as the problem has;
-//   warps 2..13   three groups of four: a group turns half a super-block of the 128 rows (a thread per row) into fp16 and puts
+//   the last warp TMA boxes of the activation rows, 128 elements per ring stage (64 for NT 256), only as many rows as the problem has;
+//   warps 2..     three groups of four: a group turns half a super-block of the 128 rows (a thread per row) into fp16 and puts
 //                 it into tensor memory with tcgen05.st; the groups take the halves in turn;
 //   warp 1        one thread issues eight tcgen05.mma (M 128, N NT, K 16) per half, A from tensor memory, B from shared memory;
-//   warps 14..17  epilogue, from two accumulators in turn (one for NT 256).
+//   the others    epilogue, one or two groups of four warps.
 // What bounds it: a tcgen05.mma with M 128 and K 16 takes 68 cycles for every N up to 128 (measured), 32 weights per cycle
 // and SM, so 512 experts of 3 M weights take 180 us whatever their rows; NT 256 doubles the work per cycle. The form before
 // this one (eight dequantising warps that loaded their rows from global memory and stored the fp16 tile swizzled into shared
@@ -29,9 +29,15 @@ namespace {
 
 using namespace tc;
 
-constexpr int WG_THREADS = 640, WG_TILE = 128, WG_MAXPROB = 1025;
-constexpr int WG_DQ0 = 2, WG_GROUPS = 3, WG_EP0 = 14, WG_XW = 18;
-constexpr int WG_NA = 4, WG_ASLOT = 64, WG_ACC = 256;   // tensor memory: four half-block operands of 64 columns, then the accumulators
+constexpr int WG_TILE = 128, WG_MAXPROB = 1025;
+constexpr int WG_DQ0 = 2, WG_GROUPS = 3, WG_NA = 4, WG_ASLOT = 64;   // tensor memory: four half-block operands of 64 columns, then the accumulators
+// Two accumulators (one of 256 columns). Items of few half blocks, the down projections', are bound by draining them: a group of four
+// epilogue warps each (228 us against 198 for 2048 rows). The gated pair's items are four times as long, and there the registers of
+// more warps cost more than they gave (288 us against 323 with a fourth dequantising group and six operands instead of the second
+// accumulator): one group serves both.
+template <int NT> __host__ __device__ constexpr int wg_nacc() { return NT == 256 ? 1 : 2; }
+template <int NT, int EPI> __host__ __device__ constexpr int wg_epg() { return EPI == WG_SWIGLU ? 1 : wg_nacc<NT>(); }
+template <int NT, int EPI> __host__ __device__ constexpr int wg_threads() { return 32 * (WG_DQ0 + 4 * WG_GROUPS + 4 * wg_epg<NT, EPI>() + 1); }
 
 template <int TYPE> __host__ __device__ constexpr int wg_raw() { return WG_TILE * (TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : TYPE == T_Q6_K ? 224 : 272); }
 // stages of raw weights: 256 columns need the room for activations, whose 64 KB per super-block set the pace there (83 us against 76)
@@ -177,10 +183,11 @@ __device__ __forceinline__ bool bar_and(int id, int threads, bool v) {
 struct Item { int expert, cnt, x_row, y_row, nt, ks; };
 
 template <int TYPE, int NT, int EPI>
-__global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_constant__ WGemmMaps maps, const WGemmParams p) {
+__global__ void __launch_bounds__(wg_threads<NT, EPI>(), 1) wgemm_kernel(const __grid_constant__ WGemmMaps maps, const WGemmParams p) {
   constexpr bool PAIR = EPI == WG_SWIGLU;
   constexpr int TROWS = PAIR ? 64 : 128;             // output rows of a tile
-  constexpr int NR = wg_nr<NT>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC, NACC = NT == 256 ? 1 : 2;
+  constexpr int NR = wg_nr<NT>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC;
+  constexpr int NACC = wg_nacc<NT>(), EPG = wg_epg<NT, EPI>(), EP0 = WG_DQ0 + 4 * WG_GROUPS, XW = EP0 + 4 * EPG, ACC = WG_NA * WG_ASLOT;
   static_assert(NX >= 2, "two activation stages at least");
   extern __shared__ uint8_t wg_smem[];
   uint8_t* raw0 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wg_smem) + 1023) & ~(uintptr_t)1023);
@@ -280,7 +287,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
     }
     if (failed)                                      // leave only once the copies in flight have landed
       for (uint32_t k = it > (uint32_t)NR ? it - NR : 0; k < it; k++) mbar_wait(&r_full[k % NR], (k / NR) & 1);
-  } else if (warp == WG_XW) {
+  } else if (warp == XW) {
     // ---- activation rows ------------------------------------------------------------------------
     uint32_t it = 0;
     for (int n = 0; n < n_items && !stopped(); n++) {
@@ -308,7 +315,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
       const Item t = item(n);
       const int n_half = 2 * (sb_begin(t.ks + 1) - sb_begin(t.ks));
       const uint32_t id = idesc_n((t.cnt + 15) & ~15);
-      const uint32_t acc = tm + WG_ACC + (ci % NACC) * NT;
+      const uint32_t acc = tm + ACC + (ci % NACC) * NT;
       if (!warp_wait(&c_empty[ci % NACC], ((ci / NACC) & 1) ^ 1)) { give_up(); break; }
       for (int h = 0; h < n_half && ok; h++, hx++) {
         const int as = hx % WG_NA;
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
         }
       }
     }
-  } else if (warp < WG_EP0) {
+  } else if (warp < EP0) {
     // ---- dequantisation ---------------------------------------------------------------------------
     const int grp = (warp - WG_DQ0) >> 2, q = warp & 3, row = q * 32 + lane;
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16);
@@ -367,14 +374,15 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
       }
       it0 += nsb; hx0 += 2 * nsb;
     }
-  } else if (warp < WG_XW) {
+  } else if (warp < XW) {
     // ---- epilogue -----------------------------------------------------------------------------------
-    const int q = warp & 3;
-    const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16) + WG_ACC;
-    uint32_t ci = 0;
+    const int q = warp & 3, eg = (warp - EP0) >> 2;    // with two groups, group eg drains accumulator eg
+    const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16) + ACC;
     int exb = 0;
-    for (int n = 0; n < n_items; n++, ci++) {
+    for (int n = 0; n < n_items; n++) {
       const Item t = item(n);
+      if (EPG == 2 && (n & 1) != eg) continue;
+      const uint32_t ci = n;
       const int cnt = t.cnt;
       // output row of column c0 + lane, fetched by the lanes side by side ahead of its use and handed round by shuffles
       auto row_of = [&](int c0) {
@@ -416,7 +424,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
             const float o = e[(up * 64 + r) * 17 + i], own = __uint_as_float(up ? v[16 + i] : v[i]);
             const float gv = up ? o : own, uv = up ? own : o;
             const int yr = __shfl_sync(0xffffffffu, my_row, up * 16 + i);
-            if (up * 16 + i < live && orow < p.N) p.y16[(int64_t)yr * p.ldy + orow] = __float2half_rn(gv * sigmoid_acc(gv) * uv);
+            if (up * 16 + i < live && orow < p.N) p.y16[(uint64_t)(uint32_t)yr * (uint32_t)p.ldy + orow] = __float2half_rn(gv * sigmoid_acc(gv) * uv);
           }
         } else {
           const int orow = t.nt * 128 + q * 32 + lane;
@@ -424,7 +432,7 @@ __global__ void __launch_bounds__(WG_THREADS, 1) wgemm_kernel(const __grid_const
 #pragma unroll
           for (int i = 0; i < 32; i++) {
             const int yr = __shfl_sync(0xffffffffu, my_row, i);
-            if (i < live && orow < p.N) y[(int64_t)yr * p.ldy] = __uint_as_float(v[i]);
+            if (i < live && orow < p.N) y[(uint64_t)(uint32_t)yr * (uint32_t)p.ldy] = __uint_as_float(v[i]);
           }
         }
       }
@@ -445,7 +453,7 @@ int launch_t(const WGemmParams& p, const WGemmMaps& maps, bool pdl, cudaStream_t
   const int n_tiles = (p.N + (EPI == WG_SWIGLU ? 63 : 127)) / (EPI == WG_SWIGLU ? 64 : 128);
   const int64_t total = ((int64_t)(p.max_count + NT - 1) / NT + (p.problems != nullptr ? p.n_problems : 0)) * n_tiles * p.ksplit;   // every problem rounds up once at most
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(total, sms))); cfg.blockDim = dim3(WG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(total, sms))); cfg.blockDim = dim3(wg_threads<NT, EPI>()); cfg.dynamicSmemBytes = smem; cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
