@@ -21,7 +21,8 @@ constexpr int QL_ENT = 64;   // entries one CTA's share may touch
 template <int TYPE, int NC> struct QlCfg {
   static constexpr int BLK = TYPE == T_Q4_K ? 144 : 176, BYTES = 16 * BLK;   // a ring slot: 16 rows x one super-block, rows BLK apart
   static constexpr int WARPS = 12;                                           // 168 registers a thread; sixteen warps of 128 measured the same
-  static constexpr int SLOTS = 216 * 1024 / WARPS / BYTES < 8 ? 216 * 1024 / WARPS / BYTES : 8;
+  static constexpr int AHEAD = 216 * 1024 / WARPS / BYTES >= 8 ? 2 : 1;      // super-blocks (four chunks) in the ring
+  static constexpr int SLOTS = 4 * AHEAD;
 };
 
 __device__ __forceinline__ void tma_box(uint32_t dst, const void* tm, int c0, int c1, uint64_t* bar) {
@@ -63,33 +64,36 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
 
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(ql_smem) + warp * (SLOTS * Cf::BYTES);
   const int n_units = u0 + warp < u1 ? (u1 - u0 - warp + Cf::WARPS - 1) / Cf::WARPS : 0;
-  // ---- the copy side walks the chunks (unit, super-block, j) ahead of the arithmetic ----
-  int f_left = n_units * nb * 4, f_unit = u0 + warp, f_sb = 0, f_j = 0, f_slot = 0, f_row = 0;
+  // ---- the copy side walks the super-blocks AHEAD of the arithmetic; a chunk's slot and its place in the unit are constants of j ----
+  int f_left = n_units * nb, f_unit = u0 + warp, f_sb = 0, f_row = 0;
   const void *fa = nullptr, *fb = nullptr;
-  auto fetch = [&](bool reused) {   // the whole warp keeps the position, one lane asks
-    if (f_left == 0) return;
-    f_left--;
-    if (f_sb == 0 && f_j == 0) {
-      const int e = f_unit / upe, ex = ent[e - e0].x;
-      f_row = (ex >= 0 ? ex * p.N : 0) + (f_unit - e * upe) * UROWS;
-      fa = ex >= 0 ? &maps.w : &maps.ws;
-      fb = !PAIR ? fa : ex >= 0 ? &maps.w2 : &maps.ws2;
-    }
-    if (elect_one()) {
-      if (reused) fence_proxy_async();
-      mbar_expect_tx(&bars[warp][f_slot], Cf::BYTES);
-      tma_box(ring + f_slot * Cf::BYTES, (f_j & 1) ? fb : fa, f_sb * Cf::BLK, f_row + (PAIR ? f_j >> 1 : f_j) * 16, &bars[warp][f_slot]);
-    }
-    if (++f_j == 4) { f_j = 0; if (++f_sb == nb) { f_sb = 0; f_unit += Cf::WARPS; } }
-    f_slot = f_slot + 1 == SLOTS ? 0 : f_slot + 1;
+  auto locate = [&]() {   // the unit that is fetched from now on
+    const int e = min(f_unit, u1 - 1) / upe, ex = ent[e - e0].x;
+    f_row = (ex >= 0 ? ex * p.N : 0) + (f_unit - e * upe) * UROWS;
+    fa = ex >= 0 ? &maps.w : &maps.ws;
+    fb = !PAIR ? fa : ex >= 0 ? &maps.w2 : &maps.ws2;
   };
-  for (int i = 0; i < SLOTS; i++) fetch(false);
+  auto fetch = [&](int slot, int j, bool reused) {   // chunk j of super-block f_sb
+    if (f_left > 0 && elect_one()) {
+      if (reused) fence_proxy_async();
+      mbar_expect_tx(&bars[warp][slot], Cf::BYTES);
+      tma_box(ring + slot * Cf::BYTES, (j & 1) ? fb : fa, f_sb * Cf::BLK, f_row + (PAIR ? j >> 1 : j) * 16, &bars[warp][slot]);
+    }
+  };
+  auto fetched = [&]() {   // a super-block's four chunks are on their way
+    if (f_left > 0) { f_left--; if (++f_sb == nb) { f_sb = 0; f_unit += Cf::WARPS; if (f_left > 0) locate(); } }
+  };
+  if (n_units > 0) locate();
+  for (int i = 0; i < Cf::AHEAD; i++) {
+    for (int j = 0; j < 4; j++) fetch(4 * i + j, j, false);
+    fetched();
+  }
 
   // mma row g is row 2g of a chunk, mma row g + 8 row 2g + 1: at a pitch of 144 or 176 bytes the eight-byte reads of four
   // neighbouring g then fall on distinct banks
   const uint32_t row_off = 2 * g * Cf::BLK;
   const uint32_t min_sel = 0x4040u | (2 * (t >> 1)) | ((2 * (t >> 1) + 1) << 8);   // two mins of this thread's pair as magic halves
-  int slot = 0, phase = 0;
+  uint32_t done = 0;   // super-blocks
   for (int i = 0; i < n_units; i++) {
     const int u = u0 + warp + i * Cf::WARPS, e = u / upe, tile = u - e * upe, le = e - e0, cnt = ent[le].z;
     const __half *xp[NC], *sp[NC];
@@ -115,7 +119,8 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
     };
     load_b(0, 0, 8);
 #pragma unroll 1
-    for (int sb = 0; sb < nb; sb++) {
+    for (int sb = 0; sb < nb; sb++, done++) {
+      const int slot0 = Cf::AHEAD == 2 ? (done & 1) * 4 : 0, phase = Cf::AHEAD == 2 ? (done >> 1) & 1 : done & 1;
       uint32_t sx0[NC], sx1[NC];
 #pragma unroll
       for (int nc = 0; nc < NC; nc++) {
@@ -124,9 +129,14 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
       }
 #pragma unroll
       for (int j = 0; j < 4; j++) {
+        const int slot = slot0 + j;
         if (!warp_wait(&bars[warp][slot], phase)) {   // a copy never landed: report, the results are void
           if (lane == 0) report_error(p.err);
-          for (int k = 1; k < SLOTS; k++) mbar_wait(&bars[warp][(slot + k) % SLOTS], phase ^ (slot + k >= SLOTS));   // leave with no copy in flight
+          // leave with no copy in flight: this super-block's other chunks, the next one's before this
+          for (int k = 0; k < SLOTS; k++) {
+            const bool ahead = Cf::AHEAD == 2 && (k >> 2) != (slot0 >> 2);
+            mbar_wait(&bars[warp][k], ahead ? (done + 1) >> 1 & 1 : k - slot0 < j ? phase ^ 1 : phase, 1u << 18);
+          }
           return;
         }
         const uint32_t base = ring + slot * Cf::BYTES + row_off;
@@ -190,9 +200,9 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
           }
         }
         __syncwarp();   // every lane has read the chunk
-        fetch(true);
-        if (++slot == SLOTS) { slot = 0; phase ^= 1; }
+        fetch(slot, j, true);
       }
+      fetched();
     }
     if constexpr (PAIR) {
       // SwiGLU (shaders/llm_moe_gemv.comp:777-781); the 32 rows are one sub-block of the down projection's input
