@@ -564,8 +564,48 @@ __global__ void __launch_bounds__(256) route_rows_kernel(RouterParams p) {
   if (tid == 0) *p.ticket = 0;
   build_work_list(p, counts, offs, eoff);
 }
+// The same with a warp per row, for passes whose rows fill the device anyway: a CTA per row spends more instructions, most of them
+// repeated in its eight warps. grid ceil(M / 8), block 256.
+__global__ void __launch_bounds__(256) route_many_kernel(RouterParams p) {
+  __shared__ int is_last;
+  __shared__ float2 cand[8][32];
+  __shared__ int counts[1025], offs[1025], eoff[1025];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, H = p.H, n = blockIdx.x * 8 + warp, used = p.used;
+  pdl_wait();
+  pdl_launch();
+  if (n < p.M) {
+    if (!p.gate_done) {
+      const __half* x = p.xn + (size_t)n * H;
+      float acc = 0.f;
+      for (int k = lane * 8; k < H; k += 256) {
+        uint4 xv = *reinterpret_cast<const uint4*>(x + k);
+        const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w};
+        float4 g0 = *reinterpret_cast<const float4*>(p.sh_gate + k), g1 = *reinterpret_cast<const float4*>(p.sh_gate + k + 4);
+        acc = fmaf(g0.x, h2f_lo(xw[0]), acc); acc = fmaf(g0.y, h2f_hi(xw[0]), acc); acc = fmaf(g0.z, h2f_lo(xw[1]), acc); acc = fmaf(g0.w, h2f_hi(xw[1]), acc);
+        acc = fmaf(g1.x, h2f_lo(xw[2]), acc); acc = fmaf(g1.y, h2f_hi(xw[2]), acc); acc = fmaf(g1.z, h2f_lo(xw[3]), acc); acc = fmaf(g1.w, h2f_hi(xw[3]), acc);
+      }
+      acc = warp_sum(acc);
+      if (lane == 0) p.topk_w[(size_t)n * (used + 1) + used] = sigmoid_acc(acc);
+    }
+    if (p.nE <= 512) route_token<16>(p, n, lane, true, cand[warp]);
+    else route_token<32>(p, n, lane, true, cand[warp]);
+    __syncwarp();
+    if (p.entries != nullptr && lane < used) p.pair_pos[(size_t)n * used + lane] = atomicAdd(p.pair_counts + __ldcg(p.topk + (size_t)n * used + lane), 1);
+  }
+  if (p.entries == nullptr) return;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) is_last = (atomicAdd(p.ticket, 1) == (int)gridDim.x - 1);
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  if (tid == 0) *p.ticket = 0;
+  build_work_list(p, counts, offs, eoff);
+}
+constexpr int ROUTE_MANY_FROM = 512;   // rows: from here on a warp per row fills the device
 int launch_route_rows(const RouterParams& p, bool pdl, cudaStream_t st) {
   if (p.nE > 1024 || p.used > 32 || p.H % 8 || p.xn == nullptr || p.pair_pos == nullptr) { set_error("route_rows: shape outside kernel limits"); return ECAPACITY; }
+  if (p.M >= ROUTE_MANY_FROM) return launch_k(route_many_kernel, dim3((p.M + 7) / 8), dim3(256), 0, pdl, st, p);
   return p.nE <= 512 ? launch_k(route_rows_kernel<2>, dim3(p.M), dim3(256), 0, pdl, st, p) : launch_k(route_rows_kernel<4>, dim3(p.M), dim3(256), 0, pdl, st, p);
 }
 
@@ -1083,11 +1123,12 @@ __global__ void __launch_bounds__(256) dn_pre_kernel(DnStepParams p) {
       *reinterpret_cast<float4*>(dn_pre_qk(p, hd, row) + 128 * kind + c) = v;
     } else {
       *reinterpret_cast<float4*>(dn_pre_v(p, hd, row) + c) = v;
-      if (lane == 0) {
-        const float alpha = __ldcg(p.ab + (size_t)row * 2 * p.Hv + hd), betar = __ldcg(p.ab + (size_t)row * 2 * p.Hv + p.Hv + hd);
-        *reinterpret_cast<float2*>(dn_pre_gb(p, hd, row)) = make_float2(expf(softplus_ref(alpha + dtb) * a_h), sigmoid_acc(betar));
-      }
     }
+  }
+  if (kind == 2 && lane < 8 && i0 + lane < i1) {   // decay and beta of the eight tokens, a lane each (one lane for all of them took half of the kernel)
+    const int row = sq.row0 + i0 + lane;
+    const float alpha = __ldcg(p.ab + (size_t)row * 2 * p.Hv + hd), betar = __ldcg(p.ab + (size_t)row * 2 * p.Hv + p.Hv + hd);
+    *reinterpret_cast<float2*>(dn_pre_gb(p, hd, row)) = make_float2(expf(softplus_ref(alpha + dtb) * a_h), sigmoid_acc(betar));
   }
 }
 

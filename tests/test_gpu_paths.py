@@ -29,11 +29,11 @@ def test_projection_of_at_most_eight_rows(pkg, orc, typ, rows, k, m):
     assert np.abs(got - want).max() <= (1e-3 if typ == 14 else 1e-5) * max(np.abs(want).max(), 1e-3)
 
 
-@pytest.mark.parametrize("n", [9, 15, 16, 17, 63, 64, 65, 127, 128, 129, 193, 257])
+@pytest.mark.parametrize("n", [9, 15, 16, 17, 63, 64, 65, 127, 128, 129, 193, 257, 513])
 def test_one_pass_is_the_passes_of_eight_rows(pkg, tiny, n):
     ids = ids_of(tiny, n, 20 + n)
-    want, _ = pkg.Graph(tiny, n_kv=320, max_tokens=8, use_cuda_graph=False).forward(ids)
-    big = pkg.Graph(tiny, n_kv=320, max_tokens=320, use_cuda_graph=False)
+    want, _ = pkg.Graph(tiny, n_kv=640, max_tokens=8, use_cuda_graph=False).forward(ids)
+    big = pkg.Graph(tiny, n_kv=640, max_tokens=640, use_cuda_graph=False)
     got, _ = big.forward(ids)
     r = compare(got, want)
     # the bounds of fp16-rounded weights with a router near-tie (as for the 300-row pass)
