@@ -44,7 +44,7 @@ int launch_row_tail(const TailParams& tp, bool pdl, cudaStream_t st);
 int launch_concat_norm(const float* e, const float* hs, const float* enorm, const float* hnorm, float eps, int H, int M, __half* xcat, bool pdl, cudaStream_t st);
 
 int launch_router(const RouterParams& p, bool pdl, cudaStream_t st);
-// selection + work list only, for passes whose logits come from launch_qgemm (the shared gate is computed here)
+// selection + work list only, for passes whose logits are in place (with the shared gate, unless the router left it)
 bool router_mma_fits(const RouterParams& p);
 int launch_router_mma(const RouterParams& p, bool pdl, cudaStream_t st);
 int launch_route_rows(const RouterParams& p, bool pdl, cudaStream_t st);
