@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
           for (int i = 0; i < 8; i++) { g[4 * i] = gn[i].x; g[4 * i + 1] = gn[i].y; g[4 * i + 2] = gn[i].z; g[4 * i + 3] = gn[i].w; }
           if (j + 32 < HD) ask(j + 32);
 #pragma unroll
-          for (int i = 0; i < 32; i++) o[i] = __fdividef(o[i], fmaf(l, __expf(fminf(-g[i], 80.f)), l));
+          for (int i = 0; i < 32; i++) o[i] = o[i] / fmaf(l, expf(-g[i]), l);
 #pragma unroll
           for (int i = 0; i < 32; i += 8)
             *reinterpret_cast<uint4*>(dst + j + i) = make_uint4(half2_of(o[i], o[i + 1]), half2_of(o[i + 2], o[i + 3]), half2_of(o[i + 4], o[i + 5]), half2_of(o[i + 6], o[i + 7]));
