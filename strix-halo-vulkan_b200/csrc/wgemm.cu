@@ -42,6 +42,17 @@ template <int NT, int EPI> __host__ __device__ constexpr int wg_threads() { retu
 template <int TYPE> __host__ __device__ constexpr int wg_raw() { return WG_TILE * (TYPE == T_Q4_K ? 144 : TYPE == T_Q5_K ? 176 : TYPE == T_Q6_K ? 224 : 272); }
 // stages of raw weights: 256 columns need the room for activations, whose 64 KB per super-block set the pace there (83 us against 76)
 template <int NT> __host__ __device__ constexpr int wg_nr() { return NT == 256 ? 2 : 3; }
+// A group has a half in two super-blocks of three. A wait by parity takes a stage's copy before last for the wanted one while the copy
+// between them is on its way, so a group has to see every copy of the stages it waits on. With as many stages as groups all that
+// it skips lies in one stage, which it never waits on; with another number every group waits for every super-block and gives its stage back.
+template <int NT> __host__ __device__ constexpr bool wg_all_wait() { return wg_nr<NT>() != WG_GROUPS; }
+__host__ __device__ constexpr uint32_t wg_half(uint32_t it, uint32_t grp) { return (grp + (WG_GROUPS - 2) * it) % WG_GROUPS; }   // group grp's half of super-block `it`; none if above 1
+__host__ __device__ constexpr bool wg_sees_all(int nr, bool all_wait) {
+  for (int g = 0; g < WG_GROUPS; g++)
+    for (int it = nr; it < nr + nr * WG_GROUPS; it++)
+      if (!all_wait && wg_half(it, g) < 2 && wg_half(it - nr, g) > 1) return false;
+  return true;
+}
 template <int NT> __host__ __device__ constexpr int wg_xc() { return NT == 256 ? 1 : 2; }   // chunks of 64 elements per activation stage
 template <int TYPE, int NT> __host__ __device__ constexpr int wg_nx() {                     // activation stages in what the raw stages leave
   return (204 * 1024 - wg_nr<NT>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) < 8 ? (204 * 1024 - wg_nr<NT>() * wg_raw<TYPE>()) / (NT * 128 * wg_xc<NT>()) : 8;
@@ -189,6 +200,7 @@ __global__ void __launch_bounds__(wg_threads<NT, EPI>(), 1) wgemm_kernel(const _
   constexpr int NR = wg_nr<NT>(), NX = wg_nx<TYPE, NT>(), RAW = wg_raw<TYPE>(), XC = wg_xc<NT>(), XST = NT * 128 * XC;
   constexpr int NACC = wg_nacc<NT>(), EPG = wg_epg<NT, EPI>(), EP0 = WG_DQ0 + 4 * WG_GROUPS, XW = EP0 + 4 * EPG, ACC = WG_NA * WG_ASLOT;
   static_assert(NX >= 2, "two activation stages at least");
+  static_assert(wg_sees_all(NR, wg_all_wait<NT>()), "a group would wait on a stage whose copy before last it has not seen");
   extern __shared__ uint8_t wg_smem[];
   uint8_t* raw0 = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(wg_smem) + 1023) & ~(uintptr_t)1023);
   uint8_t* x0 = raw0 + NR * RAW;
@@ -200,7 +212,7 @@ __global__ void __launch_bounds__(wg_threads<NT, EPI>(), 1) wgemm_kernel(const _
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    for (int s = 0; s < NR; s++) { mbar_init(&r_full[s], 1); mbar_init(&r_empty[s], 8); }
+    for (int s = 0; s < NR; s++) { mbar_init(&r_full[s], 1); mbar_init(&r_empty[s], wg_all_wait<NT>() ? 4 * WG_GROUPS : 8); }
     for (int s = 0; s < NX; s++) { mbar_init(&x_full[s], 1); mbar_init(&x_empty[s], 1); }
     for (int s = 0; s < WG_NA; s++) { mbar_init(&a_full[s], 4); mbar_init(&a_empty[s], 1); }
     for (int s = 0; s < NACC; s++) { mbar_init(&c_full[s], 1); mbar_init(&c_empty[s], 4); }
@@ -343,18 +355,23 @@ __global__ void __launch_bounds__(wg_threads<NT, EPI>(), 1) wgemm_kernel(const _
     // ---- dequantisation ---------------------------------------------------------------------------
     const int grp = (warp - WG_DQ0) >> 2, q = warp & 3, row = q * 32 + lane;
     const uint32_t lane_base = tm + ((uint32_t)(q * 32) << 16);
-    uint32_t it0 = 0, hx0 = 0;                       // super-blocks and halves before this item
+    uint32_t it = 0;                                 // super-blocks of all items
     bool ok = true;
     for (int n = 0; n < n_items && ok && !stopped(); n++) {
       const Item t = item(n);
-      const int sb0 = sb_begin(t.ks), nsb = sb_begin(t.ks + 1) - sb0;
-      for (uint32_t hx = hx0 + (grp + WG_GROUPS - hx0 % WG_GROUPS) % WG_GROUPS; hx < hx0 + 2 * nsb; hx += WG_GROUPS) {
-        const int b = (hx - hx0) >> 1, half = (hx - hx0) & 1, as = hx % WG_NA;
-        const uint32_t it = it0 + b;
-        const int s = it % NR;
+      const int sb0 = sb_begin(t.ks), sb1 = sb_begin(t.ks + 1);
+      for (int sb = sb0; sb < sb1; sb++, it++) {
+        const int s = it % NR, half = wg_half(it, grp);
+        if (half > 1 && !wg_all_wait<NT>()) continue;
         if (!warp_wait(&r_full[s], (it / NR) & 1)) { give_up(); ok = false; break; }
+        if (half > 1) {
+          if (lane == 0) arrive(&r_empty[s]);
+          continue;
+        }
+        const uint32_t hx = 2 * it + half;
+        const int as = hx % WG_NA;
         HalfBlock<TYPE> v;
-        v.load(raw0 + s * RAW, row, half, (nb * 208 + (sb0 + b) * 2) & 15);
+        v.load(raw0 + s * RAW, row, half, (nb * 208 + sb * 2) & 15);
         __syncwarp();
         if (lane == 0) arrive(&r_empty[s]);
         bool waited = false;
@@ -372,7 +389,6 @@ __global__ void __launch_bounds__(wg_threads<NT, EPI>(), 1) wgemm_kernel(const _
         __syncwarp();
         if (lane == 0) arrive(&a_full[as]);
       }
-      it0 += nsb; hx0 += 2 * nsb;
     }
   } else if (warp < XW) {
     // ---- epilogue -----------------------------------------------------------------------------------
