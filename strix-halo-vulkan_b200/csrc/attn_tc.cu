@@ -211,11 +211,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
         tmem_st32(lanes + TS + (k & 1) * AT_CELLS + 32 * hf, w);
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      // The tile before is in O, and every warp has seen so: a wait by parity would take the product before last for the last one, at the
+      // end and for the pieces below. (Free: the tensor core has the scores of the next tile to form after it.)
+      if (k > 0 && !(ok = warp_wait(&pv_done, (k - 1) & 1))) { give_up(); break; }
       if (cb + AT_CELLS > c_hi) {
         // value rows past the end hold whatever the cache held: weight zero is not enough against an infinity
         const int live = c_hi - cb;
-        // (the tile before is done with its pieces, or a slot's older phase could pass for the one waited for)
-        if (k > 0 && !(ok = warp_wait(&pv_done, (k - 1) & 1))) { give_up(); break; }
         for (int h = 0; h < VPC && ok; h++) {
           const uint32_t v = v_piece(k) + h;
           if (!(ok = warp_wait(&full[v % AT_NP], (v / AT_NP) & 1))) { give_up(); break; }

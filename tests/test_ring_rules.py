@@ -124,3 +124,57 @@ def test_two_stages_want_every_group_at_every_super_block():
     _, groups, na, _ = wgemm_numbers()
     with pytest.raises(AssertionError, match="reads super-block"):
         explore(lambda rng: wgemm_agents(rng, 2, groups, na, False), 400)
+
+
+# ---- attn_tc.cu: the softmax warps and the products of probabilities and values --------------------------------------------------------
+def attn_agents(rng, nt, every_tile):
+    s_full, p_full, pv_done = [Bar(1), Bar(1)], [Bar(4), Bar(4)], Bar(1)
+    queue, done = [], [0]                      # the tensor core's work in order; products PV in O
+
+    def forever():
+        while True:
+            yield lambda: bool(queue)
+            kind, k = queue.pop(0)
+            yield always
+            if kind == "scores":
+                s_full[k & 1].arrive()
+            else:
+                done[0] = k + 1
+                yield always
+                pv_done.arrive()
+
+    def issue():
+        queue.append(("scores", 0))
+        for k in range(nt):
+            if k + 1 < nt:
+                queue.append(("scores", k + 1))
+            yield lambda: p_full[k & 1].passed(k >> 1 & 1)
+            queue.append(("values", k))
+
+    def softmax():
+        for k in range(nt):
+            yield lambda: s_full[k & 1].passed(k >> 1 & 1)
+            if k > 0 and rng.random() < 0.3:   # a maximum grew: O is rescaled
+                yield lambda: pv_done.passed((k - 1) & 1)
+                assert done[0] == k, f"O rescaled at tile {k} holds {done[0]} products"
+            if k > 0 and every_tile:
+                yield lambda: pv_done.passed((k - 1) & 1)
+                assert done[0] == k
+            yield always
+            p_full[k & 1].arrive()
+        yield lambda: pv_done.passed((nt - 1) & 1)
+        assert done[0] == nt, f"O read with {done[0]} of {nt} products"
+
+    return [forever(), issue()] + [softmax() for _ in range(4)]
+
+
+@pytest.mark.parametrize("nt", [1, 2, 3, 4, 7])
+def test_attention_reads_o_after_its_last_product(nt):
+    s = source("attn_tc.cu")
+    wait = s.find("      if (k > 0 && !(ok = warp_wait(&pv_done, (k - 1) & 1)))")
+    explore(lambda rng: attn_agents(rng, nt, 0 <= wait < s.find("if (cb + AT_CELLS > c_hi)")), 400)
+
+
+def test_attention_warps_want_every_product():
+    with pytest.raises(AssertionError, match="O read with"):
+        explore(lambda rng: attn_agents(rng, 4, False), 400)
