@@ -246,7 +246,14 @@ int32_t b200_qgemv(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
  * many-row passes; tile_rows = activation rows per tile (64, 128 or 256). The reference's prefill GEMM
  * arithmetic: dequantised weights rounded to fp16 (shaders/llm_gemm.comp MODE 2). */
 int32_t b200_qgemm(uint32_t type, const void* host_w, int64_t rows, int64_t k, const float* host_x, int32_t m, int32_t tile_rows, float* host_y);
-/* No counterpart in the reference. The same projection for callers that cannot allocate device
+/* The gated DeltaNet recurrence of one new sequence of `rows` tokens (at least 2) as a many-row pass runs it: conv + SiLU, L2 norms,
+ * gates, delta rule (llm/deltanet.go:305-418), everything f32. proj [rows][(2 heads_k + 2 heads_v) * 128] is the projected input
+ * q | k | v | z, x [rows][n_embd] the normalised block input (rounded to fp16 as the pass holds it); alpha_w, beta_w [heads_v][n_embd],
+ * conv_w [channels][4], ssm_a and dt_bias [heads_v]. state [heads_v][128][128] goes in and comes back; out [rows][heads_v * 128] is the
+ * read-out before the gated norm. */
+int32_t b200_deltanet(int32_t heads_k, int32_t heads_v, int32_t n_embd, int32_t rows, const float* proj, const float* x, const float* alpha_w,
+                      const float* beta_w, const float* conv_w, const float* ssm_a, const float* dt_bias, float* state, float* out);
+/* No counterpart in the reference. The projection of b200_qgemv for callers that cannot allocate device
  * memory when they need it: a latency-critical thread that must not block on the allocator's lock
  * (cudaMalloc / cudaFree serialise on it and may synchronise the device), or a process whose
  * device memory was budgeted up front. All pointers are DEVICE pointers the caller already owns;

@@ -432,6 +432,42 @@ int32_t b200_qgemv_static(uint32_t type, const void* dev_w, int64_t rows, int64_
   return qgemv_static(type, dev_w, rows, k, dev_x, m, dev_y);
 }
 
+int32_t b200_deltanet(int32_t heads_k, int32_t heads_v, int32_t n_embd, int32_t rows, const float* proj, const float* x, const float* alpha_w,
+                      const float* beta_w, const float* conv_w, const float* ssm_a, const float* dt_bias, float* state, float* out) {
+  B200_TRY(need_device());
+  if (!proj || !x || !alpha_w || !beta_w || !conv_w || !ssm_a || !dt_bias || !state || !out) { set_error("deltanet: null argument"); return EINVAL_; }
+  if (heads_k < 1 || heads_v < 1 || heads_v > 256 || heads_v % heads_k || n_embd < 256 || n_embd % 256 || rows < 2 || rows > 4096) { set_error("deltanet: 2..4096 rows, heads_v a multiple of heads_k, n_embd of 256"); return EINVAL_; }
+  const size_t D = 128, Hk = heads_k, Hv = heads_v, M = rows, H = n_embd, cw = (2 * Hk + Hv) * D, ld = cw + Hv * D;
+  Scratch sc;
+  auto in = [&](const float* src, size_t n, float** dst) -> int {
+    B200_TRY(sc.get(dst, n * sizeof(float)));
+    B200_CUDA(cudaMemcpy(*dst, src, n * sizeof(float), cudaMemcpyHostToDevice));
+    return (int)OK;
+  };
+  float *d_proj, *d_x, *d_a, *d_b, *d_conv, *d_ssm, *d_dt, *d_state, *d_norm;
+  B200_TRY(in(proj, M * ld, &d_proj)); B200_TRY(in(x, M * H, &d_x)); B200_TRY(in(alpha_w, Hv * H, &d_a)); B200_TRY(in(beta_w, Hv * H, &d_b));
+  B200_TRY(in(conv_w, cw * 4, &d_conv)); B200_TRY(in(ssm_a, Hv, &d_ssm)); B200_TRY(in(dt_bias, Hv, &d_dt)); B200_TRY(in(state, Hv * D * D, &d_state));
+  const std::vector<float> ones(D, 1.f);
+  B200_TRY(in(ones.data(), D, &d_norm));
+  DnStepParams p{};
+  __half* x16 = nullptr; SeqDesc* seqs = nullptr;
+  B200_TRY(sc.get(&x16, M * H * sizeof(__half))); B200_TRY(sc.get(&p.y16, M * Hv * D * sizeof(__half))); B200_TRY(sc.get(&seqs, sizeof(SeqDesc)));
+  p.ring_slot_stride = (int64_t)(Hv * 4 * DN_RING * DN_RING_W);
+  B200_TRY(sc.get(&p.ring, p.ring_slot_stride * sizeof(float))); B200_TRY(sc.get(&p.pre, M * (Hk * 256 + Hv * 130) * sizeof(float)));
+  B200_TRY(sc.get(&p.wy, M * Hv * 192 * sizeof(float))); B200_TRY(sc.get(&p.o_raw, M * Hv * D * sizeof(float))); B200_TRY(sc.get(&p.ab, M * 2 * Hv * sizeof(float)));
+  const SeqDesc seq{0, 0, rows, 0};
+  B200_CUDA(cudaMemcpy(seqs, &seq, sizeof(seq), cudaMemcpyHostToDevice));
+  B200_TRY(quantize_rows_device(T_F16, d_x, rows, n_embd, (uint8_t*)x16, 0));
+  p.proj = d_proj; p.ldp = (int64_t)ld; p.xn = x16; p.alpha_w = d_a; p.beta_w = d_b; p.conv_w = d_conv; p.ssm_a = d_ssm; p.dt_bias = d_dt;
+  p.state = d_state; p.state_slot_stride = (int64_t)(Hv * D * D); p.seqs = seqs; p.n_seq = 1; p.norm_w = d_norm; p.pre_rows = rows;
+  p.H = n_embd; p.Hk = heads_k; p.Hv = heads_v; p.D = 128; p.conv = 4; p.eps = 1e-6f;
+  int launches = 0;
+  B200_TRY(launch_dn_scan(p, rows, rows, &launches, false, 0));
+  B200_CUDA(cudaMemcpy(out, p.o_raw, M * Hv * D * sizeof(float), cudaMemcpyDeviceToHost));
+  B200_CUDA(cudaMemcpy(state, d_state, Hv * D * D * sizeof(float), cudaMemcpyDeviceToHost));
+  return OK;
+}
+
 int32_t b200_quantize(uint32_t type, const float* host_src, int64_t rows, int64_t k, void* host_dst) {
   B200_TRY(need_device());
   const int64_t rb = gguf_row_bytes(type, k);

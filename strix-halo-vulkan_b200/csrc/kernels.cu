@@ -1227,10 +1227,13 @@ __global__ void __launch_bounds__(128) dn_scan_kernel(DnStepParams p) {
 // leaves dn_chunk_kernel, which walks the chunks, three products against the 32 state rows a CTA owns.
 //
 // The state and the recurrence are f32 throughout in the reference's device path, so the products run as split TF32: every
-// operand is hi + lo with hi rounded to TF32 and lo the exact rest, and hi hi + (hi lo + lo hi) is accumulated in f32, an
-// error of 2^-22 relative per product, that of an f32 dot product of this length. mma.sync TF32 runs at 500 multiply-adds per
-// cycle and SM, three to one here: 1.3 times the FMA pipe, at a tenth of its shared-memory reads, which is what bounded the
-// register-tiled form. 4096 tokens, 32 heads: 1706 us as one kernel on the FMA pipe.
+// operand is hi + lo with hi rounded to TF32 and lo the exact rest, and hi hi + (hi lo + lo hi) is accumulated in f32; the
+// logarithms L are summed and subtracted in f64, since their differences are what exp magnifies. Against the recurrence in f64 (2048
+// tokens, 32 heads, relative 2-norm of the outputs / of the state): 2.3e-7 / 1.7e-7 with decays as config.py draws them, 2.6e-7 / 3.1e-7
+// with a hundredth of their logarithms. The form before (f32 on the FMA pipe, f32 logarithms): 8.9e-7 / 6.3e-7 and 2.4e-7 / 3.1e-7; hi hi
+// summed by the tensor core: 4.4e-7 / 1.7e-7 and 4.7e-7 / 4.1e-7. mma.sync TF32 runs at 500 multiply-adds per cycle and SM, three to one
+// here: 1.3 times the FMA pipe, at a tenth of its shared-memory reads, which is what bounded the register-tiled form.
+// 4096 tokens, 32 heads: 1706 us as one kernel on the FMA pipe.
 // -----------------------------------------------------------------------------------------
 constexpr int DN_C = 64;                            // tokens per chunk
 // pitches (floats) of shared-memory rows: 16-byte reads of rows g at 16 kk + 4 t want 16 mod 32, 4-byte reads of rows t at
@@ -1258,9 +1261,12 @@ __device__ __forceinline__ TfB tf_b(float b0, float b1) {
   tf_split(b0, r.hi[0], r.lo[0]); tf_split(b1, r.hi[1], r.lo[1]);
   return r;
 }
-// main += hi hi, cross += hi lo + lo hi (two chains, so neither waits for the other)
+// main += hi hi, cross += hi lo + lo hi. The large term's sum is an f32 addition, not the tensor core's own, which rounds towards zero.
 __device__ __forceinline__ void mma_split(float (&main)[4], float (&cross)[4], const TfA& a, const TfB& b) {
-  mma_tf32(main, a.hi, b.hi[0], b.hi[1]);
+  float m[4] = {0.f, 0.f, 0.f, 0.f};
+  mma_tf32(m, a.hi, b.hi[0], b.hi[1]);
+#pragma unroll
+  for (int i = 0; i < 4; i++) main[i] += m[i];
   mma_tf32(cross, a.hi, b.lo[0], b.lo[1]);
   mma_tf32(cross, a.lo, b.hi[0], b.hi[1]);
 }
@@ -1308,8 +1314,8 @@ __global__ void __launch_bounds__(512, 1) dn_wy_kernel(DnStepParams p) {
   float* QK = KK + DN_C * DN_P4;
   float* Am = QK + DN_C * DN_P4;
   float* Tm = Am + DN_C * DN_P4;                // lower blocks: T; upper blocks: scratch
-  float* Lg = Tm + DN_C * DN_P4;                // [64] cumulative log decay
-  float* Bt = Lg + DN_C;                        // [64] beta
+  double* Lg = reinterpret_cast<double*>(Tm + DN_C * DN_P4);   // [64] cumulative log decay
+  float* Bt = Tm + DN_C * DN_P4 + 2 * DN_C;     // [64] beta
   float* Gm = Bt + DN_C;                        // [64] beta Gamma
   pdl_wait();
   pdl_launch();
@@ -1339,14 +1345,14 @@ __global__ void __launch_bounds__(512, 1) dn_wy_kernel(DnStepParams p) {
       float2 e0 = make_float2(1.f, 0.f), e1 = e0;
       if (t0 < n) e0 = __ldcg(reinterpret_cast<const float2*>(dn_pre_gb(p, h, row0 + t0)));
       if (t1 < n) e1 = __ldcg(reinterpret_cast<const float2*>(dn_pre_gb(p, h, row0 + t1)));
-      const float l0 = fmaxf(logf(e0.x), -87.f), l1 = fmaxf(logf(e1.x), -87.f);
-      float run = l0 + l1;                      // inclusive scan over the lanes' pair sums
+      const double l0 = fmaxf(logf(e0.x), -87.f), l1 = fmaxf(logf(e1.x), -87.f);
+      double run = l0 + l1;                     // inclusive scan over the lanes' pair sums
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const float up = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += up; }
-      const float total = __shfl_sync(0xffffffffu, run, 31), la = run - l1;
-      Lg[t0] = la; Lg[t1] = run; Bt[t0] = e0.y; Bt[t1] = e1.y; Gm[t0] = e0.y * expf(la); Gm[t1] = e1.y * expf(run);
-      if (t0 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t0)) = make_float2(expf(la), expf(total - la));
-      if (t1 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t1)) = make_float2(expf(run), expf(total - run));
+      for (int o = 1; o < 32; o <<= 1) { const double up = __shfl_up_sync(0xffffffffu, run, o); if (lane >= o) run += up; }
+      const double total = __shfl_sync(0xffffffffu, run, 31), la = run - l1;
+      Lg[t0] = la; Lg[t1] = run; Bt[t0] = e0.y; Bt[t1] = e1.y; Gm[t0] = e0.y * expf((float)la); Gm[t1] = e1.y * expf((float)run);
+      if (t0 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t0)) = make_float2(expf((float)la), expf((float)(total - la)));
+      if (t1 < n) *reinterpret_cast<float2*>(dn_pre_gb(p, h, row0 + t1)) = make_float2(expf((float)run), expf((float)(total - run)));
     }
     for (int i = tid; i < DN_C * 32; i += 512) {
       const int r = i >> 5, c = i & 31;
@@ -1356,7 +1362,7 @@ __global__ void __launch_bounds__(512, 1) dn_wy_kernel(DnStepParams p) {
     __syncthreads();
     for (int i = tid; i < DN_C * DN_C; i += 512) {
       const int r = i >> 6, c = i & 63;
-      const float ratio = c <= r ? expf(Lg[r] - Lg[c]) : 0.f;
+      const float ratio = c <= r ? expf((float)(Lg[r] - Lg[c])) : 0.f;
       Am[r * DN_P4 + c] = c < r ? Bt[r] * ratio * KK[r * DN_P4 + c] : 0.f;
       if (r < n) dn_w(p, h, row0 + r)[c] = c <= r ? ratio * QK[r * DN_P4 + c] : 0.f;
     }

@@ -397,6 +397,16 @@ def qgemm(typ, w, rows, k, x, tile_rows=64):
     return y
 
 
+def deltanet(heads_k, proj, x, alpha_w, beta_w, conv_w, ssm_a, dt_bias, state):
+    """The DeltaNet recurrence of one new sequence as a many-row pass runs it: (read-outs [rows][heads_v * 128], state after it)."""
+    a = [np.ascontiguousarray(v, dtype=np.float32) for v in (proj, x, alpha_w, beta_w, conv_w, ssm_a, dt_bias)]
+    state = np.array(state, dtype=np.float32, order="C")
+    rows, heads_v = a[0].shape[0], a[2].shape[0]
+    out = np.empty((rows, heads_v * 128), dtype=np.float32)
+    _lib.check(_lib.load().b200_deltanet(heads_k, heads_v, a[1].shape[1], rows, *(v.ctypes.data for v in a), state.ctypes.data, out.ctypes.data))
+    return out, state
+
+
 def quantize(typ, x):
     x = np.ascontiguousarray(x, dtype=np.float32)
     rows, k = int(np.prod(x.shape[:-1])), x.shape[-1]
