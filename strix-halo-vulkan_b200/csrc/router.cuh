@@ -60,6 +60,15 @@ __device__ __forceinline__ int route_token(const RouterParams& p, int n, int lan
     pv[i] = lane + 32 * i < nE ? pv[i] * inv : -1.f;
     if (write && p.probs != nullptr && lane + 32 * i < nE) p.probs[(size_t)n * nE + lane + 32 * i] = pv[i];
   }
+  // Logits that are not finite leave no probabilities to order: the first experts then, with weights that show it. The ids index
+  // counters, work lists and weights without further checks, so they lie in [0, nE) whatever the logits.
+  if (!(sum > 0.f)) {
+    if (write) {
+      if (lane < used) { p.topk[(size_t)n * used + lane] = lane; p.topk_w[(size_t)n * (used + 1) + lane] = inv; }
+      if (lane == 0 && p.margin) p.margin[n] = 0.f;
+    }
+    return want_slot < used ? want_slot : -1;
+  }
   // top-k by descending probability, ties to the lower index (llm/moe.go:249-252). The (used + 1)-th largest of the 32 lanes' own
   // maxima bounds the selection from below, and hardly more than used + 1 values reach that bound: those are put side by side, one
   // per lane in index order, and each finds its rank by comparing with all the others. (Eleven rounds of a warp-wide maximum over
@@ -207,7 +216,7 @@ __device__ __forceinline__ int route_row_cta(const RouterParams& p, int n, const
   }
   __syncthreads();
   const int nc = sm.n_cand;
-  if (nc > 32 || nc <= used) {   // many equal values (or none comparable): the one-warp form
+  if (nc > 32 || nc <= used) {   // many equal values, or none comparable (a NaN among the sums leaves no candidate): the one-warp form
     if (warp == 0) {
       const int ex = p.nE <= 512 ? route_token<16>(p, n, lane, write, sm.cand, want_slot) : route_token<32>(p, n, lane, write, sm.cand, want_slot);
       if (lane == 0) sm.expert = ex;
