@@ -141,21 +141,25 @@ __device__ __forceinline__ uint32_t half2_const(float v) {
 // Block: d, dmin (fp16), 12 bytes of packed 6-bit (scale, min), for Q5_K 32 bytes of fifth bits, 128 bytes of nibbles
 // (reference: gguf/dequant.go:238-318); 32 bytes of nibbles hold two sub-blocks, the even one low. Thread t of a quad takes
 // bytes 8t .. 8t + 7 of each such group, so that one mma step lies within one sub-block.
-// Quants enter the tensor core as they are: four or five bits in the low end of a half are the subnormal q * 2^-24, exactly,
+// Quants enter the tensor core as they are: four or five bits below a half's exponent are a subnormal q * 2^-s, exactly,
 // so a pair of weights costs one mask and no conversion, no multiply; the sub-block scale is applied to the f32 result of
-// the sub-block's two mma steps, the 2^24 (and the 16 of a high nibble left in place) with the block scale.
+// the sub-block's two mma steps, the 2^s (and the 16 of a high nibble left where it is) with the block scale.
+// How far below matters: the tensor core aligns products by the operands' exponents and a subnormal's bits lie under its own, so at
+// 2^-24 an mma has an error of 4.1e-7, at 2^-22 of 5e-8 and from 2^-20 on of 8e-9 (16 products of 0..15 with normal values). Q4_K
+// takes 2^-22 and 2^-18 with one shift more per word than 2^-24 and 2^-20, Q5_K 2^-21.
 // lo: sub-block 2G, hi: 2G + 1; of a word's four bytes the pairs are (0, 2) and (1, 3).
 template <int TYPE>
 __device__ __forceinline__ void unpack_word(uint32_t w, uint32_t fifth, int G, uint32_t& l02, uint32_t& l13, uint32_t& h02, uint32_t& h13) {
   if constexpr (TYPE == T_Q4_K) {
-    const uint32_t w8 = w >> 8;
-    l02 = w & 0x000F000Fu; h02 = w & 0x00F000F0u; l13 = w8 & 0x000F000Fu; h13 = w8 & 0x00F000F0u;
+    const uint32_t even = w << 2, odd = w >> 6;
+    l02 = even & 0x003C003Cu; h02 = even & 0x03C003C0u; l13 = odd & 0x003C003Cu; h13 = odd & 0x03C003C0u;
   } else {   // fifth bits: bit 2G of a byte belongs to its low nibble, bit 2G + 1 to the high one
     const uint32_t f = fifth >> (2 * G);
-    const uint32_t lo = (w & 0x0F0F0F0Fu) | ((f << 4) & 0x10101010u), hi = ((w >> 4) & 0x0F0F0F0Fu) | ((f << 3) & 0x10101010u);
-    l02 = lo & 0x00FF00FFu; l13 = (lo >> 8) & 0x00FF00FFu; h02 = hi & 0x00FF00FFu; h13 = (hi >> 8) & 0x00FF00FFu;
+    const uint32_t lo = ((w << 3) & 0x78787878u) | ((f << 7) & 0x80808080u), hi = ((w >> 1) & 0x78787878u) | ((f << 6) & 0x80808080u);
+    l02 = lo & 0x00F800F8u; l13 = (lo >> 8) & 0x00F800F8u; h02 = hi & 0x00F800F8u; h13 = (hi >> 8) & 0x00F800F8u;
   }
 }
+template <int TYPE> __device__ __forceinline__ constexpr float unit_scale() { return TYPE == T_Q4_K ? 4194304.f : 2097152.f; }   // 2^s of a low nibble
 // D = A B, no accumulator in
 __device__ __forceinline__ void mma16816_z(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
@@ -209,7 +213,7 @@ __device__ __forceinline__ void k45_accumulate(float (&acc)[4], uint32_t ra, uin
                           mins_half2(((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u), sel)};
   float Cm[4];
   mma16816_z(Cm, am, sx0, sx1);
-  const float d0 = h2f_lo(h0.x) * 16777216.f, n0 = h2f_hi(h0.x), d1 = h2f_lo(h1.x) * 16777216.f, n1 = h2f_hi(h1.x);
+  const float d0 = h2f_lo(h0.x) * unit_scale<TYPE>(), n0 = h2f_hi(h0.x), d1 = h2f_lo(h1.x) * unit_scale<TYPE>(), n1 = h2f_hi(h1.x);
   acc[0] = fmaf(-n0, Cm[0], fmaf(d0, a[0], acc[0])); acc[1] = fmaf(-n0, Cm[1], fmaf(d0, a[1], acc[1]));
   acc[2] = fmaf(-n1, Cm[2], fmaf(d1, a[2], acc[2])); acc[3] = fmaf(-n1, Cm[3], fmaf(d1, a[3], acc[3]));
 }

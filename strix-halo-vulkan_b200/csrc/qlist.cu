@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(QlCfg<TYPE, NC>::WARPS * 32, 1) qlist_kernel(c
         const uint32_t am[4] = {hadd2_u(__byte_perm(h0.z & 0x3F3F3F3Fu, 0x64646464u, min_sel), half2_const(-1024.f)), hadd2_u(__byte_perm(h1.z & 0x3F3F3F3Fu, 0x64646464u, min_sel), half2_const(-1024.f)),
                                 hadd2_u(__byte_perm(((h0.w >> 4) & 0x0F0F0F0Fu) | ((h0.z >> 2) & 0x30303030u), 0x64646464u, min_sel), half2_const(-1024.f)),
                                 hadd2_u(__byte_perm(((h1.w >> 4) & 0x0F0F0F0Fu) | ((h1.z >> 2) & 0x30303030u), 0x64646464u, min_sel), half2_const(-1024.f))};
-        const float d0 = h2f_lo(h0.x) * 16777216.f, n0 = h2f_hi(h0.x), d1 = h2f_lo(h1.x) * 16777216.f, n1 = h2f_hi(h1.x);
+        const float d0 = h2f_lo(h0.x) * unit_scale<TYPE>(), n0 = h2f_hi(h0.x), d1 = h2f_lo(h1.x) * unit_scale<TYPE>(), n1 = h2f_hi(h1.x);
 #pragma unroll
         for (int nc = 0; nc < NC; nc++) {
           if (nc == 0 || wide) {
