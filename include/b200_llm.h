@@ -253,6 +253,12 @@ int32_t b200_qgemm(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
  * read-out before the gated norm. */
 int32_t b200_deltanet(int32_t heads_k, int32_t heads_v, int32_t n_embd, int32_t rows, const float* proj, const float* x, const float* alpha_w,
                       const float* beta_w, const float* conv_w, const float* ssm_a, const float* dt_bias, float* state, float* out);
+/* Gated causal attention of `rows` (16 at least) query rows at the last positions of a context of `cells` cells, as a many-row pass of one
+ * sequence runs it (llm/attn.go:190-217, shaders/llm_attn_wmma.comp): q and gate [rows][n_head][head_dim] (q after norm and rotary),
+ * k and v [cells][n_head_kv][head_dim]; q, k and v are rounded to fp16 as the pass and the cache hold them, out [rows][n_head][head_dim]
+ * comes back as the fp16 values the next projection reads. parts: into how many the keys may be cut, where the rows leave SMs idle. */
+int32_t b200_attention(int32_t n_head, int32_t n_head_kv, int32_t head_dim, int32_t rows, int32_t cells, int32_t parts, const float* q, const float* k,
+                       const float* v, const float* gate, float* out);
 /* No counterpart in the reference. The projection of b200_qgemv for callers that cannot allocate device
  * memory when they need it: a latency-critical thread that must not block on the allocator's lock
  * (cudaMalloc / cudaFree serialise on it and may synchronise the device), or a process whose

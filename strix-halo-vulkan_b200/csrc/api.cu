@@ -379,7 +379,7 @@ static int finish_projection(const char* who, const float* y, const int* err, in
   int herr = 0;
   B200_CUDA(cudaMemcpy(&herr, err, sizeof(int), cudaMemcpyDeviceToHost));
   if (herr != 0) { set_error(std::string(who) + ": a bounded wait gave up"); return ETIMEOUT; }
-  B200_CUDA(cudaMemcpy(host_y, y, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
+  if (n > 0) B200_CUDA(cudaMemcpy(host_y, y, (size_t)n * sizeof(float), cudaMemcpyDeviceToHost));
   return OK;
 }
 
@@ -430,6 +430,49 @@ int32_t b200_qgemm(uint32_t type, const void* host_w, int64_t rows, int64_t k, c
 int32_t b200_qgemv_static(uint32_t type, const void* dev_w, int64_t rows, int64_t k, const float* dev_x, int32_t m, float* dev_y) {
   B200_TRY(need_device());
   return qgemv_static(type, dev_w, rows, k, dev_x, m, dev_y);
+}
+
+int32_t b200_attention(int32_t n_head, int32_t n_head_kv, int32_t head_dim, int32_t rows, int32_t cells, int32_t parts, const float* q, const float* k,
+                       const float* v, const float* gate, float* out) {
+  B200_TRY(need_device());
+  if (!q || !k || !v || !gate || !out) { set_error("attention: null argument"); return EINVAL_; }
+  if (n_head < 1 || n_head_kv < 1 || n_head % n_head_kv || !attn_tc_shape(n_head, n_head_kv, head_dim) || rows < 16 || rows > 4096 || cells < rows || cells > (1 << 20) || parts < 1 || parts > 64) {
+    set_error("attention: 16..4096 rows, rows..2^20 cells, 8 query heads per KV head of 256 dims or 4 of 128, 1..64 parts");
+    return EINVAL_;
+  }
+  const size_t M = rows, N = cells, Hq = n_head, Hkv = n_head_kv, hd = head_dim;
+  Scratch sc;
+  auto half_rows = [&](const float* src, size_t r, size_t w, __half** dst) -> int {
+    float* f = nullptr;
+    B200_TRY(sc.get(&f, r * w * sizeof(float))); B200_TRY(sc.get(dst, r * w * sizeof(__half)));
+    B200_CUDA(cudaMemcpy(f, src, r * w * sizeof(float), cudaMemcpyHostToDevice));
+    return quantize_rows_device(T_F16, f, (int64_t)r, (int64_t)w, (uint8_t*)*dst, 0);
+  };
+  AttnParams p{};
+  B200_TRY(half_rows(q, M, Hq * hd, &p.q16)); B200_TRY(half_rows(k, N, Hkv * hd, &p.kcache)); B200_TRY(half_rows(v, N, Hkv * hd, &p.vcache));
+  std::vector<float> proj(M * Hq * 2 * hd, 0.f);   // per head q | gate
+  for (size_t i = 0; i < M * Hq; i++) memcpy(&proj[(2 * i + 1) * hd], gate + i * hd, hd * sizeof(float));
+  std::vector<int> at(2 * M, 0);                   // slots, then positions
+  for (size_t i = 0; i < M; i++) at[M + i] = (int)(N - M + i);
+  float* d_proj = nullptr; int *d_at = nullptr, *err = nullptr;
+  B200_TRY(sc.get(&d_proj, proj.size() * sizeof(float))); B200_TRY(sc.get(&d_at, at.size() * sizeof(int))); B200_TRY(sc.get(&err, sizeof(int)));
+  B200_TRY(sc.get(&p.ctx16, M * Hq * hd * sizeof(__half)));
+  const int64_t room = parts > 1 ? (int64_t)(M * Hq * (hd + 2)) * parts : 0;
+  B200_TRY(sc.get(&p.partial, (size_t)room * sizeof(float)));
+  B200_CUDA(cudaMemcpy(d_proj, proj.data(), proj.size() * sizeof(float), cudaMemcpyHostToDevice));
+  B200_CUDA(cudaMemcpy(d_at, at.data(), at.size() * sizeof(int), cudaMemcpyHostToDevice));
+  B200_CUDA(cudaMemset(err, 0, sizeof(int)));
+  p.proj = d_proj; p.ldp = (int64_t)(Hq * 2 * hd); p.slot_stride = (int64_t)(N * Hkv * hd); p.row_slot = d_at; p.row_pos = d_at + M;
+  p.M = rows; p.Hq = n_head; p.Hkv = n_head_kv; p.hd = head_dim; p.n_kv = cells; p.err = err;
+  AttnTcMaps maps{};
+  B200_TRY(make_attn_maps(p.q16, rows, n_head, p.kcache, p.vcache, cells, n_head_kv, head_dim, &maps));
+  B200_TRY(launch_attn_tc(p, maps, cells - 1, room, false, 0));
+  if (p.nsplit > 0) B200_TRY(launch_attn_merge(p, false, 0));
+  std::vector<__half> h(M * Hq * hd);
+  B200_TRY(finish_projection("attention", nullptr, err, 0, nullptr));
+  B200_CUDA(cudaMemcpy(h.data(), p.ctx16, h.size() * sizeof(__half), cudaMemcpyDeviceToHost));
+  for (size_t i = 0; i < h.size(); i++) out[i] = __half2float(h[i]);
+  return OK;
 }
 
 int32_t b200_deltanet(int32_t heads_k, int32_t heads_v, int32_t n_embd, int32_t rows, const float* proj, const float* x, const float* alpha_w,

@@ -6,8 +6,10 @@
 //   warp 0     TMA: the query tile once, then keys and values in pieces of 32 KB through a ring of four;
 //   warp 1     one thread issues S = Q K^T of tile k + 1, then O += P V of tile k, so the tensor core works while tile k's softmax runs;
 //   warps 2-5  a thread per row: maximum, exponentials, row sum, and the result.
-// O is rescaled only when a row's maximum has grown by more than a factor of 2^8 since it was last adopted: until then the
-// probabilities are up to 256 instead of up to 1, which fp16 carries as exactly, and nothing is approximated.
+// O is rescaled whenever a row's maximum has grown, after the tile's exponentials, while the tensor core forms the next scores: the largest
+// probability is then exactly 1, which fp16 carries without error, and the row sum is of the probabilities as fp16 carries them, so that
+// part of what rounds them drops out of the quotient. Against f64 with peaked scores 2.17e-4 (fp16 of the exact result: 2.08e-4); with a
+// maximum kept until it had grown by 2^8, and the unrounded sum, 2.71e-4. 2048 rows take the same time either way.
 // What bounds it: a step of 128 rows x 128 cells is 2500 cycles of tcgen05.mma and 128 KB of keys and values out of L2, about as long
 // (the KV heads' tiles are read once per query tile). With mma.sync (16 rows a warp, keys and values through shared memory for every
 // warp) 2048 rows over 2 to 4 thousand cells took 752 us, this takes 117; 46 us are the tensor core's floor.
@@ -175,28 +177,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
         for (int i = 0; i < 4; i++) mx[i] = fmaxf(mx[i], s[i][j]);
       const float mn = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
-      if (k == 0) {
-        m = mn;
-      } else {
-        const bool grown = (mn - m) * c > 8.f;
-        if (__any_sync(0xffffffffu, grown)) {
-          const float f = grown ? ex2((m - mn) * c) : 1.f;
-          if (!(ok = warp_wait(&pv_done, (k - 1) & 1))) { give_up(); break; }
-          fence_after();
-#pragma unroll 1
-          for (int j = 0; j < HD; j += 32) {
-            float o[32];
-            tmem_ld32(lanes + TO + j, o);
-            tmem_ld_wait();
-            uint32_t w[32];
-#pragma unroll
-            for (int i = 0; i < 32; i++) w[i] = __float_as_uint(o[i] * f);
-            tmem_st32(lanes + TO + j, w);
-          }
-          l *= f;
-          if (grown) m = mn;
-        }
-      }
+      const bool grown = mn > m;
+      const float f = grown ? ex2((m - mn) * c) : 1.f;
+      m = mn;
       const float mc = m == -INFINITY ? 0.f : m * c;
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -205,15 +188,29 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc_kernel(const __grid_con
 #pragma unroll
         for (int j = 0; j < 32; j++) {
           const float a = ex2(fmaf(s[2 * hf + (j >> 4)][(2 * j) & 31], c, -mc)), b = ex2(fmaf(s[2 * hf + (j >> 4)][((2 * j) & 31) + 1], c, -mc));
-          sum[j & 3] += a + b;
           w[j] = half2_of(a, b);
+          const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
+          sum[j & 3] += r.x + r.y;
         }
         tmem_st32(lanes + TS + (k & 1) * AT_CELLS + 32 * hf, w);
       }
-      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      l = fmaf(l, f, (sum[0] + sum[1]) + (sum[2] + sum[3]));
       // The tile before is in O, and every warp has seen so: a wait by parity would take the product before last for the last one, at the
       // end and for the pieces below. (Free: the tensor core has the scores of the next tile to form after it.)
       if (k > 0 && !(ok = warp_wait(&pv_done, (k - 1) & 1))) { give_up(); break; }
+      if (k > 0 && __any_sync(0xffffffffu, grown)) {
+        fence_after();
+#pragma unroll 1
+        for (int j = 0; j < HD; j += 32) {
+          float o[32];
+          tmem_ld32(lanes + TO + j, o);
+          tmem_ld_wait();
+          uint32_t w[32];
+#pragma unroll
+          for (int i = 0; i < 32; i++) w[i] = __float_as_uint(o[i] * f);
+          tmem_st32(lanes + TO + j, w);
+        }
+      }
       if (cb + AT_CELLS > c_hi) {
         // value rows past the end hold whatever the cache held: weight zero is not enough against an infinity
         const int live = c_hi - cb;

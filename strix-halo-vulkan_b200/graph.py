@@ -397,6 +397,15 @@ def qgemm(typ, w, rows, k, x, tile_rows=64):
     return y
 
 
+def attention(q, k, v, gate, parts=1):
+    """Gated causal attention of query rows [rows][heads][dims] at the end of a context [cells][kv heads][dims], as a many-row pass runs it."""
+    a = [np.ascontiguousarray(x, dtype=np.float32) for x in (q, k, v, gate)]
+    rows, heads, dims = a[0].shape
+    out = np.empty_like(a[0])
+    _lib.check(_lib.load().b200_attention(heads, a[1].shape[1], dims, rows, a[1].shape[0], parts, *(x.ctypes.data for x in a), out.ctypes.data))
+    return out
+
+
 def deltanet(heads_k, proj, x, alpha_w, beta_w, conv_w, ssm_a, dt_bias, state):
     """The DeltaNet recurrence of one new sequence as a many-row pass runs it: (read-outs [rows][heads_v * 128], state after it)."""
     a = [np.ascontiguousarray(v, dtype=np.float32) for v in (proj, x, alpha_w, beta_w, conv_w, ssm_a, dt_bias)]

@@ -120,6 +120,7 @@ SYMBOLS = {
     "b200_qgemv": (I32, [U32, P, I64, I64, P, I32, P]),
     "b200_qgemv_static": (I32, [U32, P, I64, I64, P, I32, P]),
     "b200_qgemm": (I32, [U32, P, I64, I64, P, I32, I32, P]),
+    "b200_attention": (I32, [I32, I32, I32, I32, I32, I32, P, P, P, P, P]),
     "b200_deltanet": (I32, [I32, I32, I32, I32, P, P, P, P, P, P, P, P, P]),
     "b200_quantize": (I32, [U32, P, I64, I64, P]),
 }
