@@ -695,6 +695,9 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   const bool to_logits = direct && (out_logits == nullptr || out_logits_mapped);
   const bool to_h = direct && (f.want_residual ? n_lr == M && (out_resid == nullptr || out_resid_mapped) : f.want_hidden);
   *(PassOut*)stage = PassOut{to_logits ? lg_dst : logits, !to_h ? nullptr : f.want_residual ? rs_dst + (size_t)resid_off * c.n_embd : hidden_host, f.want_residual ? 0 : n_lr - 1, 0};
+  // From here on the stream reads and writes memory of the caller's: no return before it is done with that.
+  struct DrainOnError { cudaStream_t st; bool ok; ~DrainOnError() { if (!ok) cudaStreamSynchronize(st); } } drain{st, false};
+  if (f.hs != nullptr) B200_CUDA(cudaMemcpyAsync(hs_buf, f.hs, (size_t)M * c.n_embd * sizeof(float), cudaMemcpyHostToDevice, st));
   B200_CUDA(cudaEventRecord(ev0, st));
   if (single) {
     const int gkey = M * 2 + (ep_on ? 1 : 0);
@@ -726,6 +729,7 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   }
   B200_CUDA(cudaEventRecord(ev1, st));
   B200_TRY(finish_pass());
+  drain.ok = true;
   last_rows = M;
   float ms = 0.f;
   B200_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
@@ -863,13 +867,11 @@ int Graph::draft_rows(const float* hs, const int32_t* ids, int n, int vocab_k, c
   if (vocab_k <= 0 || vocab_k > c.vocab) vocab_k = c.vocab;
   if (vocab_k % 16) { set_error("draft_rows: vocab_k must be a multiple of 16"); return EINVAL_; }
   if (draft_past[dcur] + n + 1 > o.n_kv) { set_error("draft_rows: the draft cache is full"); return ECAPACITY; }
-  B200_CUDA(cudaSetDevice(m->device));
-  B200_CUDA(cudaMemcpyAsync(hs_buf, hs, (size_t)n * c.n_embd * sizeof(float), cudaMemcpyHostToDevice, st));
   draft_vocab = vocab_k;
   std::vector<int> slots(n, dcur), pos(n), lrows(n);
   for (int i = 0; i < n; i++) { pos[i] = draft_past[dcur] + i; lrows[i] = i; }
   std::vector<SeqDesc> sq{SeqDesc{dcur, 0, n, draft_past[dcur]}};
-  PassFlags f; f.draft = true; f.want_all_logits = true; f.want_residual = true;
+  PassFlags f; f.draft = true; f.want_all_logits = true; f.want_residual = true; f.hs = hs;
   resid_off = 0;
   B200_TRY(run_rows(ids, slots.data(), pos.data(), n, sq, lrows, f));
   draft_past[dcur] += n;

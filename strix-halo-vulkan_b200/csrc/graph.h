@@ -19,6 +19,7 @@ struct PassFlags {
   bool greedy = false;            // argmax + advance on the device (no host traffic)
   bool draft = false;             // the pass runs the draft layer only
   bool want_hidden = true;        // copy the last row's residual to the host (when not every row's)
+  const float* hs = nullptr;      // draft: the rows' previous residuals, host memory
 };
 
 struct Graph {

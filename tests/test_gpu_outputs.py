@@ -1,0 +1,40 @@
+"""Caller-owned buffers of a pass: which calls touch them, what a refusal leaves behind, the cache of pinned blocks."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import modelgen
+from modelgen import config
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def model(pkg):
+    return pkg.Model.open(modelgen.cached_gguf(config.variant(config.TINY, name="tiny-draft", vocab=4096, has_draft=1)))
+
+
+def ids_of(model, n, seed):
+    return np.random.default_rng(seed).integers(0, model.cfg["vocab"], n).astype(np.int32)
+
+
+def test_a_refused_draft_call_does_not_read_the_rows(pkg, model):
+    """The rows' copy is asynchronous when they are pinned, so a call that is refused may not have begun it: the caller is free to give the
+    memory back. Here it lies in a page that cannot be read at all."""
+    libc = ctypes.CDLL(None)
+    libc.mmap.restype, libc.mmap.argtypes = ctypes.c_void_p, [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_long]
+    page = libc.mmap(None, 1 << 16, 0, 0x22, -1, 0)   # PROT_NONE, MAP_PRIVATE | MAP_ANONYMOUS
+    assert page and page != ctypes.c_void_p(-1).value
+    g, L = pkg.Graph(model, n_kv=64, max_tokens=16), pkg.lib.load()
+    lg, rs = ctypes.c_void_p(), ctypes.c_void_p()
+    bad = np.array([model.cfg["vocab"]], dtype=np.int32)
+    assert L.b200_draft_rows(g._h, page, bad.ctypes.data, 1, 0, ctypes.byref(rs), ctypes.byref(lg)) == pkg.lib.EINVAL
+    small = np.empty(16, dtype=np.float32)
+    good = ids_of(model, 1, 0)
+    pkg.lib.check(L.b200_graph_set_outputs(g._h, small.ctypes.data, small.size, None, 0))
+    assert L.b200_draft_rows(g._h, page, good.ctypes.data, 1, 0, ctypes.byref(rs), ctypes.byref(lg)) == pkg.lib.ECAPACITY
+    assert g.draft_past() == 0
+    h = np.random.default_rng(1).standard_normal((1, model.cfg["n_embd"])).astype(np.float32)
+    got, want = g.draft_rows(h, good), pkg.Graph(model, n_kv=64, max_tokens=16).draft_rows(h, good)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
