@@ -78,11 +78,15 @@ HostPool& host_pool() {
   return *pool;
 }
 
-// The output buffers a caller has set hold for one call, however it ends.
+// The output buffers a caller has set hold for one call, however it ends: made before the call looks at its arguments.
 struct OutputsForOneCall {
-  Graph& g;
-  explicit OutputsForOneCall(Graph& graph) : g(graph) {}
-  ~OutputsForOneCall() { g.out_logits = g.out_resid = nullptr; g.out_logits_cap = g.out_resid_cap = 0; }
+  b200_graph* g;
+  explicit OutputsForOneCall(b200_graph* graph) : g(graph) {}
+  ~OutputsForOneCall() {
+    if (g == nullptr) return;
+    g->g.out_logits = g->g.out_resid = nullptr;
+    g->g.out_logits_cap = g->g.out_resid_cap = 0;
+  }
 };
 }  // namespace
 
@@ -179,40 +183,40 @@ int32_t b200_graph_set_outputs(b200_graph* g, float* logits, int64_t logit_float
   return OK;
 }
 int32_t b200_graph_forward(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {
+  OutputsForOneCall once(g);
   if (!g || !ids) { set_error("forward: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   B200_TRY(g->g.reset_slot(g->g.cur));
   PassFlags f;
   return g->g.extend(ids, n, f, logits, hidden);
 }
 int32_t b200_graph_extend(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {
+  OutputsForOneCall once(g);
   if (!g || !ids) { set_error("extend: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   PassFlags f;
   return g->g.extend(ids, n, f, logits, hidden);
 }
 int32_t b200_graph_extend_input(b200_graph* g, const b200_input* in, const float** logits, const float** hidden) {
+  OutputsForOneCall once(g);
   if (!g || !in || !in->ids) { set_error("extend_input: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   if (in->n_images != 0) { set_error("extend_input: this library has no vision tower; inputs with images are refused"); return EINVAL_; }
   PassFlags f;
   return g->g.extend(in->ids, in->n, f, logits, hidden);
 }
 int32_t b200_graph_extend_rows(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** residual) {
+  OutputsForOneCall once(g);
   if (!g || !ids) { set_error("extend_rows: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   PassFlags f; f.want_all_logits = true; f.want_residual = true; f.spec = g->g.speculating;
   return g->g.extend(ids, n, f, logits, residual);
 }
 int32_t b200_graph_extend_residual(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** residual) {
+  OutputsForOneCall once(g);
   if (!g || !ids) { set_error("extend_residual: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   PassFlags f; f.want_residual = true;
   return g->g.extend(ids, n, f, logits, residual);
 }
 int32_t b200_graph_decode_rows(b200_graph* g, const int32_t* slots, const int32_t* ids, int32_t n, const float** logits) {
+  OutputsForOneCall once(g);
   if (!g || !slots || !ids) { set_error("decode_rows: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   return g->g.decode_rows(slots, ids, n, logits);
 }
 int32_t b200_graph_checkpoint(b200_graph* g, int32_t* handle) { if (!g || !handle) return EINVAL_; return g->g.checkpoint(handle); }
@@ -304,8 +308,8 @@ int32_t b200_graph_timeline(b200_graph* g, int64_t* dst, int32_t max_launches) {
 int64_t b200_graph_trace(b200_graph* g, int32_t what, void* dst, int64_t nbytes) { if (!g || !dst) return -EINVAL_; return g->g.trace(what, dst, nbytes); }
 
 int32_t b200_draft_rows(b200_graph* g, const float* hs, const int32_t* ids, int32_t n, int32_t vocab_k, const float** residual, const float** logits) {
+  OutputsForOneCall once(g);
   if (!g || !hs || !ids) { set_error("draft_rows: null argument"); return EINVAL_; }
-  OutputsForOneCall once(g->g);
   return g->g.draft_rows(hs, ids, n, vocab_k, residual, logits);
 }
 int32_t b200_draft_past(const b200_graph* g) { return g ? g->g.draft_past[g->g.dcur] : 0; }

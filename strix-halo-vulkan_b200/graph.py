@@ -199,7 +199,12 @@ class Graph:
             _lib.check(L.b200_graph_set_outputs(self._h, lb and lb.ptr, lb and logits_shape[0] * logits_shape[1] or 0,
                                                 rb and rb.ptr, rb and residual_shape[0] * residual_shape[1] or 0))
         lg, rs = C.c_void_p(), C.c_void_p()
-        _lib.check(call(C.byref(lg), C.byref(rs)))
+        try:
+            status = call(C.byref(lg), C.byref(rs))
+        except BaseException:   # the call was not made: its outputs must not be another's
+            L.b200_graph_set_outputs(self._h, None, 0, None, 0)
+            raise
+        _lib.check(status)
         out = []
         for block, ptr, shape in ((lb, lg, logits_shape), (rb, rs, residual_shape)):
             if shape:

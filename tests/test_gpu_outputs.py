@@ -38,3 +38,39 @@ def test_a_refused_draft_call_does_not_read_the_rows(pkg, model):
     h = np.random.default_rng(1).standard_normal((1, model.cfg["n_embd"])).astype(np.float32)
     got, want = g.draft_rows(h, good), pkg.Graph(model, n_kv=64, max_tokens=16).draft_rows(h, good)
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+def test_outputs_hold_for_one_call_even_one_with_null_arguments(pkg, model):
+    L = pkg.lib.load()
+    g = pkg.Graph(model, n_kv=64, max_tokens=16)
+    V = model.cfg["vocab"]
+    lg, rs = ctypes.c_void_p(), ctypes.c_void_p()
+    out, one = (ctypes.byref(lg), ctypes.byref(rs)), ids_of(model, 1, 2)
+    calls = (lambda: L.b200_graph_forward(g._h, None, 1, *out), lambda: L.b200_graph_extend(g._h, None, 1, *out), lambda: L.b200_graph_extend_input(g._h, None, *out),
+             lambda: L.b200_graph_extend_rows(g._h, None, 1, *out), lambda: L.b200_graph_extend_residual(g._h, None, 1, *out),
+             lambda: L.b200_graph_decode_rows(g._h, None, one.ctypes.data, 1, out[0]), lambda: L.b200_draft_rows(g._h, None, one.ctypes.data, 1, 0, *out))
+    for call in calls:
+        mine = np.full(V, 7.0, dtype=np.float32)
+        pkg.lib.check(L.b200_graph_set_outputs(g._h, mine.ctypes.data, V, None, 0))
+        assert call() == pkg.lib.EINVAL
+        pkg.lib.check(L.b200_graph_extend(g._h, one.ctypes.data, 1, *out))
+        assert lg.value != mine.ctypes.data and (mine == 7.0).all()
+
+
+def test_outputs_of_a_call_that_was_not_made_are_dropped(pkg, model):
+    g = pkg.Graph(model, n_kv=64, max_tokens=16)
+    blocks = []
+
+    def interrupted(lg, rs):
+        blocks.append(True)
+        raise KeyboardInterrupt
+
+    big = (16, model.cfg["vocab"])   # large enough for a pinned block
+    with pytest.raises(KeyboardInterrupt):
+        g._results(interrupted, big)
+    one = ids_of(model, 1, 3)
+    lg, rs = ctypes.c_void_p(), ctypes.c_void_p()
+    pkg.lib.check(pkg.lib.load().b200_graph_extend(g._h, one.ctypes.data, 1, ctypes.byref(lg), ctypes.byref(rs)))
+    first = lg.value
+    pkg.lib.check(pkg.lib.load().b200_graph_extend(g._h, one.ctypes.data, 1, ctypes.byref(lg), ctypes.byref(rs)))
+    assert blocks and first == lg.value   # the graph's own buffer both times
