@@ -185,6 +185,7 @@ int32_t b200_graph_set_outputs(b200_graph* g, float* logits, int64_t logit_float
 int32_t b200_graph_forward(b200_graph* g, const int32_t* ids, int32_t n, const float** logits, const float** hidden) {
   OutputsForOneCall once(g);
   if (!g || !ids) { set_error("forward: null argument"); return EINVAL_; }
+  B200_TRY(g->g.outputs_fit(g->g.m->c.vocab, 0));
   B200_TRY(g->g.reset_slot(g->g.cur));
   PassFlags f;
   return g->g.extend(ids, n, f, logits, hidden);

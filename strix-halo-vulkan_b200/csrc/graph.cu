@@ -655,10 +655,13 @@ int Graph::upload_stage(int M) {
   return OK;
 }
 
-// Where this call's logits and residual rows go: the caller's buffers when it has set them, else the graph's own.
-int Graph::result_buffers(int64_t logit_floats, int64_t resid_floats, float** lg, float** rs) {
-  const b200_config& c = m->c;
+int Graph::outputs_fit(int64_t logit_floats, int64_t resid_floats) const {
   if ((out_logits != nullptr && logit_floats > out_logits_cap) || (out_resid != nullptr && resid_floats > out_resid_cap)) { set_error("the output buffers that were set are too small for this call"); return ECAPACITY; }
+  return OK;
+}
+// Where this pass's logits and residual rows go: the caller's buffers when it has set them, else the graph's own.
+int Graph::result_buffers(int64_t logit_floats, int64_t resid_floats, float** lg, float** rs) {
+  B200_TRY(outputs_fit(logit_floats, resid_floats));
   auto grow = [](float** p, int64_t* cap, int64_t need) {
     if (need <= *cap) return OK;
     if (*p != nullptr) cudaFreeHost(*p);
@@ -763,6 +766,7 @@ int Graph::extend(const int32_t* ids, int n, const PassFlags& f, const float** l
   if (f.want_all_logits && n > LR) { set_error("extend_rows: more rows than max_tokens (logits of at most 512 rows per pass)"); return ECAPACITY; }
   if (f.want_residual && n > MR) { set_error("extend_residual: more rows than max_tokens"); return ECAPACITY; }
   if (past[cur] + n > o.n_kv) { set_error("extend: the slot's context is full (" + std::to_string(past[cur]) + " + " + std::to_string(n) + " > " + std::to_string(o.n_kv) + ")"); return ECAPACITY; }
+  B200_TRY(outputs_fit((int64_t)(f.want_all_logits ? n : 1) * m->c.vocab, f.want_residual ? (int64_t)n * m->c.n_embd : 0));   // before any pass advances the slot
   resid_off = 0;
   for (int off = 0; off < n; off += MR) {
     const int M = std::min(MR, n - off);

@@ -134,6 +134,7 @@ struct Graph {
   int finish_pass();
   void place_stage(int M);
   int upload_stage(int M);
+  int outputs_fit(int64_t logit_floats, int64_t resid_floats) const;
   int result_buffers(int64_t logit_floats, int64_t resid_floats, float** lg, float** rs);
   int ep_prepare(int rank, int world);
   int ep_export(int rank, int world, void* handle64);

@@ -74,3 +74,25 @@ def test_outputs_of_a_call_that_was_not_made_are_dropped(pkg, model):
     first = lg.value
     pkg.lib.check(pkg.lib.load().b200_graph_extend(g._h, one.ctypes.data, 1, ctypes.byref(lg), ctypes.byref(rs)))
     assert blocks and first == lg.value   # the graph's own buffer both times
+
+
+@pytest.mark.parametrize("call", ["forward", "extend", "extend_residual"])
+def test_a_prompt_whose_outputs_do_not_fit_leaves_the_slot_alone(pkg, model, call):
+    """Twenty tokens are three passes of at most eight: the refusal comes before the first, not with the logits of the last."""
+    L = pkg.lib.load()
+    V, H = model.cfg["vocab"], model.cfg["n_embd"]
+    head, ids = ids_of(model, 5, 4), ids_of(model, 20, 5)
+    g, plain = (pkg.Graph(model, n_kv=64, max_tokens=8, use_cuda_graph=False) for _ in range(2))
+    for x in (g, plain):
+        x.forward(head)
+    lg, rs = ctypes.c_void_p(), ctypes.c_void_p()
+    n = 8 if call == "extend_residual" else 20   # a pass returns every row's residual, so all of them in one
+    small = np.empty(V, dtype=np.float32)
+    if call == "extend_residual":
+        rows = np.empty(n * H - 1, dtype=np.float32)
+        pkg.lib.check(L.b200_graph_set_outputs(g._h, small.ctypes.data, V, rows.ctypes.data, rows.size))
+    else:
+        pkg.lib.check(L.b200_graph_set_outputs(g._h, small.ctypes.data, V - 1, None, 0))
+    assert getattr(L, "b200_graph_" + call)(g._h, ids.ctypes.data, n, ctypes.byref(lg), ctypes.byref(rs)) == pkg.lib.ECAPACITY
+    assert g.past() == 5
+    assert np.array_equal(g.extend(ids)[0], plain.extend(ids)[0])
