@@ -32,15 +32,16 @@ struct Scratch {   // device temporaries of one call
 struct HostPool {
   static constexpr size_t POOL_MAX = (size_t)1 << 30, POOL_IDLE = (size_t)256 << 20;
   std::mutex mu;
+  struct Block { size_t size; bool idle; };
   std::multimap<size_t, void*> idle;
-  std::map<void*, size_t> size_of;
+  std::map<void*, Block> blocks;
   size_t total = 0, idle_bytes = 0;
 
   void drop_largest() {   // mu held
     auto it = std::prev(idle.end());
     cudaFreeHost(it->second);
     total -= it->first; idle_bytes -= it->first;
-    size_of.erase(it->second);
+    blocks.erase(it->second);
     idle.erase(it);
   }
   void* acquire(size_t bytes) {
@@ -51,25 +52,28 @@ struct HostPool {
       void* p = it->second;
       idle_bytes -= it->first;
       idle.erase(it);
+      blocks[p].idle = false;
       return p;
     }
     while (!idle.empty() && total + want > POOL_MAX) drop_largest();
     void* p = nullptr;
     if (total + want > POOL_MAX || cudaHostAlloc(&p, want, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     total += want;
-    size_of[p] = want;
+    blocks[p] = Block{want, false};
     return p;
   }
   bool owns(const void* p) {
     std::lock_guard<std::mutex> lock(mu);
-    return size_of.count(const_cast<void*>(p)) != 0;
+    auto it = blocks.find(const_cast<void*>(p));
+    return it != blocks.end() && !it->second.idle;
   }
   void release(void* p) {
     std::lock_guard<std::mutex> lock(mu);
-    auto it = size_of.find(p);
-    if (it == size_of.end()) return;
-    idle.emplace(it->second, p);
-    idle_bytes += it->second;
+    auto it = blocks.find(p);
+    if (it == blocks.end() || it->second.idle) return;   // not a block, or given back already
+    it->second.idle = true;
+    idle.emplace(it->second.size, p);
+    idle_bytes += it->second.size;
     while (idle_bytes > POOL_IDLE) drop_largest();
   }
 };

@@ -96,3 +96,51 @@ def test_a_prompt_whose_outputs_do_not_fit_leaves_the_slot_alone(pkg, model, cal
     assert getattr(L, "b200_graph_" + call)(g._h, ids.ctypes.data, n, ctypes.byref(lg), ctypes.byref(rs)) == pkg.lib.ECAPACITY
     assert g.past() == 5
     assert np.array_equal(g.extend(ids)[0], plain.extend(ids)[0])
+
+
+def test_a_block_given_back_twice_is_handed_out_once(pkg, model):
+    g, L = pkg.Graph(model, n_kv=16, max_tokens=8), pkg.lib.load()
+    a = L.b200_host_acquire(g._h, 3 << 20)
+    L.b200_host_release(a)
+    L.b200_host_release(a)
+    two = [L.b200_host_acquire(g._h, 3 << 20) for _ in range(2)]
+    assert all(two) and two[0] != two[1]
+    for p in two:
+        L.b200_host_release(p)
+    L.b200_host_release(None)
+    L.b200_host_release(ctypes.c_void_p(12345))   # nobody's block
+
+
+def test_the_cache_of_blocks_is_bounded(pkg, model):
+    g, L = pkg.Graph(model, n_kv=16, max_tokens=8), pkg.lib.load()
+    blocks = []
+    while len(blocks) < 9 and (p := L.b200_host_acquire(g._h, 256 << 20)):
+        blocks.append(p)
+    assert 1 <= len(blocks) <= 4 and len(set(blocks)) == len(blocks)   # 1 GiB in all, whatever other tests hold of it
+    ids = ids_of(model, 16, 6)
+    got = g.extend_rows(ids[:8])                                       # no block to be had: the graph's own buffers, copied
+    assert all(np.array_equal(a, b) for a, b in zip(got, pkg.Graph(model, n_kv=16, max_tokens=8).extend_rows(ids[:8])))
+    for p in blocks:
+        L.b200_host_release(p)
+    p = L.b200_host_acquire(g._h, 256 << 20)
+    assert p
+    L.b200_host_release(p)
+
+
+def test_pageable_and_pinned_buffers_get_the_same_results(pkg, model):
+    L = pkg.lib.load()
+    V, H, n = model.cfg["vocab"], model.cfg["n_embd"], 3
+    ids = ids_of(model, n, 7)
+    want = pkg.Graph(model, n_kv=16, max_tokens=8).extend_rows(ids)
+    g = pkg.Graph(model, n_kv=16, max_tokens=8)
+    block = L.b200_host_acquire(g._h, 4 * n * (V + H))
+    pinned = np.ctypeslib.as_array(ctypes.cast(block, ctypes.POINTER(ctypes.c_float)), (n * (V + H),))
+    for buf in (np.zeros(n * (V + H), dtype=np.float32), pinned):
+        g.reset()
+        at = buf.ctypes.data
+        pkg.lib.check(L.b200_graph_set_outputs(g._h, at, n * V, at + 4 * n * V, n * H))
+        lg, rs = ctypes.c_void_p(), ctypes.c_void_p()
+        pkg.lib.check(L.b200_graph_extend_rows(g._h, ids.ctypes.data, n, ctypes.byref(lg), ctypes.byref(rs)))
+        assert (lg.value, rs.value) == (at, at + 4 * n * V)
+        assert np.array_equal(buf[:n * V].reshape(n, V), want[0]) and np.array_equal(buf[n * V:].reshape(n, H), want[1])
+    L.b200_host_release(block)
