@@ -79,6 +79,7 @@ int Graph::init(Model* model, const b200_graph_opts& opts) {
     if (m->layers[l].is_attn) attn_index[l] = n_attn++;
     else dn_index[l] = n_dn++;
   }
+  for (int l = 0; l < c.n_layer; l++) n_rows_moe += rows_moe(m->layers[l]);
   max_entries = std::max(max_entries_for(MR, false), max_entries_for(std::min(MR, 128), false));
   B200_TRY(dalloc(&h, (size_t)MR * H)); B200_TRY(dalloc(&proj, (size_t)MR * proj_ld));
   B200_TRY(dalloc(&xn16, (size_t)MR * H)); B200_TRY(dalloc(&q16, (size_t)MR * qw)); B200_TRY(dalloc(&ctx16, (size_t)MR * qw));
@@ -234,6 +235,12 @@ bool Graph::experts_stream(const LayerW& L, int M) const {
   return !(M <= QG_FUSED_ROWS && c.n_embd <= QG_FUSED_MAX_K) && qlist_type(L.gate_exps.type) && qlist_type(L.down_exps.type) && L.down_exps.type == L.down_sh.type &&
          c.ffn_expert % 256 == 0 && qlist_fits(c.n_embd, c.ffn_expert, max_entries) && qlist_fits(c.ffn_expert, c.n_embd, max_entries);
 }
+// The experts of the fused passes: each row on its own, selected inside the expert kernel (moerow.cu)
+bool Graph::rows_moe(const LayerW& L) const {
+  const b200_config& c = m->c;
+  return L.gate_exps.type == L.up_exps.type && L.gate_exps.type == L.gate_sh.type && L.gate_sh.type == L.up_sh.type && L.down_exps.type == L.down_sh.type &&
+         moe_rows_fit(L.gate_exps.type, L.down_exps.type, c.n_embd, c.ffn_expert, c.n_expert, c.n_expert_used);
+}
 static bool pass_moe_gemm(const b200_config& c, const LayerW& L, int M, int H) {
   return pass_uses_gemm(M, H) && (int64_t)M * c.n_expert_used >= 32 * (int64_t)c.n_expert && L.gate_exps.type == L.gate_sh.type && L.down_exps.type == L.down_sh.type &&
          c.ffn_expert % 256 == 0 && c.n_embd % 128 == 0 && c.n_expert <= 1024;
@@ -273,10 +280,6 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   const int hd = c.head_dim, qw = c.n_head * hd, kvw = c.n_head_kv * hd, used = c.n_expert_used, slots1 = used + 1;
   const int xcols = std::min(M, QG_MAXCOLS);
   const bool fused = M <= QG_FUSED_ROWS && H <= QG_FUSED_MAX_K;
-  auto rows_moe = [&](const LayerW& L) {
-    return L.gate_exps.type == L.up_exps.type && L.gate_exps.type == L.gate_sh.type && L.gate_sh.type == L.up_sh.type && L.down_exps.type == L.down_sh.type &&
-           moe_rows_fit(L.gate_exps.type, L.down_exps.type, H, c.ffn_expert, c.n_expert, used);
-  };
   // expert-parallel MoE block: plain decode passes only (every rank runs the same number of rows at the same time)
   const bool epx = ep_on && ep_ready && !f.draft && !f.spec && n_seq == M;
   const int Mg = epx ? M * ep.world : M;   // rows of all ranks
@@ -487,7 +490,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     // decode and verify passes equal their rows stepped alone: llm/graph_batch_test.go:36, llm/spec_slots_test.go:199)
     const bool moe_gemm = pass_moe_gemm(c, L, M, H) && !epx;
     const bool moe_stream = !moe_gemm && experts_stream(L, M);
-    r.defer = fused && !epx && rows_moe(L); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer ? nullptr : distinct_dev;
+    r.defer = fused && !epx && rows_moe(L); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer || (fused && f.draft) ? nullptr : distinct_dev;
     if (epx) { r.entries = nullptr; r.gprob = nullptr; }   // routing only: the work list comes from the gathered routing
     // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted
     // rows (below that the column-tiled kernel, which streams each expert's weights in whole tiles, is faster)
@@ -739,8 +742,8 @@ int Graph::run_rows(const int32_t* ids, const int* slots, const int* pos, int M,
   stats.passes++; stats.rows += M; stats.launches += last_launches; stats.device_ms += ms;
   stats.host_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - host_t0).count();
   stats.last_rows = M; stats.last_launches = last_launches; stats.last_device_ms = ms;
-  // rows of fused passes select their experts inside the expert kernel: one stream per row and slot
-  if (M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !f.draft && !(ep_on && ep_ready && n_seq == M)) single_row_layers += (int64_t)M * m->c.n_layer;
+  // rows of fused passes select their experts inside the expert kernel, where it takes the layer's types: one stream per row and slot
+  if (M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !f.draft && !(ep_on && ep_ready && n_seq == M)) single_row_layers += (int64_t)M * n_rows_moe;
   return OK;
 }
 
@@ -856,7 +859,7 @@ int Graph::generate_greedy(const int32_t* slots_in, const int32_t* first, int n,
   B200_CUDA(cudaEventElapsedTime(&last_ms, ev0, ev1));
   stats.passes += steps; stats.rows += (int64_t)steps * n; stats.launches += (int64_t)steps * last_launches; stats.device_ms += last_ms;
   stats.last_rows = n; stats.last_launches = last_launches; stats.last_device_ms = last_ms / steps;
-  if (n <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !(ep_on && ep_ready)) single_row_layers += (int64_t)steps * n * m->c.n_layer;
+  if (n <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K && !(ep_on && ep_ready)) single_row_layers += (int64_t)steps * n * n_rows_moe;
   memcpy(out, ids_host, (size_t)steps * n * sizeof(int32_t));
   for (int i = 0; i < n; i++) past[slots[i]] += steps;
   spec_n = 0;

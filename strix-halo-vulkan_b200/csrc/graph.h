@@ -56,7 +56,8 @@ struct Graph {
   int *r_ticket = nullptr, *pair_counts = nullptr, *pair_pos = nullptr, *err_flag = nullptr, *n_entries = nullptr, *cols = nullptr, *row_slot = nullptr, *row_pos = nullptr, *logit_rows = nullptr, *hist_len = nullptr;
   int4* entries = nullptr;
   int64_t* distinct_dev = nullptr;     // experts streamed by the work lists built so far (device counter)
-  int64_t single_row_layers = 0;       // (row, layer) pairs of fused passes, whose experts are selected inside the expert kernel
+  int n_rows_moe = 0;                  // layers (without the draft's) whose experts a fused pass selects inside the expert kernel
+  int64_t single_row_layers = 0;       // (row, layer) pairs of fused passes in those layers
   SeqDesc* seqs = nullptr;
   float* rope = nullptr;
   int proj_ld = 0, max_entries = 0, nsplit = 0, split_cells = 0;
@@ -115,6 +116,7 @@ struct Graph {
   int max_entries_for(int M, bool stream) const;
   bool dense_tg(uint32_t type, int M, int N) const;
   bool direct_out(const PassFlags& f, int M, int n_logit_rows) const;
+  bool rows_moe(const LayerW& L) const;
   bool experts_stream(const LayerW& L, int M) const;
   int make_weight_maps();
   uint32_t fp16_weight_mask(int M, int n_logit_rows) const;

@@ -236,6 +236,7 @@ __device__ void build_work_list(const RouterParams& p, int* counts, int* offs, i
   if (M == 1) {
     if (tid < used) { p.entries[tid] = make_int4(p.topk[tid], tid, 1, 0); p.cols[tid] = tid; }
     if (tid == used) { p.entries[used] = make_int4(-1, used, 1, 0); p.cols[used] = used; *p.n_entries = used + 1; }
+    if (tid == 0 && p.distinct != nullptr) *p.distinct += used;
     tl_mark(p.tl, 6, true);
     return;
   }
