@@ -310,14 +310,14 @@ int launch_n(int cols, const TGemmParams& p, const TGemmMaps& maps, bool pdl, cu
   return EINVAL_;
 }
 
-// A warp per (row, sub-block), lane = element. grid (ceil(K / 256), rows), block 256.
+// A warp per (row, sub-block), lane = element. grid (rows, ceil(K / 256)), block 256.
 __global__ void __launch_bounds__(256) row_sums_kernel(const __half* x, int K, __half* sx) {
   pdl_wait();
   pdl_launch();
-  const int s = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int s = blockIdx.y * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (s * 32 >= K) return;
-  const float sum = warp_sum(__half2float(x[(size_t)blockIdx.y * K + s * 32 + lane]));
-  if (lane == 0) store_sub_sum(sx + (size_t)blockIdx.y * (K / 256 * TG_SX), s, sum);
+  const float sum = warp_sum(__half2float(x[(size_t)blockIdx.x * K + s * 32 + lane]));
+  if (lane == 0) store_sub_sum(sx + (size_t)blockIdx.x * (K / 256 * TG_SX), s, sum);
 }
 
 }  // namespace
@@ -370,7 +370,7 @@ int make_rows_map(const __half* x, int64_t rows, int K, int box_rows, TMap* out)
 
 int launch_row_sums(const __half* x, int rows, int K, __half* sx, bool pdl, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((K + 255) / 256, rows); cfg.blockDim = dim3(256); cfg.stream = st;
+  cfg.gridDim = dim3(rows, (K + 255) / 256); cfg.blockDim = dim3(256); cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;

@@ -16,3 +16,11 @@ def test_exact_projection(pkg, orc, typ, rows, k, m):
     w = orc.dequantize(typ, q, rows * k).reshape(rows, k).astype(np.float64)
     want = x.astype(np.float16).astype(np.float64) @ w.T
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max(), (np.abs(got - want).max(), np.abs(want).max())
+
+
+def test_more_rows_than_a_grid_is_high(pkg, orc):
+    rng = np.random.default_rng(9)
+    q = orc.quantize(12, (0.02 * rng.standard_normal((16, 256))).astype(np.float32))
+    x = rng.standard_normal((65600, 256)).astype(np.float32)
+    want = x.astype(np.float16).astype(np.float64) @ orc.dequantize(12, q, 16 * 256).reshape(16, 256).astype(np.float64).T
+    assert np.abs(pkg.qgemv(12, q, 16, 256, x) - want).max() <= 1e-5 * np.abs(want).max()
