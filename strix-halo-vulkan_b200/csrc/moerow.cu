@@ -79,19 +79,25 @@ __global__ void __launch_bounds__(256, 3) moe_gate_kernel(const __grid_constant_
   };
   tl_mark(p.tl, 2);
   int phase = 0, buf = 0;
+  bool lost = false;
   const uint32_t ra = (uint32_t)__cvta_generic_to_shared(raw) + 2 * g * BLK;
   const __half* sp = sxs + (t & 1) * (K / 32) + 2 * (t >> 1);
   for (int base = blockIdx.x * tpc; base < tiles; base += step, buf ^= 1) {
     const int tile = base + lt;
     float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-    if (tile < tiles) {
+    if (tile < tiles && !lost) {
       for (int b = 0; b < bpt; b++, phase ^= 1) {
         const int blk = ks + b * wpt;
         const uint32_t s0 = *reinterpret_cast<const uint32_t*>(sp + 8 * blk), s1 = *reinterpret_cast<const uint32_t*>(sp + 8 * blk + 4);
 #pragma unroll
         for (int m = 0; m < 2; m++) {
           if (warp_wait(&bars[warp][m], phase)) k45_accumulate<TYPE>(acc[m], ra + m * RAW, ra + m * RAW + BLK, xs + 576 * blk, s0, s1, t);
-          else if (lane == 0) report_error(p.err);   // a copy never landed: report, the results are void
+          else lost = true;
+        }
+        if (lost) {   // a copy never landed: report, the results are void; no more are asked for, and those in flight land before the CTA leaves
+          if (lane == 0) report_error(p.err);
+          for (int m = 0; m < 2; m++) mbar_wait(&bars[warp][m], phase, 1u << 18);
+          break;
         }
         __syncwarp();
         const bool more = b + 1 < bpt;
@@ -164,8 +170,9 @@ __global__ void __launch_bounds__(MD_MAXWARPS * 32) moe_down_kernel(const __grid
       const uint32_t ra = (uint32_t)__cvta_generic_to_shared(smem + u * RAW) + 2 * g * BLK;
       const __half* sp = sx + ((t & 1) ? 8 : 0) + 2 * (t >> 1);
       k45_accumulate<TYPE>(acc, ra, ra + BLK, xs, *reinterpret_cast<const uint32_t*>(sp), *reinterpret_cast<const uint32_t*>(sp + 4), t);
-    } else if (lane == 0) {
-      report_error(p.err);   // a copy never landed: report, the results are void
+    } else {   // a copy never landed: report, the results are void; leave once it has, or its limit has run out again
+      if (lane == 0) report_error(p.err);
+      mbar_wait(&bars[u], 0, 1u << 18);
     }
     if (t == 0) { yv[2 * g * ld + u] = w * acc[0]; yv[(2 * g + 1) * ld + u] = w * acc[2]; }   // every column holds the one activation row
   }

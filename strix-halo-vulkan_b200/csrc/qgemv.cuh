@@ -660,6 +660,11 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
   const int xc = GROUPED ? QG_MAXCOLS : p.xcols, chunk = GROUPED ? 1 : min(NS, 2 * QG_MAXCOLS / xc);
   const size_t plane2 = QG_WARPS * 16 * QG_MAXCOLS;   // DUAL: the second matrix's sums
   int cur = -1;
+  bool lost = false;
+  // a copy never landed: the results are void, and no more are asked for; those in flight land (or run out their limit too) before the CTA leaves
+  auto land = [&](uint64_t* bars, int it) {
+    for (int k = it; k < it + NS && k < n_units; k++) mbar_wait(&bars[k % NS], (uint32_t)((k / NS) & 1), 1u << 18);
+  };
   for (int it0 = 0; it0 < n_units; it0 += chunk) {
     const int cnt = min(chunk, n_units - it0);
     if (it0 > 0) __syncthreads();   // the sums before are read; GROUPED: every warp is done with the rows of the entry before
@@ -680,20 +685,23 @@ __global__ void __launch_bounds__(QG_THREADS, (GROUPED || TYPE == T_Q6_K) ? 3 : 
       const int tile = group_of(it) * tpc + lt;
       float acc[4] = {0.f, 0.f, 0.f, 0.f}, acc2[4] = {0.f, 0.f, 0.f, 0.f};
       if constexpr (BOXED) {
-        if (tile < tiles && kslice < nb) {
-          if (!warp_wait(&full_bar[BOXED ? warp : 0][s], (uint32_t)((it / NS) & 1))) {   // a copy never landed: report, the results are void
+        if (tile < tiles && kslice < nb && !lost) {
+          if (!warp_wait(&full_bar[BOXED ? warp : 0][s], (uint32_t)((it / NS) & 1))) {
             if (lane == 0) report_error(p.err);
+            lost = true;
+            land(full_bar[BOXED ? warp : 0], it);
           } else {
             if (it == 0) tl_mark(p.tl, 3);
             const uint8_t* row0 = stages + (size_t)s * stage_bytes + (size_t)lt * tile_bytes + 2 * g * BLK;
             for (int blk = kslice; blk < nb; blk += wpt) block_accumulate<TYPE>(acc, row0 + blk * (16 * BLK), row0 + blk * (16 * BLK) + BLK, xrow, sxrow, live, nb, blk, t);
           }
           __syncwarp();
-          if (it + NS < n_units) { fence_proxy_async(); issue_boxes(it + NS); }
+          if (it + NS < n_units && !lost) { fence_proxy_async(); issue_boxes(it + NS); }
         }
       } else {
         if (!mbar_wait(&full_bar[0][s], (uint32_t)((it / NS) & 1))) {
-          if (tid == 0) report_error(p.err);  // a copy never landed: report and leave
+          if (tid == 0) report_error(p.err);
+          land(full_bar[0], it);
           return;
         }
         if (it == 0) tl_mark(p.tl, 3);
