@@ -211,15 +211,9 @@ int Graph::max_entries_for(int M, bool stream) const {
   return std::min(M * used, m->c.n_expert + (M * used + ec - 1) / ec) + (M + ec - 1) / ec;
 }
 
-// Tile height of a many-row projection of N weight rows over M activation rows: as tall as the pass allows,
-// shrunk while the launch would leave SMs idle. 0: its tiles would cover under a third of the SMs and the
-// projection stays on the column-tiled kernel (exact weights).
-static int gemm_tile_rows(int M, int N) {
-  int tn = M <= 64 ? 64 : M <= 128 ? 128 : 256;
-  while (tn > 64 && ((N + 127) / 128) * ((M + tn - 1) / tn) < 120) tn /= 2;
-  if (((N + 127) / 128) * ((M + tn - 1) / tn) < 48) return 0;
-  return tn;
-}
+// Whether a projection of N weight rows over M activation rows runs with fp16-rounded weights (wgemm.cu): from 48 tiles of 128 x 64 on, a
+// third of the SMs. Below that it keeps its weights exact. The line decides values, not only speed: fp16_weight_mask reports it.
+static bool wgemm_covers(int M, int N) { return ((N + 127) / 128) * ((M + 63) / 64) >= 48; }
 // Router logits of passes of this many rows and more come from the column-tiled mma kernel (Q8_0 weights as
 // fp16(d * q), the reference's many-row router arithmetic: llm_gemm MODE 2), below it from per-row dot products
 constexpr int ROUTER_MMA_FROM = 16;
@@ -227,7 +221,7 @@ static bool pass_uses_gemm(int M, int H) { return !(M <= QG_FUSED_ROWS && H <= Q
 // Dense projections of passes above the fused ones that keep their weights exact - all of them below 16 rows, above that
 // those whose tiles would not fill the device as a GEMM - run on the tensor cores all the same where the type has the kernel
 bool Graph::dense_tg(uint32_t type, int M, int N) const {
-  return !(M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K) && tgemm_type(type) && !(M >= 16 && gemm_tile_rows(M, N) != 0);
+  return !(M <= QG_FUSED_ROWS && m->c.n_embd <= QG_FUSED_MAX_K) && tgemm_type(type) && !(M >= 16 && wgemm_covers(M, N));
 }
 // The experts of passes above the fused ones: warps that stream the weights (qlist.cu), where its types and shapes allow
 bool Graph::experts_stream(const LayerW& L, int M) const {
@@ -255,16 +249,16 @@ uint32_t Graph::fp16_weight_mask(int M, int n_logit_rows) const {
   const int hd = c.head_dim, qw = c.n_head * hd, kvw = c.n_head_kv * hd;
   if (!pass_uses_gemm(M, H)) return 0;
   uint32_t mask = 0;
-  if (gemm_tile_rows(M, cw)) mask |= B200_W16_DN_QKV;
-  if (gemm_tile_rows(M, vw)) mask |= B200_W16_DN_GATE;
-  if (gemm_tile_rows(M, H)) mask |= B200_W16_DN_OUT | B200_W16_ATTN_OUT;
-  if (gemm_tile_rows(M, 2 * qw)) mask |= B200_W16_ATTN_Q;
-  if (gemm_tile_rows(M, kvw)) mask |= B200_W16_ATTN_K | B200_W16_ATTN_V;
+  if (wgemm_covers(M, cw)) mask |= B200_W16_DN_QKV;
+  if (wgemm_covers(M, vw)) mask |= B200_W16_DN_GATE;
+  if (wgemm_covers(M, H)) mask |= B200_W16_DN_OUT | B200_W16_ATTN_OUT;
+  if (wgemm_covers(M, 2 * qw)) mask |= B200_W16_ATTN_Q;
+  if (wgemm_covers(M, kvw)) mask |= B200_W16_ATTN_K | B200_W16_ATTN_V;
   for (const LayerW& L : m->layers) {
     if (M >= ROUTER_MMA_FROM && L.router.type == T_Q8_0) mask |= B200_W16_ROUTER;
     if (pass_moe_gemm(c, L, M, H)) mask |= B200_W16_EXPERTS | B200_W16_SHARED;
   }
-  if (n_logit_rows == M && gemm_tile_rows(M, c.vocab)) mask |= B200_W16_HEAD;
+  if (n_logit_rows == M && wgemm_covers(M, c.vocab)) mask |= B200_W16_HEAD;
   return mask;
 }
 
@@ -333,7 +327,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   // of the SMs stays on exact weights
   const bool use_gemm = pass_uses_gemm(M, H);
   auto gemm = [&](const DTensor& w, const WMap& wm, int K, int N, const __half* x, const TMap& xm, float* y, int64_t ldy) {
-    if (gemm_tile_rows(M, N) == 0) {
+    if (!wgemm_covers(M, N)) {
       QGemvParams q = base(w, K, N, x, K);
       q.y = y; q.ldy = ldy;
       return project(w.type, PRO_F16, EPI_STORE, q);
@@ -346,7 +340,7 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
   };
   // an output projection: its planes wait in `down` for the row kernel after it, which adds them to the residual
   auto gemm_resid = [&](const DTensor& w, const WMap& wm, int K, const __half* x, const TMap& xm) {
-    if (gemm_tile_rows(M, H) == 0) {
+    if (!wgemm_covers(M, H)) {
       QGemvParams q = base(w, K, H, x, K);
       q.y = h; q.ldy = H;
       return project(w.type, PRO_F16, EPI_RESID, q);
@@ -492,8 +486,8 @@ int Graph::enqueue_pass(int M, int n_seq, int n_logit_rows, const PassFlags& f) 
     const bool moe_stream = !moe_gemm && experts_stream(L, M);
     r.defer = fused && !epx && rows_moe(L); r.ecols = entry_cols(M, moe_stream); r.distinct = r.defer || (fused && f.draft) ? nullptr : distinct_dev;
     if (epx) { r.entries = nullptr; r.gprob = nullptr; }   // routing only: the work list comes from the gathered routing
-    // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted
-    // rows (below that the column-tiled kernel, which streams each expert's weights in whole tiles, is faster)
+    // 32 rows per expert on average and more: the experts run as grouped tensor-core GEMMs over expert-sorted rows, with fp16-rounded
+    // weights; below that as exact products over a work list (qlist.cu, or the column-tiled kernel for the types it lacks)
     r.gprob = moe_gemm ? gprob : nullptr;
     if (use_gemm && M >= ROUTER_MMA_FROM && L.router.type == T_Q8_0) {
       // many rows: the router logits are one more tensor-core GEMM (the reference's prefill router is an fp16
