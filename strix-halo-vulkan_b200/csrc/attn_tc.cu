@@ -9,10 +9,10 @@
 // O is rescaled whenever a row's maximum has grown, after the tile's exponentials, while the tensor core forms the next scores: the largest
 // probability is then exactly 1, which fp16 carries without error, and the row sum is of the probabilities as fp16 carries them, so that
 // part of what rounds them drops out of the quotient. Against f64 with peaked scores 2.17e-4 (fp16 of the exact result: 2.08e-4); with a
-// maximum kept until it had grown by 2^8, and the unrounded sum, 2.71e-4. 2048 rows take the same time either way.
+// maximum kept until it had grown by 2^8, and the unrounded sum, 2.71e-4 (and 117 us).
 // What bounds it: a step of 128 rows x 128 cells is 2500 cycles of tcgen05.mma and 128 KB of keys and values out of L2, about as long
 // (the KV heads' tiles are read once per query tile). With mma.sync (16 rows a warp, keys and values through shared memory for every
-// warp) 2048 rows over 2 to 4 thousand cells took 752 us, this takes 117; 46 us are the tensor core's floor.
+// warp) 2048 rows over 2 to 4 thousand cells took 752 us, this takes 128; 46 us are the tensor core's floor.
 #include <algorithm>
 
 #include "attn_tc.cuh"

@@ -11,6 +11,8 @@
 // and SM, so 512 experts of 3 M weights take 180 us whatever their rows; NT 256 doubles the work per cycle. The form before
 // this one (eight dequantising warps that loaded their rows from global memory and stored the fp16 tile swizzled into shared
 // memory) took 1190 us at 40 rows per expert and 1366 us at 80, waiting on latencies.
+// At 40 rows per expert it issues on 67 % of the cycles, 5.4 thread instructions per gate or up weight and 7.4 per down weight
+// (counters); turning a quant into fp16 is about 2.8 of these, the rest are waits that poll, the epilogue and the items' set-up.
 //
 // How a weight is rounded: the quants become exact fp16 integers q; the factors d * sc and dmin * m are carried as fp16 hi + lo
 // pairs (hi the rounded product, lo the exact rest from one fma), and the weight is fma(q, dh, -mh) + fma(q, dl, -ml). Against
