@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1) tgemm_kernel(const __grid_const
             tmem_ld16(lane_base + cs * 2 * NMAX + NMAX + c0, m);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[c0 + i] = fmaf(-dm.y, __uint_as_float(m[i]), fmaf(dm.x, __uint_as_float(v[i]), acc[c0 + i]));
+            for (int i = 0; i < 16; i++) acc[c0 + i] += fmaf(dm.x, __uint_as_float(v[i]), -(dm.y * __uint_as_float(m[i])));
           }
         }
         fence_before();
