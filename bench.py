@@ -382,30 +382,17 @@ def main():
     prompt_len = args.prompt or (PROMPT if args.config == "a3b" else 128)
     steps, warmup = args.steps, max(args.warmup, 3)
 
+    if args.impl == "reference":
+        if rank == 0:
+            print(json.dumps({"impl": "reference", "unavailable": "a Go module over Vulkan compute: no Go toolchain, Vulkan loader or software renderer here; "
+                                                                 "the CPU restatement of its path is the cpu_baseline of the other arm"}))
+        return
     import torch
     import torch.distributed as dist
-    if args.impl == "reference" and rank != 0:
-        # rank 0 alone times the CPU implementation. The other ranks leave at once, before any process group
-        # exists: a rank parked in a barrier spins on a host core, and every OpenMP barrier of the timed code
-        # would then wait for the thread that shares that core.
-        return
-    if world > 1 and args.impl != "reference":
+    if world > 1:
         import datetime
         dist.init_process_group("nccl", device_id=torch.device("cuda", local_rank), timeout=datetime.timedelta(seconds=300))
     torch.cuda.set_device(local_rank)
-
-    if args.impl == "reference":
-        # the reference's own CPU implementation of the path (the oracle port), rank 0 only
-        if rank == 0:
-            cb, parity = cpu_baseline(pkg, cfg, local_rank, tokens=max(steps, 4) if steps <= 32 else 8)
-            line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": "tok/s", "n_gpus": args.gpus, "steps": steps,
-                    "warmup": warmup, "ms_per_step": 1e3 / cb["value"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                    "dtype": "f32", "data": "synthetic",
-                    "config": {"workload": "batch-1 greedy decode, 80B-A3B-shaped Q4_K hybrid MoE", "host": "cpu"},
-                    "cpu_baseline": cb, "e2e": {"value": cb["value"], "unit": "tok/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-                    "parity": parity}
-            print(json.dumps(line))
-        return
 
     # every rank holds the whole checkpoint; the headline step is one sequence per rank, the 64-slot measurement splits
     # its slots over the ranks and (second arm) shards the routed experts with exchanges over NVLink peer memory
