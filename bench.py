@@ -24,10 +24,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one decode step, from an ncu capture of the 4-layer prefix
-# (`--profile 1 --layers 4` under ncu's dram byte counters) scaled to 36 DeltaNet + 12 attention layers + head. The
-# figure belongs to the kernels it was captured on, and it is
-# re-captured whenever the kernels of the single-row step change (set it to None until then).
-A3B_DRAM_BYTES_PER_STEP = None
+# (`--profile 1 --layers 4` under ncu's dram byte counters, caches kept between launches): twelve times its layers
+# (36 DeltaNet and 12 attention) and the head. The figure belongs to the kernels it was captured on: it is captured again
+# whenever the kernels of the single-row step change (None until then).
+A3B_DRAM_BYTES_PER_STEP = 2629.2e6
 PROMPT = 2048
 METRIC = "decode tok/s at batch 1 (Q4_K hybrid MoE, 80B-A3B shape)"
 
